@@ -1102,6 +1102,8 @@ int decoder_create_impl(const quintrit_b200_decoder_desc_t* desc, quintrit_b200_
             d->attn_gqa = kq, d->attn_gqa_smem = bytes;
             if (const char* pad = std::getenv("QUINTRIT_B200_ATTN_SMEM_PAD")) d->attn_gqa_pad = std::min<size_t>(static_cast<size_t>(std::atoi(pad)), smem_optin - 1024 - bytes);
         }
+        d->attn_tile = attention_tile_for(group, static_cast<int>(hd), d->f32_values != 0);
+        if (d->attn_tile != nullptr && (rc = allow_max_dynamic_smem(d->attn_tile, smem_optin)) != QUINTRIT_OK) return rc;
     }
     d->use_mega = false;
     const char* mode = std::getenv("QUINTRIT_B200_DECODE");  // "kernels" keeps the one-launch-per-step path (experiments)
@@ -2365,6 +2367,7 @@ struct BatchTarget {
     __half *kc = nullptr, *vc = nullptr;  // [layers][ctx][kv_dim] of the first sequence
     const uint32_t* pos = nullptr;
     SeqIndex seq{nullptr, 0, 0};
+    size_t end = 0;                       // a prompt chunk: the positions after its last token
     bool own = true;                      // the decoder's own cache: a full chunk may be replayed as the captured graph
     const LayeredStore* layered = nullptr;  // layered models: the sequence store and the slot of a prompt's sequence
     int slot = 0;
@@ -2425,7 +2428,7 @@ int prefill_layers(quintrit_b200_decoder* d, int n, const BatchTarget& tg) {
         at.head_dim = hd, at.kv_dim = kvd, at.gqa = d->q_heads / d->kv_heads, at.ctx = d->ctx, at.f32_values = d->f32_values;
         at.scale = 1.0f / std::sqrt(static_cast<float>(hd));
         at.part_acc = d->pf.part_acc, at.b_acc = d->q_heads * 4 * hd, at.part_ms = d->pf.part_ms, at.b_ms = d->q_heads * 8;
-        launch_attention(d, at, n, s);
+        launch_attention(d, at, n, s, tg.end);
         QTB_LAUNCH_CHECK();
         AttnFinishArgs af{};
         af.part_acc = d->pf.part_acc, af.b_acc = d->q_heads * 4 * hd, af.part_ms = d->pf.part_ms, af.b_ms = d->q_heads * 8, af.pos = tg.pos, af.seq = tg.seq;
@@ -2521,9 +2524,10 @@ int decoder_prefill(quintrit_b200_decoder* d, const uint32_t* tokens, size_t cou
     int rc = prefill_buffers(d);
     if (rc != QUINTRIT_OK) return rc;
     if ((rc = decoder_gemm_prepare(d)) != QUINTRIT_OK) return rc;
-    const BatchTarget tg = target != nullptr ? *target : own_target(d);
+    BatchTarget tg = target != nullptr ? *target : own_target(d);
     for (size_t c0 = 0; c0 < count; c0 += kPrefillMax) {
         const int n = static_cast<int>(std::min<size_t>(kPrefillMax, count - c0));
+        tg.end = pos0 + c0 + n;
         QTB_CUDA(cudaMemcpyAsync(d->pf.tokens, tokens + c0, size_t(n) * sizeof(uint32_t), cudaMemcpyHostToDevice, d->stream));
         if (tg.own) QTB_CUDA(cudaMemcpyAsync(d->d_history + pos0 + c0, d->pf.tokens, size_t(n) * sizeof(uint32_t), cudaMemcpyDeviceToDevice, d->stream));
         if ((rc = enqueue_prefill_chunk(d, n, pos0 + static_cast<uint32_t>(c0), c0 + n == count, tg)) != QUINTRIT_OK) return rc;

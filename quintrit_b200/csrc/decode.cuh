@@ -411,6 +411,7 @@ struct AttnArgs {
     float* part_ms;           // [q_heads][4][2]: M and S per chunk (S = 0 marks an empty chunk)
     int b_q, b_acc, b_ms;     // batch of tokens: token blockIdx.z uses q + z * b_q, part_acc + z * b_acc, part_ms + z * b_ms
     SeqIndex seq;             // its position and KV cache
+    int tokens;               // of the batch (attention_tile_kernel)
 };
 
 constexpr int kAttnThreads = 1024;

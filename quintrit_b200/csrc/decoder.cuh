@@ -10,6 +10,7 @@
 #include "decode.cuh"
 #include "gemv_lut.cuh"
 #include "megakernel.cuh"
+#include "prompt_attention.cuh"
 
 namespace qtb {
 struct LayeredDecoder;  // layered.cuh: a model whose layers differ from one another
@@ -51,6 +52,7 @@ struct quintrit_b200_decoder {
     bool attn_v2 = false;
     qtb::AttnGqaKernel attn_gqa = nullptr;     // one-launch-per-step and batched paths: the grouped attention kernel, if this model's shape has one
     size_t attn_gqa_smem = 0;
+    qtb::AttnGqaKernel attn_tile = nullptr;    // prompt chunks: eight tokens per block, if this model's shape has that kernel
     size_t attn_gqa_pad = 0;                   // experiments: extra shared memory per block, which lowers the number of resident blocks
     float* attn_out = nullptr;
     float *fac = nullptr, *fac_M = nullptr;
@@ -172,8 +174,17 @@ inline int decoder_gemv_bs(quintrit_b200_decoder* d, int layer, int first, const
     return QUINTRIT_OK;
 }
 
-// Attention of n tokens: all query heads of a KV head in one block where an instantiation exists, else one query head per block.
-inline void launch_attention(quintrit_b200_decoder* d, const AttnArgs& at, int n, cudaStream_t s) {
+// Attention of n tokens: all query heads of a KV head in one block where an instantiation exists, else one query head per block. `end`: positions
+// after the last token of a prompt chunk (0 for tokens of several sequences). A chunk's tokens go eight to a block where that fills the machine:
+// with 64 tokens or more once the cache is divided into four chunks (end above 512), which are blocks of their own, and with full chunks of 256
+// anywhere. Passes of four layers with 12 / 4 heads of 256 and F16 accumulators: 256 tokens at position 900 2713 -> 1654 us, at 0 1067 -> 1045; 64
+// at 900 997 -> 752, but at 200 714 -> 737; 32 at 900 731 -> 718, at 200 574 -> 672. With 8 / 2 heads of 128: 64 at 900 674 -> 628, 48 560 -> 596.
+inline void launch_attention(quintrit_b200_decoder* d, AttnArgs at, int n, cudaStream_t s, size_t end = 0) {
+    if (d->attn_tile != nullptr && end != 0 && (n >= 256 || (n >= 64 && end > 512))) {
+        at.tokens = n;
+        d->attn_tile<<<dim3(d->kv_heads, 4, n / kTokenTile + 2), kTokenTileThreads, attn_tile_smem(d->q_heads / d->kv_heads, d->head_dim), s>>>(at);
+        return;
+    }
     // several tokens: the query heads of a KV head share one pass over its rows; one token: more, wider blocks pull the rows faster
     if (d->attn_gqa != nullptr && n > 1)
         d->attn_gqa<<<dim3(d->kv_heads, 4, n), kAttnGqaThreads, d->attn_gqa_smem + d->attn_gqa_pad, s>>>(at);
