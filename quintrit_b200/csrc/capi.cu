@@ -1042,7 +1042,8 @@ int decoder_create_impl(const quintrit_b200_decoder_desc_t* desc, quintrit_b200_
         QTB_CUDA(cudaFuncSetAttribute(norm_quant_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big_bs));
         QTB_CUDA(cudaFuncSetAttribute(attn_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big_bs));
         QTB_CUDA(cudaFuncSetAttribute(act_quant_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big_bs));
-        QTB_CUDA(cudaFuncSetAttribute(lm_head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big_bs));
+        QTB_CUDA(cudaFuncSetAttribute(lm_head_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big_bs));
+        QTB_CUDA(cudaFuncSetAttribute(lm_head_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big_bs));
         QTB_CUDA(cudaFuncSetAttribute(attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(attention_smem(256))));
         d->use_mega = false;
         QTB_CUDA(cudaDeviceSynchronize());
@@ -1088,8 +1089,9 @@ int decoder_create_impl(const quintrit_b200_decoder_desc_t* desc, quintrit_b200_
     if ((rc = allow_max_dynamic_smem(norm_quant_kernel, smem_optin)) != QUINTRIT_OK) return rc;
     if ((rc = allow_max_dynamic_smem(attn_finish_kernel, smem_optin)) != QUINTRIT_OK) return rc;
     if ((rc = allow_max_dynamic_smem(act_quant_kernel, smem_optin)) != QUINTRIT_OK) return rc;
-    if ((rc = allow_max_dynamic_smem(lm_head_kernel, smem_optin)) != QUINTRIT_OK) return rc;
-    if ((rc = allow_max_dynamic_smem(lm_head_batch_kernel, smem_optin)) != QUINTRIT_OK) return rc;
+    if ((rc = allow_max_dynamic_smem(lm_head_kernel<false>, smem_optin)) != QUINTRIT_OK || (rc = allow_max_dynamic_smem(lm_head_kernel<true>, smem_optin)) != QUINTRIT_OK) return rc;
+    for (int tg : {1, 2, 4})
+        if ((rc = allow_max_dynamic_smem(lm_head_batch_for(tg, d->bf16_tables), smem_optin)) != QUINTRIT_OK) return rc;
     if ((rc = allow_max_dynamic_smem(attention_kernel, smem_optin)) != QUINTRIT_OK) return rc;
     // attention for all query heads of a KV head at once, where the group size and the head size allow it
     d->attn_gqa = nullptr, d->attn_gqa_smem = 0;
@@ -2506,7 +2508,7 @@ int enqueue_prefill_chunk(quintrit_b200_decoder* d, int n, uint32_t pos0, bool w
         nf.y16_out = d->x16, nf.y16_bf16 = d->bf16_tables;
         norm_quant_kernel<<<1, kRowThreads, H * sizeof(float), s>>>(nf);
         QTB_LAUNCH_CHECK();
-        lm_head_kernel<<<d->sm_count * 8, 256, H * sizeof(float), s>>>(d->lm_head, d->x16, H, d->vocab, d->logits, d->bf16_tables);
+        launch_lm_head(d->lm_head, d->x16, H, d->vocab, d->logits, d->bf16_tables, d->sm_count, s);
         QTB_LAUNCH_CHECK();
         argmax_kernel<<<1, 1024, 0, s>>>(d->logits, d->vocab, d->d_token);
         QTB_LAUNCH_CHECK();
@@ -2719,7 +2721,7 @@ extern "C" int quintrit_b200_moe_create_shard(uint32_t device_index, uint32_t hi
         if (out_moe == nullptr) return fail(QUINTRIT_ERR_NULL_POINTER, "out_moe is NULL");
         *out_moe = nullptr;
         if (router_bf16 == nullptr || gate_up == nullptr || down == nullptr || scales == nullptr) return fail(QUINTRIT_ERR_NULL_POINTER, "router_bf16, gate_up, down or scales is NULL");
-        if (hidden == 0 || hidden % 128 != 0 || lm_head_batch_smem(static_cast<int>(hidden)) > 200 * 1024)
+        if (hidden == 0 || hidden % 128 != 0 || hidden > 3200)
             return fail(QUINTRIT_ERR_UNSUPPORTED, "the hidden size %u must be a multiple of 128, at most 3200", hidden);
         if (inter == 0 || inter % 16 != 0 || inter > 49152) return fail(QUINTRIT_ERR_UNSUPPORTED, "the expert width %u must be a multiple of 16, at most 49152", inter);
         if (n_experts == 0 || n_experts > 1024 || top_k == 0 || top_k > n_experts || top_k > 64) return fail(QUINTRIT_ERR_INVALID_ARGUMENT, "%u experts with top-%u routing are not supported (at most 1024 experts, top-64)", n_experts, top_k);
@@ -2744,8 +2746,7 @@ extern "C" int quintrit_b200_moe_create_shard(uint32_t device_index, uint32_t hi
         if ((rc = gemv_kernel_for_device(static_cast<int>(device_index), &k)) != QUINTRIT_OK) return rc;
         int smem_optin = 0;
         QTB_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, static_cast<int>(device_index)));
-        if ((rc = allow_max_dynamic_smem(lm_head_batch_kernel, smem_optin)) != QUINTRIT_OK || (rc = allow_max_dynamic_smem(moe_prepare_kernel, smem_optin)) != QUINTRIT_OK ||
-            (rc = allow_max_dynamic_smem(moe_act_quant_kernel, smem_optin)) != QUINTRIT_OK)
+        if ((rc = allow_max_dynamic_smem(moe_prepare_kernel, smem_optin)) != QUINTRIT_OK || (rc = allow_max_dynamic_smem(moe_act_quant_kernel, smem_optin)) != QUINTRIT_OK)
             return rc;
         quintrit_b200_moe* m = new quintrit_b200_moe();
         m->magic = kMagicMoe, m->device = static_cast<int>(device_index), m->sm_count = prop.multiProcessorCount;
@@ -2998,13 +2999,13 @@ int batch_head(quintrit_b200_batch* b, int n) {
     nf.y16_out = b->x16, nf.b_y16 = H, nf.y16_bf16 = d->bf16_tables;
     norm_quant_kernel<<<dim3(1, 1, n), kRowThreads, H * sizeof(float), s>>>(nf);
     QTB_LAUNCH_CHECK();
-    if (H % 128 == 0 && lm_head_batch_smem(H) <= 200 * 1024) {
-        lm_head_batch_kernel<<<dim3(d->sm_count, (n + kHeadTokens - 1) / kHeadTokens), kHeadThreads, lm_head_batch_smem(H), s>>>(d->lm_head, b->x16, H, d->vocab, n, b->logits,
-                                                                                                                                  d->bf16_tables);
+    if (n > 1 && H % kHeadCols == 0) {
+        const int tg = lm_head_token_groups(n);
+        lm_head_batch_for(tg, d->bf16_tables)<<<dim3(d->sm_count, (n + tg * kHeadTokens - 1) / (tg * kHeadTokens)), kHeadThreads, lm_head_batch_smem(tg), s>>>(d->lm_head, b->x16, H, d->vocab, n, b->logits);
         QTB_LAUNCH_CHECK();
-    } else {  // a hidden size the grouped kernel does not take: token by token
+    } else {  // one token, or a hidden size the grouped kernel does not take: token by token
         for (int t = 0; t < n; ++t) {
-            lm_head_kernel<<<d->sm_count * 8, 256, H * sizeof(float), s>>>(d->lm_head, b->x16 + size_t(t) * H, H, d->vocab, b->logits + size_t(t) * d->vocab, d->bf16_tables);
+            launch_lm_head(d->lm_head, b->x16 + size_t(t) * H, H, d->vocab, b->logits + size_t(t) * d->vocab, d->bf16_tables, d->sm_count, s);
             QTB_LAUNCH_CHECK();
         }
     }

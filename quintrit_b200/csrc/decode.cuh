@@ -12,6 +12,8 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include "packed_f32.cuh"
+
 namespace qtb {
 
 constexpr int kRowThreads = 1024;  // one block walks a whole activation vector
@@ -1080,106 +1082,156 @@ __global__ void __cluster_dims__(kActClusterSize, 1, 1) __launch_bounds__(kActCl
     cluster.sync();  // no block leaves while its partial results may still be read
 }
 
-// ---- output head: one warp per vocabulary row, ggml_vec_dot_f16 order (model.rs:346-375, ops.rs:970-1014) --------------
-__global__ void __launch_bounds__(256) lm_head_kernel(const __half* __restrict__ w, const __half* __restrict__ x16, int hidden, int vocab,
-                                                      float* __restrict__ logits, bool bf16) {
-    extern __shared__ float x_s[];  // hidden floats
-    for (int i = threadIdx.x; i < hidden; i += blockDim.x) x_s[i] = table_to_float(x16[i], bf16);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    const int np = hidden & ~31;  // hidden is a multiple of 32 (checked at creation): no scalar tail
-    for (int row = blockIdx.x * warps + (threadIdx.x >> 5); row < vocab; row += gridDim.x * warps) {
-        const __half* wr = w + static_cast<size_t>(row) * hidden;
-        float acc = 0.0f;
-        if (bf16) {  // ggml_vec_dot_bf16: product and sum rounded separately (ops.rs:694-700)
-#pragma unroll 8
-            for (int i = 0; i < np; i += 32) acc = __fadd_rn(acc, __fmul_rn(x_s[i + lane], bf16_bits_to_float(__half_as_ushort(wr[i + lane]))));
-        } else {
-#pragma unroll 8
-            for (int i = 0; i < np; i += 32) acc = __fmaf_rn(x_s[i + lane], __half2float(wr[i + lane]), acc);
-        }
-        const float sum = bf16 ? dot_lane_reduce_bf16(acc) : dot_lane_reduce_f16(acc);
-        if (lane == 0) logits[row] = sum;
-    }
+// ---- output head: ggml_vec_dot_f16 / _bf16 order (model.rs:346-375, ops.rs:970-1014) --------------------------------------
+// Accumulator lane l of a row's dot product takes the elements 32 i + l in the order of i; then the lanes are added: 16, 8 and
+// 4 apart, then neighbours and the two sums (F16), or 2 apart and neighbours (BF16). A BF16 product and its sum are rounded
+// separately (ops.rs:694-700).
+template <bool BF16>
+__device__ __forceinline__ unsigned long long head_widen(uint32_t two) {
+    return BF16 ? widen_bf162(two) : widen_half2(two);
+}
+template <bool BF16>
+__device__ __forceinline__ unsigned long long head_step(unsigned long long w, unsigned long long x, unsigned long long acc) {
+    return BF16 ? add_f32x2(acc, mul_f32x2(x, w)) : fma_f32x2(x, w, acc);
 }
 
-// ---- output head for several tokens at once ------------------------------------------------------------------------------
-// The same dot products as lm_head_kernel (lane l of a warp owns the elements 32 i + l of a row and adds them in the order of
-// i, then the lanes are reduced), for up to kHeadTokens tokens against kHeadRows vocabulary rows per warp at a time: a row
-// element is read from HBM once per token group instead of once per token, and an activation read from shared memory serves
-// kHeadRows rows. The activations sit in shared memory as F32, laid out so that a lane reads its elements of four consecutive
-// steps with one 16-byte load: float4 index (t * hidden / 128 + k) * 32 + lane holds steps 4k .. 4k + 3.
-constexpr int kHeadTokens = 16, kHeadRows = 4, kHeadThreads = 256;
-__host__ __device__ constexpr size_t lm_head_batch_smem(int hidden) { return static_cast<size_t>(kHeadTokens) * hidden * sizeof(float); }
-
-__global__ void __launch_bounds__(kHeadThreads, 1) lm_head_batch_kernel(const __half* __restrict__ w, const __half* __restrict__ x16, int hidden, int vocab, int n,
-                                                                         float* __restrict__ logits, bool bf16) {
-    extern __shared__ float4 x4[];
-    float* xs = reinterpret_cast<float*>(x4);
-    const int t0 = blockIdx.y * kHeadTokens, nt = min(kHeadTokens, n - t0), k4 = hidden / 128;
-    for (int idx = threadIdx.x; idx < kHeadTokens * hidden; idx += kHeadThreads) {
-        const int t = idx / hidden, e = idx - t * hidden, step = e >> 5, l = e & 31;
-        const float v = t < nt ? table_to_float(x16[static_cast<size_t>(t0 + t) * hidden + e], bf16) : 0.0f;
-        xs[((static_cast<size_t>(t) * k4 + (step >> 2)) * 32 + l) * 4 + (step & 3)] = v;
-    }
+// One token. Four threads share a row: each owns eight neighbouring lanes, that is one 16-byte load per 32 elements, and a warp
+// reads eight rows at a time. Bound by HBM: 32768 x 3072 F16 (201 MB) HEAD1_TIME
+constexpr int kHeadOneThreads = 256, kHeadOneRows = 8;  // rows of a warp
+template <bool BF16>
+__global__ void __launch_bounds__(kHeadOneThreads) lm_head_kernel(const __half* __restrict__ w, const __half* __restrict__ x16, int hidden, int vocab, float* __restrict__ logits) {
+    extern __shared__ __align__(16) float x_s[];  // hidden floats
+    for (int i = threadIdx.x; i < hidden; i += kHeadOneThreads) x_s[i] = table_to_float(x16[i], BF16);
     __syncthreads();
-    const int lane = threadIdx.x & 31, warps = kHeadThreads / 32;
-    for (int row0 = (blockIdx.x * warps + (threadIdx.x >> 5)) * kHeadRows; row0 < vocab; row0 += gridDim.x * warps * kHeadRows) {
-        const __half* wr[kHeadRows];
+    const int lane = threadIdx.x & 31, quarter = lane & 3, steps = hidden / 32;  // (hidden is a multiple of 32: checked at creation)
+    for (int row0 = (blockIdx.x * (kHeadOneThreads / 32) + (threadIdx.x >> 5)) * kHeadOneRows; row0 < vocab; row0 += gridDim.x * (kHeadOneThreads / 32) * kHeadOneRows) {
+        const int row = row0 + (lane >> 2);
+        const uint4* wr = reinterpret_cast<const uint4*>(w + static_cast<size_t>(min(row, vocab - 1)) * hidden) + quarter;
+        const ulonglong2* xr = reinterpret_cast<const ulonglong2*>(x_s) + quarter * 2;
+        unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
+        auto step = [&](const uint4& h, int i) {
+            const ulonglong2 x0 = xr[i * 8], x1 = xr[i * 8 + 1];
+            acc[0] = head_step<BF16>(head_widen<BF16>(h.x), x0.x, acc[0]);
+            acc[1] = head_step<BF16>(head_widen<BF16>(h.y), x0.y, acc[1]);
+            acc[2] = head_step<BF16>(head_widen<BF16>(h.z), x1.x, acc[2]);
+            acc[3] = head_step<BF16>(head_widen<BF16>(h.w), x1.y, acc[3]);
+        };
+        int i = 0;
+        for (; i + 8 <= steps; i += 8) {
+            uint4 h[8];
 #pragma unroll
-        for (int r = 0; r < kHeadRows; ++r) wr[r] = w + static_cast<size_t>(min(row0 + r, vocab - 1)) * hidden + lane;
-        float acc[kHeadTokens][kHeadRows];
+            for (int k = 0; k < 8; ++k) h[k] = __ldg(wr + (i + k) * 4);
 #pragma unroll
-        for (int t = 0; t < kHeadTokens; ++t)
+            for (int k = 0; k < 8; ++k) step(h[k], i + k);
+        }
+        for (; i < steps; ++i) step(wr[i * 4], i);
 #pragma unroll
-            for (int r = 0; r < kHeadRows; ++r) acc[t][r] = 0.0f;
-        unsigned short raw[kHeadRows][4];
+        for (int k = 0; k < 4; ++k) acc[k] = add_f32x2(acc[k], shfl_xor_f32x2(acc[k], 2));  // lanes 16 apart
 #pragma unroll
-        for (int r = 0; r < kHeadRows; ++r)
+        for (int k = 0; k < 4; ++k) acc[k] = add_f32x2(acc[k], shfl_xor_f32x2(acc[k], 1));  // 8 apart
+        const float2 lo = unpack_f32x2(add_f32x2(acc[0], acc[2])), hi = unpack_f32x2(add_f32x2(acc[1], acc[3]));  // 4 apart
+        const float sum = BF16 ? __fadd_rn(__fadd_rn(lo.x, hi.x), __fadd_rn(lo.y, hi.y)) : __fadd_rn(__fadd_rn(lo.x, lo.y), __fadd_rn(hi.x, hi.y));
+        if (quarter == 0 && row < vocab) logits[row] = sum;
+    }
+}
+inline void launch_lm_head(const __half* w, const __half* x16, int hidden, int vocab, float* logits, bool bf16, int sm_count, cudaStream_t s) {
+    const int blocks = std::min(sm_count * 4, (vocab + 63) / 64);
+    if (bf16)
+        lm_head_kernel<true><<<blocks, kHeadOneThreads, hidden * sizeof(float), s>>>(w, x16, hidden, vocab, logits);
+    else
+        lm_head_kernel<false><<<blocks, kHeadOneThreads, hidden * sizeof(float), s>>>(w, x16, hidden, vocab, logits);
+}
+
+// Several tokens: a block walks tiles of vocabulary rows; rows and activations of 128 columns at a time come through a ring of
+// asynchronous copies, and a row is read from HBM once for 32 tokens. Sixteen threads share the accumulator lanes of a dot
+// product (two each, packed); a thread holds eight rows times eight tokens, so a row element and an activation loaded and
+// widened serve eight operations each. The eight warps are spread over the groups of eight tokens that there are (TG = 1, 2 or
+// 4) and, with the rest, over rows: 16 rows a warp. The lanes are added by halving exchanges. Bound by issue slots:
+// 1.75 per packed operation (measured HEADB_TIME).
+constexpr int kHeadThreads = 256, kHeadCols = 128, kHeadTokens = 8;
+constexpr int kHeadRowStride = kHeadCols * 2 + 64;  // bytes: the rows of a warp's two halves are neighbours, half the banks apart
+__host__ __device__ constexpr int head_tile_rows(int tg) { return 16 * (kHeadThreads / 32 / tg); }
+__host__ __device__ constexpr int head_stages(int tg) { return tg == 4 ? 8 : 4; }  // 147 KB of a 32-token block's small stages, 172 KB and 98 KB of the others
+__host__ __device__ constexpr size_t head_stage_bytes(int tg) { return static_cast<size_t>(head_tile_rows(tg)) * kHeadRowStride + tg * kHeadTokens * kHeadCols * 2; }
+
+template <int TG, bool BF16>
+__global__ void __launch_bounds__(kHeadThreads, 1) lm_head_batch_kernel(const __half* __restrict__ w, const __half* __restrict__ x16, int hidden, int vocab, int n, float* __restrict__ logits) {
+    constexpr int kRows = head_tile_rows(TG), kTok = TG * kHeadTokens, kPieces = kHeadCols / 8, kHeadStages = head_stages(TG);
+    extern __shared__ __align__(16) unsigned char head_smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, j = lane & 15, half = lane >> 4;
+    const int t0 = blockIdx.y * kTok, group = warp % TG, wrow = (warp / TG) * 16;
+    const int chunks = hidden / kHeadCols, tiles = (vocab + kRows - 1) / kRows;
+    const int mine = blockIdx.x < static_cast<unsigned>(tiles) ? (tiles - 1 - static_cast<int>(blockIdx.x)) / static_cast<int>(gridDim.x) + 1 : 0;
+    const int total = mine * chunks;
+    auto issue = [&](int it) {  // 128 columns of a tile's rows and of the tokens; rows and tokens past the end repeat the last one
+        if (it < total) {
+            unsigned char* st = head_smem + (it % kHeadStages) * head_stage_bytes(TG);
+            const int row0 = (static_cast<int>(blockIdx.x) + it / chunks * static_cast<int>(gridDim.x)) * kRows, c0 = it % chunks * kHeadCols;
+            for (int i = tid; i < kRows * kPieces; i += kHeadThreads)
+                attn_cp16(st + (i / kPieces) * kHeadRowStride + (i % kPieces) * 16, w + static_cast<size_t>(min(row0 + i / kPieces, vocab - 1)) * hidden + c0 + (i % kPieces) * 8);
+            unsigned char* sx = st + kRows * kHeadRowStride;
+            for (int i = tid; i < kTok * kPieces; i += kHeadThreads)
+                attn_cp16(sx + i * 16, x16 + static_cast<size_t>(min(t0 + i / kPieces, n - 1)) * hidden + c0 + (i % kPieces) * 8);
+        }
+        attn_cp_commit();
+    };
 #pragma unroll
-            for (int j = 0; j < 4; ++j) raw[r][j] = __half_as_ushort(wr[r][j * 32]);
-        for (int k = 0; k < k4; ++k) {
-            float wv[kHeadRows][4];
+    for (int k = 0; k < kHeadStages - 1; ++k) issue(k);
+    unsigned long long acc[64];  // [row][token]
 #pragma unroll
-            for (int r = 0; r < kHeadRows; ++r)
+    for (int k = 0; k < 64; ++k) acc[k] = 0ull;
+    for (int it = 0; it < total; ++it) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kHeadStages - 2) : "memory");
+        __syncthreads();
+        issue(it + kHeadStages - 1);
+        const unsigned char* st = head_smem + (it % kHeadStages) * head_stage_bytes(TG);
+        const unsigned char* sw = st + (wrow + half) * kHeadRowStride + j * 4;
+        const unsigned char* sx = st + kRows * kHeadRowStride + group * kHeadTokens * kHeadCols * 2 + j * 4;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) wv[r][j] = table_to_float(__ushort_as_half(raw[r][j]), bf16);
-            if (k + 1 < k4) {  // the next steps' row elements are requested before this step's arithmetic
+        for (int i = 0; i < kHeadCols / 32; ++i) {
+            unsigned long long wf[8];
 #pragma unroll
-                for (int r = 0; r < kHeadRows; ++r)
+            for (int r = 0; r < 8; ++r) wf[r] = head_widen<BF16>(*reinterpret_cast<const uint32_t*>(sw + 2 * r * kHeadRowStride + i * 64));
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) raw[r][j] = __half_as_ushort(wr[r][(4 * (k + 1) + j) * 32]);
-            }
-            const float4* xk = x4 + static_cast<size_t>(k) * 32 + lane;
-            if (bf16) {  // ggml_vec_dot_bf16: product and sum rounded separately (ops.rs:694-700)
+            for (int t = 0; t < kHeadTokens; ++t) {
+                const unsigned long long x = head_widen<BF16>(*reinterpret_cast<const uint32_t*>(sx + t * kHeadCols * 2 + i * 64));
 #pragma unroll
-                for (int t = 0; t < kHeadTokens; ++t) {
-                    const float4 x = xk[static_cast<size_t>(t) * k4 * 32];
-                    const float xv[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-#pragma unroll
-                        for (int r = 0; r < kHeadRows; ++r) acc[t][r] = __fadd_rn(acc[t][r], __fmul_rn(xv[j], wv[r][j]));
-                }
-            } else {
-#pragma unroll
-                for (int t = 0; t < kHeadTokens; ++t) {
-                    const float4 x = xk[static_cast<size_t>(t) * k4 * 32];
-                    const float xv[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-#pragma unroll
-                        for (int r = 0; r < kHeadRows; ++r) acc[t][r] = __fmaf_rn(xv[j], wv[r][j], acc[t][r]);
-                }
+                for (int r = 0; r < 8; ++r) acc[r * 8 + t] = head_step<BF16>(wf[r], x, acc[r * 8 + t]);
             }
         }
+        if ((it + 1) % chunks == 0) {
+            halve_f32x2(acc, 64, 8, (j & 8) != 0);   // lanes 16 apart: the thread bit is the top bit of the row index
+            halve_f32x2(acc, 32, 4, (j & 4) != 0);   // 8 apart: the next bit of the row index
+            halve_f32x2(acc, 16, 2, (j & 2) != 0);   // 4 apart: its last bit
+            const int row = (static_cast<int>(blockIdx.x) + it / chunks * static_cast<int>(gridDim.x)) * kRows + wrow + half + 2 * (((j >> 3) & 1) * 4 + ((j >> 2) & 1) * 2 + ((j >> 1) & 1));
 #pragma unroll
-        for (int t = 0; t < kHeadTokens; ++t)
-#pragma unroll
-            for (int r = 0; r < kHeadRows; ++r) {
-                const float sum = bf16 ? dot_lane_reduce_bf16(acc[t][r]) : dot_lane_reduce_f16(acc[t][r]);
-                if (lane == 0 && t < nt && row0 + r < vocab) logits[static_cast<size_t>(t0 + t) * vocab + row0 + r] = sum;
+            for (int t = 0; t < kHeadTokens; ++t) {
+                float sum;
+                if constexpr (BF16) {  // 2 apart, then neighbours
+                    const float2 f = unpack_f32x2(add_f32x2(acc[t], shfl_xor_f32x2(acc[t], 1)));
+                    sum = __fadd_rn(f.x, f.y);
+                } else {
+                    const float2 f = unpack_f32x2(acc[t]);
+                    sum = __fadd_rn(f.x, f.y);
+                    sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, 1));
+                }
+                const int tok = t0 + group * kHeadTokens + t;
+                if ((t & 1) == (j & 1) && row < vocab && tok < n) logits[static_cast<size_t>(tok) * vocab + row] = sum;
             }
+#pragma unroll
+            for (int k = 0; k < 64; ++k) acc[k] = 0ull;
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+inline size_t lm_head_batch_smem(int tg) { return head_stages(tg) * head_stage_bytes(tg); }
+inline int lm_head_token_groups(int n) { return n <= kHeadTokens ? 1 : n <= 2 * kHeadTokens ? 2 : 4; }
+using LmHeadBatchKernel = void (*)(const __half*, const __half*, int, int, int, float*);
+inline LmHeadBatchKernel lm_head_batch_for(int tg, bool bf16) {
+    switch (tg) {
+        case 1: return bf16 ? lm_head_batch_kernel<1, true> : lm_head_batch_kernel<1, false>;
+        case 2: return bf16 ? lm_head_batch_kernel<2, true> : lm_head_batch_kernel<2, false>;
+        default: return bf16 ? lm_head_batch_kernel<4, true> : lm_head_batch_kernel<4, false>;
     }
 }
 

@@ -337,7 +337,7 @@ inline int enqueue_token(quintrit_b200_decoder* d, bool with_head) {
         nf.block_scaled = bs;
         norm_quant_kernel<<<1, kRowThreads, H * sizeof(float), s>>>(nf);
         QTB_LAUNCH_CHECK();
-        lm_head_kernel<<<d->sm_count * 8, 256, H * sizeof(float), s>>>(d->lm_head, d->x16, H, d->vocab, d->logits, d->bf16_tables);
+        launch_lm_head(d->lm_head, d->x16, H, d->vocab, d->logits, d->bf16_tables, d->sm_count, s);
         QTB_LAUNCH_CHECK();
         argmax_kernel<<<1, 1024, 0, s>>>(d->logits, d->vocab, d->d_token);
         QTB_LAUNCH_CHECK();

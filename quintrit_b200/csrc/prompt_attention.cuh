@@ -14,6 +14,7 @@
 // prompt of a 4-layer Falcon3-10B shape: 8.03 -> 6.11 ms against a block per token (attention_gqa_kernel).
 #pragma once
 #include "decode.cuh"
+#include "packed_f32.cuh"
 
 namespace qtb {
 
@@ -23,35 +24,6 @@ __host__ __device__ constexpr size_t attn_tile_smem(int g, int hd) {
     return static_cast<size_t>(kTokenTileRows) * (attn_tile_key_stride(hd) + hd * 2) + static_cast<size_t>(kTokenTile) * g * (hd * 4 + kTokenTileRows * 12);
 }
 
-__device__ __forceinline__ unsigned long long pack_f32x2(float a, float b) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 unpack_f32x2(unsigned long long v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ unsigned long long fma_f32x2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ unsigned long long mul_f32x2(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ unsigned long long add_f32x2(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ unsigned long long widen_half2(uint32_t h) {
-    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
-    return pack_f32x2(f.x, f.y);
-}
 template <bool F32>
 __device__ __forceinline__ unsigned long long value_round2(unsigned long long v) {  // value_round of both halves
     if constexpr (F32) return v;
@@ -59,21 +31,6 @@ __device__ __forceinline__ unsigned long long value_round2(unsigned long long v)
     const float2 r = __half22float2(__floats2half2_rn(f.x, f.y));
     return pack_f32x2(r.x, r.y);
 }
-__device__ __forceinline__ unsigned long long shfl_xor_f32x2(unsigned long long v, int mask) { return __shfl_xor_sync(0xffffffffu, v, mask); }
-
-// One halving step over the thread bit `mask`: threads with the bit clear keep the first half of the values, the others the
-// second half, each added to the partner's copy.
-template <int N>
-__device__ __forceinline__ void halve_f32x2(unsigned long long (&v)[N], int n, int mask, bool upper) {
-#pragma unroll
-    for (int k = 0; k < N / 2; ++k) {
-        if (k < n / 2) {
-            const unsigned long long keep = upper ? v[k + n / 2] : v[k], send = upper ? v[k] : v[k + n / 2];
-            v[k] = add_f32x2(keep, shfl_xor_f32x2(send, mask));
-        }
-    }
-}
-
 // Grid (kv_heads, 4 chunks, token tiles). Token tiles are aligned to positions that are multiples of eight, so that the
 // tokens of a tile agree on the division of the cache into chunks (it changes at multiples of 256).
 template <int G, int E, bool F32>  // query heads per KV head, head_dim / 32
