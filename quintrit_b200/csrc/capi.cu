@@ -2101,7 +2101,7 @@ extern "C" int quintrit_b200_decoder_trace_step(quintrit_b200_decoder_t* decoder
 namespace {
 
 std::mutex g_gemm_lock;
-constexpr int kGemmMaxParts = 8;
+constexpr int kGemmMaxParts = kAccPartsMax;
 constexpr size_t kGemmSmemLimit = 227 * 1024;  // dynamic shared memory a CTA may ask for on this device
 // Makes the two-bit copy of the weights and the call buffers of a matrix the first time it is used by the batched projection.
 int gemm_prepare(quintrit_b200_matrix* m) {
@@ -2400,8 +2400,8 @@ int prefill_layers(quintrit_b200_decoder* d, int n, const BatchTarget& tg) {
         if (l > 0) n1.acc_prev = d->pf.acc_down, n1.b_acc = H, n1.scale_prev = d->pf.s_i, n1.ws_prev = d->scales[(l - 1) * 7 + 6];
         n1.norm_w = d->norms[l * 4 + 0], n1.eps = d->eps, n1.n = H;
         n1.q_out = d->pf.a8_h, n1.b_q = H, n1.scale_out = d->pf.s_h, n1.b_scale = 1;
-        if (l > 0) n1.v_prev = v_down;
-        norm_quant_kernel<<<dim3(1, 1, n), kRowThreads, H * sizeof(float), s>>>(n1);
+        if (l > 0) n1.v_prev = defer ? v_down : AccView{d->pf.acc_down, 1, 0, H};
+        launch_norm_quant_rows(n1, n, s);
         QTB_LAUNCH_CHECK();
         if (quintrit_b200_matrix* sq = d->pf.stack[size_t(l) * 2]) {  // q | k | v as one product
             if ((rc = gemm_launch(sq, d->pf.a8_h, n, d->pf.acc_qkv, s, qkv, &v_q, st, d->pf.parts[0])) != QUINTRIT_OK) return rc;
@@ -2437,15 +2437,15 @@ int prefill_layers(quintrit_b200_decoder* d, int n, const BatchTarget& tg) {
         af.q_heads = d->q_heads, af.head_dim = hd, af.ctx = d->ctx;
         af.sub_norm_w = d->norms[l * 4 + 2], af.eps = d->eps;
         af.q_out = d->pf.a8_q, af.b_q = qd, af.scale_out = d->pf.s_q, af.b_scale = 1;
-        attn_finish_kernel<<<dim3(1, 1, n), kRowThreads, qd * sizeof(float), s>>>(af);
+        launch_attn_finish_rows(af, n, s);
         QTB_LAUNCH_CHECK();
         if ((rc = gemm_launch(mat(l, 3), d->pf.a8_q, n, d->pf.acc_o, s, 0, view(&v_o), st, d->pf.parts[3])) != QUINTRIT_OK) return rc;
         NormQuantArgs n2{};
         n2.x = d->pf.x, n2.b_x = H, n2.acc_prev = d->pf.acc_o, n2.b_acc = H, n2.scale_prev = d->pf.s_q, n2.ws_prev = sc[3];
         n2.norm_w = d->norms[l * 4 + 1], n2.eps = d->eps, n2.n = H;
         n2.q_out = d->pf.a8_h, n2.b_q = H, n2.scale_out = d->pf.s_h, n2.b_scale = 1;
-        if (defer) n2.v_prev = v_o;
-        norm_quant_kernel<<<dim3(1, 1, n), kRowThreads, H * sizeof(float), s>>>(n2);
+        n2.v_prev = defer ? v_o : AccView{d->pf.acc_o, 1, 0, H};
+        launch_norm_quant_rows(n2, n, s);
         QTB_LAUNCH_CHECK();
         if (quintrit_b200_matrix* sg = d->pf.stack[size_t(l) * 2 + 1]) {  // gate | up as one product
             if ((rc = gemm_launch(sg, d->pf.a8_h, n, d->pf.acc_gu, s, 2 * I, &v_gate, st, d->pf.parts[4])) != QUINTRIT_OK) return rc;
@@ -2461,11 +2461,8 @@ int prefill_layers(quintrit_b200_decoder* d, int n, const BatchTarget& tg) {
         aq.n = I, aq.relu2 = d->arch == QUINTRIT_B200_ARCH_BITNET;
         aq.sub_norm_w = d->norms[l * 4 + 3], aq.eps = d->eps;
         aq.q_out = d->pf.a8_i, aq.b_q = I, aq.scale_out = d->pf.s_i;
-        if (gu_views) aq.v_gate = v_gate, aq.v_up = v_up;
-        if (std::getenv("QUINTRIT_B200_ACT_CLUSTER_OFF") == nullptr)
-            act_quant_cluster_kernel<<<dim3(kActClusterSize, 1, n), kActClusterThreads, act_cluster_slice(I) * sizeof(float), s>>>(aq);
-        else
-            act_quant_kernel<<<dim3(1, 1, n), kRowThreads, I * sizeof(float), s>>>(aq);
+        aq.v_gate = gu_views ? v_gate : AccView{aq.acc_gate, 1, 0, aq.b_acc}, aq.v_up = gu_views ? v_up : AccView{aq.acc_up, 1, 0, aq.b_acc};
+        launch_act_quant_rows(aq, n, s);
         QTB_LAUNCH_CHECK();
         if ((rc = gemm_launch(mat(l, 6), d->pf.a8_i, n, d->pf.acc_down, s, 0, l + 1 < d->layers ? view(&v_down) : nullptr, st, d->pf.parts[6])) != QUINTRIT_OK) return rc;
     }
@@ -2996,8 +2993,9 @@ int batch_head(quintrit_b200_batch* b, int n) {
     NormQuantArgs nf{};
     nf.x = d->pf.x, nf.b_x = H, nf.acc_prev = d->pf.acc_down, nf.b_acc = H, nf.scale_prev = d->pf.s_i, nf.b_scale = 1;
     nf.ws_prev = d->scales[(d->layers - 1) * 7 + 6], nf.norm_w = d->out_norm, nf.eps = d->eps, nf.n = H;
+    nf.v_prev = AccView{d->pf.acc_down, 1, 0, H};
     nf.y16_out = b->x16, nf.b_y16 = H, nf.y16_bf16 = d->bf16_tables;
-    norm_quant_kernel<<<dim3(1, 1, n), kRowThreads, H * sizeof(float), s>>>(nf);
+    launch_norm_quant_rows(nf, n, s);
     QTB_LAUNCH_CHECK();
     if (n > 1 && H % kHeadCols == 0) {
         const int tg = lm_head_token_groups(n);

@@ -11,6 +11,7 @@
 #include "gemv_lut.cuh"
 #include "megakernel.cuh"
 #include "prompt_attention.cuh"
+#include "row_kernels.cuh"
 
 namespace qtb {
 struct LayeredDecoder;  // layered.cuh: a model whose layers differ from one another
