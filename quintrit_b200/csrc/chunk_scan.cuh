@@ -30,9 +30,23 @@ struct ChunkWork {
     bf16* qk;      // hgrn2: [head][chunk][q hi, q lo, k hi, k lo][16][rows]
     float* a;      // hgrn2: [head][chunk][16][16]
     float* fe;     // hgrn2: [head][chunk][rows]
-    int v_pad, rows;
+    float* starts; // [head][segment][v_pad][rows]: the state a segment starts from; before the carry, from the second segment on, what the one before it adds
+    float* decay;  // [head][segment][rows] (mamba2: one value): how much of a state is left after the segment
+    int v_pad, rows, segments, per;  // segments of a head's chunks that are scanned side by side, chunks of a segment
 };
-inline size_t chunk_work(char* base, bool mamba, int heads, int vdim, int n, int groups, int tokens, ChunkWork* w) {
+
+// Segments of a prompt's chunks. A block a head and 64 columns walks its chunks one after another (1.2-1.4 us each, a chain of dependent
+// products), and a few dozen such blocks leave most of the machine idle. Scanned in segments, a segment's own contribution to the state comes
+// first (all but the last, from a state of zero), then a pass over the segments gives the states they start from, then all segments scan side by
+// side: about 1.6 times the products, on as many blocks as give every multiprocessor two, and two more launches. Below kSegmentChunks chunks a
+// segment, or with fewer than three segments, the launches cost more than the shorter chain saves. 2048 tokens: 64 heads of 64 x 128 in 4 segments
+// 179 -> 105 us (local 31, carry 6, scan 68), 16 heads of 128 x 128 in 9 segments 144 -> 60 us (18, 8, 34).
+constexpr int kSegmentChunks = 8;
+inline int chunk_segments(int blocks, int chunks, int sm_count) {
+    const int most = 2 * sm_count / blocks, worth = chunks / kSegmentChunks, s = most < worth ? most : worth;
+    return s < 3 ? 1 : s;
+}
+inline size_t chunk_work(char* base, bool mamba, int heads, int vdim, int n, int groups, int tokens, int sm_count, ChunkWork* w) {
     const size_t t = size_t(chunk_count(tokens)) * kChunkT, c = chunk_count(tokens);
     size_t at = 0;
     auto take = [&](size_t bytes) {
@@ -51,6 +65,12 @@ inline size_t chunk_work(char* base, bool mamba, int heads, int vdim, int n, int
         w->qk = reinterpret_cast<bf16*>(take(c * heads * 64 * w->rows * 2));
         w->a = reinterpret_cast<float*>(take(c * heads * 256 * 4));
         w->fe = reinterpret_cast<float*>(take(c * heads * w->rows * 4));
+    }
+    const int chunks = static_cast<int>(c), most = chunk_segments(heads * (w->v_pad / kChunkV), chunks, sm_count);
+    w->per = (chunks + most - 1) / most, w->segments = (chunks + w->per - 1) / w->per;
+    if (w->segments > 1) {  // (room for `most`, which never falls as the tokens get more: the space made for the longest launch serves every other)
+        w->starts = reinterpret_cast<float*>(take(size_t(heads) * most * w->v_pad * w->rows * 4));
+        w->decay = reinterpret_cast<float*>(take(size_t(heads) * most * w->rows * 4));
     }
     return at;
 }
@@ -213,33 +233,40 @@ __global__ void __launch_bounds__(128) hgrn_prep_kernel(const __grid_constant__ 
     }
 }
 
-template <int KIND> inline size_t chunk_scan_smem(int rows) {
-    const size_t stage = size_t(KIND == kScanMamba2 ? 2 : 4) * kChunkT * (rows + 8) * 2 + size_t(kChunkT) * (kChunkV + 8) * 2 + 256 * 4 + (KIND == kScanMamba2 ? 32 : rows) * 4;
-    return kChunkStages * stage;
+// Operand tiles of a chunk: C (q hi, q lo), then B (k hi, k lo); a segment's own contribution needs neither the first ones nor A.
+template <int KIND, bool LOCAL> __host__ __device__ constexpr int chunk_scan_ops() { return (KIND == kScanMamba2 ? 2 : 4) / (LOCAL ? 2 : 1); }
+template <int KIND, int ROWS, bool LOCAL> __host__ __device__ constexpr size_t chunk_scan_stage() {
+    return size_t(chunk_scan_ops<KIND, LOCAL>()) * kChunkT * (ROWS + 8) * 2 + size_t(kChunkT) * (kChunkV + 8) * 2 + (LOCAL ? 0 : 256 * 4) + (KIND == kScanMamba2 ? 32 : ROWS) * 4;
 }
+template <int KIND, int ROWS, bool LOCAL> __host__ __device__ constexpr size_t chunk_scan_smem() { return kChunkStages * chunk_scan_stage<KIND, ROWS, LOCAL>(); }
 
-// grid: (heads, ceil(vdim / 64)); warp w owns the state columns 16 w .. 16 w + 15 of the block's 64. y: without mamba2's silu(z), which the
-// kernel that norms y applies.
-template <int KIND, int ROWS>
+// grid: (heads, ceil(vdim / 64), segments); warp w owns the state columns 16 w .. 16 w + 15 of the block's 64. y: without mamba2's silu(z), which the
+// kernel that norms y applies. LOCAL: no outputs, only what the chunks of the segment add to a state and how much they leave of it (one segment fewer).
+template <int KIND, int ROWS, bool LOCAL>
 __global__ void __launch_bounds__(128) chunk_scan_kernel(const __grid_constant__ ScanArgs a, const __grid_constant__ ChunkWork w) {
     extern __shared__ __align__(16) unsigned char cs_sm[];
-    constexpr int kOps = KIND == kScanMamba2 ? 2 : 4, kPitch = ROWS + 8, kVPitch = kChunkV + 8, kTail = KIND == kScanMamba2 ? 32 : ROWS;
-    constexpr size_t kStage = size_t(kOps) * kChunkT * kPitch * 2 + size_t(kChunkT) * kVPitch * 2 + 256 * 4 + kTail * 4;
+    constexpr int kOps = chunk_scan_ops<KIND, LOCAL>(), kPitch = ROWS + 8, kVPitch = kChunkV + 8, kTail = KIND == kScanMamba2 ? 32 : ROWS, kMat = LOCAL ? 0 : 64;  // (float4s of A)
+    constexpr int kFirstK = LOCAL ? 0 : kOps / 2;  // the first tile of B or k
+    constexpr size_t kStage = chunk_scan_stage<KIND, ROWS, LOCAL>();
     const int head = blockIdx.x, v0 = blockIdx.y * kChunkV, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
     const int chunks = (a.tokens + kChunkT - 1) / kChunkT, inner = a.heads * a.vdim, group = KIND == kScanMamba2 ? head / (a.heads / a.groups) : 0;
     const uint32_t pos0 = seq_position(a.seq, a.pos, 0);
     const int vw = v0 + warp * 16;
     float* state = a.state + size_t(head) * a.vdim * a.n;
+    const int seg = blockIdx.z, from = seg * w.per, to = min(from + w.per, chunks);
+    auto start = [&](int s, int v, int d) { return w.starts + ((size_t(head) * w.segments + s) * w.v_pad + v) * ROWS + d; };
     float S[ROWS / 8][4];
 #pragma unroll
     for (int j = 0; j < ROWS / 8; ++j)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int v = vw + g + (e >> 1) * 8, d = 8 * j + 2 * c + (e & 1);
-            S[j][e] = pos0 > 0 && v < a.vdim && d < a.n ? state[size_t(v) * a.n + d] : 0.0f;
+            if (LOCAL) S[j][e] = 0.0f;
+            else if (w.segments > 1) S[j][e] = v < a.vdim ? *start(seg, v, d) : 0.0f;
+            else S[j][e] = pos0 > 0 && v < a.vdim && d < a.n ? state[size_t(v) * a.n + d] : 0.0f;
         }
     auto fetch = [&](int chunk) {
-        if (chunk >= chunks) {
+        if (chunk >= to) {
             cp_async_commit_group();  // (an empty group keeps the count of groups in step with the chunks)
             return;
         }
@@ -249,9 +276,9 @@ __global__ void __launch_bounds__(128) chunk_scan_kernel(const __grid_constant__
         float* mat = reinterpret_cast<float*>(xs + kChunkT * kVPitch);
         constexpr int kVec = ROWS / 8;
         for (int i = tid; i < kOps * kChunkT * kVec; i += 128) {
-            const int op = i / (kChunkT * kVec), t = i / kVec % kChunkT, p = i % kVec;
-            const bf16* src = KIND == kScanMamba2 ? w.bc + ((size_t(chunk * kChunkT + t) * 2 + (1 - op)) * a.groups + group) * ROWS + p * 8
-                                                  : w.qk + ((size_t(head) * chunks + chunk) * 64 + op * kChunkT + t) * ROWS + p * 8;
+            const int op = i / (kChunkT * kVec), all = LOCAL ? op + kOps : op, t = i / kVec % kChunkT, p = i % kVec;
+            const bf16* src = KIND == kScanMamba2 ? w.bc + ((size_t(chunk * kChunkT + t) * 2 + (1 - all)) * a.groups + group) * ROWS + p * 8
+                                                  : w.qk + ((size_t(head) * chunks + chunk) * 64 + all * kChunkT + t) * ROWS + p * 8;
             cp_async16(ops + (op * kChunkT + t) * kPitch + p * 8, src, true);
         }
         for (int i = tid; i < kChunkT * (kChunkV / 8); i += 128) {
@@ -260,70 +287,77 @@ __global__ void __launch_bounds__(128) chunk_scan_kernel(const __grid_constant__
         }
         const float* m = KIND == kScanMamba2 ? w.gram + (size_t(chunk) * a.groups + group) * 256 : w.a + (size_t(head) * chunks + chunk) * 256;
         const float* tail = KIND == kScanMamba2 ? w.dt + (size_t(head) * chunks + chunk) * 32 : w.fe + (size_t(head) * chunks + chunk) * ROWS;
-        for (int i = tid; i < 64 + kTail / 4; i += 128) cp_async16(mat + i * 4, i < 64 ? m + i * 4 : tail + (i - 64) * 4, true);
+        for (int i = tid; i < kMat + kTail / 4; i += 128) cp_async16(mat + i * 4, i < kMat ? m + i * 4 : tail + (i - kMat) * 4, true);
         cp_async_commit_group();
     };
-    for (int i = 0; i < kChunkStages - 1; ++i) fetch(i);
-    for (int chunk = 0; chunk < chunks; ++chunk) {
+    float left = KIND == kScanMamba2 ? 0.0f : 1.0f;  // LOCAL: sum of the log decays, product of the decays of state row tid
+    for (int i = 0; i < kChunkStages - 1; ++i) fetch(from + i);
+    for (int chunk = from; chunk < to; ++chunk) {
         unsigned char* st = cs_sm + (chunk % kChunkStages) * kStage;
         cp_async_wait_group<kChunkStages - 2>();
         __syncthreads();
         fetch(chunk + kChunkStages - 1);  // into the stage of the chunk before this one, which every warp has left
+        const bf16* ops = reinterpret_cast<const bf16*>(st);
+        const bf16* xs = ops + kOps * kChunkT * kPitch;
+        const float* mat = reinterpret_cast<const float*>(xs + kChunkT * kVPitch);
+        const float* tail = mat + 4 * kMat;  // mamba2: dt, running sums; hgrn2: F_16
+        if constexpr (LOCAL) {
+            if (KIND == kScanMamba2) left += tail[16 + 15];
+            else if (tid < ROWS) left *= tail[tid];
+        }
         if (vw < a.vdim) {
-            const bf16* ops = reinterpret_cast<const bf16*>(st);
-            const bf16* xs = ops + kOps * kChunkT * kPitch;
-            const float* mat = reinterpret_cast<const float*>(xs + kChunkT * kVPitch);
-            const float* tail = mat + 256;  // mamba2: dt, running sums; hgrn2: F_16
             uint32_t xv[4];                 // x as a B operand: columns 0..7 (0, 1) and 8..15 (2, 3); transposed it is the A operand {0, 2, 1, 3}
             load_frag_b(xv, xs + warp * 16, kVPitch);
-            float O[2][4] = {}, P[3][2][4] = {};  // independent sums: a product waits for the one before it in the same registers
+            if constexpr (!LOCAL) {
+                float O[2][4] = {}, P[3][2][4] = {};  // independent sums: a product waits for the one before it in the same registers
 #pragma unroll
-            for (int ks = 0; ks < ROWS / 16; ++ks) {
-                uint32_t q[4], ql[4], h[4], l[4];
-                load_frag_a(q, ops + ks * 16, kPitch);
-                split_bf16(S[2 * ks][0], S[2 * ks][1], &h[0], &l[0]), split_bf16(S[2 * ks + 1][0], S[2 * ks + 1][1], &h[1], &l[1]);
-                split_bf16(S[2 * ks][2], S[2 * ks][3], &h[2], &l[2]), split_bf16(S[2 * ks + 1][2], S[2 * ks + 1][3], &h[3], &l[3]);
-                if (ks & 1) mma_16816(P[0][0], q, h[0], h[1]), mma_16816(P[0][1], q, h[2], h[3]);
-                else mma_16816(O[0], q, h[0], h[1]), mma_16816(O[1], q, h[2], h[3]);
-                mma_16816(P[1][0], q, l[0], l[1]), mma_16816(P[1][1], q, l[2], l[3]);
-                if (KIND == kScanHgrn2) {
-                    load_frag_a(ql, ops + kChunkT * kPitch + ks * 16, kPitch);
-                    mma_16816(P[2][0], ql, h[0], h[1]), mma_16816(P[2][1], ql, h[2], h[3]);
+                for (int ks = 0; ks < ROWS / 16; ++ks) {
+                    uint32_t q[4], ql[4], h[4], l[4];
+                    load_frag_a(q, ops + ks * 16, kPitch);
+                    split_bf16(S[2 * ks][0], S[2 * ks][1], &h[0], &l[0]), split_bf16(S[2 * ks + 1][0], S[2 * ks + 1][1], &h[1], &l[1]);
+                    split_bf16(S[2 * ks][2], S[2 * ks][3], &h[2], &l[2]), split_bf16(S[2 * ks + 1][2], S[2 * ks + 1][3], &h[3], &l[3]);
+                    if (ks & 1) mma_16816(P[0][0], q, h[0], h[1]), mma_16816(P[0][1], q, h[2], h[3]);
+                    else mma_16816(O[0], q, h[0], h[1]), mma_16816(O[1], q, h[2], h[3]);
+                    mma_16816(P[1][0], q, l[0], l[1]), mma_16816(P[1][1], q, l[2], l[3]);
+                    if (KIND == kScanHgrn2) {
+                        load_frag_a(ql, ops + kChunkT * kPitch + ks * 16, kPitch);
+                        mma_16816(P[2][0], ql, h[0], h[1]), mma_16816(P[2][1], ql, h[2], h[3]);
+                    }
                 }
-            }
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
+                for (int i = 0; i < 2; ++i)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) O[i][e] += P[0][i][e] + (P[1][i][e] + P[2][i][e]);
-            // the sums inside the chunk
-            float A[8];  // A rows t = g, g + 8 at s = 2c, 2c + 1 | 2c + 8, 2c + 9, in operand order
+                    for (int e = 0; e < 4; ++e) O[i][e] += P[0][i][e] + (P[1][i][e] + P[2][i][e]);
+                // the sums inside the chunk
+                float A[8];  // A rows t = g, g + 8 at s = 2c, 2c + 1 | 2c + 8, 2c + 9, in operand order
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const int t = g + ((e >> 1) & 1) * 8, s = 2 * c + (e & 1) + (e >> 2) * 8;
-                A[e] = s <= t ? mat[t * 16 + s] : 0.0f;
-                if (KIND == kScanMamba2 && s <= t) A[e] *= expf(tail[16 + t] - tail[16 + s]) * tail[s];
-            }
-            if (KIND == kScanMamba2) {
-                const float e0 = expf(tail[16 + g]), e1 = expf(tail[16 + g + 8]);
-#pragma unroll
-                for (int i = 0; i < 2; ++i) O[i][0] *= e0, O[i][1] *= e0, O[i][2] *= e1, O[i][3] *= e1;
-            }
-            uint32_t ah[4], al[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) split_bf16(A[2 * e], A[2 * e + 1], &ah[e], &al[e]);
-            mma_16816(O[0], ah, xv[0], xv[1]), mma_16816(O[1], ah, xv[2], xv[3]);
-            mma_16816(O[0], al, xv[0], xv[1]), mma_16816(O[1], al, xv[2], xv[3]);
-            const float skip = KIND == kScanMamba2 ? a.d_skip[head] : 0.0f;
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int tl = g + (e >> 1) * 8, t = chunk * kChunkT + tl, vl = warp * 16 + i * 8 + 2 * c + (e & 1);
-                    if (t >= a.tokens || v0 + vl >= a.vdim) continue;
-                    float y = O[i][e];
-                    if (KIND == kScanMamba2) y += skip * __bfloat162float(xs[tl * kVPitch + vl]);
-                    a.y[size_t(t) * inner + head * a.vdim + v0 + vl] = y;
+                for (int e = 0; e < 8; ++e) {
+                    const int t = g + ((e >> 1) & 1) * 8, s = 2 * c + (e & 1) + (e >> 2) * 8;
+                    A[e] = s <= t ? mat[t * 16 + s] : 0.0f;
+                    if (KIND == kScanMamba2 && s <= t) A[e] *= expf(tail[16 + t] - tail[16 + s]) * tail[s];
                 }
+                if (KIND == kScanMamba2) {
+                    const float e0 = expf(tail[16 + g]), e1 = expf(tail[16 + g + 8]);
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) O[i][0] *= e0, O[i][1] *= e0, O[i][2] *= e1, O[i][3] *= e1;
+                }
+                uint32_t ah[4], al[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) split_bf16(A[2 * e], A[2 * e + 1], &ah[e], &al[e]);
+                mma_16816(O[0], ah, xv[0], xv[1]), mma_16816(O[1], ah, xv[2], xv[3]);
+                mma_16816(O[0], al, xv[0], xv[1]), mma_16816(O[1], al, xv[2], xv[3]);
+                const float skip = KIND == kScanMamba2 ? a.d_skip[head] : 0.0f;
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int tl = g + (e >> 1) * 8, t = chunk * kChunkT + tl, vl = warp * 16 + i * 8 + 2 * c + (e & 1);
+                        if (t >= a.tokens || v0 + vl >= a.vdim) continue;
+                        float y = O[i][e];
+                        if (KIND == kScanMamba2) y += skip * __bfloat162float(xs[tl * kVPitch + vl]);
+                        a.y[size_t(t) * inner + head * a.vdim + v0 + vl] = y;
+                    }
+            }
             // the state after the chunk
             if (KIND == kScanMamba2) {
                 const float total = tail[16 + 15], decay = expf(total);
@@ -337,7 +371,7 @@ __global__ void __launch_bounds__(128) chunk_scan_kernel(const __grid_constant__
 #pragma unroll
                 for (int j = 0; j < ROWS / 8; j += 2) {
                     uint32_t k[4];
-                    load_frag_b(k, ops + kChunkT * kPitch + j * 8, kPitch);
+                    load_frag_b(k, ops + kFirstK * kChunkT * kPitch + j * 8, kPitch);
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
 #pragma unroll
@@ -351,8 +385,8 @@ __global__ void __launch_bounds__(128) chunk_scan_kernel(const __grid_constant__
 #pragma unroll
                 for (int j = 0; j < ROWS / 8; j += 2) {
                     uint32_t kh[4], kl[4];
-                    load_frag_b(kh, ops + 2 * kChunkT * kPitch + j * 8, kPitch);
-                    load_frag_b(kl, ops + 3 * kChunkT * kPitch + j * 8, kPitch);
+                    load_frag_b(kh, ops + kFirstK * kChunkT * kPitch + j * 8, kPitch);
+                    load_frag_b(kl, ops + (kFirstK + 1) * kChunkT * kPitch + j * 8, kPitch);
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         const float2 fe = *reinterpret_cast<const float2*>(tail + (j + h) * 8 + 2 * c);
@@ -364,6 +398,16 @@ __global__ void __launch_bounds__(128) chunk_scan_kernel(const __grid_constant__
             }
         }
     }
+    if constexpr (LOCAL) {
+        if (blockIdx.y == 0 && tid < ROWS) w.decay[(size_t(head) * w.segments + seg) * ROWS + tid] = KIND == kScanMamba2 ? expf(left) : left;
+#pragma unroll
+        for (int j = 0; j < ROWS / 8; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (vw + g + 8 * h < a.vdim) *reinterpret_cast<float2*>(start(seg + 1, vw + g + 8 * h, 8 * j + 2 * c)) = make_float2(S[j][2 * h], S[j][2 * h + 1]);
+        return;
+    }
+    if (to < chunks) return;
 #pragma unroll
     for (int j = 0; j < ROWS / 8; ++j)
 #pragma unroll
@@ -371,6 +415,45 @@ __global__ void __launch_bounds__(128) chunk_scan_kernel(const __grid_constant__
             const int v = vw + g + (e >> 1) * 8, d = 8 * j + 2 * c + (e & 1);
             if (v < a.vdim && d < a.n) state[size_t(v) * a.n + d] = S[j][e];
         }
+}
+
+// The states that the segments start from: S of segment s + 1 = what is left of S after segment s + what segment s adds. grid: (ceil(vdim * rows / 512),
+// heads), 128 threads of four rows of a column. The reads do not depend on the sums, so they are in flight together (64 heads of 64 x 128, 4 segments: 5.5 us).
+__global__ void __launch_bounds__(128) chunk_carry_kernel(const __grid_constant__ ScanArgs a, const __grid_constant__ ChunkWork w) {
+    const int i = (blockIdx.x * 128 + threadIdx.x) * 4, v = i / w.rows, d = i % w.rows, head = blockIdx.y;
+    if (v >= a.vdim) return;
+    float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (seq_position(a.seq, a.pos, 0) > 0) {
+        const float* state = a.state + (size_t(head) * a.vdim + v) * a.n + d;
+        if (d < a.n) s.x = state[0];
+        if (d + 1 < a.n) s.y = state[1];
+        if (d + 2 < a.n) s.z = state[2];
+        if (d + 3 < a.n) s.w = state[3];
+    }
+    const size_t step = size_t(w.v_pad) * w.rows;
+    float* at = w.starts + size_t(head) * w.segments * step + size_t(v) * w.rows + d;
+    const float* decay = w.decay + size_t(head) * w.segments * w.rows + d;
+    *reinterpret_cast<float4*>(at) = s;
+#pragma unroll 4
+    for (int k = 1; k < w.segments; ++k) {
+        const float4 add = *reinterpret_cast<const float4*>(at + k * step), f = *reinterpret_cast<const float4*>(decay + (k - 1) * w.rows);
+        s.x = fmaf(s.x, f.x, add.x), s.y = fmaf(s.y, f.y, add.y), s.z = fmaf(s.z, f.z, add.z), s.w = fmaf(s.w, f.w, add.w);
+        *reinterpret_cast<float4*>(at + k * step) = s;
+    }
+}
+
+// The launches of a scan over prepared chunks.
+struct ChunkScanKernels {
+    void (*local)(ScanArgs, ChunkWork);
+    void (*scan)(ScanArgs, ChunkWork);
+    size_t local_smem, smem;
+};
+template <int KIND, int ROWS> ChunkScanKernels chunk_scan_kernels_of() {
+    return {chunk_scan_kernel<KIND, ROWS, true>, chunk_scan_kernel<KIND, ROWS, false>, chunk_scan_smem<KIND, ROWS, true>(), chunk_scan_smem<KIND, ROWS, false>()};
+}
+inline ChunkScanKernels chunk_scan_kernels(bool mamba, int rows) {
+    if (mamba) return rows == 32 ? chunk_scan_kernels_of<kScanMamba2, 32>() : rows == 64 ? chunk_scan_kernels_of<kScanMamba2, 64>() : chunk_scan_kernels_of<kScanMamba2, 128>();
+    return rows == 32 ? chunk_scan_kernels_of<kScanHgrn2, 32>() : rows == 64 ? chunk_scan_kernels_of<kScanHgrn2, 64>() : chunk_scan_kernels_of<kScanHgrn2, 128>();
 }
 
 }  // namespace qtb

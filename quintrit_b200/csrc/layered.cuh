@@ -469,7 +469,7 @@ inline int layered_decoder_setup(quintrit_b200_decoder* d, const std::shared_ptr
                 if (m.f32) continue;
                 if (l.kind == MixerKind::kRetention && retention_chunked(l)) work = std::max(work, retention_work(nullptr, l.heads, l.dim, l.vdim, kLayeredChunk, &rw));
                 else if (l.kind != MixerKind::kRetention && chunk_scan_rows(l.key_dim()) != 0)
-                    work = std::max(work, chunk_work(nullptr, l.kind == MixerKind::kMamba2, l.heads, l.vdim, l.key_dim(), l.groups, kLayeredChunk, &cw));
+                    work = std::max(work, chunk_work(nullptr, l.kind == MixerKind::kMamba2, l.heads, l.vdim, l.key_dim(), l.groups, kLayeredChunk, m.sm_count, &cw));
                 continue;
             }
             if (l.kind == MixerKind::kLogistic) queries = std::max(queries, size_t(l.heads) * round_up(l.dim, 64));
@@ -538,14 +538,16 @@ inline int layered_decoder_setup(quintrit_b200_decoder* d, const std::shared_ptr
                              reinterpret_cast<const void*>(dense_gemm_tc_kernel<128, kDenseDual>), reinterpret_cast<const void*>(dense_gemm_tc_kernel<128, kDensePlain>),
                              reinterpret_cast<const void*>(dense_gemm_tc_kernel<256, kDensePlain>), reinterpret_cast<const void*>(dense_gemm_tc_kernel<128, kDenseGrouped>),
                              reinterpret_cast<const void*>(dense_gemm_tc_kernel<256, kDenseGrouped>),
-                             reinterpret_cast<const void*>(chunk_scan_kernel<kScanMamba2, 32>), reinterpret_cast<const void*>(chunk_scan_kernel<kScanMamba2, 64>),
-                             reinterpret_cast<const void*>(chunk_scan_kernel<kScanMamba2, 128>), reinterpret_cast<const void*>(chunk_scan_kernel<kScanHgrn2, 32>),
-                             reinterpret_cast<const void*>(chunk_scan_kernel<kScanHgrn2, 64>), reinterpret_cast<const void*>(chunk_scan_kernel<kScanHgrn2, 128>),
                              reinterpret_cast<const void*>(pooled_attention_mma_kernel<32>), reinterpret_cast<const void*>(pooled_attention_mma_kernel<64>),
                              reinterpret_cast<const void*>(pooled_attention_mma_kernel<128>)};
     for (int heads : {1, 4, 8})
         for (LogisticStep k : {logistic_step_for<bf16, true>(heads), logistic_step_for<float, true>(heads), logistic_step_for<float, false>(heads)}) kernels.push_back(reinterpret_cast<const void*>(k));
     kernels.push_back(reinterpret_cast<const void*>(logistic_mma_kernel<kLogisticMmaDims>)), kernels.push_back(reinterpret_cast<const void*>(logistic_tc_kernel));
+    for (bool mamba : {false, true})
+        for (int rows : {32, 64, 128}) {
+            const ChunkScanKernels f = chunk_scan_kernels(mamba, rows);
+            kernels.push_back(reinterpret_cast<const void*>(f.local)), kernels.push_back(reinterpret_cast<const void*>(f.scan));
+        }
     for (int rows : {32, 64, 128, 256}) {
         kernels.push_back(reinterpret_cast<const void*>(retention_kernels(rows, 64).state));
         for (int cols : {64, 128, 256}) kernels.push_back(reinterpret_cast<const void*>(retention_kernels(rows, cols).out));
@@ -635,7 +637,7 @@ inline int layered_chunk_scan(quintrit_b200_decoder* d, const MixerSpec& l, cons
     cudaStream_t s = d->stream;
     const bool mamba = l.kind == MixerKind::kMamba2;
     ChunkWork w;
-    chunk_work(d->lay->work, mamba, l.heads, l.vdim, a.n, l.groups, a.tokens, &w);
+    chunk_work(d->lay->work, mamba, l.heads, l.vdim, a.n, l.groups, a.tokens, d->lay->model->sm_count, &w);
     const int chunks = chunk_count(a.tokens), rows = w.rows;
     if (mamba) {
         const dim3 cgrid((l.heads * w.v_pad + 2 * l.groups * rows + 127) / 128, chunks);
@@ -649,16 +651,17 @@ inline int layered_chunk_scan(quintrit_b200_decoder* d, const MixerSpec& l, cons
         rows == 32 ? prep(hgrn_prep_kernel<32>) : rows == 64 ? prep(hgrn_prep_kernel<64>) : prep(hgrn_prep_kernel<128>);
         QTB_LAUNCH_CHECK();
     }
-    const dim3 grid(l.heads, w.v_pad / kChunkV);
-    auto go = [&](auto kernel, size_t smem) { kernel<<<grid, 128, smem, s>>>(a, w); };
+    const ChunkScanKernels f = chunk_scan_kernels(mamba, rows);
+    if (w.segments > 1) {
+        f.local<<<dim3(l.heads, w.v_pad / kChunkV, w.segments - 1), 128, f.local_smem, s>>>(a, w);
+        QTB_LAUNCH_CHECK();
+        chunk_carry_kernel<<<dim3((l.vdim * rows + 511) / 512, l.heads), 128, 0, s>>>(a, w);
+        QTB_LAUNCH_CHECK();
+    }
+    f.scan<<<dim3(l.heads, w.v_pad / kChunkV, w.segments), 128, f.smem, s>>>(a, w);
     if (mamba) {
-        const size_t smem = chunk_scan_smem<kScanMamba2>(rows);
-        rows == 32 ? go(chunk_scan_kernel<kScanMamba2, 32>, smem) : rows == 64 ? go(chunk_scan_kernel<kScanMamba2, 64>, smem) : go(chunk_scan_kernel<kScanMamba2, 128>, smem);
         QTB_LAUNCH_CHECK();
         conv_tail_kernel<<<(l.conv_dim() + 255) / 256, 256, 0, s>>>(a);
-    } else {
-        const size_t smem = chunk_scan_smem<kScanHgrn2>(rows);
-        rows == 32 ? go(chunk_scan_kernel<kScanHgrn2, 32>, smem) : rows == 64 ? go(chunk_scan_kernel<kScanHgrn2, 64>, smem) : go(chunk_scan_kernel<kScanHgrn2, 128>, smem);
     }
     QTB_LAUNCH_CHECK();
     return QUINTRIT_OK;
