@@ -7,7 +7,9 @@
 // turn; two sets of accumulators let the ending of a tile overlap the products of the next. Tiles run over the tokens first, so the blocks
 // that are at work together share weight rows.
 //
-// The dual form makes two products of one tile, W_o y and W_down m, in two accumulators and ends with both gates and the residual sum.
+// The dual form makes two products of one tile, W_o y and W_down m, in two accumulators and ends with both gates and the residual sum. Its rows are
+// only the model's width, so its tiles are few and long. 2048 tokens, 2048 rows, K = 4096 + 5632: 256 tiles of 128 tokens are two waves of which the
+// second is half empty, 110 us; 128 tiles of 256 tokens, with one set of accumulators, 75 us.
 // The grouped form multiplies runs of consecutive activation rows, each with its own range of weight rows (the experts of a mixture); which
 // runs there are is read from device memory.
 // Every wait is bounded, as in gemm_tc.cuh, whose mbarrier, descriptor and status conventions are used here.
@@ -153,7 +155,8 @@ __global__ void __launch_bounds__(kDenseThreads, 1) dense_gemm_tc_kernel(const _
     extern __shared__ unsigned char dense_smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(dense_smem_raw) + 1023) & ~uintptr_t(1023));
     constexpr int S = dense_stages(N), kStage = dense_stage_bytes(N), kAcc = DUAL ? 2 * N : N;  // kAcc: tensor-memory columns of a tile
-    static_assert(2 * kAcc <= 512, "two sets of accumulators fit tensor memory");
+    constexpr int kSets = 2 * kAcc <= 512 ? 2 : 1;  // sets of accumulators in tensor memory: with one, a block's next tile waits for the ending
+    static_assert(kSets * kAcc <= 512);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S * kStage);
     const uint32_t bar0 = smem_u32(bars), tiles0 = smem_u32(smem);
     auto loaded = [&](int s) { return bar0 + 8u * s; };
@@ -237,8 +240,8 @@ __global__ void __launch_bounds__(kDenseThreads, 1) dense_gemm_tc_kernel(const _
                 int prob, row0, token0;
                 locate(item, &prob, &row0, &token0);
                 const int steps0 = a.k_steps[prob], steps = DUAL ? steps0 + a.k_steps[1] : steps0;
-                const int set = j & 1;
-                if (!(okay = mbar_wait(acc_empty(set), ((j >> 1) & 1) ^ 1, abort_flag, a.spin_limit))) break;
+                const int set = j % kSets;
+                if (!(okay = mbar_wait(acc_empty(set), ((j / kSets) & 1) ^ 1, abort_flag, a.spin_limit))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 for (int k = 0; k < steps; ++k) {
                     if (!(okay = mbar_wait(loaded(s), ph, abort_flag, a.spin_limit))) break;
@@ -262,9 +265,9 @@ __global__ void __launch_bounds__(kDenseThreads, 1) dense_gemm_tc_kernel(const _
         for (int item = blockIdx.x; item < items; item += gridDim.x, ++j) {
             int prob, row0, token0;
             locate(item, &prob, &row0, &token0);
-            const int set = j & 1;
+            const int set = j % kSets;
             bool okay = true;
-            if (lane == 0) okay = mbar_wait(acc_full(set), (j >> 1) & 1, abort_flag, a.spin_limit) && *abort_flag == 0;
+            if (lane == 0) okay = mbar_wait(acc_full(set), (j / kSets) & 1, abort_flag, a.spin_limit) && *abort_flag == 0;
             okay = __shfl_sync(0xffffffffu, okay ? 1 : 0, 0) != 0;
             if (!okay) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -333,6 +336,13 @@ __global__ void __launch_bounds__(kDenseThreads, 1) dense_gemm_tc_kernel(const _
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
     }
+}
+
+// Tokens of a tile of the dual form and of the plain one: the fewer waves, a 256-token tile counted as 1.25 (long K: 0.36 against 0.45 us a 64-column
+// slice, weights are read for twice the tokens) or 1.6 (short K: mostly ending) of a 128-token one.
+inline int dense_waves(int tokens, int n, int row_tiles, int sm_count) { return ((tokens + n - 1) / n * row_tiles + sm_count - 1) / sm_count; }
+inline int dense_tile(int tokens, int row_tiles, int sm_count, double wide) {
+    return tokens > kDenseBox && wide * dense_waves(tokens, 256, row_tiles, sm_count) <= dense_waves(tokens, 128, row_tiles, sm_count) ? 256 : 128;
 }
 
 // ---- 32-bit products ------------------------------------------------------------------------------------------------------------------

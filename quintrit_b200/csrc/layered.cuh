@@ -535,7 +535,7 @@ inline int layered_decoder_setup(quintrit_b200_decoder* d, const std::shared_ptr
                              reinterpret_cast<const void*>(gated_scan_kernel<kScanRetention>),
                              reinterpret_cast<const void*>(pooled_attention_kernel<bf16, true>), reinterpret_cast<const void*>(pooled_attention_kernel<bf16, false>),
                              reinterpret_cast<const void*>(pooled_attention_kernel<float, true>), reinterpret_cast<const void*>(pooled_attention_kernel<float, false>),
-                             reinterpret_cast<const void*>(dense_gemm_tc_kernel<128, kDenseDual>), reinterpret_cast<const void*>(dense_gemm_tc_kernel<128, kDensePlain>),
+                             reinterpret_cast<const void*>(dense_gemm_tc_kernel<128, kDenseDual>), reinterpret_cast<const void*>(dense_gemm_tc_kernel<256, kDenseDual>), reinterpret_cast<const void*>(dense_gemm_tc_kernel<128, kDensePlain>),
                              reinterpret_cast<const void*>(dense_gemm_tc_kernel<256, kDensePlain>), reinterpret_cast<const void*>(dense_gemm_tc_kernel<128, kDenseGrouped>),
                              reinterpret_cast<const void*>(dense_gemm_tc_kernel<256, kDenseGrouped>),
                              reinterpret_cast<const void*>(pooled_attention_mma_kernel<32>), reinterpret_cast<const void*>(pooled_attention_mma_kernel<64>),
@@ -788,10 +788,10 @@ int layered_gemm(quintrit_b200_decoder* d, int n, const LayeredMatrix* const (&w
     for (int i = 0; i < n_stack; ++i) a.stack[i] = st[i], a.k_steps[i] = w[i]->pitch / kDenseK, a.row_tiles[i] = w[i]->rows_pad / kDenseM, tiles += a.row_tiles[i];
     const int j = n_stack > 1 ? 1 : 0;
     if constexpr (sizeof(T) == 2)
-        if (n > kDenseBox)
+        if (dense_tile(n, tiles, d->sm_count, 1.6) == 256)
             dense_gemm_tc_kernel<256, kDensePlain><<<std::min(d->sm_count, (n + 255) / 256 * tiles), kDenseThreads, dense_smem(256), d->stream>>>(w[0]->map, *hmap[0], w[j]->map, *hmap[j], a);
         else
-            dense_gemm_tc_kernel<128, kDensePlain><<<std::min(d->sm_count, tiles), kDenseThreads, dense_smem(128), d->stream>>>(w[0]->map, *hmap[0], w[j]->map, *hmap[j], a);
+            dense_gemm_tc_kernel<128, kDensePlain><<<std::min(d->sm_count, (n + 127) / 128 * tiles), kDenseThreads, dense_smem(128), d->stream>>>(w[0]->map, *hmap[0], w[j]->map, *hmap[j], a);
     else
         dense_gemm_f32_kernel<kDensePlain><<<dim3((n + kF32Tile - 1) / kF32Tile, tiles * (kDenseM / kF32Tile)), 256, 0, d->stream>>>(
             static_cast<const float*>(w[0]->w), static_cast<const float*>(h[0]), w[0]->pitch, static_cast<const float*>(w[j]->w), static_cast<const float*>(h[j]), w[j]->pitch, a);
@@ -808,11 +808,14 @@ int layered_add(quintrit_b200_decoder* d, int n, const LayeredMatrix* o, const C
     a.k_steps[0] = o->pitch / kDenseK, a.k_steps[1] = down != nullptr ? down->pitch / kDenseK : 0, a.row_tiles[0] = o->rows_pad / kDenseM;
     a.width = d->lay->model->spec.width;
     if (down == nullptr) down = o, map_down = map_o, act_down = act_o;
-    if constexpr (sizeof(T) == 2)
-        dense_gemm_tc_kernel<128, kDenseDual><<<std::min(d->sm_count, (n + 127) / 128 * a.row_tiles[0]), kDenseThreads, dense_smem(128), d->stream>>>(o->map, *map_o, down->map, *map_down, a);
-    else
+    if constexpr (sizeof(T) == 2) {
+        const int tile = dense_tile(n, a.row_tiles[0], d->sm_count, 1.25);
+        auto go = [&](auto kernel) { kernel<<<std::min(d->sm_count, (n + tile - 1) / tile * a.row_tiles[0]), kDenseThreads, dense_smem(tile), d->stream>>>(o->map, *map_o, down->map, *map_down, a); };
+        tile == 256 ? go(dense_gemm_tc_kernel<256, kDenseDual>) : go(dense_gemm_tc_kernel<128, kDenseDual>);
+    } else {
         dense_gemm_f32_kernel<kDenseDual><<<dim3((n + kF32Tile - 1) / kF32Tile, a.row_tiles[0] * (kDenseM / kF32Tile)), 256, 0, d->stream>>>(
             static_cast<const float*>(o->w), static_cast<const float*>(act_o), o->pitch, static_cast<const float*>(down->w), static_cast<const float*>(act_down), down->pitch, a);
+    }
     QTB_LAUNCH_CHECK();
     return QUINTRIT_OK;
 }
