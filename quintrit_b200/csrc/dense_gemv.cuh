@@ -478,14 +478,47 @@ __global__ void __launch_bounds__(kProjectThreads, 4) out_project_kernel(const _
 }
 
 // ---- batched counterparts of the steps around the projections ------------------------------------------------------------------------------
-// x = embed[token] * scale + pos[position] (pos may be nullptr)
+// Four consecutive elements of a vector (e a multiple of 4, rows 16-byte aligned).
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const bf16* p) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+}
+__device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store4(bf16* p, float4 v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+__device__ __forceinline__ float4 norm_value4(const NormParams& n, float4 x, float inv, int i) {
+    const float4 w = load4(n.w + i);
+    if (n.b == nullptr) return make_float4(x.x * inv * w.x, x.y * inv * w.y, x.z * inv * w.z, x.w * inv * w.w);
+    const float4 b = load4(n.b + i);
+    return make_float4(tanhf(n.alpha * x.x) * w.x + b.x, tanhf(n.alpha * x.y) * w.y + b.y, tanhf(n.alpha * x.z) * w.z + b.z, tanhf(n.alpha * x.w) * w.w + b.w);
+}
+
+// x = embed[token] * scale + pos[position] (pos may be nullptr); a thread takes four elements where the width is a multiple of four.
 template <typename T>
 __global__ void embed_scaled_kernel(const T* embed, int pitch, const T* pos_table, const uint32_t* tokens, const uint32_t* pos, SeqIndex seq, float scale, int width, float* x) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, t = blockIdx.y;
-    if (i >= width) return;
-    float v = from_storage(embed[size_t(tokens[t]) * pitch + i]) * scale;
-    if (pos_table != nullptr) v += from_storage(pos_table[size_t(seq_position(seq, pos, t)) * width + i]);
-    x[size_t(t) * width + i] = v;
+    const int n = blockIdx.x * blockDim.x + threadIdx.x, t = blockIdx.y;
+    const T* row = embed + size_t(tokens[t]) * pitch;
+    const T* at = pos_table != nullptr ? pos_table + size_t(seq_position(seq, pos, t)) * width : nullptr;
+    if (width % 4 == 0) {
+        const int i = n * 4;
+        if (i >= width) return;
+        float4 v = load4(row + i);
+        v.x *= scale, v.y *= scale, v.z *= scale, v.w *= scale;
+        if (at != nullptr) {
+            const float4 p = load4(at + i);
+            v.x += p.x, v.y += p.y, v.z += p.z, v.w += p.w;
+        }
+        store4(x + size_t(t) * width + i, v);
+        return;
+    }
+    for (int i = n; i < width; i += gridDim.x * blockDim.x) {
+        float v = from_storage(row[i]) * scale;
+        if (at != nullptr) v += from_storage(at[i]);
+        x[size_t(t) * width + i] = v;
+    }
 }
 
 // h_s = norm s of x, in the storage type; rows (optional) picks tokens
@@ -504,6 +537,41 @@ __global__ void __launch_bounds__(256) norm_rows_kernel(const float* x, int widt
         h0[size_t(t) * pitch + i] = to_storage<T>(norm_value(n0, xr[i], inv, i));
         if (h1 != nullptr) h1[size_t(t) * pitch + i] = to_storage<T>(norm_value(n1, xr[i], inv, i));
     }
+}
+
+// The same where the width is a multiple of four and at most 1024 TURNS: a thread keeps its elements in registers between the sum and the results, all
+// loads in flight, four elements to a store (2048 tokens of 2048, two norms: 22 -> 9.4 us, 32 MB).
+template <typename T, int TURNS>
+__global__ void __launch_bounds__(256) norm_rows4_kernel(const float* __restrict__ x, int width, float eps, NormParams n0, T* __restrict__ h0, NormParams n1, T* __restrict__ h1, int pitch,
+                                                         const uint32_t* __restrict__ rows) {
+    __shared__ float red[8];
+    const int t = blockIdx.x;
+    const float* xr = x + size_t(rows != nullptr ? rows[t] : t) * width;
+    float4 v[TURNS];
+    float ss = 0.0f, inv = 1.0f;
+#pragma unroll
+    for (int k = 0; k < TURNS; ++k) {
+        const int i = (threadIdx.x + 256 * k) * 4;
+        v[k] = i < width ? load4(xr + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
+    }
+    if (n0.b == nullptr) inv = 1.0f / sqrtf(block_sum(ss, red) / static_cast<float>(width) + eps);
+#pragma unroll
+    for (int k = 0; k < TURNS; ++k) {
+        const int i = (threadIdx.x + 256 * k) * 4;
+        if (i >= width) continue;
+        store4(h0 + size_t(t) * pitch + i, norm_value4(n0, v[k], inv, i));
+        if (h1 != nullptr) store4(h1 + size_t(t) * pitch + i, norm_value4(n1, v[k], inv, i));
+    }
+}
+template <typename T>
+inline void launch_norm_rows(int tokens, cudaStream_t s, const float* x, int width, float eps, const NormParams& n0, T* h0, const NormParams& n1, T* h1, int pitch, const uint32_t* rows) {
+    const auto bits = [](const NormParams& n) { return reinterpret_cast<uintptr_t>(n.w) | reinterpret_cast<uintptr_t>(n.b); };
+    auto go = [&](auto kernel) { kernel<<<tokens, 256, 0, s>>>(x, width, eps, n0, h0, n1, h1, pitch, rows); };
+    if (width % 4 != 0 || width > 4096 || (reinterpret_cast<uintptr_t>(x) | bits(n0) | bits(n1)) % 16 != 0) go(norm_rows_kernel<T>);
+    else if (width <= 1024) go(norm_rows4_kernel<T, 1>);
+    else if (width <= 2048) go(norm_rows4_kernel<T, 2>);
+    else go(norm_rows4_kernel<T, 4>);
 }
 
 // x = norm(embed[token]), also written to `first` (the first of the vectors that depth averages run over; may be nullptr), and h = next(x)
@@ -655,6 +723,56 @@ __global__ void __launch_bounds__(256) finish_rows_kernel(const float* y, const 
     if (parts > 0 && w != nullptr) parts_norm<float, false>(act_smem, inner, inner, parts, eps, w, w_len, nullptr, red);
     else if (parts > 0) parts_norm<float, true>(act_smem, inner, inner, parts, eps, nullptr, 1, gate_after != nullptr ? gate_after + size_t(t) * gate_ld : nullptr, red);
     for (int i = threadIdx.x; i < inner; i += blockDim.x) out[size_t(t) * pitch + i] = to_storage<T>(act_smem[i]);
+}
+
+// The same for whole parts of four-element multiples, at most 128 TURNS long: a warp takes a part and keeps it in registers. Without a norm (parts = 0)
+// pieces of 128 elements are converted. 2048 tokens: 4096 in 8 parts with mamba2's gate 30 -> 21 us (80 MB), 2048 in 16 parts 20 -> 7.9 us.
+template <typename T, int TURNS>
+__global__ void __launch_bounds__(256) finish_rows4_kernel(const float* __restrict__ y, const float* __restrict__ gate, int gate_ld, int inner, int parts, float eps, const float* __restrict__ w, int w_len,
+                                                           T* __restrict__ out, int pitch) {
+    const int t = blockIdx.x, lane = threadIdx.x & 31, len = parts > 0 ? inner / parts : 128, pieces = (inner + len - 1) / len;
+    for (int p = threadIdx.x >> 5; p < pieces; p += 8) {
+        const int begin = p * len, end = min(begin + len, inner);
+        float4 v[TURNS], g[TURNS];
+#pragma unroll
+        for (int k = 0; k < TURNS; ++k) {
+            const int i = begin + (lane + 32 * k) * 4;
+            v[k] = i < end ? load4(y + size_t(t) * inner + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (gate != nullptr) g[k] = i < end ? load4(gate + size_t(t) * gate_ld + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        float ss = 0.0f;
+#pragma unroll
+        for (int k = 0; k < TURNS; ++k) {
+            if (gate != nullptr) v[k].x *= silu_f(g[k].x), v[k].y *= silu_f(g[k].y), v[k].z *= silu_f(g[k].z), v[k].w *= silu_f(g[k].w);
+            ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
+        }
+        const float inv = parts > 0 ? 1.0f / sqrtf(warp_sum(ss) / static_cast<float>(len) + eps) : 1.0f;
+#pragma unroll
+        for (int k = 0; k < TURNS; ++k) {
+            const int i = begin + (lane + 32 * k) * 4;
+            if (i >= end) continue;
+            float4 r = make_float4(v[k].x * inv, v[k].y * inv, v[k].z * inv, v[k].w * inv);
+            if (parts > 0 && w != nullptr) {
+                const float4 f = load4(w + i % w_len);
+                r.x *= f.x, r.y *= f.y, r.z *= f.z, r.w *= f.w;
+            }
+            store4(out + size_t(t) * pitch + i, r);
+        }
+    }
+}
+template <typename T>
+inline void launch_finish_rows(int tokens, cudaStream_t s, const float* y, const float* gate, const float* gate_after, int gate_ld, int inner, int parts, float eps, const float* w, int w_len, T* out,
+                               int pitch) {
+    const int len = parts > 0 ? inner / parts : 128;
+    const bool aligned = (reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(w)) % 16 == 0;
+    if (gate_after != nullptr || !aligned || inner % 4 != 0 || len % 4 != 0 || len > 512 || (gate != nullptr && gate_ld % 4 != 0) || (w != nullptr && w_len % 4 != 0)) {
+        finish_rows_kernel<T><<<tokens, 256, size_t(inner) * sizeof(float), s>>>(y, gate, gate_after, gate_ld, inner, parts, eps, w, w_len, out, pitch);
+        return;
+    }
+    auto go = [&](auto kernel) { kernel<<<tokens, 256, 0, s>>>(y, gate, gate_ld, inner, parts, eps, w, w_len, out, pitch); };
+    if (len <= 128) go(finish_rows4_kernel<T, 1>);
+    else if (len <= 256) go(finish_rows4_kernel<T, 2>);
+    else go(finish_rows4_kernel<T, 4>);
 }
 
 }  // namespace qtb

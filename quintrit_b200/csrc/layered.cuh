@@ -855,15 +855,15 @@ int layered_parallel_layer(quintrit_b200_decoder* d, size_t li, int n, const Lay
         QTB_LAUNCH_CHECK();
         return QUINTRIT_OK;
     }
-    norm_rows_kernel<T><<<n, 256, 0, s>>>(y.x, W, m.spec.eps, l.norm1, static_cast<T*>(y.h1), l.norm2, n_stack > 1 ? static_cast<T*>(y.h2) : nullptr, wp, nullptr);
+    launch_norm_rows<T>(n, s, y.x, W, m.spec.eps, l.norm1, static_cast<T*>(y.h1), l.norm2, n_stack > 1 ? static_cast<T*>(y.h2) : nullptr, wp, nullptr);
     QTB_LAUNCH_CHECK();
     const LayeredMatrix* const ws[2] = {&l.in1, &l.in2};
     const CUtensorMap* const hm[2] = {&y.map_h1, &y.map_h2};
     const void* const hs[2] = {y.h1, y.h2};
     if ((rc = layered_gemm<T>(d, n, ws, hm, hs, st, n_stack)) != QUINTRIT_OK || (rc = layered_mixer<T>(d, li, 0, n, tg, &ready)) != QUINTRIT_OK) return rc;
     const float* gate = sizeof(T) == 2 && x.spec.kind == MixerKind::kMamba2 && !tg.step() && n > kChunkT / 2 && chunk_scan_rows(x.spec.state) != 0 ? y.p1 : nullptr;  // silu(z)
-    finish_rows_kernel<T><<<n, 256, size_t(x.spec.inner()) * sizeof(float), s>>>(y.y[0], gate, nullptr, l.spec.in_rows(), x.spec.inner(), parts, m.spec.eps, x.mix_norm, norm_len,
-                                                                                 static_cast<T*>(y.y_t[0]), x.o.pitch);
+    launch_finish_rows<T>(n, s, y.y[0], gate, nullptr, l.spec.in_rows(), x.spec.inner(), parts, m.spec.eps, x.mix_norm, norm_len, static_cast<T*>(y.y_t[0]),
+                          x.o.pitch);
     QTB_LAUNCH_CHECK();
     DenseGemmArgs a{};
     a.x = y.x;
@@ -996,7 +996,7 @@ int layered_sequential_layer(quintrit_b200_decoder* d, size_t li, int n, const L
     DenseStack st[2] = {};
     layered_in_stacks(y, l, st);
     if (!*normed) {
-        norm_rows_kernel<T><<<n, 256, 0, s>>>(y.x, W, m.spec.eps, l.norm1, static_cast<T*>(y.h1), NormParams{}, nullptr, wp, nullptr);
+        launch_norm_rows<T>(n, s, y.x, W, m.spec.eps, l.norm1, static_cast<T*>(y.h1), NormParams{}, nullptr, wp, nullptr);
         QTB_LAUNCH_CHECK();
     }
     *normed = true;
@@ -1012,8 +1012,8 @@ int layered_sequential_layer(quintrit_b200_decoder* d, size_t li, int n, const L
         if ((rc = layered_mixer<T>(d, li, k, n, tg, &ready)) != QUINTRIT_OK) return rc;
         if (ready) continue;
         const float* gate = x.spec.kind == MixerKind::kRetention ? y.p1 + x.col + x.spec.gate_col() : nullptr;
-        finish_rows_kernel<T><<<n, 256, size_t(x.spec.inner()) * sizeof(float), s>>>(y.y[k], nullptr, gate, l.spec.in_rows(), x.spec.inner(), layered_norm_parts(x.spec), m.spec.eps, nullptr, 1,
-                                                                                     static_cast<T*>(y.y_t[k]), x.o.pitch);
+        launch_finish_rows<T>(n, s, y.y[k], nullptr, gate, l.spec.in_rows(), x.spec.inner(), layered_norm_parts(x.spec), m.spec.eps, nullptr, 1, static_cast<T*>(y.y_t[k]),
+                              x.o.pitch);
         QTB_LAUNCH_CHECK();
     }
     RowsArgs r{};
@@ -1066,7 +1066,7 @@ int layered_layers(quintrit_b200_decoder* d, const uint32_t* tokens, int n, cons
         embed_norm_kernel<T><<<n, 256, size_t(W) * sizeof(float), s>>>(static_cast<const T*>(m.embed.w), wp, tokens, W, m.spec.eps, m.embed_norm, y.x, y.past, m.layers[0].norm1,
                                                                       static_cast<T*>(n > 1 ? y.h1 : nullptr));
     else
-        embed_scaled_kernel<T><<<dim3((W + 255) / 256, n), 256, 0, s>>>(static_cast<const T*>(m.embed.w), wp, static_cast<const T*>(m.pos_table), tokens, tg.pos, tg.seq, m.spec.embed_scale, W, y.x);
+        embed_scaled_kernel<T><<<dim3((W + 1023) / 1024, n), 256, 0, s>>>(static_cast<const T*>(m.embed.w), wp, static_cast<const T*>(m.pos_table), tokens, tg.pos, tg.seq, m.spec.embed_scale, W, y.x);
     QTB_LAUNCH_CHECK();
     bool normed = m.embed_norm.w != nullptr;  // y.h1 holds the next layer's first norm
     for (size_t li = 0; li < m.layers.size(); ++li) {
@@ -1098,7 +1098,7 @@ template <typename T>
 int layered_head_rows(quintrit_b200_decoder* d, const uint32_t* rows, int first, int n, float* logits) {
     LayeredDecoder& y = *d->lay;
     const LayeredModel& m = *y.model;
-    norm_rows_kernel<T><<<n, 256, 0, d->stream>>>(y.x + size_t(first) * m.spec.width, m.spec.width, m.spec.eps, m.out_norm, static_cast<T*>(y.h_head), NormParams{}, nullptr, m.head.pitch, rows);
+    launch_norm_rows<T>(n, d->stream, y.x + size_t(first) * m.spec.width, m.spec.width, m.spec.eps, m.out_norm, static_cast<T*>(y.h_head), NormParams{}, nullptr, m.head.pitch, rows);
     QTB_LAUNCH_CHECK();
     DenseStack st[2] = {layered_stack(m.head), {}};
     st[0].n_seg = 1, st[0].seg[0] = DenseSeg{0, m.spec.vocab, kSegPlain, m.spec.vocab, logits, nullptr, nullptr};

@@ -313,3 +313,14 @@ def test_trace_replay(tmp_path):
     for step, want in ((0, wa[[24, 3]]), (2, wa[[25, 39]]), (3, wb[[0, 1]])):
         check(np.fromfile(tmp_path / f"{step}.f32", "<f4").reshape(-1, 71), want, "float32")
     assert not (tmp_path / "1.f32").exists()
+
+
+# Norms a token's row at a time, four elements to a thread: one, two and four turns of a block's threads, rows beyond them; output norms in parts of one, two
+# and four turns of a warp and beyond.
+@pytest.mark.parametrize("width,layers", [(1028, [M(5, 80, 16, groups=1, conv=2, norm_groups=2, ff=24)]), (2052, [M(4, 160, 16, groups=2, conv=2, norm_groups=2)]),
+                                          (4100, [M(3, 360, 16, groups=1, conv=2, norm_groups=2), H(2, 16, 36)]), (30, [H(3, 16, 22), M(3, 10, 16, groups=1, conv=2, norm_groups=3)])])
+def test_rows_of_many_lengths(tmp_path, width, layers):
+    config = mf.lasosun_config(layers, width, 41, 64, eps=3e-5)
+    model, w = build(tmp_path, config, width, "bfloat16")
+    ids = ids_for(7, 19, 41)
+    check(model.new_session().feed(ids, range(len(ids))), plain.lasosun(config, w, ids), "bfloat16")
