@@ -181,18 +181,31 @@ int gemv_kernel_for_device(int dev, GemvKernel* out) {
     return QUINTRIT_OK;
 }
 
+// dependent: the launch before this one in the stream is zero_kernel, which this one need not wait for until it adds.
 int launch_gemv(const GemvItem* d_items, int n_items, const int8_t* d_act, int32_t* d_out, unsigned int* d_counters, int sm_count,
-                cudaStream_t stream) {
+                cudaStream_t stream, bool dependent = false) {
     int dev = 0;
     QTB_CUDA(cudaGetDevice(&dev));
     GemvKernel k = nullptr;
     int rc = gemv_kernel_for_device(dev, &k);
     if (rc != QUINTRIT_OK) return rc;
     const int grid = std::max(1, std::min(n_items, sm_count * kCtasPerSm));
-    k<<<grid, kGemvThreads, kGemvSmemBytes, stream>>>(d_items, n_items, d_act, d_out, d_counters);
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization, attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3(grid), cfg.blockDim = dim3(kGemvThreads), cfg.dynamicSmemBytes = kGemvSmemBytes, cfg.stream = stream;
+    cfg.attrs = &attr, cfg.numAttrs = dependent ? 1 : 0;
+    ++g_launches;
+    QTB_CUDA(cudaLaunchKernelEx(&cfg, k, d_items, n_items, d_act, d_out, d_counters));
+    return QUINTRIT_OK;
+}
+
+// The same with the results cleared first, `out_count` of them (at least one).
+int launch_gemv_cleared(const GemvItem* d_items, int n_items, const int8_t* d_act, int32_t* d_out, size_t out_count, unsigned int* d_counters, int sm_count, cudaStream_t stream) {
+    zero_kernel<<<static_cast<unsigned>(std::min<size_t>((out_count + 1023) / 1024, static_cast<size_t>(sm_count))), 256, 0, stream>>>(d_out, out_count);
     ++g_launches;
     QTB_CUDA(cudaGetLastError());
-    return QUINTRIT_OK;
+    return launch_gemv(d_items, n_items, d_act, d_out, d_counters, sm_count, stream, true);
 }
 
 // After a synchronisation: did the kernel refuse to run because its table-base constant was wrong?
@@ -522,8 +535,7 @@ extern "C" int quintrit_b200_gemv_i32_device(const quintrit_b200_matrix_t* matri
         if (d_activations == nullptr || d_out == nullptr) return fail(QUINTRIT_ERR_NULL_POINTER, "a device pointer is NULL");
         DeviceGuard g(matrix->device);
         cudaStream_t s = static_cast<cudaStream_t>(stream);
-        QTB_CUDA(cudaMemsetAsync(d_out, 0, matrix->rows * sizeof(int32_t), s));
-        rc = launch_gemv(matrix->d_items, matrix->n_items, d_activations, d_out, matrix->d_counters, matrix->sm_count, s);
+        rc = launch_gemv_cleared(matrix->d_items, matrix->n_items, d_activations, d_out, matrix->rows, matrix->d_counters, matrix->sm_count, s);
         return rc == QUINTRIT_OK ? ok() : rc;
     });
 }
@@ -812,8 +824,7 @@ extern "C" int quintrit_b200_plan_launch(quintrit_b200_plan_t* plan, void* strea
         if (rc != QUINTRIT_OK) return rc;
         DeviceGuard g(plan->device);
         cudaStream_t s = static_cast<cudaStream_t>(stream);
-        QTB_CUDA(cudaMemsetAsync(plan->d_out, 0, plan->out_total * sizeof(int32_t), s));
-        rc = launch_gemv(plan->d_items, plan->n_items, plan->d_act, plan->d_out, plan->d_counters, plan->sm_count, s);
+        rc = launch_gemv_cleared(plan->d_items, plan->n_items, plan->d_act, plan->d_out, plan->out_total, plan->d_counters, plan->sm_count, s);
         return rc == QUINTRIT_OK ? ok() : rc;
     });
 }

@@ -24,7 +24,7 @@
 // Work decomposition: an item is (block pair, range of row tiles). A CTA builds the 64 KB table of the pair (256 byte
 // values x 2 blocks x 32 columns x int32), then its 8 warps stream the tiles; every lane adds its row's partial sum to
 // the output with one red.global.add (the K dimension is split over items, so the output is cleared beforehand).
-// The kernel is persistent: CTAs take items from a global counter until none is left, three CTAs per SM.
+// The kernel is persistent: after its first three items a CTA takes more from a global counter until none is left, three CTAs per SM.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -281,11 +281,12 @@ gemv_lut_kernel(const GemvItem* __restrict__ items, int n_items, const int8_t* _
         asm volatile("mov.b32 %0, %1;" : "=r"(creg[q]) : "r"(v));
     }
 
-    // Prologue: indices of the first three items, descriptors of the first two, activations of the first.
-    if (tid < 3) s_idx[tid] = static_cast<int>(atomicAdd(&counters[0], 1u));
-    __syncthreads();
+    // Prologue: the first three items are dealt out by block index, the others by the counter. (With all of them taken from the counter the blocks that
+    // came first took three items each before the others had one: a launch of two items a block ran three rounds on two thirds of the blocks. And a
+    // launch of less than one item a block need not wait for a counter at all.)
+    if (tid < 3) s_idx[tid] = static_cast<int>(blockIdx.x + tid * gridDim.x);
     if (tid < 8) {
-        const int k = tid >> 2, idx = s_idx[k];
+        const int k = tid >> 2, idx = static_cast<int>(blockIdx.x + k * gridDim.x);
         if (idx < n_items) reinterpret_cast<uint4*>(&s_items[k])[tid & 3] = reinterpret_cast<const uint4*>(items + idx)[tid & 3];
     }
     __syncthreads();
@@ -317,7 +318,7 @@ gemv_lut_kernel(const GemvItem* __restrict__ items, int n_items, const int8_t* _
         if (tag_a < 0) preload(ra, tag_a, i, warp, item, s_items, s_idx, n_items, warp, lane);
         // index of item i + 3 (kept in a register until the end of the iteration so that nothing waits on it here)
         unsigned int fetched = 0;
-        if (tid == 0) fetched = atomicAdd(&counters[0], 1u);
+        if (tid == 0) fetched = atomicAdd(&counters[0], 1u) + 3 * gridDim.x;
         // descriptor of item i + 2
         const int idx2 = s_idx[(i + 2) & 3];
         if (tid < 4 && idx2 < n_items) {
@@ -340,6 +341,7 @@ gemv_lut_kernel(const GemvItem* __restrict__ items, int n_items, const int8_t* _
             fill_table(tab, a, tid);
         }
         __syncthreads();
+        if (i == 0) asm volatile("griddepcontrol.wait;" ::: "memory");  // the results are cleared (zero_kernel, where this launch depends on it)
 
         int t = warp;
         while (tag_a == i) {
@@ -377,6 +379,18 @@ gemv_lut_kernel(const GemvItem* __restrict__ items, int n_items, const int8_t* _
             __threadfence();
         }
     }
+}
+
+// Clears the results before a launch that adds to them. The launch behind it may start at once (programmatic dependent launch): it brings its
+// weights and builds its first table meanwhile and waits before it adds.
+__global__ void __launch_bounds__(256) zero_kernel(int32_t* __restrict__ out, size_t n) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const size_t tid = blockIdx.x * size_t(256) + threadIdx.x, threads = gridDim.x * size_t(256);
+    const size_t lead = (16 - reinterpret_cast<uintptr_t>(out) % 16) % 16 / 4, head = lead < n ? lead : n, quads = (n - head) / 4;  // (the caller's pointer need not be aligned)
+    int4* q = reinterpret_cast<int4*>(out + head);
+    for (size_t i = tid; i < quads; i += threads) q[i] = make_int4(0, 0, 0, 0);
+    if (tid < head) out[tid] = 0;
+    if (head + quads * 4 + tid < n) out[head + quads * 4 + tid] = 0;
 }
 
 // Reports the shared-window address of dynamic shared memory for a kernel without static shared memory.
