@@ -25,6 +25,7 @@ namespace qtb {
 
 constexpr int kDenseM = 128, kDenseBox = 128, kDenseK = 64;  // kDenseBox: rows of an activation box; a tile's N is a multiple of it
 constexpr int kDenseEndWarps = 8;
+constexpr int kDenseRanks = 8;  // blocks that may share a tile (the dual form)
 constexpr int kDenseThreads = 64 + 32 * kDenseEndWarps;  // TMA warp, MMA warp, warps for the ending
 __host__ __device__ constexpr int dense_stages(int n) { return n > 128 ? 4 : 6; }
 __host__ __device__ constexpr int dense_stage_bytes(int n) { return (kDenseM + n) * kDenseK * 2; }
@@ -144,9 +145,22 @@ __device__ __forceinline__ void tmem_load16(uint32_t taddr, uint32_t (&v)[16]) {
           "=r"(v[14]), "=r"(v[15])
         : "r"(taddr));
 }
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 cluster_load4(uint32_t addr, int rank) {  // sixteen bytes at the same place in the shared memory of a block of the cluster
+    uint32_t there;
+    float4 v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(there));
+    return v;
+}
 }  // namespace dense_detail
 
-template <int N, int FORM>
+// SPLIT (dual form): the blocks of a cluster share a tile, each takes a range of the K slices of both products; they add their gated sums through
+// distributed shared memory, a block for a range of the tokens, in the order of the ranks. The grid is exactly the tiles times the cluster's size.
+template <int N, int FORM, bool SPLIT = false>
 __global__ void __launch_bounds__(kDenseThreads, 1) dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap w0, const __grid_constant__ CUtensorMap h0, const __grid_constant__ CUtensorMap w1,
                                                                          const __grid_constant__ CUtensorMap h1, const __grid_constant__ DenseGemmArgs a) {
     using namespace gemm_detail;
@@ -156,7 +170,8 @@ __global__ void __launch_bounds__(kDenseThreads, 1) dense_gemm_tc_kernel(const _
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(dense_smem_raw) + 1023) & ~uintptr_t(1023));
     constexpr int S = dense_stages(N), kStage = dense_stage_bytes(N), kAcc = DUAL ? 2 * N : N;  // kAcc: tensor-memory columns of a tile
     constexpr int kSets = 2 * kAcc <= 512 ? 2 : 1;  // sets of accumulators in tensor memory: with one, a block's next tile waits for the ending
-    static_assert(kSets * kAcc <= 512);
+    static_assert(kSets * kAcc <= 512 && (DUAL || !SPLIT));
+    static_assert(!SPLIT || size_t(N) * kDenseM * 4 <= size_t(S) * kStage, "the sums of a tile fit the ring's memory");
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S * kStage);
     const uint32_t bar0 = smem_u32(bars), tiles0 = smem_u32(smem);
     auto loaded = [&](int s) { return bar0 + 8u * s; };
@@ -168,6 +183,12 @@ __global__ void __launch_bounds__(kDenseThreads, 1) dense_gemm_tc_kernel(const _
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int token_tiles = (a.tokens + N - 1) / N;
+    int rank = 0, ranks = 1;
+    if constexpr (SPLIT) {
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+        asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+    }
+    const int item0 = blockIdx.x / ranks, item_step = gridDim.x / ranks;
     const int items = GROUPED ? *a.n_runs * a.row_tiles[0] : token_tiles * (a.row_tiles[0] + (!DUAL && a.n_prob > 1 ? a.row_tiles[1] : 0));
     // tile `item`: its problem, first row and first token
     auto locate = [&](int item, int* prob, int* row0, int* token0) {
@@ -208,11 +229,11 @@ __global__ void __launch_bounds__(kDenseThreads, 1) dense_gemm_tc_kernel(const _
             int it = 0, s = 0;
             uint32_t ph = 0;
             bool okay = true;
-            for (int item = blockIdx.x; item < items && okay; item += gridDim.x) {
+            for (int item = item0; item < items && okay; item += item_step) {
                 int prob, row0, token0;
                 locate(item, &prob, &row0, &token0);
                 const int steps0 = a.k_steps[prob], steps = DUAL ? steps0 + a.k_steps[1] : steps0;
-                for (int k = 0; k < steps; ++k, ++it) {
+                for (int k = steps * rank / ranks; k < steps * (rank + 1) / ranks; ++k, ++it) {
                     if (!(okay = mbar_wait(empty(s), ph ^ 1, abort_flag, a.spin_limit))) break;
                     const bool second = DUAL ? k >= steps0 : prob != 0;
                     const int x = (DUAL && second ? k - steps0 : k) * kDenseK;
@@ -236,20 +257,20 @@ __global__ void __launch_bounds__(kDenseThreads, 1) dense_gemm_tc_kernel(const _
             int s = 0, j = 0;
             uint32_t ph = 0;
             bool okay = true;
-            for (int item = blockIdx.x; item < items && okay; item += gridDim.x, ++j) {
+            for (int item = item0; item < items && okay; item += item_step, ++j) {
                 int prob, row0, token0;
                 locate(item, &prob, &row0, &token0);
                 const int steps0 = a.k_steps[prob], steps = DUAL ? steps0 + a.k_steps[1] : steps0;
-                const int set = j % kSets;
+                const int set = j % kSets, k_begin = steps * rank / ranks;
                 if (!(okay = mbar_wait(acc_empty(set), ((j / kSets) & 1) ^ 1, abort_flag, a.spin_limit))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int k = 0; k < steps; ++k) {
+                for (int k = k_begin; k < steps * (rank + 1) / ranks; ++k) {
                     if (!(okay = mbar_wait(loaded(s), ph, abort_flag, a.spin_limit))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t at = tiles0 + s * kStage;
                     const uint64_t da = smem_desc(at, 16, 1024, 2), db = smem_desc(at + kDenseM * kDenseK * 2, 16, 1024, 2);  // 128-byte swizzle, 8-row groups 1024 bytes apart
                     const uint32_t acc = tmem_base + set * kAcc + (DUAL && k >= steps0 ? N : 0);
-                    const bool first = k == 0 || (DUAL && k == steps0);
+                    const bool first = k == k_begin || (DUAL && k == steps0);
 #pragma unroll
                     for (int q = 0; q < kDenseK / 16; ++q) mma_bf16(acc, da + 2 * q, db + 2 * q, idesc, first && q == 0 ? 0u : 1u);
                     mma_commit(empty(s));
@@ -262,7 +283,7 @@ __global__ void __launch_bounds__(kDenseThreads, 1) dense_gemm_tc_kernel(const _
         // the ending: a warp reads the 32 lanes of tensor memory that its index modulo 4 selects; the two warps of a quarter take 16-column pieces in turn
         const int r = (warp & 3) * 32 + lane, turn = (warp - 2) >> 2;
         int j = 0;
-        for (int item = blockIdx.x; item < items; item += gridDim.x, ++j) {
+        for (int item = item0; item < items; item += item_step, ++j) {
             int prob, row0, token0;
             locate(item, &prob, &row0, &token0);
             const int set = j % kSets;
@@ -273,7 +294,39 @@ __global__ void __launch_bounds__(kDenseThreads, 1) dense_gemm_tc_kernel(const _
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t acc = tmem_base + (uint32_t((warp & 3) * 32) << 16) + set * kAcc;
             const int n_here = GROUPED ? a.runs[item / a.row_tiles[0]].tokens : min(N, a.tokens - token0);
-            if constexpr (DUAL) {
+            if constexpr (SPLIT) {
+                float* part = reinterpret_cast<float*>(smem);  // [token][row]; the products that read the ring are done
+                const int row = row0 + r, total = a.k_steps[0] + a.k_steps[1];
+                const bool has1 = total * rank / ranks < a.k_steps[0], has2 = total * (rank + 1) / ranks > a.k_steps[0];
+                for (int c0 = turn * 16; c0 < n_here; c0 += 32) {
+                    // the gates of sixteen tokens in flight: no condition stands before a load, what lies beyond the last token or row reads their gate
+                    const size_t at = size_t(token0 + c0) * a.width + min(row, a.width - 1);
+                    const int last = min(15, n_here - c0 - 1);
+                    float g1[16], g2[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) g1[i] = g2[i] = 1.0f;
+                    if (has1 && a.gate1 != nullptr) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) g1[i] = a.gate1[at + min(i, last) * size_t(a.width)];
+                    } else if (has1 && a.token_gate != nullptr) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) g1[i] = a.token_gate[token0 + c0 + min(i, last)];
+                    }
+                    if (has2 && a.gate2 != nullptr) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) g2[i] = a.gate2[at + min(i, last) * size_t(a.width)];
+                    }
+                    uint32_t v1[16], v2[16];
+                    if (has1) tmem_load16(acc + c0, v1);
+                    if (has2) tmem_load16(acc + N + c0, v2);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        const float add = has1 ? __uint_as_float(v1[i]) * g1[i] : 0.0f;
+                        part[(c0 + i) * kDenseM + r] = has2 ? fmaf(__uint_as_float(v2[i]), g2[i], add) : add;
+                    }
+                }
+            } else if constexpr (DUAL) {
                 const int row = row0 + r;
                 const bool has2 = a.k_steps[1] > 0;
                 for (int c0 = turn * 16; c0 < n_here; c0 += 32) {
@@ -329,6 +382,34 @@ __global__ void __launch_bounds__(kDenseThreads, 1) dense_gemm_tc_kernel(const _
             if (lane == 0) mbar_arrive(acc_empty(set));
         }
     }
+    if constexpr (SPLIT) {  // every thread of the cluster comes here, after a failed wait too
+        __syncwarp();
+        cluster_sync();
+        int prob, row0, token0;
+        locate(item0, &prob, &row0, &token0);
+        const int per = N / ranks, end = min((rank + 1) * per, a.tokens - token0), row = row0 + lane * 4;
+        for (int t = rank * per + warp; t < end; t += kDenseThreads / 32) {  // a warp takes a token: four rows a lane, all ranks' sums requested together
+            float4 v[kDenseRanks];
+#pragma unroll
+            for (int q = 0; q < kDenseRanks; ++q) v[q] = q < ranks ? cluster_load4(tiles0 + t * (kDenseM * 4) + lane * 16, q) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            float4 sum = v[0];
+#pragma unroll
+            for (int q = 1; q < kDenseRanks; ++q) sum.x += v[q].x, sum.y += v[q].y, sum.z += v[q].z, sum.w += v[q].w;
+            float* x = a.x + size_t(token0 + t) * a.width + row;
+            const float add[4] = {sum.x, sum.y, sum.z, sum.w};
+            if (a.width % 4 == 0) {
+                if (row < a.width) {
+                    const float4 old = *reinterpret_cast<const float4*>(x);
+                    *reinterpret_cast<float4*>(x) = make_float4(old.x + add[0], old.y + add[1], old.z + add[2], old.w + add[3]);
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (row + e < a.width) x[e] += add[e];
+            }
+        }
+        cluster_sync();  // no block leaves while its sums may still be read
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (tid == 0 && *abort_flag) atomicExch(a.status, kGemmStatusTimeout);
@@ -343,6 +424,17 @@ __global__ void __launch_bounds__(kDenseThreads, 1) dense_gemm_tc_kernel(const _
 inline int dense_waves(int tokens, int n, int row_tiles, int sm_count) { return ((tokens + n - 1) / n * row_tiles + sm_count - 1) / sm_count; }
 inline int dense_tile(int tokens, int row_tiles, int sm_count, double wide) {
     return tokens > kDenseBox && wide * dense_waves(tokens, 256, row_tiles, sm_count) <= dense_waves(tokens, 128, row_tiles, sm_count) ? 256 : 128;
+}
+
+// Blocks that share a tile of the dual form where its tiles of 128 tokens leave more than half of the machine idle: as many as fit in one wave (clusters do
+// not quite fill it) with at least kRankSlices 64-column slices each, fewer of which the exchange would not pay
+// for. By ncu: 300 tokens of width 1024, K = 2048 + 2816, 24 tiles on four blocks each 35 -> 19 us.
+constexpr int kRankSlices = 8;
+inline int dense_ranks(int tokens, int row_tiles, int slices, int sm_count) {
+    const int tiles = (tokens + 127) / 128 * row_tiles;
+    int ranks = kDenseRanks;
+    while (ranks > 1 && (ranks * tiles > sm_count * 9 / 10 || slices / ranks < kRankSlices)) ranks /= 2;
+    return ranks;
 }
 
 // ---- 32-bit products ------------------------------------------------------------------------------------------------------------------

@@ -535,7 +535,8 @@ inline int layered_decoder_setup(quintrit_b200_decoder* d, const std::shared_ptr
                              reinterpret_cast<const void*>(gated_scan_kernel<kScanRetention>),
                              reinterpret_cast<const void*>(pooled_attention_kernel<bf16, true>), reinterpret_cast<const void*>(pooled_attention_kernel<bf16, false>),
                              reinterpret_cast<const void*>(pooled_attention_kernel<float, true>), reinterpret_cast<const void*>(pooled_attention_kernel<float, false>),
-                             reinterpret_cast<const void*>(dense_gemm_tc_kernel<128, kDenseDual>), reinterpret_cast<const void*>(dense_gemm_tc_kernel<256, kDenseDual>), reinterpret_cast<const void*>(dense_gemm_tc_kernel<128, kDensePlain>),
+                             reinterpret_cast<const void*>(dense_gemm_tc_kernel<128, kDenseDual>), reinterpret_cast<const void*>(dense_gemm_tc_kernel<256, kDenseDual>),
+                             reinterpret_cast<const void*>(dense_gemm_tc_kernel<128, kDenseDual, true>), reinterpret_cast<const void*>(dense_gemm_tc_kernel<128, kDensePlain>),
                              reinterpret_cast<const void*>(dense_gemm_tc_kernel<256, kDensePlain>), reinterpret_cast<const void*>(dense_gemm_tc_kernel<128, kDenseGrouped>),
                              reinterpret_cast<const void*>(dense_gemm_tc_kernel<256, kDenseGrouped>),
                              reinterpret_cast<const void*>(pooled_attention_mma_kernel<32>), reinterpret_cast<const void*>(pooled_attention_mma_kernel<64>),
@@ -809,6 +810,16 @@ int layered_add(quintrit_b200_decoder* d, int n, const LayeredMatrix* o, const C
     a.width = d->lay->model->spec.width;
     if (down == nullptr) down = o, map_down = map_o, act_down = act_o;
     if constexpr (sizeof(T) == 2) {
+        if (const int ranks = dense_ranks(n, a.row_tiles[0], a.k_steps[0] + a.k_steps[1], d->sm_count); ranks > 1) {
+            cudaLaunchConfig_t cfg{};
+            cudaLaunchAttribute attr{};
+            attr.id = cudaLaunchAttributeClusterDimension, attr.val.clusterDim.x = ranks, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+            cfg.gridDim = dim3((n + 127) / 128 * a.row_tiles[0] * ranks), cfg.blockDim = dim3(kDenseThreads), cfg.dynamicSmemBytes = dense_smem(128), cfg.stream = d->stream;
+            cfg.attrs = &attr, cfg.numAttrs = 1;
+            QTB_CUDA(cudaLaunchKernelEx(&cfg, dense_gemm_tc_kernel<128, kDenseDual, true>, o->map, *map_o, down->map, *map_down, a));
+            QTB_LAUNCH_CHECK();
+            return QUINTRIT_OK;
+        }
         const int tile = dense_tile(n, a.row_tiles[0], d->sm_count, 1.25);
         auto go = [&](auto kernel) { kernel<<<std::min(d->sm_count, (n + tile - 1) / tile * a.row_tiles[0]), kDenseThreads, dense_smem(tile), d->stream>>>(o->map, *map_o, down->map, *map_down, a); };
         tile == 256 ? go(dense_gemm_tc_kernel<256, kDenseDual>) : go(dense_gemm_tc_kernel<128, kDenseDual>);
