@@ -147,16 +147,18 @@ void build_items(std::vector<GemvItem>& items, const uint4* w, size_t act_off, s
     }
 }
 
-using GemvKernel = void (*)(const GemvItem*, int, const int8_t*, int32_t*, unsigned int*);
+using GemvKernel = void (*)(const GemvItem*, int, const int8_t*, int32_t*, unsigned int*, int);
+struct GemvKernels { GemvKernel add = nullptr, clear = nullptr; };  // adds to results that are cleared; clears them itself
+template <uint32_t BASE> GemvKernels gemv_kernels() { return {gemv_lut_kernel<BASE, false>, gemv_lut_kernel<BASE, true>}; }
 
 // Picks the kernel instantiation whose table-base constant equals the shared-window address this device gives to
 // dynamic shared memory (measured once per device with smem_base_kernel).
-int gemv_kernel_for_device(int dev, GemvKernel* out) {
-    static GemvKernel chosen[64] = {};
+int gemv_kernel_for_device(int dev, GemvKernels* out) {
+    static GemvKernels chosen[64];
     static std::mutex lock;  // first calls on a device from several host threads must not race on the cache
     if (dev < 0 || dev >= 64) return fail(QUINTRIT_ERR_DEVICE, "device index %d out of range", dev);
     std::lock_guard<std::mutex> hold(lock);
-    if (chosen[dev] == nullptr) {
+    if (chosen[dev].add == nullptr) {
         unsigned int* d_base = nullptr;
         unsigned int base = 0xFFFFFFFFu;
         QTB_CUDA(cudaMalloc(&d_base, sizeof(unsigned int)));
@@ -165,29 +167,30 @@ int gemv_kernel_for_device(int dev, GemvKernel* out) {
         if (e == cudaSuccess) e = cudaMemcpy(&base, d_base, sizeof base, cudaMemcpyDeviceToHost);
         cudaFree(d_base);
         if (e != cudaSuccess) return cuda_fail(e, "smem_base_kernel");
-        GemvKernel k = nullptr;
+        GemvKernels k;
         switch (base) {
-            case 0: k = gemv_lut_kernel<0>; break;
-            case 1024: k = gemv_lut_kernel<1024>; break;
-            case 2048: k = gemv_lut_kernel<2048>; break;
-            case 3072: k = gemv_lut_kernel<3072>; break;
-            case 4096: k = gemv_lut_kernel<4096>; break;
+            case 0: k = gemv_kernels<0>(); break;
+            case 1024: k = gemv_kernels<1024>(); break;
+            case 2048: k = gemv_kernels<2048>(); break;
+            case 3072: k = gemv_kernels<3072>(); break;
+            case 4096: k = gemv_kernels<4096>(); break;
             default: return fail(QUINTRIT_ERR_DEVICE, "unexpected shared-memory base %u on CUDA device %d: no kernel was built for it", base, dev);
         }
-        QTB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvSmemBytes));
+        for (GemvKernel f : {k.add, k.clear}) QTB_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvSmemBytes));
         chosen[dev] = k;
     }
     *out = chosen[dev];
     return QUINTRIT_OK;
 }
 
-// dependent: the launch before this one in the stream is zero_kernel, which this one need not wait for until it adds.
+// dependent: the launch before this one in the stream is zero_kernel, which this one need not wait for until it adds. clear: results that the launch
+// clears itself (0: they are cleared).
 int launch_gemv(const GemvItem* d_items, int n_items, const int8_t* d_act, int32_t* d_out, unsigned int* d_counters, int sm_count,
-                cudaStream_t stream, bool dependent = false) {
+                cudaStream_t stream, bool dependent = false, int clear = 0) {
     int dev = 0;
     QTB_CUDA(cudaGetDevice(&dev));
-    GemvKernel k = nullptr;
-    int rc = gemv_kernel_for_device(dev, &k);
+    GemvKernels ks;
+    int rc = gemv_kernel_for_device(dev, &ks);
     if (rc != QUINTRIT_OK) return rc;
     const int grid = std::max(1, std::min(n_items, sm_count * kCtasPerSm));
     cudaLaunchConfig_t cfg{};
@@ -196,12 +199,13 @@ int launch_gemv(const GemvItem* d_items, int n_items, const int8_t* d_act, int32
     cfg.gridDim = dim3(grid), cfg.blockDim = dim3(kGemvThreads), cfg.dynamicSmemBytes = kGemvSmemBytes, cfg.stream = stream;
     cfg.attrs = &attr, cfg.numAttrs = dependent ? 1 : 0;
     ++g_launches;
-    QTB_CUDA(cudaLaunchKernelEx(&cfg, k, d_items, n_items, d_act, d_out, d_counters));
+    QTB_CUDA(cudaLaunchKernelEx(&cfg, clear > 0 ? ks.clear : ks.add, d_items, n_items, d_act, d_out, d_counters, clear));
     return QUINTRIT_OK;
 }
 
 // The same with the results cleared first, `out_count` of them (at least one).
 int launch_gemv_cleared(const GemvItem* d_items, int n_items, const int8_t* d_act, int32_t* d_out, size_t out_count, unsigned int* d_counters, int sm_count, cudaStream_t stream) {
+    if (out_count <= static_cast<size_t>(kSelfClearMax)) return launch_gemv(d_items, n_items, d_act, d_out, d_counters, sm_count, stream, false, static_cast<int>(out_count));
     zero_kernel<<<static_cast<unsigned>(std::min<size_t>((out_count + 1023) / 1024, static_cast<size_t>(sm_count))), 256, 0, stream>>>(d_out, out_count);
     ++g_launches;
     QTB_CUDA(cudaGetLastError());
@@ -1089,7 +1093,7 @@ int decoder_create_impl(const quintrit_b200_decoder_desc_t* desc, quintrit_b200_
     if ((rc = dev_upload(d, &d->d_items, items.data(), items.size())) != QUINTRIT_OK) return rc;
 
     // one-time kernel set-up, before any stream capture
-    GemvKernel k = nullptr;
+    GemvKernels k;
     if ((rc = gemv_kernel_for_device(d->device, &k)) != QUINTRIT_OK) return rc;
     // The limit is a property of the kernel, shared by every decoder of the process: it is set to the most the device allows, so that a
     // later, smaller model does not lower it under an earlier, larger one.
@@ -1994,11 +1998,11 @@ int noalloc_setup(int dev, NoAllocDevice** out) {
         if (e == cudaSuccess) e = cudaMemcpy(&base, ptr + 12, sizeof base, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return cuda_fail(e, "smem_base_kernel");
         switch (base) {
-            case 0: s.kernel = gemv_lut_kernel<0>; break;
-            case 1024: s.kernel = gemv_lut_kernel<1024>; break;
-            case 2048: s.kernel = gemv_lut_kernel<2048>; break;
-            case 3072: s.kernel = gemv_lut_kernel<3072>; break;
-            case 4096: s.kernel = gemv_lut_kernel<4096>; break;
+            case 0: s.kernel = gemv_lut_kernel<0, false>; break;
+            case 1024: s.kernel = gemv_lut_kernel<1024, false>; break;
+            case 2048: s.kernel = gemv_lut_kernel<2048, false>; break;
+            case 3072: s.kernel = gemv_lut_kernel<3072, false>; break;
+            case 4096: s.kernel = gemv_lut_kernel<4096, false>; break;
             default: return fail(QUINTRIT_ERR_DEVICE, "unexpected shared-memory base %u on CUDA device %d: no kernel was built for it", base, dev);
         }
         QTB_CUDA(cudaFuncSetAttribute(s.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvSmemBytes));
@@ -2038,7 +2042,7 @@ extern "C" int quintrit_b200_gemv_i32_noalloc(const quintrit_b200_matrix_t* matr
         const int grid = static_cast<int>(std::max<size_t>(1, std::min(n_items, slots)));
         s->kernel<<<grid, kGemvThreads, kGemvSmemBytes, st>>>(reinterpret_cast<const GemvItem*>(s->scratch + kNoAllocHeaderBytes),
                                                              static_cast<int>(n_items), d_activations, d_out,
-                                                             reinterpret_cast<unsigned int*>(s->scratch));
+                                                             reinterpret_cast<unsigned int*>(s->scratch), 0);
         ++g_launches;
         QTB_CUDA(cudaGetLastError());
         return ok();
@@ -2750,7 +2754,7 @@ extern "C" int quintrit_b200_moe_create_shard(uint32_t device_index, uint32_t hi
         }
         DeviceGuard g(static_cast<int>(device_index));
         if ((rc = upload_exp2_table()) != QUINTRIT_OK) return rc;
-        GemvKernel k = nullptr;
+        GemvKernels k;
         if ((rc = gemv_kernel_for_device(static_cast<int>(device_index), &k)) != QUINTRIT_OK) return rc;
         int smem_optin = 0;
         QTB_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, static_cast<int>(device_index)));

@@ -142,3 +142,23 @@ def test_plan_runs_many_projections_in_one_launch(oracle, monkeypatch, segments)
         for (rows, cols), planar, a, r in zip(shapes, planars, acts, res):
             assert np.array_equal(r, oracle.gemv_planar(planar, rows, cols, a)), (rows, cols)
         acts = [rng.integers(-128, 128, c).astype(np.int8) for _, c in shapes]
+
+
+# Results that the launch clears itself (up to 8192 of them) or that a launch before it clears, at every alignment a caller's pointer can have, over values left there.
+@pytest.mark.parametrize("rows", [1, 3, 8191, 8192, 8193])
+@pytest.mark.parametrize("shift", [0, 1, 3])
+def test_results_are_cleared_at_any_alignment(oracle, rows, shift):
+    import torch
+
+    rng = np.random.default_rng(rows + shift)
+    cols = 330
+    trits = rng.integers(-1, 2, (rows, cols)).astype(np.int8)
+    m = q.Matrix(oracle.pack_planar(trits, rows, cols), rows, cols)
+    act = rng.integers(-128, 128, cols).astype(np.int8)
+    x = torch.from_numpy(act).cuda()
+    out = torch.full((rows + 8,), -7, dtype=torch.int32, device="cuda")
+    for _ in range(3):
+        m.gemv_i32_device(x.data_ptr(), out.data_ptr() + 4 * shift, torch.cuda.current_stream().cuda_stream)
+    got = out.cpu().numpy()
+    assert np.array_equal(got[shift:shift + rows], trits.astype(np.int32) @ act.astype(np.int32))
+    assert np.all(got[:shift] == -7) and np.all(got[shift + rows:] == -7)
