@@ -2597,6 +2597,10 @@ struct quintrit_b200_moe {
     float* pairs = nullptr;      // [max_batch * top_k][hidden]: every pair's down result as floats (zeros for pairs of experts held elsewhere)
     int expert_first = 0, expert_count = 0, n_local = 0, last_batch = 0;  // this GPU's experts; the local pairs of the last forward
     GemvItem *gu_items = nullptr, *down_items = nullptr;
+    // What a forward hands back lies in one piece of device memory - counters, tie, chosen, weights, out, in this order - and comes down in one copy
+    // into pinned memory; behind it is room for the inputs on their way up.
+    char *pack = nullptr, *host = nullptr;
+    size_t pack_out = 0, host_x = 0;  // bytes in front of `out`; bytes in front of the inputs
     cudaStream_t stream = nullptr;
 };
 
@@ -2614,6 +2618,7 @@ void destroy_moe(quintrit_b200_moe* m) {
     DeviceGuard g(m->device);
     if (m->stream) cudaStreamDestroy(m->stream);
     for (void* p : m->allocs) cudaFree(p);
+    if (m->host) cudaFreeHost(m->host);
     m->magic = 0;
     delete m;
 }
@@ -2643,23 +2648,29 @@ int moe_enqueue(quintrit_b200_moe* m, int batch) {
     return QUINTRIT_OK;
 }
 // The experts of the local pairs (m->local_z, m->n_local: set by the caller from the chosen ids) up to every pair's down result as floats.
-int moe_enqueue_experts(quintrit_b200_moe* m, int batch) {
+// combine: the weighted sum in m->out as well (a block that holds every expert).
+int moe_enqueue_experts(quintrit_b200_moe* m, int batch, bool combine = false) {
     cudaStream_t s = m->stream;
     const int H = m->hidden, I = m->inter, K = m->top_k, nz = batch * K, nl = m->n_local;
     const int pairs_gu = ((H + kBlockTrits - 1) / kBlockTrits + 1) / 2, pairs_d = ((I + kBlockTrits - 1) / kBlockTrits + 1) / 2;
     const int n_gu = nl * pairs_gu, n_d = nl * pairs_d * m->chunks_down;
-    QTB_CUDA(cudaMemsetAsync(m->acc_down, 0, size_t(nz) * H * sizeof(int32_t), s));
     if (nl > 0) {
-        moe_items_kernel<<<(n_gu + n_d + 255) / 256, 256, 0, s>>>(m->experts, m->chosen, m->local_z, nl, K, H, I, m->inter_pad, m->chunks_down, m->gu_items, m->down_items);
+        const size_t n_gu4 = size_t(nz) * 2 * I / 4, n_d4 = size_t(nz) * H / 4;
+        moe_items_kernel<<<std::max((n_gu + n_d + 255) / 256, m->sm_count), 256, 0, s>>>(m->experts, m->chosen, m->local_z, nl, K, H, I, m->inter_pad, m->chunks_down, m->gu_items, m->down_items,
+                                                                                       reinterpret_cast<int4*>(m->acc_gu), n_gu4, reinterpret_cast<int4*>(m->acc_down), n_d4);
         QTB_LAUNCH_CHECK();
-        QTB_CUDA(cudaMemsetAsync(m->acc_gu, 0, size_t(nz) * 2 * I * sizeof(int32_t), s));
         int rc = launch_gemv(m->gu_items, n_gu, m->a8_x, m->acc_gu, m->counters, m->sm_count, s);
         if (rc != QUINTRIT_OK) return rc;
         moe_act_quant_kernel<<<nl, kRowThreads, I * sizeof(float), s>>>(m->acc_gu, m->experts, m->chosen, m->local_z, m->s_x, K, I, m->inter_pad, m->a8_i, m->s_i);
         QTB_LAUNCH_CHECK();
         if ((rc = launch_gemv(m->down_items, n_d, m->a8_i, m->acc_down, m->counters, m->sm_count, s)) != QUINTRIT_OK) return rc;
+    } else {
+        QTB_CUDA(cudaMemsetAsync(m->acc_down, 0, size_t(nz) * H * sizeof(int32_t), s));
     }
-    moe_scale_pairs_kernel<<<dim3((H + 255) / 256, nz), 256, 0, s>>>(m->acc_down, m->experts, m->chosen, m->s_i, H, m->pairs);
+    if (combine)
+        moe_scale_combine_kernel<<<dim3((H + 127) / 128, batch), 128, 0, s>>>(m->acc_down, m->experts, m->chosen, m->s_i, m->weights, K, H, m->pairs, m->out);
+    else
+        moe_scale_pairs_kernel<<<dim3((H + 255) / 256, nz), 256, 0, s>>>(m->acc_down, m->experts, m->chosen, m->s_i, H, m->pairs);
     QTB_LAUNCH_CHECK();
     return QUINTRIT_OK;
 }
@@ -2669,24 +2680,14 @@ int moe_enqueue_combine(quintrit_b200_moe* m, int batch) {
     return QUINTRIT_OK;
 }
 
-// Router, selection (with the host's std::sort for tokens with equal probabilities), the list of local pairs, the local experts: everything up
-// to the pairs' results, then a synchronisation.
-int moe_partial(quintrit_b200_moe* m, const float* x, size_t batch) {
-    cudaStream_t s = m->stream;
-    const int B = static_cast<int>(batch), K = m->top_k, E = m->n_experts;
-    QTB_CUDA(cudaMemcpyAsync(m->x, x, batch * m->hidden * sizeof(float), cudaMemcpyHostToDevice, s));
-    int rc = moe_enqueue(m, B);
-    if (rc != QUINTRIT_OK) return rc;
-    // Experts with exactly equal probabilities: std::sort (the reference's choice, hybrid.rs:828-831) orders them by its algorithm. The
-    // device ranks such ties by id and flags the token; the host then sorts that token's experts with the standard library's std::sort
-    // and replaces the device's choice and weights.
-    std::vector<unsigned int> tie(batch);
-    std::vector<uint32_t> chosen(batch * K);
-    QTB_CUDA(cudaMemcpyAsync(tie.data(), m->tie, batch * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
-    QTB_CUDA(cudaMemcpyAsync(chosen.data(), m->chosen, batch * K * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    QTB_CUDA(cudaStreamSynchronize(s));
-    for (int b = 0; b < B; ++b) {
+// Experts with exactly equal probabilities: std::sort (the reference's choice, hybrid.rs:828-831) orders them by its algorithm. The
+// device ranks such ties by id and flags the token; the host then sorts that token's experts with the standard library's std::sort
+// and replaces the device's choice and weights. Everything on the stream is done when this is called.
+int moe_break_ties(quintrit_b200_moe* m, const unsigned int* tie, uint32_t* chosen, int batch, bool* any) {
+    const int K = m->top_k, E = m->n_experts;
+    for (int b = 0; b < batch; ++b) {
         if (tie[b] == 0) continue;
+        if (any) *any = true;
         std::vector<float> p(E);
         QTB_CUDA(cudaMemcpy(p.data(), m->probs + size_t(b) * E, E * sizeof(float), cudaMemcpyDeviceToHost));
         std::vector<uint32_t> order(E);
@@ -2700,6 +2701,23 @@ int moe_partial(quintrit_b200_moe* m, const float* x, size_t batch) {
         QTB_CUDA(cudaMemcpy(m->chosen + size_t(b) * K, order.data(), K * sizeof(uint32_t), cudaMemcpyHostToDevice));
         QTB_CUDA(cudaMemcpy(m->weights + size_t(b) * K, w.data(), K * sizeof(float), cudaMemcpyHostToDevice));
     }
+    return QUINTRIT_OK;
+}
+
+// Router, selection (with the host's std::sort for tokens with equal probabilities), the list of local pairs, the local experts: everything up
+// to the pairs' results, then a synchronisation.
+int moe_partial(quintrit_b200_moe* m, const float* x, size_t batch) {
+    cudaStream_t s = m->stream;
+    const int B = static_cast<int>(batch), K = m->top_k;
+    QTB_CUDA(cudaMemcpyAsync(m->x, x, batch * m->hidden * sizeof(float), cudaMemcpyHostToDevice, s));
+    int rc = moe_enqueue(m, B);
+    if (rc != QUINTRIT_OK) return rc;
+    std::vector<unsigned int> tie(batch);
+    std::vector<uint32_t> chosen(batch * K);
+    QTB_CUDA(cudaMemcpyAsync(tie.data(), m->tie, batch * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+    QTB_CUDA(cudaMemcpyAsync(chosen.data(), m->chosen, batch * K * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    QTB_CUDA(cudaStreamSynchronize(s));
+    if ((rc = moe_break_ties(m, tie.data(), chosen.data(), B, nullptr)) != QUINTRIT_OK) return rc;
     std::vector<uint32_t> local;
     for (size_t z = 0; z < chosen.size(); ++z)
         if (chosen[z] >= static_cast<uint32_t>(m->expert_first) && chosen[z] < static_cast<uint32_t>(m->expert_first + m->expert_count)) local.push_back(static_cast<uint32_t>(z));
@@ -2710,6 +2728,33 @@ int moe_partial(quintrit_b200_moe* m, const float* x, size_t batch) {
     QTB_CUDA(cudaMemcpyAsync(&flag, m->counters + 2, sizeof flag, cudaMemcpyDeviceToHost, s));
     QTB_CUDA(cudaStreamSynchronize(s));  // (also keeps `local` alive until its copy is done)
     if (flag != 0) return fail(QUINTRIT_ERR_DEVICE, "GEMV kernel on the CUDA device found its shared-memory table at an unexpected address");
+    return QUINTRIT_OK;
+}
+
+// A block that holds every expert: the device goes on with its own choice, results and flags come down in one copy, and only a token with a tie (the
+// host decides) sends the experts through again. One synchronisation instead of three, copies from and to pinned memory.
+int moe_whole(quintrit_b200_moe* m, const float* x, size_t batch, float* out, uint32_t* out_experts, float* out_weights) {
+    cudaStream_t s = m->stream;
+    const int B = static_cast<int>(batch), K = m->top_k;
+    const size_t x_bytes = batch * m->hidden * sizeof(float), bytes = m->pack_out + x_bytes;
+    std::memcpy(m->host + m->host_x, x, x_bytes);
+    QTB_CUDA(cudaMemcpyAsync(m->x, m->host + m->host_x, x_bytes, cudaMemcpyHostToDevice, s));
+    int rc = moe_enqueue(m, B);
+    if (rc != QUINTRIT_OK) return rc;
+    m->n_local = B * K, m->last_batch = B;  // (local_z counts up from zero in such a block)
+    auto at = [&](const void* p) { return m->host + (static_cast<const char*>(p) - m->pack); };
+    for (bool again = false;; again = true) {
+        if ((rc = moe_enqueue_experts(m, B, true)) != QUINTRIT_OK) return rc;
+        QTB_CUDA(cudaMemcpyAsync(m->host, m->pack, bytes, cudaMemcpyDeviceToHost, s));
+        QTB_CUDA(cudaStreamSynchronize(s));
+        if (reinterpret_cast<unsigned int*>(at(m->counters))[2] != 0) return fail(QUINTRIT_ERR_DEVICE, "GEMV kernel on the CUDA device found its shared-memory table at an unexpected address");
+        bool ties = false;
+        if (!again && (rc = moe_break_ties(m, reinterpret_cast<unsigned int*>(at(m->tie)), reinterpret_cast<uint32_t*>(at(m->chosen)), B, &ties)) != QUINTRIT_OK) return rc;
+        if (!ties) break;
+    }
+    std::memcpy(out, at(m->out), x_bytes);
+    if (out_experts) std::memcpy(out_experts, at(m->chosen), batch * K * sizeof(uint32_t));
+    if (out_weights) std::memcpy(out_weights, at(m->weights), batch * K * sizeof(float));
     return QUINTRIT_OK;
 }
 
@@ -2775,15 +2820,24 @@ extern "C" int quintrit_b200_moe_create_shard(uint32_t device_index, uint32_t hi
         };
         if ((rc = moe_alloc(m, &m->router, E * H)) != QUINTRIT_OK || (rc = moe_alloc(m, &m->experts, E)) != QUINTRIT_OK || (rc = moe_alloc(m, &m->x, B * H)) != QUINTRIT_OK ||
             (rc = moe_alloc(m, &m->x16, B * H)) != QUINTRIT_OK || (rc = moe_alloc(m, &m->a8_x, B * H + 256)) != QUINTRIT_OK || (rc = moe_alloc(m, &m->s_x, B)) != QUINTRIT_OK ||
-            (rc = moe_alloc(m, &m->logits, B * E)) != QUINTRIT_OK || (rc = moe_alloc(m, &m->probs, B * E)) != QUINTRIT_OK || (rc = moe_alloc(m, &m->chosen, Z)) != QUINTRIT_OK ||
-            (rc = moe_alloc(m, &m->weights, Z)) != QUINTRIT_OK || (rc = moe_alloc(m, &m->tie, B)) != QUINTRIT_OK || (rc = moe_alloc(m, &m->counters, 4)) != QUINTRIT_OK ||
+            (rc = moe_alloc(m, &m->logits, B * E)) != QUINTRIT_OK || (rc = moe_alloc(m, &m->probs, B * E)) != QUINTRIT_OK ||
             (rc = moe_alloc(m, &m->acc_gu, Z * 2 * I)) != QUINTRIT_OK || (rc = moe_alloc(m, &m->a8_i, Z * m->inter_pad + 256)) != QUINTRIT_OK || (rc = moe_alloc(m, &m->s_i, Z)) != QUINTRIT_OK ||
-            (rc = moe_alloc(m, &m->acc_down, Z * H)) != QUINTRIT_OK || (rc = moe_alloc(m, &m->out, B * H)) != QUINTRIT_OK || (rc = moe_alloc(m, &m->gu_items, Z * pairs_gu)) != QUINTRIT_OK ||
+            (rc = moe_alloc(m, &m->acc_down, Z * H)) != QUINTRIT_OK || (rc = moe_alloc(m, &m->gu_items, Z * pairs_gu)) != QUINTRIT_OK ||
             (rc = moe_alloc(m, &m->down_items, Z * pairs_d * m->chunks_down)) != QUINTRIT_OK || (rc = moe_alloc(m, &m->local_z, Z)) != QUINTRIT_OK ||
             (rc = moe_alloc(m, &m->pairs, Z * H)) != QUINTRIT_OK)
             return bail(rc);
+        const auto words = [](size_t n) { return (n + 3) / 4 * 16; };  // bytes of n words, rounded up to 16
+        m->pack_out = words(4) + words(B) + 2 * words(Z), m->host_x = m->pack_out + words(B * H);
+        if ((rc = moe_alloc(m, &m->pack, m->host_x)) != QUINTRIT_OK) return bail(rc);
+        m->counters = reinterpret_cast<unsigned int*>(m->pack), m->tie = reinterpret_cast<unsigned int*>(m->pack + words(4));
+        m->chosen = reinterpret_cast<uint32_t*>(m->pack + words(4) + words(B)), m->weights = reinterpret_cast<float*>(m->pack + words(4) + words(B) + words(Z));
+        m->out = reinterpret_cast<float*>(m->pack + m->pack_out);
+        std::vector<uint32_t> every(Z);
+        for (size_t z = 0; z < Z; ++z) every[z] = static_cast<uint32_t>(z);
         cudaError_t e = cudaMemcpy(m->router, router_bf16, E * H * sizeof(uint16_t), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(m->experts, refs.data(), E * sizeof(MoeExpertRef), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy(m->local_z, every.data(), Z * sizeof(uint32_t), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&m->host), m->host_x + B * H * sizeof(float));
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
         if (e != cudaSuccess) {
             destroy_moe(m);
@@ -2820,8 +2874,7 @@ extern "C" int quintrit_b200_moe_forward(quintrit_b200_moe_t* moe, const float* 
         if ((rc = moe_check_batch(moe, batch)) != QUINTRIT_OK) return rc;
         if (moe->expert_count != moe->n_experts) return fail(QUINTRIT_ERR_INVALID_ARGUMENT, "this block holds experts %d .. %d of %d: run quintrit_b200_moe_forward_partial, add the pairs of all GPUs, then quintrit_b200_moe_finish", moe->expert_first, moe->expert_first + moe->expert_count, moe->n_experts);
         DeviceGuard g(moe->device);
-        if ((rc = moe_partial(moe, x, batch)) != QUINTRIT_OK) return rc;
-        if ((rc = moe_finish(moe, batch, out, out_experts, out_weights)) != QUINTRIT_OK) return rc;
+        if ((rc = moe_whole(moe, x, batch, out, out_experts, out_weights)) != QUINTRIT_OK) return rc;
         return ok();
     });
 }
@@ -2875,8 +2928,9 @@ extern "C" int quintrit_b200_moe_time(quintrit_b200_moe_t* moe, size_t batch, ui
         QTB_CUDA(cudaEventRecord(e0, m->stream));
         for (uint32_t r = 0; r < repeats && rc == QUINTRIT_OK; ++r) {
             rc = moe_enqueue(m, static_cast<int>(batch));
-            if (rc == QUINTRIT_OK) rc = moe_enqueue_experts(m, static_cast<int>(batch));
-            if (rc == QUINTRIT_OK) rc = moe_enqueue_combine(m, static_cast<int>(batch));
+            const bool whole = m->expert_count == m->n_experts;
+            if (rc == QUINTRIT_OK) rc = moe_enqueue_experts(m, static_cast<int>(batch), whole);
+            if (rc == QUINTRIT_OK && !whole) rc = moe_enqueue_combine(m, static_cast<int>(batch));
         }
         cudaEventRecord(e1, m->stream);
         cudaError_t e = cudaStreamSynchronize(m->stream);

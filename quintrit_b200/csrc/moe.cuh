@@ -48,7 +48,8 @@ __global__ void __launch_bounds__(kRowThreads) moe_prepare_kernel(const float* _
 // over many small blocks instead of the head kernel's few large ones.
 __global__ void __launch_bounds__(128) moe_router_kernel(const __half* __restrict__ router, const __half* __restrict__ x16, int hidden, int n_experts, int batch,
                                                          float* __restrict__ logits) {
-    // grid (rows / 4, tokens / 4): a warp takes one expert row and four tokens; the elements of eight steps are requested together
+    // grid (rows / 4, tokens / 4): a warp takes one expert row and four tokens; the elements of sixteen steps are requested together
+    constexpr int kSteps = 16;
     const int lane = threadIdx.x & 31, row = blockIdx.x * 4 + (threadIdx.x >> 5), b0 = blockIdx.y * 4;
     if (row >= n_experts) return;
     const __half* w = router + static_cast<size_t>(row) * hidden + lane;
@@ -56,17 +57,17 @@ __global__ void __launch_bounds__(128) moe_router_kernel(const __half* __restric
     const __half* x[4];
 #pragma unroll
     for (int t = 0; t < 4; ++t) x[t] = x16 + static_cast<size_t>(min(b0 + t, batch - 1)) * hidden + lane;
-    for (int i0 = 0; i0 < hidden; i0 += 256) {
-        unsigned short wr[8], xr[4][8];
+    for (int i0 = 0; i0 < hidden; i0 += 32 * kSteps) {
+        unsigned short wr[kSteps], xr[4][kSteps];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < kSteps; ++k) {
             const int i = i0 + 32 * k;
             wr[k] = i < hidden ? __half_as_ushort(w[i]) : 0;
 #pragma unroll
             for (int t = 0; t < 4; ++t) xr[t][k] = i < hidden ? __half_as_ushort(x[t][i]) : 0;
         }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < kSteps; ++k) {
             if (i0 + 32 * k < hidden) {
                 const float wv = bf16_bits_to_float(wr[k]);
 #pragma unroll
@@ -93,19 +94,28 @@ __global__ void __launch_bounds__(256) moe_select_kernel(const float* __restrict
     for (int i = tid; i < n_experts; i += 256) p_s[i] = logits[b * n_experts + i];
     if (tid == 0) tie[b] = 0u;
     __syncthreads();
-    __shared__ float s_mx, s_inv;
-    if (tid == 0) {
-        float mx = p_s[0];
-        for (int i = 1; i < n_experts; ++i)
-            if (p_s[i] > mx) mx = p_s[i];
-        s_mx = mx;
-    }
+    __shared__ float s_inv, warp_mx[8];
+    // The maximum as the reference's loop leaves it (a NaN in the first place stays, others are passed over): any order gives it.
+    float mx = -INFINITY;
+    for (int i = tid; i < n_experts; i += 256) mx = fmaxf(mx, p_s[i]);
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((tid & 31) == 0) warp_mx[tid >> 5] = mx;
+    const float first = p_s[0];
     __syncthreads();
-    for (int i = tid; i < n_experts; i += 256) p_s[i] = device_expf(__fsub_rn(p_s[i], s_mx));  // (every exponential on its own: any thread may take it)
+#pragma unroll
+    for (int w = 0; w < 8; ++w) mx = fmaxf(mx, warp_mx[w]);
+    if (first != first) mx = first;
+    for (int i = tid; i < n_experts; i += 256) p_s[i] = device_expf(__fsub_rn(p_s[i], mx));  // (every exponential on its own: any thread may take it)
     __syncthreads();
     if (tid == 0) {
         double sum = 0.0;
-        for (int i = 0; i < n_experts; ++i) sum += static_cast<double>(p_s[i]);  // in the order of the experts, as the reference adds them
+        for (int i0 = 0; i0 < n_experts; i0 += 32) {  // in the order of the experts, as the reference adds them; the values of 32 are read together
+            float v[32];
+#pragma unroll
+            for (int k = 0; k < 32; ++k) v[k] = i0 + k < n_experts ? p_s[i0 + k] : 0.0f;  // (adding zero changes nothing: every value is >= 0, or NaN)
+#pragma unroll
+            for (int k = 0; k < 32; ++k) sum += static_cast<double>(v[k]);
+        }
         s_inv = sum > 0.0 ? __double2float_rn(1.0 / sum) : 1.0f;
     }
     __syncthreads();
@@ -116,6 +126,7 @@ __global__ void __launch_bounds__(256) moe_select_kernel(const float* __restrict
         probs[b * n_experts + i] = p;
         int rank = 0;
         bool tied = false;
+#pragma unroll 16
         for (int j = 0; j < n_experts; ++j) {
             const float q = p_s[j];
             rank += (q > p || (q == p && j < i)) ? 1 : 0;
@@ -141,7 +152,10 @@ __global__ void __launch_bounds__(256) moe_select_kernel(const float* __restrict
 // intermediate columns, the row tiles in `chunks_down` ranges). Same decomposition as build_items on the host.
 // `local_z` lists the n_z pairs whose expert this GPU holds (all pairs on one GPU; a share of them under expert parallelism).
 __global__ void moe_items_kernel(const MoeExpertRef* __restrict__ experts, const uint32_t* __restrict__ chosen, const uint32_t* __restrict__ local_z, int n_z, int top_k, int hidden,
-                                 int inter, int inter_pad, int chunks_down, GemvItem* __restrict__ gu_items, GemvItem* __restrict__ down_items) {
+                                 int inter, int inter_pad, int chunks_down, GemvItem* __restrict__ gu_items, GemvItem* __restrict__ down_items, int4* __restrict__ zero_gu, size_t n_gu4,
+                                 int4* __restrict__ zero_down, size_t n_down4) {
+    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n_gu4 + n_down4; i += size_t(gridDim.x) * blockDim.x)  // the results that the two launches add to
+        (i < n_gu4 ? zero_gu[i] : zero_down[i - n_gu4]) = make_int4(0, 0, 0, 0);
     const int blocks_gu = (hidden + kBlockTrits - 1) / kBlockTrits, pairs_gu = (blocks_gu + 1) / 2, tiles_gu = (2 * inter + kTileRows - 1) / kTileRows;
     const int blocks_d = (inter + kBlockTrits - 1) / kBlockTrits, pairs_d = (blocks_d + 1) / 2, tiles_d = (hidden + kTileRows - 1) / kTileRows;
     const int n_gu = n_z * pairs_gu, n_d = n_z * pairs_d * chunks_down;
@@ -200,15 +214,45 @@ __global__ void __launch_bounds__(kRowThreads) moe_act_quant_kernel(const int32_
 // pairs[z][h] = the down result of pair z as floats: one multiply by weight_scale / act_scale, zero for a zero activation scale
 // (layer.rs:143-150) and for a pair whose expert another GPU holds (that GPU writes the value; the exchange adds the shares, of which
 // exactly one is not zero).
+__device__ __forceinline__ float moe_pair_value(int32_t acc, const MoeExpertRef& e, float s_i) {
+    const bool live = e.w_down != nullptr && s_i > 0.0f;
+    return live ? __fmul_rn(static_cast<float>(acc), __fdiv_rn(e.ws_down, s_i)) : 0.0f;
+}
 __global__ void moe_scale_pairs_kernel(const int32_t* __restrict__ acc_down, const MoeExpertRef* __restrict__ experts, const uint32_t* __restrict__ chosen,
                                        const float* __restrict__ s_i, int hidden, float* __restrict__ pairs) {
     const size_t z = blockIdx.y;
-    const MoeExpertRef& e = experts[chosen[z]];
+    const MoeExpertRef e = experts[chosen[z]];
     const float s = s_i[z];
-    const bool live = e.w_down != nullptr && s > 0.0f;
-    const float post = live ? __fdiv_rn(e.ws_down, s) : 0.0f;
-    for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < hidden; h += gridDim.x * blockDim.x)
-        pairs[z * hidden + h] = live ? __fmul_rn(static_cast<float>(acc_down[z * hidden + h]), post) : 0.0f;
+    for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < hidden; h += gridDim.x * blockDim.x) pairs[z * hidden + h] = moe_pair_value(acc_down[z * hidden + h], e, s);
+}
+
+// Both in one launch where one GPU holds every expert: the pairs and, in selection order, their weighted sum (hybrid.rs:853-857). The factors of a
+// token's pairs are made once a block (an element that looks up its expert, scale and weight for itself waits for three reads in a row).
+constexpr int kMoeMaxTop = 64;
+__global__ void __launch_bounds__(128) moe_scale_combine_kernel(const int32_t* __restrict__ acc_down, const MoeExpertRef* __restrict__ experts, const uint32_t* __restrict__ chosen,
+                                                                const float* __restrict__ s_i, const float* __restrict__ weights, int top_k, int hidden, float* __restrict__ pairs, float* __restrict__ out) {
+    __shared__ float post[kMoeMaxTop], weight[kMoeMaxTop];
+    __shared__ bool live[kMoeMaxTop];
+    const size_t z0 = static_cast<size_t>(blockIdx.y) * top_k;
+    if (const int i = threadIdx.x; i < top_k) {  // (top_k is at most kMoeMaxTop: checked at creation)
+        const float s = s_i[z0 + i], ws = experts[chosen[z0 + i]].ws_down;
+        live[i] = s > 0.0f;
+        post[i] = s > 0.0f ? __fdiv_rn(ws, s) : 0.0f;
+        weight[i] = weights[z0 + i];
+    }
+    __syncthreads();
+    const int h = blockIdx.x * 128 + threadIdx.x;
+    if (h >= hidden) return;
+    float o = 0.0f;
+#pragma unroll 8
+    for (int i = 0; i < top_k; ++i) {
+        const int32_t acc = acc_down[(z0 + i) * hidden + h];
+        const float p = live[i] ? __fmul_rn(static_cast<float>(acc), post[i]) : 0.0f;
+        pairs[(z0 + i) * hidden + h] = p;
+        const float v = __fmul_rn(p, weight[i]);
+        o = i == 0 ? v : __fadd_rn(o, v);
+    }
+    out[static_cast<size_t>(blockIdx.y) * hidden + h] = o;
 }
 
 // out[token][h] = the pairs' results weighted and added in selection order, the first one assigned (hybrid.rs:853-857).
