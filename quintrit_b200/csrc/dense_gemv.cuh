@@ -203,7 +203,9 @@ struct NormProjectArgs {
     PairSum pair;               // added to x first; the first block writes the sum to x_out (not x itself)
     float* x_out;
     void* h_out;                // the first norm's result in the storage type, [tokens][pitch]; may be nullptr
+    int staged;                 // the norms' vectors lie in shared memory behind the activations: brought before the wait (widths that are multiples of four, at most kStagedWidth)
 };
+constexpr int kStagedWidth = 2048;  // two turns of 256 threads with four elements each
 
 constexpr int kProjectThreads = 256;
 
@@ -237,6 +239,15 @@ __global__ void __launch_bounds__(kProjectThreads, 4) norm_project_kernel(NormPr
         if (a.norm[0].b != nullptr) l2_prefetch(a.norm[0].b, bytes);
         if (a.pair.r[0] != nullptr) l2_prefetch(a.pair.w[0], bytes), l2_prefetch(a.pair.w[1], bytes);
     }
+    float* const vectors = act_smem + a.n_stack * pitch;  // staged: the weights of either norm, or weights and bias of the one
+    const bool staged = FORM != kProjectAny && a.staged != 0;
+    if (staged) {
+        const float* const src[2] = {a.norm[0].w, FORM == kProjectTanh ? a.norm[0].b : a.norm[1].w};
+        const int n = FORM == kProjectTanh || a.n_stack > 1 ? 2 : 1;
+        for (int k = 0; k < n; ++k)
+            for (int i = tid * 4; i < a.width; i += kProjectThreads * 4) attn_cp16(vectors + k * a.width + i, src[k] + i);
+        attn_cp_commit();
+    }
     pdl_wait();
     if (FORM == kProjectAny && a.pair.r[0] != nullptr) {
         float* sum = act_smem + a.n_stack * pitch;
@@ -255,23 +266,59 @@ __global__ void __launch_bounds__(kProjectThreads, 4) norm_project_kernel(NormPr
         }
         x = sum;  // (each thread reads back what it wrote)
     }
-    float inv = 1.0f;
-    if (FORM == kProjectRms || (FORM == kProjectAny && a.norm[0].b == nullptr)) {
+    if (staged) {
+        float4 xv[2];
         float ss = 0.0f;
-#pragma unroll 4
-        for (int i = tid; i < a.width; i += kProjectThreads) ss += x[i] * x[i];
-        inv = 1.0f / sqrtf(block_sum(ss, red) / static_cast<float>(a.width) + a.eps);
-    }
-    for (int s = 0; s < a.n_stack; ++s)
-#pragma unroll 4
-        for (int i = tid; i < pitch; i += kProjectThreads) {
-            const float v = i < a.width ? round_to<T>(FORM == kProjectRms    ? x[i] * inv * a.norm[s].w[i]
-                                                        : FORM == kProjectTanh ? tanhf(a.norm[s].alpha * x[i]) * a.norm[s].w[i] + a.norm[s].b[i]
-                                                                               : norm_value(a.norm[s], x[i], inv, i))
-                                          : 0.0f;
-            act_smem[s * pitch + act_index<T>(i, pitch)] = v;
-            if (FORM != kProjectRms && a.h_out != nullptr && s == 0 && blockIdx.x == 0) static_cast<T*>(a.h_out)[size_t(token) * pitch + i] = to_storage<T>(v);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int i = (tid + kProjectThreads * k) * 4;
+            xv[k] = i < a.width ? *reinterpret_cast<const float4*>(x + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            ss += xv[k].x * xv[k].x + xv[k].y * xv[k].y + xv[k].z * xv[k].z + xv[k].w * xv[k].w;
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");  // (a thread reads back what it brought)
+        const float inv = FORM == kProjectRms ? 1.0f / sqrtf(block_sum(ss, red) / static_cast<float>(a.width) + a.eps) : 1.0f;
+        for (int s = 0; s < a.n_stack; ++s)
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int i = (tid + kProjectThreads * k) * 4;
+                if (i >= pitch) continue;
+                float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (i < a.width) {
+                    const float4 w = *reinterpret_cast<const float4*>(vectors + (FORM == kProjectRms ? s * a.width : 0) + i);
+                    if (FORM == kProjectRms) {
+                        v = make_float4(xv[k].x * inv * w.x, xv[k].y * inv * w.y, xv[k].z * inv * w.z, xv[k].w * inv * w.w);
+                    } else {
+                        const float4 b = *reinterpret_cast<const float4*>(vectors + a.width + i);
+                        const float alpha = a.norm[0].alpha;
+                        v = make_float4(tanhf(alpha * xv[k].x) * w.x + b.x, tanhf(alpha * xv[k].y) * w.y + b.y, tanhf(alpha * xv[k].z) * w.z + b.z, tanhf(alpha * xv[k].w) * w.w + b.w);
+                    }
+                    v = make_float4(round_to<T>(v.x), round_to<T>(v.y), round_to<T>(v.z), round_to<T>(v.w));
+                }
+                act_put4<T>(act_smem + s * pitch, i, pitch, v);
+                if (FORM != kProjectRms && a.h_out != nullptr && blockIdx.x == 0) {
+                    T* h = static_cast<T*>(a.h_out) + size_t(token) * pitch + i;
+                    h[0] = to_storage<T>(v.x), h[1] = to_storage<T>(v.y), h[2] = to_storage<T>(v.z), h[3] = to_storage<T>(v.w);
+                }
+            }
+    } else {
+        float inv = 1.0f;
+        if (FORM == kProjectRms || (FORM == kProjectAny && a.norm[0].b == nullptr)) {
+            float ss = 0.0f;
+#pragma unroll 4
+            for (int i = tid; i < a.width; i += kProjectThreads) ss += x[i] * x[i];
+            inv = 1.0f / sqrtf(block_sum(ss, red) / static_cast<float>(a.width) + a.eps);
+        }
+        for (int s = 0; s < a.n_stack; ++s)
+#pragma unroll 4
+            for (int i = tid; i < pitch; i += kProjectThreads) {
+                const float v = i < a.width ? round_to<T>(FORM == kProjectRms    ? x[i] * inv * a.norm[s].w[i]
+                                                            : FORM == kProjectTanh ? tanhf(a.norm[s].alpha * x[i]) * a.norm[s].w[i] + a.norm[s].b[i]
+                                                                                   : norm_value(a.norm[s], x[i], inv, i))
+                                              : 0.0f;
+                act_smem[s * pitch + act_index<T>(i, pitch)] = v;
+                if (FORM != kProjectRms && a.h_out != nullptr && s == 0 && blockIdx.x == 0) static_cast<T*>(a.h_out)[size_t(token) * pitch + i] = to_storage<T>(v);
+            }
+    }
     __syncthreads();
     for (int s = 0; s < a.n_stack; ++s)
         for (int k = 0; k < a.stack[s].n_seg; ++k) {
@@ -354,15 +401,19 @@ struct FinishProjectArgs {
     const float *gate1, *gate2; // sigmoids, [tokens][width]; nullptr: no gate
 };
 
-template <typename T>
-__global__ void __launch_bounds__(kProjectThreads, 4) finish_project_kernel(FinishProjectArgs a) {
+// What a block waits for is latency, not bandwidth. BOTH (where the grid leaves a block's registers): the first pieces of a row of either matrix are on their way before the wait; the residual stream and the
+// gates of a warp's first row follow right behind it instead of at the end. With the norms' vectors staged in norm_project_kernel: a step of six Lasosun
+// layers of width 1024 190 -> 175 us, of six Tosevik layers 293 -> 283 us.
+template <typename T, bool BOTH>
+__global__ void __launch_bounds__(kProjectThreads, BOTH ? 2 : 4) finish_project_kernel(FinishProjectArgs a) {
     extern __shared__ float act_smem[];
     __shared__ float red[kProjectThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31, token = blockIdx.y;
     float *y = act_smem, *m = act_smem + a.o_pitch;
     const int warps = gridDim.x * (kProjectThreads / 32);
     pdl_trigger();
-    RowHead<1> head;
+    RowHead<1> head, spare;
+    RowHead<1>& head2 = BOTH ? spare : head;
     bool first = true;
     if (const int row = blockIdx.x * (kProjectThreads / 32) + (tid >> 5); row < a.width) {
         load_pieces<T, 1>(head, static_cast<const T*>(a.o) + size_t(row) * a.o_pitch, a.o_pitch, lane);
@@ -371,7 +422,16 @@ __global__ void __launch_bounds__(kProjectThreads, 4) finish_project_kernel(Fini
             if (a.m != nullptr) l2_prefetch(static_cast<const T*>(a.down) + size_t(row) * a.down_pitch, a.down_pitch * sizeof(T));
         }
     }
+    const int row0 = blockIdx.x * (kProjectThreads / 32) + (tid >> 5);
+    if (BOTH && row0 < a.width && a.m != nullptr) load_pieces<T, 1>(head2, static_cast<const T*>(a.down) + size_t(row0) * a.down_pitch, a.down_pitch, lane);
     pdl_wait();
+    float x0 = 0.0f, g10 = 1.0f, g20 = 1.0f;
+    if (BOTH && row0 < a.width && lane == 0) {
+        const size_t at = size_t(token) * a.width + row0;
+        x0 = a.x[at];
+        if (a.gate1 != nullptr) g10 = a.gate1[at];
+        if (a.gate2 != nullptr) g20 = a.gate2[at];
+    }
     const float* yt = a.y + size_t(token) * a.inner;
     const bool norm = a.norm_parts > 0;
     if (a.inner % 4 == 0) {
@@ -397,17 +457,18 @@ __global__ void __launch_bounds__(kProjectThreads, 4) finish_project_kernel(Fini
     for (int row = blockIdx.x * (kProjectThreads / 32) + (tid >> 5); row < a.width; row += warps) {
         float so[1], sd[1] = {0.0f};
         const T *o_row = static_cast<const T*>(a.o) + size_t(row) * a.o_pitch, *d_row = static_cast<const T*>(a.down) + size_t(row) * a.down_pitch;
+        const bool begun = BOTH && first;
         if (!first) load_pieces<T, 1>(head, o_row, a.o_pitch, lane);
         first = false;
         dot_rows<T, 1>(o_row, a.o_pitch, y, head, so);
         if (a.m != nullptr) {
-            load_pieces<T, 1>(head, d_row, a.down_pitch, lane);
-            dot_rows<T, 1>(d_row, a.down_pitch, m, head, sd);
+            if (!begun) load_pieces<T, 1>(head2, d_row, a.down_pitch, lane);
+            dot_rows<T, 1>(d_row, a.down_pitch, m, head2, sd);
         }
         if (lane == 0) {
             const size_t at = size_t(token) * a.width + row;
-            const float g1 = a.gate1 != nullptr ? a.gate1[at] : 1.0f, g2 = a.gate2 != nullptr ? a.gate2[at] : 1.0f;
-            a.x[at] += so[0] * g1 + sd[0] * g2;
+            const float g1 = begun ? g10 : a.gate1 != nullptr ? a.gate1[at] : 1.0f, g2 = begun ? g20 : a.gate2 != nullptr ? a.gate2[at] : 1.0f;
+            a.x[at] = (begun ? x0 : a.x[at]) + (so[0] * g1 + sd[0] * g2);
         }
     }
 }
@@ -444,6 +505,11 @@ __global__ void __launch_bounds__(kProjectThreads, 4) out_project_kernel(const _
         if (lane == 0) l2_prefetch(w, m.pitch * sizeof(T));
     }
     pdl_wait();
+    float old = 0.0f;  // what the first row adds to, on its way from here on
+    if (unit0 < units && lane == 0) {
+        const OutProjectArgs::Mixer& m = a.mix[unit0 >= a.width ? 1 : 0];
+        if (m.add) old = m.out[size_t(token) * a.width + unit0 % a.width];
+    }
     float* gates = act_smem + a.mix[0].pitch + (a.n > 1 ? a.mix[1].pitch : 0);
     for (int k = 0; k < a.n; ++k) {
         const OutProjectArgs::Mixer& m = a.mix[k];
@@ -472,7 +538,7 @@ __global__ void __launch_bounds__(kProjectThreads, 4) out_project_kernel(const _
         dot_rows<T, 1>(w, m.pitch, act_smem + (k > 0 ? a.mix[0].pitch : 0), head, v);
         if (lane == 0) {
             float* out = m.out + size_t(token) * a.width + row;
-            *out = m.add ? *out + v[0] : v[0];
+            *out = m.add ? (unit == unit0 ? old : *out) + v[0] : v[0];
         }
     }
 }

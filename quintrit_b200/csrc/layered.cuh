@@ -524,7 +524,8 @@ inline int layered_decoder_setup(quintrit_b200_decoder* d, const std::shared_ptr
     std::vector<const void*> kernels = {reinterpret_cast<const void*>(norm_project_kernel<bf16, kProjectRms>), reinterpret_cast<const void*>(norm_project_kernel<float, kProjectRms>),
                              reinterpret_cast<const void*>(norm_project_kernel<bf16, kProjectTanh>), reinterpret_cast<const void*>(norm_project_kernel<float, kProjectTanh>),
                              reinterpret_cast<const void*>(norm_project_kernel<bf16, kProjectAny>), reinterpret_cast<const void*>(norm_project_kernel<float, kProjectAny>),
-                             reinterpret_cast<const void*>(finish_project_kernel<bf16>), reinterpret_cast<const void*>(finish_project_kernel<float>),
+                             reinterpret_cast<const void*>(finish_project_kernel<bf16, false>), reinterpret_cast<const void*>(finish_project_kernel<float, false>),
+                             reinterpret_cast<const void*>(finish_project_kernel<bf16, true>), reinterpret_cast<const void*>(finish_project_kernel<float, true>),
                              reinterpret_cast<const void*>(finish_rows_kernel<bf16>), reinterpret_cast<const void*>(finish_rows_kernel<float>),
                              reinterpret_cast<const void*>(out_project_kernel<bf16>), reinterpret_cast<const void*>(out_project_kernel<float>),
                              reinterpret_cast<const void*>(rows_kernel<bf16>), reinterpret_cast<const void*>(rows_kernel<float>),
@@ -589,6 +590,15 @@ inline DenseStack layered_stack(const LayeredMatrix& w) {
 template <typename T> void (*layered_project_kernel(const NormProjectArgs& a))(NormProjectArgs) {
     if (a.pair.r[0] != nullptr || (a.norm[0].b == nullptr && a.h_out != nullptr)) return norm_project_kernel<T, kProjectAny>;
     return a.norm[0].b != nullptr ? norm_project_kernel<T, kProjectTanh> : norm_project_kernel<T, kProjectRms>;
+}
+
+// Whether the norms' vectors of a launch are staged in shared memory; returns the bytes this takes.
+inline size_t layered_stage_vectors(NormProjectArgs* a) {
+    const auto bits = [](const void* p) { return reinterpret_cast<uintptr_t>(p); };
+    const bool plain = a->pair.r[0] == nullptr && !(a->norm[0].b == nullptr && a->h_out != nullptr) && (a->norm[0].b == nullptr || a->n_stack == 1);  // (the kernels with a form of their own)
+    if (!plain || a->width % 4 != 0 || a->width > kStagedWidth || (bits(a->x) | bits(a->norm[0].w) | bits(a->norm[0].b) | (a->n_stack > 1 ? bits(a->norm[1].w) : 0)) % 16 != 0) return 0;
+    a->staged = 1;
+    return size_t(a->norm[0].b != nullptr || a->n_stack > 1 ? 2 : 1) * a->width * sizeof(float);
 }
 
 // The two stacks of a layer's projections with their endings; returns how many there are.
@@ -854,7 +864,8 @@ int layered_parallel_layer(quintrit_b200_decoder* d, size_t li, int n, const Lay
             for (int k = 0; k < st[i].n_seg; ++k) units += (st[i].seg[k].rows + 1) / 2;
         }
         const int warps = kProjectThreads / 32;
-        launch_dependent(layered_project_kernel<T>(a), dim3(std::min((units + warps - 1) / warps, 4 * m.sm_count)), kProjectThreads, size_t(n_stack) * wp * sizeof(float), s, a);
+        const size_t vectors = layered_stage_vectors(&a);
+        launch_dependent(layered_project_kernel<T>(a), dim3(std::min((units + warps - 1) / warps, 4 * m.sm_count)), kProjectThreads, size_t(n_stack) * wp * sizeof(float) + vectors, s, a);
         QTB_LAUNCH_CHECK();
         if ((rc = layered_mixer<T>(d, li, 0, n, tg, &ready)) != QUINTRIT_OK) return rc;
         FinishProjectArgs f{};
@@ -862,7 +873,9 @@ int layered_parallel_layer(quintrit_b200_decoder* d, size_t li, int n, const Lay
         f.o = x.o.w, f.o_pitch = x.o.pitch;
         if (n_stack > 1) f.m = y.m, f.down = l.down.w, f.down_pitch = l.down.pitch;
         if (l.spec.gated_residual) f.gate1 = y.g1, f.gate2 = y.g2;
-        launch_dependent(finish_project_kernel<T>, dim3(std::min((W + warps - 1) / warps, 4 * m.sm_count)), kProjectThreads, (size_t(f.o_pitch) + f.down_pitch) * sizeof(float), s, f);
+        const int blocks = std::min((W + warps - 1) / warps, 4 * m.sm_count);
+        launch_dependent(blocks <= 2 * m.sm_count ? finish_project_kernel<T, true> : finish_project_kernel<T, false>, dim3(blocks), kProjectThreads,
+                         (size_t(f.o_pitch) + f.down_pitch) * sizeof(float), s, f);
         QTB_LAUNCH_CHECK();
         return QUINTRIT_OK;
     }
@@ -906,7 +919,9 @@ int layered_sequential_step(quintrit_b200_decoder* d, size_t li, const LayeredTa
         int units = 0;
         for (int k = 0; k < a.stack[0].n_seg; ++k) units += (a.stack[0].seg[k].rows + 1) / 2;
         a.eps = m.spec.eps, a.width = W, a.n_stack = 1;
-        launch_dependent(layered_project_kernel<T>(a), dim3(std::min((units + warps - 1) / warps, 4 * m.sm_count)), kProjectThreads, size_t(a.pair.r[0] != nullptr ? 2 : 1) * wp * sizeof(float), s, a);
+        const size_t vectors = layered_stage_vectors(&a);
+        launch_dependent(layered_project_kernel<T>(a), dim3(std::min((units + warps - 1) / warps, 4 * m.sm_count)), kProjectThreads,
+                         size_t(a.pair.r[0] != nullptr ? 2 : 1) * wp * sizeof(float) + vectors, s, a);
         QTB_LAUNCH_CHECK();
         return QUINTRIT_OK;
     };
@@ -1099,7 +1114,8 @@ int layered_head(quintrit_b200_decoder* d, int row, float* logits) {
     a.stack[0] = layered_stack(m.head);
     a.stack[0].n_seg = 1, a.stack[0].seg[0] = DenseSeg{0, m.spec.vocab, kSegPlain, m.spec.vocab, logits, nullptr, nullptr};
     const int warps = kProjectThreads / 32;
-    launch_dependent(layered_project_kernel<T>(a), dim3(std::min((m.spec.vocab / 2 + warps) / warps, 4 * m.sm_count)), kProjectThreads, size_t(m.head.pitch) * sizeof(float), d->stream, a);
+    const size_t vectors = layered_stage_vectors(&a);
+    launch_dependent(layered_project_kernel<T>(a), dim3(std::min((m.spec.vocab / 2 + warps) / warps, 4 * m.sm_count)), kProjectThreads, size_t(m.head.pitch) * sizeof(float) + vectors, d->stream, a);
     QTB_LAUNCH_CHECK();
     return QUINTRIT_OK;
 }
