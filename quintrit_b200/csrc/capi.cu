@@ -177,6 +177,8 @@ int gemv_kernel_for_device(int dev, GemvKernels* out) {
             default: return fail(QUINTRIT_ERR_DEVICE, "unexpected shared-memory base %u on CUDA device %d: no kernel was built for it", base, dev);
         }
         for (GemvKernel f : {k.add, k.clear}) QTB_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvSmemBytes));
+        cudaFuncAttributes loaded;  // (a kernel is loaded when it is first asked for: here, not in a user's first call)
+        QTB_CUDA(cudaFuncGetAttributes(&loaded, zero_kernel));
         chosen[dev] = k;
     }
     *out = chosen[dev];

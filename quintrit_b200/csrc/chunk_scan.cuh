@@ -153,10 +153,11 @@ __global__ void __launch_bounds__(256) ssd_gram_kernel(const __grid_constant__ S
     w.gram[(size_t(chunk) * a.groups + g) * 256 + tid] = s;
 }
 
-// hgrn2: gates, A, scaled operands. grid: (heads, chunks), 128 threads; n <= ROWS
+// hgrn2: gates, A, scaled operands. grid: (heads, chunks), 128 threads; n <= ROWS. Bound by reads of shared memory and, with few blocks, by the chain of 16
+// decays; so a thread takes four rows of the state at a time for A and two for the operands (16 heads of 128 x 128, 2048 tokens: 51 -> 40 us).
 template <int ROWS>
 __global__ void __launch_bounds__(128) hgrn_prep_kernel(const __grid_constant__ ScanArgs a, const __grid_constant__ ChunkWork w) {
-    extern __shared__ float prep_sm[];
+    extern __shared__ __align__(16) float prep_sm[];
     const int head = blockIdx.x, chunk = blockIdx.y, chunks = gridDim.y, tid = threadIdx.x, n = a.n;
     constexpr int rows = ROWS;
     float *q = prep_sm, *k = q + kChunkT * rows, *f = k + kChunkT * rows;
@@ -195,34 +196,43 @@ __global__ void __launch_bounds__(128) hgrn_prep_kernel(const __grid_constant__ 
     __syncthreads();
     const size_t at = size_t(head) * chunks + chunk;
     bf16* qk = w.qk + at * 64 * rows;
-    auto put = [&](int which, int t, int d, float v) {
-        const bf16 hi = __float2bfloat16_rn(v);
-        qk[((which)*kChunkT + t) * rows + d] = hi;
-        qk[((which + 1) * kChunkT + t) * rows + d] = __float2bfloat16_rn(v - __bfloat162float(hi));
+    auto put = [&](int which, int t, int d, float2 v) {
+        uint32_t hi, lo;
+        split_bf16(v.x, v.y, &hi, &lo);
+        *reinterpret_cast<uint32_t*>(qk + (which * kChunkT + t) * rows + d) = hi;
+        *reinterpret_cast<uint32_t*>(qk + ((which + 1) * kChunkT + t) * rows + d) = lo;
     };
-    for (int d = tid; d < rows; d += 128) {
-        float prod = 1.0f;
-        for (int t = 0; t < kChunkT; ++t) {
-            prod *= f[t * rows + d];
-            put(0, t, d, q[t * rows + d] * prod);
-        }
-        w.fe[at * rows + d] = prod;
-        float rest = 1.0f;
-        for (int t = kChunkT - 1; t >= 0; --t) {
-            put(2, t, d, k[t * rows + d] * rest);
-            rest *= f[t * rows + d];
+    auto at2 = [&](const float* p, int t, int d) { return *reinterpret_cast<const float2*>(p + t * rows + d); };
+    for (int d = (tid & 63) * 2; d < rows; d += 128) {  // two neighbouring rows a thread; the first half of the block takes q, the second k
+        float2 prod = make_float2(1.0f, 1.0f);
+        if (tid < 64) {
+#pragma unroll
+            for (int t = 0; t < kChunkT; ++t) {
+                const float2 ft = at2(f, t, d), qt = at2(q, t, d);
+                prod.x *= ft.x, prod.y *= ft.y;
+                put(0, t, d, make_float2(qt.x * prod.x, qt.y * prod.y));
+            }
+            *reinterpret_cast<float2*>(w.fe + at * rows + d) = prod;
+        } else {
+#pragma unroll
+            for (int t = kChunkT - 1; t >= 0; --t) {
+                const float2 ft = at2(f, t, d), kt = at2(k, t, d);
+                put(2, t, d, make_float2(kt.x * prod.x, kt.y * prod.y));
+                prod.x *= ft.x, prod.y *= ft.y;
+            }
         }
     }
-    const int s = tid >> 3, dg = tid & 7;  // A: a thread takes a column s and every eighth row of the state
+    const int s = tid >> 3, dg = tid & 7;  // A: a thread takes a column s and four of every 32 rows of the state (rows beyond n hold zeros)
     float acc[kChunkT];
 #pragma unroll
     for (int t = 0; t < kChunkT; ++t) acc[t] = 0.0f;
-    for (int d = dg; d < n; d += 8) {
-        float r = k[s * rows + d];
+    for (int d = dg * 4; d < rows; d += 32) {
+        float4 r = load4(k + s * rows + d);
 #pragma unroll
         for (int t = 0; t < kChunkT; ++t) {
-            if (t > s) r *= f[t * rows + d];
-            if (t >= s) acc[t] = fmaf(q[t * rows + d], r, acc[t]);
+            const float4 ft = load4(f + t * rows + d), qt = load4(q + t * rows + d);
+            if (t > s) r.x *= ft.x, r.y *= ft.y, r.z *= ft.z, r.w *= ft.w;
+            if (t >= s) acc[t] = fmaf(qt.x, r.x, fmaf(qt.y, r.y, fmaf(qt.z, r.z, fmaf(qt.w, r.w, acc[t]))));
         }
     }
 #pragma unroll
