@@ -225,7 +225,8 @@ inline int enqueue_token(quintrit_b200_decoder* d, bool with_head) {
         n1.zero_a = d->acc_qkv;
         n1.zero_a_n = bs ? 0 : qd + 2 * kvd;
         n1.block_scaled = bs, n1.q8_d = d->q8_d;
-        norm_quant_kernel<<<1, kRowThreads, H * sizeof(float), s>>>(n1);
+        if (bs) launch_norm_blocks(n1, s);
+        else norm_quant_kernel<<<1, kRowThreads, H * sizeof(float), s>>>(n1);
         QTB_LAUNCH_CHECK();
         int rc;
         if (bs) {
@@ -295,7 +296,8 @@ inline int enqueue_token(quintrit_b200_decoder* d, bool with_head) {
         n2.zero_a = d->acc_gu;
         n2.zero_a_n = bs ? 0 : 2 * I;
         n2.block_scaled = bs, n2.q8_d = d->q8_d;
-        norm_quant_kernel<<<1, kRowThreads, H * sizeof(float), s>>>(n2);
+        if (bs) launch_norm_blocks(n2, s);
+        else norm_quant_kernel<<<1, kRowThreads, H * sizeof(float), s>>>(n2);
         QTB_LAUNCH_CHECK();
         if (bs) {
             float* f = reinterpret_cast<float*>(d->acc_gu);
@@ -336,7 +338,8 @@ inline int enqueue_token(quintrit_b200_decoder* d, bool with_head) {
         nf.y16_out = d->x16;
         nf.y16_bf16 = d->bf16_tables;
         nf.block_scaled = bs;
-        norm_quant_kernel<<<1, kRowThreads, H * sizeof(float), s>>>(nf);
+        if (bs) launch_norm_blocks(nf, s);
+        else norm_quant_kernel<<<1, kRowThreads, H * sizeof(float), s>>>(nf);
         QTB_LAUNCH_CHECK();
         launch_lm_head(d->lm_head, d->x16, H, d->vocab, d->logits, d->bf16_tables, d->sm_count, s);
         QTB_LAUNCH_CHECK();

@@ -1,4 +1,5 @@
-// The steps between the projections of a prompt chunk or of a step of several sequences (per-tensor models), a token's vector at a time:
+// The steps between the projections of a prompt chunk or of a step of several sequences (per-tensor models), a token's vector at a time (and the norm of
+// a block-scaled model's step):
 // residual + norm + codes, combination of the KV chunks + codes, activation + codes. Operation for operation those of norm_quant_kernel,
 // attn_finish_kernel and act_quant_kernel (decode.cuh), which single steps use; here a thread takes four neighbouring elements at a time and
 // keeps them in registers from the load to the codes.
@@ -69,8 +70,27 @@ inline int row_turns(int n) {
     return turns <= 4 ? turns : 0;
 }
 
-// Grid (1, 1, tokens). a.v_prev holds the previous projection's sums where there is one (a.acc_prev only says that there is).
-template <int TURNS>
+// Q8_0 codes (quantize_q8_0_block) of four neighbouring values: eight neighbouring lanes hold a block of 32. Every lane of the warp calls it.
+__device__ __forceinline__ uint32_t quantize_q8_0_4(const float (&y)[4], bool store_scale, float* scale) {
+    float m = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) m = fmaxf(m, fabsf(y[e]));  // (f32::max ignores a NaN, and so does fmaxf)
+    for (int o = 4; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (store_scale) *scale = __half2float(__float2half_rn(__fdiv_rn(m, 127.0f)));
+    const float id = m != 0.0f ? __fdiv_rn(127.0f, m) : 0.0f;
+    uint32_t out = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float r = rintf(__fmul_rn(y[e], id));
+        const int q = r == r ? static_cast<int>(fminf(fmaxf(r, -128.0f), 127.0f)) : 0;
+        out |= (static_cast<uint32_t>(q) & 0xffu) << (8 * e);
+    }
+    return out;
+}
+
+// Grid (1, 1, tokens). a.v_prev holds the previous projection's sums where there is one (a.acc_prev only says that there is). BLOCKS: a step of a
+// block-scaled model, whose projections leave floats (a.acc_prev) and take Q8_0 blocks.
+template <int TURNS, bool BLOCKS = false>
 __global__ void __launch_bounds__(1024) norm_quant_rows_kernel(const __grid_constant__ NormQuantArgs a) {
     __shared__ double sh_d[32];
     __shared__ float sh_f[32];
@@ -85,11 +105,11 @@ __global__ void __launch_bounds__(1024) norm_quant_rows_kernel(const __grid_cons
         const bool there = i < a.n;
         xv[k] = there ? *reinterpret_cast<const float4*>(x + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         wv[k] = there ? *reinterpret_cast<const float4*>(a.norm_w + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        sums[k] = prev && there ? acc_view_read4(a.v_prev, z, i) : make_int4(0, 0, 0, 0);
+        sums[k] = !prev || !there ? make_int4(0, 0, 0, 0) : BLOCKS ? *reinterpret_cast<const int4*>(a.acc_prev + z * a.b_acc + i) : acc_view_read4(a.v_prev, z, i);
     }
     float post = 0.0f;
     bool live = false;
-    if (prev) {
+    if (prev && !BLOCKS) {
         const float s = a.scale_prev[a.b_scale ? z : 0];
         live = s > 0.0f;  // layer.rs:148-150: a zero activation scale gives a zero projection
         post = live ? __fdiv_rn(a.ws_prev, s) : 0.0f;
@@ -103,7 +123,7 @@ __global__ void __launch_bounds__(1024) norm_quant_rows_kernel(const __grid_cons
         if (prev) {
             const int c[4] = {sums[k].x, sums[k].y, sums[k].z, sums[k].w};
 #pragma unroll
-            for (int e = 0; e < 4; ++e) y[k][e] = __fadd_rn(y[k][e], live ? __fmul_rn(static_cast<float>(c[e]), post) : 0.0f);
+            for (int e = 0; e < 4; ++e) y[k][e] = __fadd_rn(y[k][e], BLOCKS ? __int_as_float(c[e]) : live ? __fmul_rn(static_cast<float>(c[e]), post) : 0.0f);
             if (i < a.n) *reinterpret_cast<float4*>(x + i) = make_float4(y[k][0], y[k][1], y[k][2], y[k][3]);
         }
 #pragma unroll
@@ -129,6 +149,15 @@ __global__ void __launch_bounds__(1024) norm_quant_rows_kernel(const __grid_cons
 #pragma unroll
             for (int e = 0; e < 4; ++e) h[e] = a.y16_bf16 ? float_to_bf16_bits(y[k][e]) : __half_as_ushort(__float2half_rn(y[k][e]));
             *reinterpret_cast<ushort4*>(a.y16_out + z * a.b_y16 + i) = make_ushort4(h[0], h[1], h[2], h[3]);
+        }
+        return;
+    }
+    if constexpr (BLOCKS) {
+#pragma unroll
+        for (int k = 0; k < TURNS; ++k) {
+            const int i = (threadIdx.x + k * blockDim.x) * 4;
+            const uint32_t codes = quantize_q8_0_4(y[k], i < a.n && (threadIdx.x & 7) == 0, a.q8_d + i / 32);
+            if (i < a.n) *reinterpret_cast<uint32_t*>(a.q_out + z * a.b_q + i) = codes;
         }
         return;
     }
@@ -342,6 +371,16 @@ inline void launch_norm_quant_rows(const NormQuantArgs& a, int n, cudaStream_t s
         case 2: return go(norm_quant_rows_kernel<2>);
         case 3: case 4: return go(norm_quant_rows_kernel<4>);
         default: norm_quant_kernel<<<dim3(1, 1, n), kRowThreads, a.n * sizeof(float), s>>>(a);
+    }
+}
+// One token of a block-scaled model (hidden a multiple of 32). One block's chain of reads, sums and codes: 3072 values: a step of two layers (five of them)
+// 284 -> 277 us.
+inline void launch_norm_blocks(const NormQuantArgs& a, cudaStream_t s) {
+    switch (row_turns(a.n)) {
+        case 1: norm_quant_rows_kernel<1, true><<<1, row_threads(a.n), 0, s>>>(a); return;
+        case 2: norm_quant_rows_kernel<2, true><<<1, row_threads(a.n), 0, s>>>(a); return;
+        case 3: case 4: norm_quant_rows_kernel<4, true><<<1, row_threads(a.n), 0, s>>>(a); return;
+        default: norm_quant_kernel<<<1, kRowThreads, a.n * sizeof(float), s>>>(a);
     }
 }
 inline void launch_attn_finish_rows(const AttnFinishArgs& a, int n, cudaStream_t s) {

@@ -29,3 +29,23 @@ def test_prompt_equals_single_steps(arch, hidden, inter, heads, kv_heads, head_d
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32)) and got_next == want_next
     (x, tx), (y, ty) = a.forward(want_next, n), b.forward(got_next, n)
     assert np.array_equal(x.view(np.uint32), y.view(np.uint32)) and tx == ty
+
+
+@pytest.mark.parametrize("hidden", [64, 960, 4160])  # lanes of a warp without elements, several warps, a second turn of the threads
+def test_block_scaled_steps(oracle, hidden):
+    """The norm of a block-scaled model's step (norm_quant_rows_kernel with BLOCKS) against the oracle."""
+    from quintrit_b200 import gguf_io
+
+    spec = synth.make_model(q.ARCH_LLAMA, True, hidden, 704, 2, 4, 2, 64, 300, 256, 500000.0, 1e-5, config=hidden % 89, random_norms=True)
+    shapes = [(256, hidden), (128, hidden), (128, hidden), (hidden, 256), (704, hidden), (704, hidden), (hidden, 704)]
+    rng = np.random.default_rng(hidden)
+    payloads, block_scales = [], []
+    for l in range(2):
+        for p, (r, c) in enumerate(shapes):
+            sc = rng.uniform(0.5, 2.0, r * c // 64).astype(np.float16)
+            payloads.append((q.SRC_Q2_0, gguf_io.encode_q2_0(synth.trits(synth.seed_for(hidden % 89, l, p, 0), r * c).reshape(r, c), sc)))
+            block_scales.append(sc.astype(np.float32))
+    dec, ref = q.Decoder(dict(spec, weights=payloads)), oracle.Model(dict(spec, block_scales=block_scales))
+    for pos, tok in enumerate(synth.prompt_tokens(5, 4, spec["vocab"])):
+        want, got = ref.forward(int(tok), pos), dec.forward(int(tok), pos)[0]
+        assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), pos
