@@ -1053,15 +1053,19 @@ int decoder_create_impl(const quintrit_b200_decoder_desc_t* desc, quintrit_b200_
         return rc;
 
     if ((rc = dev_alloc(d, &d->q8_d, std::max<size_t>({H, I, qd}) / 32 + 1)) != QUINTRIT_OK) return rc;
+    // The limit is a property of the kernel, shared by every decoder of the process: it is set to the most the device allows, so that a
+    // later, smaller model does not lower it under an earlier, larger one.
+    int smem_optin = 0;
+    QTB_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, d->device));
+    const size_t big = std::max<size_t>({H, I, qd}) * sizeof(float);
+    if (big + 1024 > static_cast<size_t>(smem_optin)) return fail(QUINTRIT_ERR_UNSUPPORTED, "a vector of %zu bytes does not fit the shared memory of a multiprocessor (%d bytes)", big, smem_optin);
+    if ((rc = allow_max_dynamic_smem(norm_quant_kernel, smem_optin)) != QUINTRIT_OK) return rc;
+    if ((rc = allow_max_dynamic_smem(attn_finish_kernel, smem_optin)) != QUINTRIT_OK) return rc;
+    if ((rc = allow_max_dynamic_smem(act_quant_kernel, smem_optin)) != QUINTRIT_OK) return rc;
+    if ((rc = allow_max_dynamic_smem(lm_head_kernel<false>, smem_optin)) != QUINTRIT_OK || (rc = allow_max_dynamic_smem(lm_head_kernel<true>, smem_optin)) != QUINTRIT_OK) return rc;
+    if ((rc = allow_max_dynamic_smem(attention_kernel, smem_optin)) != QUINTRIT_OK) return rc;
     if (block_scaled) {  // no work items: the block-scaled projections are plain launches; one kernel per step
         QTB_CUDA(block_scaled_allow_smem());
-        const int big_bs = static_cast<int>(std::max<size_t>({H, I, qd}) * sizeof(float));
-        QTB_CUDA(cudaFuncSetAttribute(norm_quant_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big_bs));
-        QTB_CUDA(cudaFuncSetAttribute(attn_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big_bs));
-        QTB_CUDA(cudaFuncSetAttribute(act_quant_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big_bs));
-        QTB_CUDA(cudaFuncSetAttribute(lm_head_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big_bs));
-        QTB_CUDA(cudaFuncSetAttribute(lm_head_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big_bs));
-        QTB_CUDA(cudaFuncSetAttribute(attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(attention_smem(256))));
         d->use_mega = false;
         QTB_CUDA(cudaDeviceSynchronize());
         return QUINTRIT_OK;
@@ -1097,19 +1101,8 @@ int decoder_create_impl(const quintrit_b200_decoder_desc_t* desc, quintrit_b200_
     // one-time kernel set-up, before any stream capture
     GemvKernels k;
     if ((rc = gemv_kernel_for_device(d->device, &k)) != QUINTRIT_OK) return rc;
-    // The limit is a property of the kernel, shared by every decoder of the process: it is set to the most the device allows, so that a
-    // later, smaller model does not lower it under an earlier, larger one.
-    int smem_optin = 0;
-    QTB_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, d->device));
-    const size_t big = std::max<size_t>({H, I, qd}) * sizeof(float);
-    if (big + 1024 > static_cast<size_t>(smem_optin)) return fail(QUINTRIT_ERR_UNSUPPORTED, "a vector of %zu bytes does not fit the shared memory of a multiprocessor (%d bytes)", big, smem_optin);
-    if ((rc = allow_max_dynamic_smem(norm_quant_kernel, smem_optin)) != QUINTRIT_OK) return rc;
-    if ((rc = allow_max_dynamic_smem(attn_finish_kernel, smem_optin)) != QUINTRIT_OK) return rc;
-    if ((rc = allow_max_dynamic_smem(act_quant_kernel, smem_optin)) != QUINTRIT_OK) return rc;
-    if ((rc = allow_max_dynamic_smem(lm_head_kernel<false>, smem_optin)) != QUINTRIT_OK || (rc = allow_max_dynamic_smem(lm_head_kernel<true>, smem_optin)) != QUINTRIT_OK) return rc;
     for (int tg : {1, 2, 4})
         if ((rc = allow_max_dynamic_smem(lm_head_batch_for(tg, d->bf16_tables), smem_optin)) != QUINTRIT_OK) return rc;
-    if ((rc = allow_max_dynamic_smem(attention_kernel, smem_optin)) != QUINTRIT_OK) return rc;
     // attention for all query heads of a KV head at once, where the group size and the head size allow it
     d->attn_gqa = nullptr, d->attn_gqa_smem = 0;
     if (hd % 32 == 0 && hd <= 256 && std::getenv("QUINTRIT_B200_ATTN_GQA_OFF") == nullptr) {
@@ -1166,7 +1159,9 @@ void mega_phase_items(std::vector<GemvItem>& items, const quintrit_b200_matrix* 
 template <uint32_t BASE>
 int mega_bind(quintrit_b200_decoder* d) {
     d->mega_kernel = decode_token_kernel<BASE>;
-    QTB_CUDA(cudaFuncSetAttribute(decode_token_kernel<BASE>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(d->mega_smem)));
+    int smem_optin = 0, rc;
+    QTB_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, d->device));
+    if ((rc = allow_max_dynamic_smem(decode_token_kernel<BASE>, smem_optin)) != QUINTRIT_OK) return rc;  // (for every decoder of the process)
     int per_sm = 0;
     QTB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_token_kernel<BASE>, kMegaThreads, d->mega_smem));
     if (per_sm < 1) return fail(QUINTRIT_ERR_DEVICE, "the decode kernel does not fit one CTA per multiprocessor on this CUDA device");
