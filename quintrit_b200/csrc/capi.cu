@@ -2598,6 +2598,7 @@ struct quintrit_b200_moe {
     // into pinned memory; behind it is room for the inputs on their way up.
     char *pack = nullptr, *host = nullptr;
     size_t pack_out = 0, host_x = 0;  // bytes in front of `out`; bytes in front of the inputs
+    char* on_host(const void* p) const { return host + (static_cast<const char*>(p) - pack); }  // where a part of the piece lies in the host's copy
     cudaStream_t stream = nullptr;
 };
 
@@ -2679,24 +2680,33 @@ int moe_enqueue_combine(quintrit_b200_moe* m, int batch) {
 
 // Experts with exactly equal probabilities: std::sort (the reference's choice, hybrid.rs:828-831) orders them by its algorithm. The
 // device ranks such ties by id and flags the token; the host then sorts that token's experts with the standard library's std::sort
-// and replaces the device's choice and weights. Everything on the stream is done when this is called.
-int moe_break_ties(quintrit_b200_moe* m, const unsigned int* tie, uint32_t* chosen, int batch, bool* any) {
+// and replaces the device's choice and weights. Everything on the stream is done when this is called; m->host holds the choice (tie,
+// chosen, weights), and what the host decided goes up on the block's own stream, in front of the launches that read it: the stream does not wait
+// for the default one, on which an ordinary copy would go.
+int moe_break_ties(quintrit_b200_moe* m, int batch, bool* any) {
     const int K = m->top_k, E = m->n_experts;
+    const unsigned int* tie = reinterpret_cast<const unsigned int*>(m->on_host(m->tie));
+    uint32_t* chosen = reinterpret_cast<uint32_t*>(m->on_host(m->chosen));
+    float* weights = reinterpret_cast<float*>(m->on_host(m->weights));
+    *any = false;
+    std::vector<float> p(E);
+    std::vector<uint32_t> order(E);
     for (int b = 0; b < batch; ++b) {
         if (tie[b] == 0) continue;
-        if (any) *any = true;
-        std::vector<float> p(E);
-        QTB_CUDA(cudaMemcpy(p.data(), m->probs + size_t(b) * E, E * sizeof(float), cudaMemcpyDeviceToHost));
-        std::vector<uint32_t> order(E);
+        *any = true;
+        QTB_CUDA(cudaMemcpyAsync(p.data(), m->probs + size_t(b) * E, E * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+        QTB_CUDA(cudaStreamSynchronize(m->stream));
         for (int i = 0; i < E; ++i) order[i] = static_cast<uint32_t>(i);
         std::sort(order.begin(), order.end(), [&](uint32_t a, uint32_t c) { return p[a] > p[c]; });
-        std::vector<float> w(K);
+        float* w = weights + size_t(b) * K;
         double sum = 0.0;
         for (int i = 0; i < K; ++i) w[i] = p[order[i]], sum += static_cast<double>(w[i]);
         const float sc = std::max(static_cast<float>(sum), 6.103515625e-5f);
         for (int i = 0; i < K; ++i) w[i] /= sc, chosen[size_t(b) * K + i] = order[i];
-        QTB_CUDA(cudaMemcpy(m->chosen + size_t(b) * K, order.data(), K * sizeof(uint32_t), cudaMemcpyHostToDevice));
-        QTB_CUDA(cudaMemcpy(m->weights + size_t(b) * K, w.data(), K * sizeof(float), cudaMemcpyHostToDevice));
+    }
+    if (*any) {  // (the tokens without a tie get back what they had)
+        QTB_CUDA(cudaMemcpyAsync(m->chosen, chosen, size_t(batch) * K * sizeof(uint32_t), cudaMemcpyHostToDevice, m->stream));
+        QTB_CUDA(cudaMemcpyAsync(m->weights, weights, size_t(batch) * K * sizeof(float), cudaMemcpyHostToDevice, m->stream));
     }
     return QUINTRIT_OK;
 }
@@ -2709,14 +2719,13 @@ int moe_partial(quintrit_b200_moe* m, const float* x, size_t batch) {
     QTB_CUDA(cudaMemcpyAsync(m->x, x, batch * m->hidden * sizeof(float), cudaMemcpyHostToDevice, s));
     int rc = moe_enqueue(m, B);
     if (rc != QUINTRIT_OK) return rc;
-    std::vector<unsigned int> tie(batch);
-    std::vector<uint32_t> chosen(batch * K);
-    QTB_CUDA(cudaMemcpyAsync(tie.data(), m->tie, batch * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
-    QTB_CUDA(cudaMemcpyAsync(chosen.data(), m->chosen, batch * K * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    QTB_CUDA(cudaMemcpyAsync(m->host, m->pack, m->pack_out, cudaMemcpyDeviceToHost, s));
     QTB_CUDA(cudaStreamSynchronize(s));
-    if ((rc = moe_break_ties(m, tie.data(), chosen.data(), B, nullptr)) != QUINTRIT_OK) return rc;
+    bool ties = false;
+    if ((rc = moe_break_ties(m, B, &ties)) != QUINTRIT_OK) return rc;
+    const uint32_t* chosen = reinterpret_cast<const uint32_t*>(m->on_host(m->chosen));
     std::vector<uint32_t> local;
-    for (size_t z = 0; z < chosen.size(); ++z)
+    for (size_t z = 0; z < batch * K; ++z)
         if (chosen[z] >= static_cast<uint32_t>(m->expert_first) && chosen[z] < static_cast<uint32_t>(m->expert_first + m->expert_count)) local.push_back(static_cast<uint32_t>(z));
     m->n_local = static_cast<int>(local.size()), m->last_batch = B;
     if (!local.empty()) QTB_CUDA(cudaMemcpyAsync(m->local_z, local.data(), local.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
@@ -2739,19 +2748,18 @@ int moe_whole(quintrit_b200_moe* m, const float* x, size_t batch, float* out, ui
     int rc = moe_enqueue(m, B);
     if (rc != QUINTRIT_OK) return rc;
     m->n_local = B * K, m->last_batch = B;  // (local_z counts up from zero in such a block)
-    auto at = [&](const void* p) { return m->host + (static_cast<const char*>(p) - m->pack); };
     for (bool again = false;; again = true) {
         if ((rc = moe_enqueue_experts(m, B, true)) != QUINTRIT_OK) return rc;
         QTB_CUDA(cudaMemcpyAsync(m->host, m->pack, bytes, cudaMemcpyDeviceToHost, s));
         QTB_CUDA(cudaStreamSynchronize(s));
-        if (reinterpret_cast<unsigned int*>(at(m->counters))[2] != 0) return fail(QUINTRIT_ERR_DEVICE, "GEMV kernel on the CUDA device found its shared-memory table at an unexpected address");
+        if (reinterpret_cast<unsigned int*>(m->on_host(m->counters))[2] != 0) return fail(QUINTRIT_ERR_DEVICE, "GEMV kernel on the CUDA device found its shared-memory table at an unexpected address");
         bool ties = false;
-        if (!again && (rc = moe_break_ties(m, reinterpret_cast<unsigned int*>(at(m->tie)), reinterpret_cast<uint32_t*>(at(m->chosen)), B, &ties)) != QUINTRIT_OK) return rc;
+        if (!again && (rc = moe_break_ties(m, B, &ties)) != QUINTRIT_OK) return rc;
         if (!ties) break;
     }
-    std::memcpy(out, at(m->out), x_bytes);
-    if (out_experts) std::memcpy(out_experts, at(m->chosen), batch * K * sizeof(uint32_t));
-    if (out_weights) std::memcpy(out_weights, at(m->weights), batch * K * sizeof(float));
+    std::memcpy(out, m->on_host(m->out), x_bytes);
+    if (out_experts) std::memcpy(out_experts, m->on_host(m->chosen), batch * K * sizeof(uint32_t));
+    if (out_weights) std::memcpy(out_weights, m->on_host(m->weights), batch * K * sizeof(float));
     return QUINTRIT_OK;
 }
 
@@ -2836,6 +2844,7 @@ extern "C" int quintrit_b200_moe_create_shard(uint32_t device_index, uint32_t hi
         if (e == cudaSuccess) e = cudaMemcpy(m->local_z, every.data(), Z * sizeof(uint32_t), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&m->host), m->host_x + B * H * sizeof(float));
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaDeviceSynchronize();  // (the clearing and the copies above are on the default stream, which m->stream does not wait for)
         if (e != cudaSuccess) {
             destroy_moe(m);
             return cuda_fail(e, "set-up of the mixture-of-experts block");

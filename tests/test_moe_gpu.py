@@ -58,6 +58,31 @@ def test_equal_probabilities_are_ordered_as_std_sort_orders_them():
     block.free()
 
 
+@pytest.mark.parametrize("shard", [False, True])
+def test_the_hosts_order_of_equals_is_what_the_experts_run_with(shard):
+    """All experts equally probable: what std::sort makes of that is not the order of their ids, so a pass that still reads the device's choice gives
+    other experts. Fresh blocks and repeated calls, whole and with one share holding everything but the last expert."""
+    hidden, inter, n_experts, top_k, batch = 256, 64, 64, 5, 16
+    rng, router, gu, dn, scales = _block(21, hidden, inter, n_experts)
+    r = np.tile(np.asarray(router, np.uint16).reshape(n_experts, hidden)[:1], (n_experts, 1))
+    held = n_experts - 1 if shard else n_experts
+    for _ in range(3):
+        block = q.Moe(hidden, inter, top_k, r, gu[:held], dn[:held], scales[:held], n_experts=n_experts)
+        for call in range(6):
+            x = rng.standard_normal((batch, hidden)).astype(np.float32)
+            if shard:
+                block.forward_partial(x)
+                out, ids, w = block.finish()
+            else:
+                out, ids, w = block.forward(x)
+            assert np.array_equal(ids, np.tile(ids[:1], (batch, 1))) and list(ids[0]) != list(range(top_k)) and n_experts - 1 not in ids[0]
+            assert np.all(w == w[0][0]) and abs(float(w[0].sum()) - 1.0) < 1e-6
+            for b in (0, 7, batch - 1):
+                pairs = [omoe.expert(x[b], gu[e], dn[e], hidden, inter, *scales[e]) for e in ids[b]]
+                assert np.array_equal(out[b].view(np.uint32), omoe.combine(pairs, w[b]).view(np.uint32)), (call, b)
+        block.free()
+
+
 def test_arguments():
     rng, router, gu, dn, scales = _block(9, 256, 64, 4)
     with pytest.raises(q.QuintritError) as e:
