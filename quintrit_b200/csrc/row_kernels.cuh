@@ -8,6 +8,10 @@
 // loads, parts included, are all requested before the first is used (one element at a time in a loop that stores to the residual stream, the parts
 // of an element were fetched one after another), block-wide results take two rounds of shuffles, codes leave four to a store. 256 tokens of the
 // Falcon3-10B shape (12 heads of 256, 23040 channels), by ncu: norm 17.5 -> 7.4 us, KV chunks 16.2 -> 9.9 us, activation 71 -> 30 us.
+//
+// Longer vectors, events around 20 launches, 32 tokens, against the kernels of decode.cuh: norm of 8192 / 16384 values 9.4 -> 6.6 / 12.4 -> 10.4 us; KV
+// chunks of 8192 / 10240 / 16384 values 23 -> 8.3 / 29 -> 14.4 / 41 -> 14.5 us; 256 tokens of 16384 25 -> 17 and 70 -> 30 us. (At 1024 threads the long
+// forms spill: 16 bytes a thread of the norm with four turns, 64 and 288 of the KV chunks with two and four. They are ahead all the same.)
 #pragma once
 #include "decode.cuh"
 
@@ -394,13 +398,16 @@ inline void launch_attn_finish_rows(const AttnFinishArgs& a, int n, cudaStream_t
     }
 }
 inline void launch_act_quant_rows(const ActQuantArgs& a, int n, cudaStream_t s) {
-    const int turns = (act_cluster_slice(a.n) + 1023) / 1024;  // of 256 threads with four elements each
+    // Turns of 256 threads with four elements each. Past four, blocks of 512 threads: eight turns a thread do not fit the registers (36864 channels,
+    // 32 tokens: 35 us against 12.4; 256 tokens: 192 against 66). A model's vector is at most 51200 long, seven turns; longer ones take the
+    // general kernel.
+    const int turns = (act_cluster_slice(a.n) + 1023) / 1024;
     auto go = [&](auto kernel, int threads) { kernel<<<dim3(kActClusterSize, 1, n), threads, 0, s>>>(a); };
     if (turns <= 1) go(act_quant_rows_kernel<1, 256>, 256);
     else if (turns == 2) go(act_quant_rows_kernel<2, 256>, 256);
     else if (turns == 3) go(act_quant_rows_kernel<3, 256>, 256);
     else if (turns == 4) go(act_quant_rows_kernel<4, 256>, 256);
-    else if (turns <= 16) go(act_quant_rows_kernel<8, 512>, 512);
+    else if (turns <= 8) go(act_quant_rows_kernel<4, 512>, 512);
     else act_quant_kernel<<<dim3(1, 1, n), kRowThreads, a.n * sizeof(float), s>>>(a);
 }
 

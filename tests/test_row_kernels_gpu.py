@@ -17,6 +17,9 @@ pytestmark = pytest.mark.gpu
     (q.ARCH_LLAMA, 4128, 16416, 5, 1, 256),  # a second turn of the norm's threads, a third of the activation's
     (q.ARCH_LLAMA, 128, 24608, 34, 2, 128),  # a second turn of the attention's threads, a fourth of the activation's
     (q.ARCH_BITNET, 128, 32800, 2, 1, 64),   # the activation step with blocks of 512 threads
+    (q.ARCH_BITNET, 128, 51200, 2, 1, 64),   # the longest vector a model may have: a fourth turn of those
+    (q.ARCH_LLAMA, 8224, 64, 2, 1, 64),      # a third turn of the norm's threads
+    (q.ARCH_LLAMA, 128, 128, 68, 17, 128),   # a third turn of the attention's threads
 ])
 def test_prompt_equals_single_steps(arch, hidden, inter, heads, kv_heads, head_dim):
     spec = synth.make_model(arch, False, hidden, inter, 2, heads, kv_heads, head_dim, 300, 1024, 500000.0, 1e-5, config=hidden % 97, random_norms=True, tied=arch == q.ARCH_BITNET)
