@@ -82,9 +82,11 @@ __global__ void __launch_bounds__(128) moe_router_kernel(const __half* __restric
     }
 }
 
-// One block per token: softmax of the router logits as ops.rs:274-298 writes it (one thread, in order), every expert's rank by
+// One block per token: softmax of the router logits as ops.rs:274-298 writes it (the sum by one thread, in order), every expert's rank by
 // counting (descending probability; equal probabilities by lower id, and the token is flagged: std::sort decides such ties by its
-// algorithm, which the host then runs), the first top_k chosen, their probabilities divided by their sum.
+// algorithm, which the host then runs), the first top_k chosen, their probabilities divided by their sum. Equals that all rank behind the chosen
+// ones (a peaked router leaves many experts exactly zero) do not flag the token: whatever their order, the choice is the same. Only beside a NaN,
+// which has no rank, every tie does.
 __global__ void __launch_bounds__(256) moe_select_kernel(const float* __restrict__ logits, int n_experts, int top_k, float* __restrict__ probs,
                                                          uint32_t* __restrict__ chosen, float* __restrict__ weights, unsigned int* __restrict__ tie) {
     extern __shared__ float p_s[];  // n_experts probabilities, then top_k selected ones
@@ -95,6 +97,7 @@ __global__ void __launch_bounds__(256) moe_select_kernel(const float* __restrict
     if (tid == 0) tie[b] = 0u;
     __syncthreads();
     __shared__ float s_inv, warp_mx[8];
+    __shared__ bool s_nan;
     // The maximum as the reference's loop leaves it (a NaN in the first place stays, others are passed over): any order gives it.
     float mx = -INFINITY;
     for (int i = tid; i < n_experts; i += 256) mx = fmaxf(mx, p_s[i]);
@@ -116,6 +119,7 @@ __global__ void __launch_bounds__(256) moe_select_kernel(const float* __restrict
 #pragma unroll
             for (int k = 0; k < 32; ++k) sum += static_cast<double>(v[k]);
         }
+        s_nan = sum != sum;
         s_inv = sum > 0.0 ? __double2float_rn(1.0 / sum) : 1.0f;
     }
     __syncthreads();
@@ -124,15 +128,17 @@ __global__ void __launch_bounds__(256) moe_select_kernel(const float* __restrict
     for (int i = tid; i < n_experts; i += 256) {
         const float p = p_s[i];
         probs[b * n_experts + i] = p;
-        int rank = 0;
+        int above = 0, equal_before = 0;  // (the first of a group of equals has rank `above`)
         bool tied = false;
 #pragma unroll 16
         for (int j = 0; j < n_experts; ++j) {
             const float q = p_s[j];
-            rank += (q > p || (q == p && j < i)) ? 1 : 0;
+            above += q > p ? 1 : 0;
+            equal_before += q == p && j < i ? 1 : 0;
             tied |= q == p && j != i;
         }
-        if (tied) atomicOr(tie + b, 1u);
+        const int rank = above + equal_before;
+        if (tied && (above < top_k || s_nan)) atomicOr(tie + b, 1u);
         if (rank < top_k) {
             chosen[b * top_k + rank] = static_cast<uint32_t>(i);
             w_s[rank] = p;

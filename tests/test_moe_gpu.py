@@ -83,6 +83,35 @@ def test_the_hosts_order_of_equals_is_what_the_experts_run_with(shard):
         block.free()
 
 
+def test_equal_probabilities_below_the_cut_cost_no_second_pass():
+    """A peaked router leaves many experts a probability of exactly zero. A group of equals that begins at or past rank top_k changes neither the
+    choice nor its order, so the experts run once; one that reaches into the choice sends them through again with the host's order."""
+    hidden, inter, n_experts, top_k = 256, 64, 16, 3
+    rng, _, gu, dn, scales = _block(12, hidden, inter, n_experts)
+    x = np.ones((2, hidden), np.float32)
+
+    def launches(levels):  # the router's rows are constant: logits in the order of `levels`, 256 apart for a step of one
+        r = oracle.f32_to_bf16_bits(np.repeat(np.asarray(levels, np.float32), hidden))
+        block = q.Moe(hidden, inter, top_k, r, gu, dn, scales, max_batch=4)
+        q.launch_count(reset=True)
+        out, ids, w = block.forward(x)
+        n = q.launch_count()
+        for b in range(2):
+            want, want_ids, want_w = omoe.forward(x[b], r, gu, dn, scales, hidden, inter, top_k)
+            assert list(ids[b]) == list(want_ids)
+            assert np.array_equal(w[b].view(np.uint32), want_w.view(np.uint32)) and np.array_equal(out[b].view(np.uint32), want.view(np.uint32))
+        block.free()
+        return n
+
+    level = [-0.01 * i for i in range(n_experts)]  # exp(-2.56 i): all different
+    once = launches(level)
+    assert launches(level[:3] + [-2.0] * 13) == once   # thirteen zeros behind the three chosen
+    assert launches(level[:5] + [level[5]] * 11) == once  # a group that begins at rank 5
+    assert launches(level[:3] + [level[3]] * 13) == once  # exactly at the cut
+    assert launches(level[:2] + [level[2]] * 14) > once  # the third place is one of fourteen equals
+    assert launches([0.0, 0.0] + level[2:]) > once       # the first two are equal: their order is std::sort's
+
+
 def test_arguments():
     rng, router, gu, dn, scales = _block(9, 256, 64, 4)
     with pytest.raises(q.QuintritError) as e:
