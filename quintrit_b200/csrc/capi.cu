@@ -152,7 +152,8 @@ struct GemvKernels { GemvKernel add = nullptr, clear = nullptr; };  // adds to r
 template <uint32_t BASE> GemvKernels gemv_kernels() { return {gemv_lut_kernel<BASE, false>, gemv_lut_kernel<BASE, true>}; }
 
 // Picks the kernel instantiation whose table-base constant equals the shared-window address this device gives to
-// dynamic shared memory (measured once per device with smem_base_kernel).
+// dynamic shared memory (measured once per device with smem_base_kernel). The first time on a device it allocates, waits and loads
+// modules; creating a matrix does that, so that the calls on it are launches only and the first of them can be captured.
 int gemv_kernel_for_device(int dev, GemvKernels* out) {
     static GemvKernels chosen[64];
     static std::mutex lock;  // first calls on a device from several host threads must not race on the cache
@@ -177,7 +178,7 @@ int gemv_kernel_for_device(int dev, GemvKernels* out) {
             default: return fail(QUINTRIT_ERR_DEVICE, "unexpected shared-memory base %u on CUDA device %d: no kernel was built for it", base, dev);
         }
         for (GemvKernel f : {k.add, k.clear}) QTB_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvSmemBytes));
-        cudaFuncAttributes loaded;  // (a kernel is loaded when it is first asked for: here, not in a user's first call)
+        cudaFuncAttributes loaded;  // (a kernel is loaded when it is first asked for)
         QTB_CUDA(cudaFuncGetAttributes(&loaded, zero_kernel));
         chosen[dev] = k;
     }
@@ -479,6 +480,12 @@ extern "C" int quintrit_b200_matrix_upload(uint32_t device_index, int32_t source
         if ((e = cudaMalloc(&m->d_outf, rows * sizeof(float))) != cudaSuccess) return bail(e, "cudaMalloc(results f32)");
         if ((e = cudaMemcpy(m->d_items, items.data(), items.size() * sizeof(GemvItem), cudaMemcpyHostToDevice)) != cudaSuccess) return bail(e, "cudaMemcpy(items)");
         if ((e = cudaMemset(m->d_counters, 0, 4 * sizeof(unsigned int))) != cudaSuccess) return bail(e, "cudaMemset(counters)");
+        GemvKernels kernels;
+        if ((rc = gemv_kernel_for_device(m->device, &kernels)) != QUINTRIT_OK) {
+            destroy_matrix(m);
+            return rc;
+        }
+        if ((e = cudaStreamSynchronize(nullptr)) != cudaSuccess) return bail(e, "set-up");  // (a caller's stream need not wait for the default one)
         *out_matrix = m;
         return ok();
     });
@@ -785,6 +792,7 @@ extern "C" int quintrit_b200_plan_create(const quintrit_b200_matrix_t* const* ma
         for (auto& sg : p->segments)
             if ((e = cudaEventCreateWithFlags(&sg.up, cudaEventDisableTiming)) != cudaSuccess || (e = cudaEventCreateWithFlags(&sg.done, cudaEventDisableTiming)) != cudaSuccess)
                 return bail(e, "cudaEventCreate");
+        if ((e = cudaStreamSynchronize(nullptr)) != cudaSuccess) return bail(e, "set-up");  // (a caller's stream need not wait for the default one)
         *out_plan = p;
         return ok();
     });

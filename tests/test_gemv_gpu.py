@@ -162,3 +162,47 @@ def test_results_are_cleared_at_any_alignment(oracle, rows, shift):
     got = out.cpu().numpy()
     assert np.array_equal(got[shift:shift + rows], trits.astype(np.int32) @ act.astype(np.int32))
     assert np.all(got[:shift] == -7) and np.all(got[shift + rows:] == -7)
+
+
+FIRST_CALL = """
+import numpy as np, torch
+import quintrit_b200 as q
+rows, cols, kind = {rows}, 320, "{kind}"
+rng = np.random.default_rng(1)
+trits = rng.integers(-1, 2, rows * cols).astype(np.int8)
+act = rng.integers(-128, 128, cols).astype(np.int8)
+m = q.Matrix.from_trits(trits, rows, cols)
+plan = q.Plan([m]) if kind == "plan" else None
+x, out = torch.from_numpy(act).cuda(), torch.full((rows,), 7, dtype=torch.int32, device="cuda")
+torch.cuda.synchronize()
+graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+with torch.cuda.graph(graph, stream=side):
+    if plan is not None:
+        plan.launch(side.cuda_stream)
+    else:
+        m.gemv_i32_device(x.data_ptr(), out.data_ptr(), side.cuda_stream)
+want = trits.reshape(rows, cols).astype(np.int64) @ act.astype(np.int64)
+if plan is None:
+    for _ in range(2):
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(out.cpu().numpy(), want)
+else:  # the plan's activations are zeros until a program writes them
+    graph.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(plan.run(plan.pack_activations([act]))[:rows], want)
+del graph
+"""
+
+
+@pytest.mark.parametrize("kind", ["matrix", "plan"])
+@pytest.mark.parametrize("rows", [70, 9000])  # results cleared by the launch itself, and by a launch in front of it
+def test_the_first_call_of_a_process_can_be_captured(rows, kind):
+    """Creating a matrix sets the device up (the kernel for its shared-memory base, module loading): a user's first call is launches and nothing else."""
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", FIRST_CALL.format(rows=rows, kind=kind)], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
