@@ -144,6 +144,7 @@ int quintrit_b200_gemv_f32(const quintrit_b200_matrix_t* matrix, const int8_t* a
 /*
  * The same GEMV on device pointers, enqueued on `stream` (a cudaStream_t, NULL = default stream) without waiting:
  * the device seam of quintrit-cuda/src/gemv.rs:191-226 (Gemv::plain). d_activations: cols int8; d_out: rows int32.
+ * Since it does not wait, a launch that gave up (QUINTRIT_ERR_DEVICE) is reported by the next host-buffer call on the matrix.
  */
 int quintrit_b200_gemv_i32_device(const quintrit_b200_matrix_t* matrix, const int8_t* d_activations, int32_t* d_out, void* stream);
 
@@ -190,7 +191,8 @@ int quintrit_b200_plan_layout(const quintrit_b200_plan_t* plan, size_t index, si
                               size_t* out_act_total, size_t* out_out_total);
 /* Device pointers of the plan's activation (int8) and result (int32) buffers, for callers that fill them on the device. */
 int quintrit_b200_plan_buffers(const quintrit_b200_plan_t* plan, int8_t** out_d_activations, int32_t** out_d_results);
-/* Enqueues result clearing and the persistent GEMV kernel on `stream` (NULL = default); does not wait. */
+/* Enqueues result clearing and the persistent GEMV kernel on `stream` (NULL = default); does not wait (a launch that gave up is
+ * reported by the next quintrit_b200_plan_run). */
 int quintrit_b200_plan_launch(quintrit_b200_plan_t* plan, void* stream);
 /* Host-buffer form: copies `activations` (act_total bytes) in, launches, copies out_total int32 back and waits. */
 int quintrit_b200_plan_run(quintrit_b200_plan_t* plan, const int8_t* activations, size_t activations_len, int32_t* out,
@@ -359,6 +361,12 @@ int quintrit_b200_decoder_trace_step(quintrit_b200_decoder_t* decoder, uint64_t*
  * failure path (expected: ctas). The device stays usable.
  */
 int quintrit_b200_selftest_barrier(uint32_t device_index, uint32_t ctas, uint32_t spin_limit, uint32_t* out_released);
+/*
+ * The same for the wait in the GEMV that clears its own results: a launch in which no block clears them, so that every
+ * block's wait runs out after `spin_limit` polls (1..2^20). Returns QUINTRIT_ERR_DEVICE with the message a host-buffer call
+ * gives for the same condition; *out_kept receives the number of results that no block added to (expected: all 64).
+ */
+int quintrit_b200_selftest_clear(uint32_t device_index, uint32_t spin_limit, uint32_t* out_kept);
 
 /*
  * Prompt ingestion: `count` tokens at positions pos .. pos + count - 1 in chunks of up to 256, every projection of a chunk as one

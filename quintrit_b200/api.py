@@ -134,6 +134,7 @@ def load_library(build_if_missing: bool = True) -> C.CDLL:
     l.quintrit_b200_decoder_time_token.argtypes = [C.c_void_p, C.c_uint32, C.c_uint32, C.POINTER(C.c_float)]
     l.quintrit_b200_decoder_trace_step.argtypes = [C.c_void_p, C.POINTER(C.c_uint64), _sz, C.POINTER(_sz)]
     l.quintrit_b200_selftest_barrier.argtypes = [C.c_uint32, C.c_uint32, C.c_uint32, C.POINTER(C.c_uint32)]
+    l.quintrit_b200_selftest_clear.argtypes = [C.c_uint32, C.c_uint32, C.POINTER(C.c_uint32)]
     l.quintrit_b200_launch_count.restype = C.c_uint64
     l.quintrit_b200_launch_count.argtypes = [C.c_int]
     _lib = l

@@ -147,7 +147,7 @@ void build_items(std::vector<GemvItem>& items, const uint4* w, size_t act_off, s
     }
 }
 
-using GemvKernel = void (*)(const GemvItem*, int, const int8_t*, int32_t*, unsigned int*, int);
+using GemvKernel = void (*)(const GemvItem*, int, const int8_t*, int32_t*, unsigned int*, int, unsigned int);
 struct GemvKernels { GemvKernel add = nullptr, clear = nullptr; };  // adds to results that are cleared; clears them itself
 template <uint32_t BASE> GemvKernels gemv_kernels() { return {gemv_lut_kernel<BASE, false>, gemv_lut_kernel<BASE, true>}; }
 
@@ -187,9 +187,9 @@ int gemv_kernel_for_device(int dev, GemvKernels* out) {
 }
 
 // dependent: the launch before this one in the stream is zero_kernel, which this one need not wait for until it adds. clear: results that the launch
-// clears itself (0: they are cleared).
+// clears itself (0: they are cleared); clear_spins: how long its blocks wait for that.
 int launch_gemv(const GemvItem* d_items, int n_items, const int8_t* d_act, int32_t* d_out, unsigned int* d_counters, int sm_count,
-                cudaStream_t stream, bool dependent = false, int clear = 0) {
+                cudaStream_t stream, bool dependent = false, int clear = 0, unsigned int clear_spins = kClearSpins) {
     int dev = 0;
     QTB_CUDA(cudaGetDevice(&dev));
     GemvKernels ks;
@@ -202,7 +202,7 @@ int launch_gemv(const GemvItem* d_items, int n_items, const int8_t* d_act, int32
     cfg.gridDim = dim3(grid), cfg.blockDim = dim3(kGemvThreads), cfg.dynamicSmemBytes = kGemvSmemBytes, cfg.stream = stream;
     cfg.attrs = &attr, cfg.numAttrs = dependent ? 1 : 0;
     ++g_launches;
-    QTB_CUDA(cudaLaunchKernelEx(&cfg, clear > 0 ? ks.clear : ks.add, d_items, n_items, d_act, d_out, d_counters, clear));
+    QTB_CUDA(cudaLaunchKernelEx(&cfg, clear > 0 ? ks.clear : ks.add, d_items, n_items, d_act, d_out, d_counters, clear, clear_spins));
     return QUINTRIT_OK;
 }
 
@@ -215,12 +215,20 @@ int launch_gemv_cleared(const GemvItem* d_items, int n_items, const int8_t* d_ac
     return launch_gemv(d_items, n_items, d_act, d_out, d_counters, sm_count, stream, true);
 }
 
-// After a synchronisation: did the kernel refuse to run because its table-base constant was wrong?
-int check_kernel_status(unsigned int* d_counters) {
-    unsigned int flag = 0;
-    QTB_CUDA(cudaMemcpy(&flag, d_counters + 2, sizeof flag, cudaMemcpyDeviceToHost));
+// The status word of the GEMV kernel (d_counters[2]) as an error of the C ABI. A wait that ran out belongs to a launch that is over: the word is
+// cleared, so that the matrix or plan stays usable. It may be the word of an earlier launch on device buffers, which did not wait and look.
+int gemv_status_error(unsigned int flag, unsigned int* d_counters) {
+    if (flag == kGemvStatusClear) {
+        QTB_CUDA(cudaMemset(d_counters + 2, 0, sizeof(unsigned int)));
+        return fail(QUINTRIT_ERR_DEVICE, "the GEMV kernel on the CUDA device gave up waiting for its results to be cleared (this call or an earlier one on device buffers)");
+    }
     if (flag != 0) return fail(QUINTRIT_ERR_DEVICE, "GEMV kernel on the CUDA device found its shared-memory table at an unexpected address");
     return QUINTRIT_OK;
+}
+int check_kernel_status(unsigned int* d_counters) {  // after a synchronisation
+    unsigned int flag = 0;
+    QTB_CUDA(cudaMemcpy(&flag, d_counters + 2, sizeof flag, cudaMemcpyDeviceToHost));
+    return gemv_status_error(flag, d_counters);
 }
 
 struct DeviceGuard {
@@ -873,8 +881,8 @@ extern "C" int quintrit_b200_plan_run(quintrit_b200_plan_t* plan, const int8_t* 
         QTB_CUDA(cudaMemcpyAsync(&flag, plan->d_counters + 2, sizeof flag, cudaMemcpyDeviceToHost, plan->s_copy));
         QTB_CUDA(cudaStreamSynchronize(plan->s_copy));
         QTB_CUDA(cudaStreamSynchronize(plan->s_run));
-        if (flag != 0) return fail(QUINTRIT_ERR_DEVICE, "GEMV kernel on the CUDA device found its shared-memory table at an unexpected address");
-        return ok();
+        rc = gemv_status_error(flag, plan->d_counters);
+        return rc == QUINTRIT_OK ? ok() : rc;
     });
 }
 
@@ -2047,7 +2055,7 @@ extern "C" int quintrit_b200_gemv_i32_noalloc(const quintrit_b200_matrix_t* matr
         const int grid = static_cast<int>(std::max<size_t>(1, std::min(n_items, slots)));
         s->kernel<<<grid, kGemvThreads, kGemvSmemBytes, st>>>(reinterpret_cast<const GemvItem*>(s->scratch + kNoAllocHeaderBytes),
                                                              static_cast<int>(n_items), d_activations, d_out,
-                                                             reinterpret_cast<unsigned int*>(s->scratch), 0);
+                                                             reinterpret_cast<unsigned int*>(s->scratch), 0, 0u);
         ++g_launches;
         QTB_CUDA(cudaGetLastError());
         return ok();
@@ -2081,6 +2089,35 @@ extern "C" int quintrit_b200_selftest_barrier(uint32_t device_index, uint32_t ct
         if (e != cudaSuccess) return cuda_fail(e, "barrier self-test");
         for (uint32_t i = 0; i < ctas; ++i) *out_released += host[17 + i];
         rc = kernel_status_error(host[16]);
+        return rc == QUINTRIT_OK ? ok() : rc;
+    });
+}
+
+// Runs the self-clearing GEMV with the first ticket gone, so that no block clears the results: every wait runs out after `spin_limit` polls.
+// Expected outcome: QUINTRIT_ERR_DEVICE ("gave up waiting for its results") and *out_kept == 64, i.e. no block added to what it found.
+extern "C" int quintrit_b200_selftest_clear(uint32_t device_index, uint32_t spin_limit, uint32_t* out_kept) {
+    return guard([&]() -> int {
+        if (out_kept == nullptr) return fail(QUINTRIT_ERR_NULL_POINTER, "out_kept is NULL");
+        *out_kept = 0;
+        if (spin_limit == 0 || spin_limit > kClearSpins) return fail(QUINTRIT_ERR_INVALID_ARGUMENT, "spin_limit must be 1..2^20 polls");
+        constexpr size_t kRows = 64, kCols = 800;
+        const std::vector<uint8_t> planar(kRows * quintrit_b200_planar_row_bytes(kCols), uint8_t(250));  // every trit +1
+        const std::vector<int8_t> act(kCols, int8_t(1));
+        quintrit_b200_matrix* m = nullptr;
+        int rc = quintrit_b200_matrix_upload(device_index, kSrcPlanar, planar.data(), planar.size(), kRows, kCols, &m);
+        if (rc != QUINTRIT_OK) return rc;
+        DeviceGuard g(m->device);
+        const unsigned int taken = 1;
+        std::vector<int32_t> out(kRows);
+        cudaError_t e = cudaMemcpy(m->d_act, act.data(), kCols, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy(m->d_counters + 3, &taken, sizeof taken, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemset(m->d_out, 0x55, kRows * sizeof(int32_t));
+        if (e == cudaSuccess) rc = launch_gemv(m->d_items, m->n_items, m->d_act, m->d_out, m->d_counters, m->sm_count, nullptr, false, static_cast<int>(kRows), spin_limit);
+        if (e == cudaSuccess && rc == QUINTRIT_OK) e = cudaMemcpy(out.data(), m->d_out, kRows * sizeof(int32_t), cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess) rc = cuda_fail(e, "self-test of the clearing");
+        if (rc == QUINTRIT_OK) rc = check_kernel_status(m->d_counters);
+        for (int32_t v : out) *out_kept += v == 0x55555555 ? 1u : 0u;
+        destroy_matrix(m);
         return rc == QUINTRIT_OK ? ok() : rc;
     });
 }

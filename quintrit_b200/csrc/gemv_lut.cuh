@@ -253,18 +253,21 @@ __device__ __forceinline__ void unpack_acts(const PackedActs& p, int a[5]) {
 // CLEAR: the launch clears its `out_count` results itself. The CTA that draws the first ticket does it (it runs, whatever the others do) while the
 // others bring their weights and build their first table; they look at the flag it sets before they add. That saves a launch (1024 to 3072
 // results: 11.9 -> 8.9 us a call); past kSelfClearMax one CTA takes longer than the launch of zero_kernel (23040 results: 13.5 against 12.9 us). counters[3]: tickets in the low half, the flag on top.
+// The wait for the flag is bounded (`clear_spins` polls, about a second): a CTA whose wait runs out says so in counters[2] and leaves without
+// adding anything.
 constexpr int kSelfClearMax = 8192;
-constexpr unsigned int kClearedBit = 0x80000000u, kClearSpins = 1u << 24;
+constexpr unsigned int kClearedBit = 0x80000000u, kClearSpins = 1u << 20;
+constexpr unsigned int kGemvStatusBase = 1, kGemvStatusClear = 5;  // counters[2]: table base, wait for the clearing (2 to 4: other kernels' time-outs)
 template <uint32_t BASE, bool CLEAR>
 __global__ void __launch_bounds__(kGemvThreads, kCtasPerSm)
 gemv_lut_kernel(const GemvItem* __restrict__ items, int n_items, const int8_t* __restrict__ act_base, int32_t* __restrict__ out_base,
-                unsigned int* __restrict__ counters, int out_count) {
+                unsigned int* __restrict__ counters, int out_count, unsigned int clear_spins) {
     extern __shared__ __align__(1024) int tab[];
     GemvItem* s_items = reinterpret_cast<GemvItem*>(reinterpret_cast<char*>(tab) + kTableBytes);
     int* s_idx = reinterpret_cast<int*>(reinterpret_cast<char*>(tab) + kTableBytes + 4 * sizeof(GemvItem));
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (static_cast<uint32_t>(__cvta_generic_to_shared(tab)) != BASE) {
-        if (tid == 0) atomicExch(&counters[2], 1u);
+        if (tid == 0) atomicExch(&counters[2], kGemvStatusBase);
         return;
     }
 
@@ -364,13 +367,18 @@ gemv_lut_kernel(const GemvItem* __restrict__ items, int n_items, const int8_t* _
         __syncthreads();
         if (!CLEAR && i == 0) asm volatile("griddepcontrol.wait;" ::: "memory");  // the results are cleared (zero_kernel, where this launch depends on it)
         if (CLEAR && i == 0) {
+            bool late = false;
             if (tid == 0) {
                 unsigned int seen = 0, spins = 0;
                 do asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counters + 3) : "memory");
-                while ((seen & kClearedBit) == 0 && ++spins < kClearSpins);
-                if ((seen & kClearedBit) == 0) atomicExch(&counters[2], 1u);
+                while ((seen & kClearedBit) == 0 && ++spins < clear_spins);
+                late = (seen & kClearedBit) == 0;
+                if (late) atomicExch(&counters[2], kGemvStatusClear);
             }
-            __syncthreads();
+            if (__syncthreads_or(late)) {
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                break;
+            }
         }
 
         int t = warp;

@@ -164,6 +164,19 @@ def test_results_are_cleared_at_any_alignment(oracle, rows, shift):
     assert np.all(got[:shift] == -7) and np.all(got[shift + rows:] == -7)
 
 
+def test_a_wait_for_cleared_results_that_runs_out_adds_nothing_and_says_so(oracle):
+    """A launch that clears its own results, with the ticket of the block that does so gone: every block's bounded wait runs out."""
+    kept = C.c_uint32(0)
+    lib = q.load_library()
+    assert lib.quintrit_b200_selftest_clear(0, 2000, C.byref(kept)) == 15
+    assert b"gave up waiting for its results" in lib.quintrit_last_error_message()
+    assert kept.value == 64  # what lay in the result buffer is still there
+    rng = np.random.default_rng(2)
+    trits, act = rng.integers(-1, 2, 40 * 320).astype(np.int8), rng.integers(-128, 128, 320).astype(np.int8)
+    m = q.Matrix.from_trits(trits, 40, 320)  # the device stays usable
+    assert np.array_equal(m.gemv_i32(act).astype(np.int64), oracle.gemv_bruteforce(trits, 40, 320, act))
+
+
 FIRST_CALL = """
 import numpy as np, torch
 import quintrit_b200 as q
