@@ -1143,7 +1143,7 @@ int decoder_create_impl(const quintrit_b200_decoder_desc_t* desc, quintrit_b200_
                  d->kv_heads * (hd / kV2Dims) < static_cast<uint32_t>(d->sm_count);  // some CTAs must stay free to compute the softmax factors
     if (const char* v2 = std::getenv("QUINTRIT_B200_ATTN_V2")) d->attn_v2 = d->attn_v2 && v2[0] != '0';  // experiments: "0" keeps the first form
     auto bytes_for = [&](bool v2) {
-        return mega_smem_bytes(mega_attn_region(d->ctx, gqa_n, hd, v2), static_cast<int>(std::max<size_t>(H, qd_full)), static_cast<int>(H), static_cast<int>(L));
+        return mega_smem_bytes(mega_attn_region(d->ctx, gqa_n, hd, H, v2), static_cast<int>(std::max<size_t>(H, qd_full)), static_cast<int>(H), static_cast<int>(L));
     };
     if (d->attn_v2 && bytes_for(true) > static_cast<size_t>(smem_optin)) d->attn_v2 = false;
     const size_t mega_bytes = bytes_for(d->attn_v2);
@@ -1251,7 +1251,7 @@ int mega_setup(quintrit_b200_decoder* d, const quintrit_b200_decoder_desc_t* des
     a.xa = d->xa, a.xb = d->xb;
     a.acc_qkv = d->acc_qkv, a.acc_o = d->acc_o, a.acc_gu = d->acc_gu, a.acc_down = d->acc_down;
     a.v_inter = d->v_inter, a.amax_bits = d->amax_bits, a.part_acc = d->part_acc, a.part_ms = d->part_ms, a.logits = d->logits;
-    a.scores = d->scores, a.attn_region = static_cast<unsigned int>(mega_attn_region(d->ctx, d->q_heads / d->kv_heads, d->head_dim, d->attn_v2));
+    a.scores = d->scores, a.attn_region = static_cast<unsigned int>(mega_attn_region(d->ctx, d->q_heads / d->kv_heads, d->head_dim, d->hidden, d->attn_v2));
     a.attn_v2 = d->attn_v2 ? 1 : 0, a.attn_out = d->attn_out;
     a.fac = d->fac, a.fac_flags = d->fac_flags, a.fac_M = d->fac_M, a.fac_done = d->fac_done, a.fac_stride = fac_stride;
     a.bf16_tables = d->bf16_tables ? 1 : 0;

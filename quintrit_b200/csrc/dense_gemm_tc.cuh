@@ -8,8 +8,8 @@
 // that are at work together share weight rows.
 //
 // The dual form makes two products of one tile, W_o y and W_down m, in two accumulators and ends with both gates and the residual sum. Its rows are
-// only the model's width, so its tiles are few and long. 2048 tokens, 2048 rows, K = 4096 + 5632: 256 tiles of 128 tokens are two waves of which the
-// second is half empty, 110 us; 128 tiles of 256 tokens, with one set of accumulators, 75 us.
+// only the model's width, so its tiles are few and long. 2048 tokens, 2048 rows, K = 4096 + 5632: 256 tiles of 128 tokens are two waves on 148
+// multiprocessors, the second a quarter empty, 110 us; 128 tiles of 256 tokens are one wave, with one set of accumulators, 75 us.
 // The grouped form multiplies runs of consecutive activation rows, each with its own range of weight rows (the experts of a mixture); which
 // runs there are is read from device memory.
 // Every wait is bounded, as in gemm_tc.cuh, whose mbarrier, descriptor and status conventions are used here.

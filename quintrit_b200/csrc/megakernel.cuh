@@ -1238,13 +1238,17 @@ __device__ __noinline__ void mega_values2_unit(const MegaArgs& a, const MegaLaye
 
 // Shared-memory plan of the token kernel (bytes from the dynamic base): attention region (its first 64 KiB double as the
 // GEMV table) | y (floats) | a8 | small. The attention region holds whichever is largest: a scores unit (staged key block,
-// the group's queries, the new key/value rows), a values unit for the longest chunk, or the lm_head rings.
-__host__ __device__ constexpr size_t mega_attn_region(int ctx, int gqa, int head_dim, bool v2) {
+// the group's queries, the new key/value rows), a values unit for the longest chunk, or the output head's activations (floats).
+// It is never smaller than kMegaRegionMin, which together with the vectors behind it decides which models take this kernel: wider ones
+// (past 8 to 9 thousand values) have not been run through it and take one kernel per step.
+constexpr size_t kMegaRegionMin = 129 * 1024;
+__host__ __device__ constexpr size_t mega_attn_region(int ctx, int gqa, int head_dim, int hidden, bool v2) {
     const int len_max = ctx < 512 ? ctx : (ctx + 3) / 4;
     size_t need = static_cast<size_t>(kAttnBlockBytes) + static_cast<size_t>(gqa) * head_dim * 4 + static_cast<size_t>(head_dim) * 4 + 64;
-    const size_t vals = v2 ? values2_bytes(ctx, gqa) : values_unit_bytes(len_max, gqa), head = static_cast<size_t>(kMegaWarps) * 4 * 1024 * 2 + 1024;
+    const size_t vals = v2 ? values2_bytes(ctx, gqa) : values_unit_bytes(len_max, gqa), head = static_cast<size_t>(hidden) * 4;
     if (vals > need) need = vals;
     if (head > need) need = head;
+    if (kMegaRegionMin > need) need = kMegaRegionMin;
     return (need + 1023) / 1024 * 1024;
 }
 // After the small arrays: the norm weights of the next norm (hidden floats) and a copy of every layer's descriptor.
