@@ -1078,7 +1078,8 @@ int decoder_create_impl(const quintrit_b200_decoder_desc_t* desc, quintrit_b200_
     if ((rc = allow_max_dynamic_smem(norm_quant_kernel, smem_optin)) != QUINTRIT_OK) return rc;
     if ((rc = allow_max_dynamic_smem(attn_finish_kernel, smem_optin)) != QUINTRIT_OK) return rc;
     if ((rc = allow_max_dynamic_smem(act_quant_kernel, smem_optin)) != QUINTRIT_OK) return rc;
-    if ((rc = allow_max_dynamic_smem(lm_head_kernel<false>, smem_optin)) != QUINTRIT_OK || (rc = allow_max_dynamic_smem(lm_head_kernel<true>, smem_optin)) != QUINTRIT_OK) return rc;
+    for (bool few : {false, true})
+        if ((rc = allow_max_dynamic_smem(lm_head_for(few, d->bf16_tables), smem_optin)) != QUINTRIT_OK) return rc;
     if ((rc = allow_max_dynamic_smem(attention_kernel, smem_optin)) != QUINTRIT_OK) return rc;
     if (block_scaled) {  // no work items: the block-scaled projections are plain launches; one kernel per step
         QTB_CUDA(block_scaled_allow_smem());

@@ -1810,6 +1810,42 @@ __device__ __forceinline__ void head_rows(const MegaArgs& a, const float* xs, fl
     }
 }
 
+// The same with sixteen threads to a row, as lm_head_few_kernel computes them, sixteen loads ahead of the sixteen at work: where a warp has at most
+// kHeadFew rows, the waits of a long row are what takes the time. Out of line, so that the registers of the form above stay its own. One layer of width
+// 8192, 4000 rows (two a warp): 157 -> 143 us a token (149 with the ring of copies); of width 4096, 8000 rows 119 -> 114, 9400 rows (four a warp) no
+// difference, which is where the line lies.
+constexpr int kHeadFew = 4;
+template <bool BF16>
+__device__ __noinline__ void head_rows_few(const MegaArgs& a, const float* xs, float& bv, unsigned int& bi) {
+    constexpr int kAhead = 16;
+    const int lane = threadIdx.x & 31, part = lane & 15, H = a.hidden, steps = H / 32;
+    const int warp = blockIdx.x * kMegaWarps + (threadIdx.x >> 5), warps = gridDim.x * kMegaWarps;
+    const int begin = static_cast<int>(static_cast<long long>(a.vocab) * warp / warps), end = static_cast<int>(static_cast<long long>(a.vocab) * (warp + 1) / warps);
+    const unsigned long long* xr = reinterpret_cast<const unsigned long long*>(xs) + part;
+    for (int row0 = begin; row0 < end; row0 += 2) {
+        const int row = row0 + (lane >> 4);
+        const uint32_t* wr = reinterpret_cast<const uint32_t*>(a.lm_head + static_cast<size_t>(min(row, end - 1)) * H) + part;
+        unsigned long long acc = 0ull;
+        uint32_t now[kAhead], next[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) now[k] = k < steps ? __ldg(wr + k * 16) : 0u;
+        for (int i = 0; i < steps; i += kAhead) {
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) next[k] = i + kAhead + k < steps ? __ldg(wr + (i + kAhead + k) * 16) : 0u;
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) {
+                if (i + k < steps) acc = head_step<BF16>(head_widen<BF16>(now[k]), xr[(i + k) * 16], acc);
+                now[k] = next[k];
+            }
+        }
+        const float sum = head_few_sum<BF16>(acc);
+        if (part == 0 && row < end) {
+            a.logits[row] = sum;
+            argmax_merge(bv, bi, sum, static_cast<unsigned int>(row + a.vocab_base));
+        }
+    }
+}
+
 // Final norm (model.rs:326-331), output head, greedy candidate of this CTA.
 __device__ __noinline__ bool phase_head(const MegaArgs& a, unsigned int seq_base, unsigned char* smem) {
     const MegaSmem v = mega_smem_views(smem, a);
@@ -1834,8 +1870,13 @@ __device__ __noinline__ bool phase_head(const MegaArgs& a, unsigned int seq_base
     __syncthreads();
     float bv = -INFINITY;
     unsigned int bi = 0xFFFFFFFFu;
-    if (bf16) head_rows<true>(a, xs, bv, bi);
-    else head_rows<false>(a, xs, bv, bi);
+    if (a.vocab <= kHeadFew * G * kMegaWarps) {
+        if (bf16) head_rows_few<true>(a, xs, bv, bi);
+        else head_rows_few<false>(a, xs, bv, bi);
+    } else {
+        if (bf16) head_rows<true>(a, xs, bv, bi);
+        else head_rows<false>(a, xs, bv, bi);
+    }
     for (int o = 4; o < 32; o <<= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
         argmax_merge(bv, bi, ov, __shfl_xor_sync(0xffffffffu, bi, o));
