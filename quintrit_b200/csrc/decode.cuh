@@ -1116,8 +1116,9 @@ inline void launch_lm_head(const __half* w, const __half* x16, int hidden, int v
 // asynchronous copies, and a row is read from HBM once for 32 tokens. Sixteen threads share the accumulator lanes of a dot
 // product (two each, packed); a thread holds eight rows times eight tokens, so a row element and an activation loaded and
 // widened serve eight operations each. The eight warps are spread over the groups of eight tokens that there are (TG = 1, 2 or
-// 4) and, with the rest, over rows: 16 rows a warp. The lanes are added by halving exchanges. Bound by issue slots:
-// 1.75 per packed operation (32 tokens x 32768 x 3072: 226 us by ncu; two warps a scheduler waiting for 64-byte loads: about 330).
+// 4) and, with the rest, over rows: 16 rows a warp. The lanes are added by halving exchanges. Bound by the
+// heavy half of the FMA pipe, which takes conversions beside its share of the packed operations (ncu, 32 tokens x 32768 x 3072: 229 us, that pipe 66 % busy,
+// issue slots 47 %, 2.4 instructions per packed operation; two warps a scheduler waiting for 64-byte loads: about 330 us).
 constexpr int kHeadThreads = 256, kHeadCols = 128, kHeadTokens = 8;
 constexpr int kHeadRowStride = kHeadCols * 2 + 64;  // bytes: the rows of a warp's two halves are neighbours, half the banks apart
 __host__ __device__ constexpr int head_tile_rows(int tg) { return 16 * (kHeadThreads / 32 / tg); }

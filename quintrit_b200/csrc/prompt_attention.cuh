@@ -9,9 +9,10 @@
 //  B. a warp turns its own token's scores into the factors ms / vs with a warp scan;
 //  C. the same warp runs all value chains of its token: a lane owns head_dim / 32 coordinates, two to a packed operation
 //     (fma.rn.f32x2 rounds each half on its own; one conversion rounds both accumulators to F16).
-// Bound by instruction issue and, in C, by the pipe that converts between F16 and F32 (ncu: 54 % of the issue slots and 57 % of that pipe's at
-// 12 / 4 heads of 256 and two blocks a multiprocessor): about 9 slots per score, 22 per head, position and 8 coordinates. The 1000-token
-// prompt of a 4-layer Falcon3-10B shape: 8.03 -> 6.11 ms against a block per token (attention_gqa_kernel).
+// Bound by instruction issue and, in C, by the heavy half of the FMA pipe, which converts between F16 and F32 (ncu, 232 tokens at positions 768 to 999, 12 /
+// 4 heads of 256: 201 us, while a multiprocessor is active 54 % of the issue slots and 58 % of that pipe; 40 warp instructions per token, head and
+// position with the tiles' overhang, of which the source has 9 in a score and 22 in the chains). The 1000-token prompt of a 4-layer Falcon3-10B shape:
+// 8.03 -> 6.11 ms against a block per token (attention_gqa_kernel).
 #pragma once
 #include "decode.cuh"
 #include "packed_f32.cuh"
