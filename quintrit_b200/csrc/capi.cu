@@ -42,8 +42,7 @@ struct quintrit_b200_matrix {
     float* d_as = nullptr;   // cols / 32 activation block scales
     // batched projection on the tensor cores (gemm_tc.cuh): two-bit block-major copy of the weights and call buffers, made on first use
     uint8_t* d_gemm_w = nullptr;
-    size_t gemm_rows_padded = 0;
-    int8_t* d_gemm_act = nullptr;     // kGemmMaxN x whole 128-column blocks, zero padded
+    int8_t* d_gemm_act = nullptr;     // kGemmMaxN x whole stages of 256 columns, zero padded
     int8_t* d_gemm_in = nullptr;      // host-call staging: kGemmMaxN x cols
     int32_t* d_gemm_out = nullptr;    // host-call staging: kGemmMaxN x rows
     unsigned int* d_gemm_status = nullptr;
@@ -2161,18 +2160,25 @@ namespace {
 std::mutex g_gemm_lock;
 constexpr int kGemmMaxParts = kAccPartsMax;
 constexpr size_t kGemmSmemLimit = 227 * 1024;  // dynamic shared memory a CTA may ask for on this device
+// Writes a matrix into a two-bit copy from row tile `tile0` on; the copy's bytes are 0x55 (on the default stream, before).
+cudaError_t gemm_copy_weights(const quintrit_b200_matrix* m, uint8_t* copy, int tile0) {
+    const size_t warps = size_t(m->blocks) * m->tiles;
+    stream_to_two_bit_kernel<<<static_cast<int>(std::min<size_t>((warps + 7) / 8, size_t(m->sm_count) * 16)), 256>>>(
+        m->d_w, reinterpret_cast<uint32_t*>(copy), static_cast<int>(m->rows), static_cast<int>(m->cols), static_cast<int>(gemm_blocks(m->cols)) * (kGemmStageCols / 64),
+        static_cast<int>(m->blocks), static_cast<int>(m->tiles), tile0);
+    ++g_launches;
+    return cudaGetLastError();
+}
 // Makes the two-bit copy of the weights and the call buffers of a matrix the first time it is used by the batched projection.
 int gemm_prepare(quintrit_b200_matrix* m) {
     std::lock_guard<std::mutex> hold(g_gemm_lock);
     if (m->d_gemm_w != nullptr) return QUINTRIT_OK;
     if (m->block_scaled) return fail(QUINTRIT_ERR_UNSUPPORTED, "the batched projection takes per-tensor ternary matrices, not block-scaled (Q2_0) ones");
-    const size_t rows_padded = (m->rows + kGemmM - 1) / kGemmM * kGemmM, gblocks = (m->cols + kGemmBlockCols - 1) / kGemmBlockCols, k_pad = gblocks * kGemmBlockCols;
+    const size_t gblocks = gemm_blocks(m->cols), k_pad = gblocks * kGemmStageCols, bytes = gemm_copy_bytes(m->rows, m->cols);
     uint8_t* w = nullptr;
-    QTB_CUDA(cudaMalloc(&w, gblocks * rows_padded * 32));
-    const size_t bytes = gblocks * rows_padded * 32;
-    stream_to_two_bit_kernel<<<static_cast<int>(std::min<size_t>((bytes + 255) / 256, 148 * 32)), 256>>>(m->d_w, w, m->rows, m->cols, rows_padded, gblocks, m->blocks, m->tiles, 0, rows_padded);
-    ++g_launches;
-    cudaError_t e = cudaGetLastError();
+    QTB_CUDA(cudaMalloc(&w, bytes));
+    cudaError_t e = cudaMemsetAsync(w, 0x55, bytes, nullptr);
+    if (e == cudaSuccess) e = gemm_copy_weights(m, w, 0);
     if (e == cudaSuccess) e = cudaMalloc(&m->d_gemm_act, size_t(kGemmMaxN) * k_pad);
     if (e == cudaSuccess) e = cudaMalloc(&m->d_gemm_status, 4096);  // the status word; the rest is used by debug builds only
     if (e == cudaSuccess) e = cudaMemset(m->d_gemm_status, 0, 4096);
@@ -2182,7 +2188,6 @@ int gemm_prepare(quintrit_b200_matrix* m) {
         cudaFree(w);
         return cuda_fail(e, "set-up of the batched projection");
     }
-    m->gemm_rows_padded = rows_padded;
     m->d_gemm_w = w;
     return QUINTRIT_OK;
 }
@@ -2199,11 +2204,11 @@ int gemm_launch(quintrit_b200_matrix* m, const int8_t* d_act, int batch, int32_t
     TensorMapEncodeFn encode = nullptr;
     int rc = tensor_map_encoder(&encode);
     if (rc != QUINTRIT_OK) return rc;
-    const int gblocks = static_cast<int>((m->cols + kGemmBlockCols - 1) / kGemmBlockCols);
-    const int n = std::max(16, (batch + 15) / 16 * 16), k_pad = gblocks * kGemmBlockCols;
+    const int gblocks = static_cast<int>(gemm_blocks(m->cols));
+    const int n = (batch + 31) / 32 * 32, k_pad = gblocks * kGemmStageCols;  // the pair's instruction takes multiples of 32
     // The TMA reads the caller's vectors in place when their pitch and address allow it (columns and vectors beyond the matrix read as zeros);
-    // otherwise they are first copied into a zero-padded matrix with a pitch of whole blocks.
-    const bool in_place = m->cols % 32 == 0 && reinterpret_cast<uintptr_t>(d_act) % 16 == 0;
+    // otherwise they are first copied into a zero-padded matrix with a pitch of whole stages.
+    const bool in_place = m->cols % 16 == 0 && reinterpret_cast<uintptr_t>(d_act) % 16 == 0;
     const void* base = d_act;
     cuuint64_t pitch = m->cols, vectors = static_cast<cuuint64_t>(batch);
     if (!in_place) {
@@ -2211,37 +2216,36 @@ int gemm_launch(quintrit_b200_matrix* m, const int8_t* d_act, int batch, int32_t
         ++g_launches;
         base = m->d_gemm_act, pitch = static_cast<cuuint64_t>(k_pad), vectors = static_cast<cuuint64_t>(n);
     }
-    // the activations as a 3-D tensor: 32 bytes of a K tile, the vectors, the K tiles of a vector; a box is 32 x n x 4 (the four tiles of a block)
+    // a box is half a stage of half the vectors: 128 bytes x n / 2
     CUtensorMap map;
-    const cuuint64_t dims[3] = {32, vectors, pitch / 32};
-    const cuuint64_t strides[2] = {pitch, 32};  // bytes between vectors and between K tiles: multiples of 16
-    const cuuint32_t box[3] = {32, static_cast<cuuint32_t>(n), 4}, elem[3] = {1, 1, 1};
-    const CUresult cr = encode(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B,
+    const cuuint64_t dims[2] = {pitch, vectors}, strides[1] = {pitch};
+    const cuuint32_t box[2] = {128, static_cast<cuuint32_t>(n / 2)}, elem[2] = {1, 1};
+    const CUresult cr = encode(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (cr != CUDA_SUCCESS) return fail(QUINTRIT_ERR_DEVICE, "cuTensorMapEncodeTiled failed with CUDA driver error %d", static_cast<int>(cr));
     GemmArgs a;
     a.w = m->d_gemm_w, a.out = d_out, a.status = status != nullptr ? status : m->d_gemm_status;
-    a.rows = static_cast<int>(m->rows), a.rows_padded = static_cast<int>(m->gemm_rows_padded), a.blocks = gblocks;
+    a.rows = static_cast<int>(m->rows), a.pairs = static_cast<int>(gemm_row_tiles(m->rows) / 2), a.blocks = gblocks;
     a.n = n, a.batch = batch, a.ldo = ldo;
     a.stages = gemm_stages_for(n, kGemmSmemLimit);
-    if (const char* v = std::getenv("QUINTRIT_B200_GEMM_STAGES")) a.stages = std::max(2, std::min(std::atoi(v), a.stages));  // experiments: fewer stages (at least two: see the decode groups)
+    if (const char* v = std::getenv("QUINTRIT_B200_GEMM_STAGES")) a.stages = std::max(kGemmGroups, std::min(std::atoi(v), a.stages));  // experiments: fewer stages (one a decode group at least)
     a.spin_limit = 1u << 16;  // polls of up to 20 us each: about a second before a wait gives up
-    // Work items are (row tile, K part); K is split (at least four blocks a part, at most kGemmMaxParts parts) where the items of whole tiles would
-    // leave SMs idle: the cost of a split is the largest number of items an SM gets times the blocks of an item plus about one block for its
-    // epilogue, plus the pass that adds the parts (its bytes at about 3 TB/s against 0.4 us a block).
-    const int m_tiles = a.rows_padded / kGemmM;
+    // Work items are (pair of row tiles, K part); K is split (at most kGemmMaxParts parts) where the items of whole rows would leave multiprocessors idle: the cost of a split, in
+    // cycles, is the largest number of items a pair gets times (the stages of an item at four cycles a vector, or what handing them on takes, plus an end), plus the
+    // bytes of the partial sums, written here and read by the consumer, at about 4 TB/s.
+    const int sm_pairs = m->sm_count / 2;
+    const long stage = std::max(4 * n + 36, 700), end = 2000 + 16 * n;
     int ksplit = 1;
     long best = -1;
-    for (int ks = 1; ks <= std::min(kGemmMaxParts, std::max(1, a.blocks / 4)); ++ks) {
+    for (int ks = 1; ks <= std::min(kGemmMaxParts, a.blocks); ++ks) {
         const int per = (a.blocks + ks - 1) / ks, parts = (a.blocks + per - 1) / per;
-        const long waves = (long(m_tiles) * parts + m->sm_count - 1) / m->sm_count;
-        const long add_pass = parts > 1 ? long((parts + 1) * double(batch) * double(m->rows) * 4.0 / 1.2e6) + 3 : 0;  // bytes the second kernel moves, in units of a block's time
-        const long cost = waves * (per + 1) + add_pass;
+        const long waves = (long(a.pairs) * parts + sm_pairs - 1) / sm_pairs;
+        const long cost = waves * (per * stage + end) + (parts > 1 ? static_cast<long>(2.0 * parts * double(batch) * double(m->rows) * 4.0 / 2160.0) : 0);
         if (best < 0 || cost < best) best = cost, ksplit = parts;
     }
     if (const char* v = std::getenv("QUINTRIT_B200_GEMM_KSPLIT")) ksplit = std::max(1, std::min({std::atoi(v), a.blocks, kGemmMaxParts}));
-    a.blocks_per_cta = (a.blocks + ksplit - 1) / ksplit;
-    ksplit = (a.blocks + a.blocks_per_cta - 1) / a.blocks_per_cta;
+    a.blocks_per_item = (a.blocks + ksplit - 1) / ksplit;
+    ksplit = (a.blocks + a.blocks_per_item - 1) / a.blocks_per_item;
     if (ksplit > 1) {
         if (parts == nullptr) {
             if (m->d_gemm_parts == nullptr) {
@@ -2252,7 +2256,7 @@ int gemm_launch(quintrit_b200_matrix* m, const int8_t* d_act, int batch, int32_t
         }
         a.out = parts, a.ldo = static_cast<int>(m->rows);
     }
-    gemm_i8_tcgen05_kernel<<<std::min(m_tiles * ksplit, m->sm_count), kGemmThreads, gemm_smem_bytes(n, a.stages), stream>>>(map, a);
+    gemm_i8_tcgen05_kernel<<<2 * std::min(a.pairs * ksplit, sm_pairs), kGemmThreads, gemm_smem_bytes(n, a.stages), stream>>>(map, a);
     ++g_launches;
     if (ksplit > 1 && defer != nullptr) {
         *defer = AccView{parts, ksplit, size_t(batch) * m->rows, static_cast<int>(m->rows)};
@@ -2352,24 +2356,20 @@ int decoder_gemm_prepare(quintrit_b200_decoder* d) {
             rows += m->rows;
         }
         const quintrit_b200_matrix* m0 = mat(l, first);
-        const size_t gblocks = (m0->cols + kGemmBlockCols - 1) / kGemmBlockCols;
         uint8_t* w = nullptr;
-        int r = dev_alloc(d, &w, gblocks * rows * 32, false);
+        int r = dev_alloc(d, &w, gemm_copy_bytes(rows, m0->cols), false);
         if (r != QUINTRIT_OK) return r;
-        size_t off = 0;
+        QTB_CUDA(cudaMemsetAsync(w, 0x55, gemm_copy_bytes(rows, m0->cols), nullptr));
+        size_t tile = 0;
         for (int k = first; k < first + count; ++k) {
-            const quintrit_b200_matrix* m = mat(l, k);
-            const size_t bytes = gblocks * m->rows * 32;
-            stream_to_two_bit_kernel<<<static_cast<int>(std::min<size_t>((bytes + 255) / 256, 148 * 32)), 256>>>(m->d_w, w, m->rows, m->cols, m->rows, gblocks, m->blocks, m->tiles, off, rows);
-            ++g_launches;
-            off += m->rows;
+            QTB_CUDA(gemm_copy_weights(mat(l, k), w, static_cast<int>(tile)));
+            tile += mat(l, k)->rows / kGemmM;
         }
-        QTB_CUDA(cudaGetLastError());
         quintrit_b200_matrix* sm = new quintrit_b200_matrix();
         sm->magic = kMagicMatrix, sm->device = d->device, sm->sm_count = d->sm_count;
         sm->rows = rows, sm->cols = m0->cols, sm->blocks = m0->blocks, sm->tiles = 0;
         sm->d_w = nullptr, sm->w_bytes = 0, sm->d_items = nullptr, sm->n_items = 0, sm->d_counters = nullptr, sm->d_act = nullptr, sm->d_out = nullptr, sm->d_outf = nullptr;
-        sm->d_gemm_w = w, sm->gemm_rows_padded = rows;
+        sm->d_gemm_w = w;
         d->pf.stacked_objects.push_back(sm);
         *out = sm;
         return QUINTRIT_OK;

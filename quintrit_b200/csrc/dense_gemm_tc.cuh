@@ -124,9 +124,6 @@ __device__ __forceinline__ void dense_end16(const DenseSeg& g, int row, int toke
 }
 
 namespace dense_detail {
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
-}
 // kind::f16 with bf16 operands: F32 accumulator (1 at bit 4), BF16 A and B (1 at bits 7 and 10), both K-major, N / 8 at bit 17, M / 16 at bit 24.
 __device__ __forceinline__ uint32_t instr_desc_bf16(int m, int n) { return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(m >> 4) << 24); }
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {

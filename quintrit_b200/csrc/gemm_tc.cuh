@@ -8,29 +8,36 @@
 //
 // Shape on a B200. The batch-1 kernel streams velurex bytes (0.2 bytes per weight); turning those into int8 operands costs a table lookup and
 // a byte transposition per weight byte, which would leave the tensor pipe waiting. This kernel therefore reads its own copy of the weights,
-// made on the device the first time a matrix is used here: two bits per trit (0.25 bytes per weight), four consecutive columns per byte, so
-// that one lookup turns a byte into four int8 operands that are already in K order. The product runs as tcgen05.mma.kind::i8 with the
-// accumulator in tensor memory:
-//   * a work item is 128 weight rows (the M of the instruction) times a range of 128-column blocks (K); the batch is the N (16..256);
-//   * warps 2..17 decode, in four groups that take the blocks round-robin: a thread takes a row's 32 bytes of a block from shared memory,
-//     looks every byte up in a 256-entry table of int8x4 words (32 copies, one per shared-memory bank, so lookups never collide) and
-//     writes the row's 128 int8 operands into its lane of TENSOR MEMORY with tcgen05.st (32 columns a group). Operands that threads
+// made on the device the first time a matrix is used here: two bits per trit (0.25 bytes per weight), placed so that a mask, at most two shifts and one
+// byte permute turn a quarter of a word into four int8 operands that are already in K order. The product runs as tcgen05.mma.kind::i8 on pairs of
+// multiprocessors (cta_group::2) with the accumulator in tensor memory:
+//   * a work item is 256 weight rows (the M of the instruction, 128 a block of the pair) times a range of 256-column stages (K); the batch is the N
+//     (32..256). Each block of a pair holds half of the batch's activations, so a stage costs it n / 2 x 256 + 8192 bytes of shared memory and of L2 traffic: with a
+//     block for itself (n x 256 + 8192) the activations' way through L2 would be longer than the products;
+//   * sixteen warps decode, in four groups that take the stages round-robin: a thread takes a row's 64 bytes of a stage from shared memory and writes the row's
+//     256 int8 operands into its lane of TENSOR MEMORY with tcgen05.st (64 columns a group). Operands that threads
 //     store to shared memory need a proxy fence before the tensor cores may read them, and that fence was measured at more than a
 //     thousand cycles a block; operands in tensor memory need none;
-//   * two loader threads (warp 0 and the last warp) fetch, per block, the tile's 4096 weight bytes (one bulk copy) and the matching four
-//     32-byte-wide slices of the activation matrix (one 3-D TMA box, 32-byte swizzle, in place from the caller's vectors where their
-//     pitch allows it), both completing on one mbarrier;
-//   * one thread of warp 1 issues four MMAs (128 x N x 32, A from tensor memory, B from shared memory) per block and releases the stage
-//     and the group's operand columns with tcgen05.commit; a ring of 3 to 8 stages (as many as fit beside the batch) keeps the loads ahead;
-//   * the kernel is persistent: a CTA takes items round-robin;
-//   * at the end of an item the decode warps read the accumulator with tcgen05.ld (a row per thread, the column chunks shared between the
-//     four warps of a lane quarter) and write out[b][row] (when K was split over several items, so that matrices with few rows still fill
-//     the chip, each part writes its partial sums and a small second kernel adds the parts: exact integers in any order).
-// Every wait on an mbarrier is bounded: after `spin_limit` polls the thread raises an abort flag that the other roles see, the kernel
+//   * two load warps, taking the stages in turn, fetch the tile's 8192 weight bytes (one bulk copy) and the matching activations (two
+//     TMA boxes of n / 2 vectors x 128 bytes, 128-byte swizzle, in place from the caller's vectors where their pitch allows it), completing on one mbarrier;
+//   * one thread of the pair's first block issues eight MMAs (256 x N x 32, A from tensor memory, B from shared memory) per stage and releases the stage
+//     and the group's operand columns in both blocks with tcgen05.commit; a ring of 5 to 12 stages (as many as fit) keeps the loads ahead;
+//   * the kernel is persistent: a pair takes items round-robin;
+//   * at the end of an item the decode warps read the accumulator with tcgen05.ld (a row per thread, a quarter of the columns a group), release it and write
+//     out[b][row] (when K was split over several items, so that matrices with few rows still fill the chip, each part writes its partial sums and the
+//     consumer or a small second kernel adds the parts: exact integers in any order). A group decodes its first stage of the next item before that, so
+//     the tensor cores wait for the reading of the accumulator only.
+// Bound by the products at 256 vectors (1060 cycles a stage of 256 x 256 x 256, 1024 of them the tensor cores'), by what hands a stage on (about 700 cycles) at 32. Events around
+// 24 launches of the Falcon3-10B shapes, weights from HBM, against the former kernel (a block a tile, 128-column stages, table lookups):
+//   46080 x 3072, 256 vectors  59.7 -> 37.0 us;  32 vectors  43 -> 22.7 us
+//   3072 x 23040, 256 vectors  27 -> 19.2 us;    32 vectors  21 -> 12.4 us
+//   5120 x 3072, 256 vectors   22 -> 12.4 us;    32 vectors  10 -> 8.3 us
+// Every wait on an mbarrier is bounded: after `spin_limit` polls the thread raises an abort flag that the other roles (of both blocks) see, the kernel
 // sets its status word, waits (bounded) for its own copies in flight, frees its tensor memory and returns.
 //
-// Weight copy ("two-bit block-major"): byte j of block g of row r at (g * rows_padded + r) * 32 + j holds the columns g * 128 + 4 j + i,
-// i = 0..3, as (trit + 1) << 2 i; rows are padded to 128 and columns to whole blocks with code 1 (trit 0).
+// Weight copy: the 16 bytes at ((tile * chunks + c) * 128 + r) * 16 hold columns 64 c .. 64 c + 63 of row r of a tile of 128 rows, 16 columns a
+// 32-bit word: column k of a word as trit + 1 at bit 4 k for k < 8, at bit 4 (k - 8) + 2 for the others. Rows are padded to pairs of tiles and columns to
+// whole stages with code 1 (trit 0).
 #pragma once
 #include <cstdint>
 
@@ -41,62 +48,90 @@
 
 namespace qtb {
 
-constexpr int kGemmM = 128;
+constexpr int kGemmM = 128;     // weight rows of a block; a pair takes two such tiles
 constexpr int kGemmDecodeWarps = 16;
-constexpr int kGemmGroups = 4;  // the decode warps work in groups of four; group g decodes the blocks it, it + 4, ... of the CTA's sequence on its own
-constexpr int kGemmThreads = 64 + 32 * kGemmDecodeWarps + 32;  // weight loader warp, MMA warp, decode warps, activation loader warp
-constexpr int kGemmMaxStages = 8;
-constexpr int kGemmMaxN = 256;  // 256 accumulator columns + 4 x 32 operand columns fit the 512 columns of tensor memory
-constexpr int kGemmBlockCols = 128;           // columns (K) of one block of the two-bit copy: 32 bytes a row
-constexpr int kGemmLutBytes = 256 * 32 * 4;  // 32 copies of the byte -> int8x4 table, one per shared-memory bank: lookups never collide
+constexpr int kGemmGroups = 4;  // the decode warps work in groups of four; group g decodes the stages it, it + 4, ... of the pair's sequence on its own
+constexpr int kGemmLoadWarps = 2;  // load warp w fetches the stages w, w + 4, ...: the fixed cost of a stage (about 600 cycles in one warp) would bound small batches
+constexpr int kGemmThreads = 32 * (kGemmDecodeWarps + 1 + kGemmLoadWarps);  // decode warps, the MMA warp, load warps
+constexpr int kGemmMaxStages = 12;
+constexpr int kGemmMaxN = 256;  // 256 accumulator columns + 4 x 64 operand columns are the 512 columns of tensor memory
+constexpr int kGemmStageCols = 256;                            // columns (K) of one stage
+constexpr int kGemmStageBytes = kGemmM * kGemmStageCols / 4;   // its weight bytes for one tile
 constexpr unsigned int kGemmStatusTimeout = 4;
 
 struct GemmArgs {
-    const uint8_t* w;      // two-bit block-major weights
-    int32_t* out;          // [batch][rows]; with K split over several items: the partial sums [part][batch][rows] that gemm_reduce_parts_kernel adds up
+    const uint8_t* w;      // the two-bit copy
+    int32_t* out;          // [batch][rows]; with K split over several items: the partial sums [part][batch][rows]
     unsigned int* status;  // set to kGemmStatusTimeout when a wait ran out
-    int rows, rows_padded, blocks;
+    int rows, pairs;       // weight rows; pairs of row tiles
+    int blocks;            // stages (256 columns) of a row
     int ldo;               // elements between the results of consecutive vectors in `out` (rows, or more when the results go into a wider row)
-    int n;                 // instruction N: the batch rounded up to a multiple of 16
+    int n;                 // instruction N: the batch rounded up to a multiple of 32
     int batch;             // activation vectors actually present (columns of the accumulator that are written out)
-    int blocks_per_cta;    // blocks of one work item (a row tile x a K part)
+    int blocks_per_item;   // stages of one work item (a pair of row tiles x a K part)
     int stages;
     unsigned int spin_limit;
 };
 
-// Stages that fit the shared memory of an SM for a batch of n: as many as possible (at most kGemmMaxStages), because the blocks in flight have to
-// cover the latency of the weight bytes from HBM.
+// Stages that fit the shared memory of an SM for a batch of n: as many as possible (at most kGemmMaxStages), because the stages in flight have to
+// cover the latency of the weight bytes from HBM. Five at n = 256.
+inline size_t gemm_stage_bytes(int n) { return size_t(n / 2) * kGemmStageCols + kGemmStageBytes; }
 inline int gemm_stages_for(int n, size_t smem_limit) {
-    const size_t fixed = kGemmLutBytes + 256 + 1024, stage = size_t(n) * kGemmBlockCols + kGemmM * 32;
-    const size_t fit = smem_limit > fixed ? (smem_limit - fixed) / stage : 0;
+    const size_t fixed = 512 + 1024, fit = smem_limit > fixed ? (smem_limit - fixed) / gemm_stage_bytes(n) : 0;
     return static_cast<int>(fit < size_t(kGemmMaxStages) ? fit : size_t(kGemmMaxStages));
 }
-inline size_t gemm_smem_bytes(int n, int stages) {
-    return size_t(stages) * (size_t(n) * kGemmBlockCols + kGemmM * 32) + kGemmLutBytes + 256 + 1024;  // + barriers + alignment slack
-}
+inline size_t gemm_smem_bytes(int n, int stages) { return size_t(stages) * gemm_stage_bytes(n) + 512 + 1024; }  // + barriers + alignment slack
+inline size_t gemm_row_tiles(size_t rows) { return (rows + 2 * kGemmM - 1) / (2 * kGemmM) * 2; }
+inline size_t gemm_blocks(size_t cols) { return (cols + kGemmStageCols - 1) / kGemmStageCols; }
+inline size_t gemm_copy_bytes(size_t rows, size_t cols) { return gemm_row_tiles(rows) * gemm_blocks(cols) * kGemmStageBytes; }
 
-// stream layout (gemv_lut.cuh) -> two-bit block-major; `blocks` counts 128-column blocks here, `vblocks` the 160-trit velurex blocks of a row
-// The copy may be one of several matrices stacked row-wise into one (q | k | v, gate | up): its rows start at row_off of rows_total.
-__global__ void stream_to_two_bit_kernel(const uint4* __restrict__ stream, uint8_t* __restrict__ out, size_t rows, size_t cols, size_t rows_padded, size_t blocks, size_t vblocks,
-                                         size_t tiles, size_t row_off, size_t rows_total) {
-    const size_t total = blocks * rows_padded * 32;
-    const uint8_t* s = reinterpret_cast<const uint8_t*>(stream);
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
-        const size_t g = i / (rows_padded * 32), rem = i % (rows_padded * 32), r = rem / 32, j = rem % 32;
-        unsigned int byte = 0;
-        for (int q = 0; q < 4; ++q) {
-            const size_t col = g * 128 + j * 4 + q;
-            unsigned int code = 1;  // trit 0 beyond the matrix
-            if (r < rows && col < cols) {
-                const size_t vb = col / 160, p = (col % 160) / 32, jj = col % 32, t = r / 32, l = r % 32, pos = (jj + 32 - l) % 32;  // planar byte jj sits at position pos of the rotated row
-                const unsigned int v = s[((vb * tiles + t) * 2 + pos / 16) * 512 + l * 16 + pos % 16];
-                const unsigned int d4 = v / 84, r4 = v - 84 * d4, d3 = r4 / 28, r3 = r4 - 28 * d3, d2 = r3 / 9, r2 = r3 - 9 * d2, d1 = r2 / 3, d0 = r2 - 3 * d1;
-                const unsigned int digits[5] = {d0, d1, d2, d3, d4};
-                code = v <= 250 ? digits[p] : 1;
-            }
-            byte |= code << (2 * q);
+// stream layout (gemv_lut.cuh) -> the two-bit copy, whose bytes are all 0x55 (code 1) before; `chunks` 16-byte units a row, `vblocks` 160-trit velurex blocks
+// a row. The copy may be one of several matrices stacked row-wise into one (q | k | v, gate | up): its rows start at tile `tile0`. A warp takes a velurex
+// block of 32 rows, a row a lane: 32 bytes in two 16-byte loads, a table lookup per byte for its five codes, ten words out. (A word a thread from single bytes took
+// 4 ms longer over the four layers of a Falcon3-10B-shaped model's first prompt.)
+__global__ void stream_to_two_bit_kernel(const uint4* __restrict__ stream, uint32_t* __restrict__ out, int rows, int cols, int chunks, int vblocks, int tiles, int tile0) {
+    __shared__ unsigned short codes[256];  // byte -> its five codes, two bits each
+    for (int v = threadIdx.x; v < 256; v += blockDim.x) {
+        unsigned int d = 0x155;
+        if (v <= 250) {
+            const int d4 = v / 84, r4 = v - 84 * d4, d3 = r4 / 28, r3 = r4 - 28 * d3, d2 = r3 / 9, r2 = r3 - 9 * d2, d1 = r2 / 3;
+            d = (r2 - 3 * d1) | d1 << 2 | d2 << 4 | d3 << 6 | d4 << 8;
         }
-        out[(g * rows_total + row_off + r) * 32 + j] = static_cast<uint8_t>(byte);
+        codes[v] = static_cast<unsigned short>(d);
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
+    for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < vblocks * tiles; i += warps) {
+        const int vb = i / tiles, t = i - vb * tiles, r = t * 32 + lane;
+        const uint4* src = stream + (static_cast<size_t>(i) * 2) * 32 + lane;
+        const uint4 x = src[0], y = src[32];
+        const uint32_t words[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+        uint32_t lo[5] = {0, 0, 0, 0, 0}, hi[5] = {0, 0, 0, 0, 0};  // columns 32 p .. 32 p + 15 and the sixteen behind them
+#pragma unroll
+        for (int k = 0; k < 32; ++k) {
+            const unsigned int c = codes[(words[k >> 2] >> (8 * (k & 3))) & 0xffu];
+            const int j = (k + lane) & 31, jj = j & 15, at = jj < 8 ? 4 * jj : 4 * (jj - 8) + 2;  // position k of a row holds planar byte (k + row) mod 32
+#pragma unroll
+            for (int p = 0; p < 5; ++p) {
+                const uint32_t bits = ((c >> (2 * p)) & 3u) << at;
+                lo[p] |= j < 16 ? bits : 0u;
+                hi[p] |= j < 16 ? 0u : bits;
+            }
+        }
+        if (r >= rows) continue;
+        uint32_t* dst = out + (static_cast<size_t>(tile0 + r / kGemmM) * chunks * kGemmM + r % kGemmM) * 4;
+#pragma unroll
+        for (int w = 0; w < 10; ++w) {
+            const int col = vb * 160 + w * 16, left = cols - col;
+            uint32_t word = w & 1 ? hi[w >> 1] : lo[w >> 1];
+            if (left <= 0) break;
+            if (left < 16) {  // the columns behind the matrix stay code 1
+                uint32_t keep = 0;
+                for (int k = 0; k < left; ++k) keep |= 3u << (k < 8 ? 4 * k : 4 * (k - 8) + 2);
+                word = (word & keep) | (0x55555555u & ~keep);
+            }
+            dst[static_cast<size_t>(col / 64) * (kGemmM * 4) + (col % 64) / 16] = word;
+        }
     }
 }
 
@@ -120,16 +155,6 @@ __global__ void gemm_pad_activations_kernel(const int8_t* __restrict__ act, int8
 }
 
 namespace gemm_detail {
-
-#ifdef QTB_GEMM_TRACE
-// Debug build only: cycle stamps of CTA 0, role `who` (0 loader, 1 MMA thread, 2 decode warp 0), event `ev`, block `k` < 16, at status + 64 + ...
-#define QTB_GEMM_STAMP(who, ev, k)                                                                                              \
-    do {                                                                                                                        \
-        if (blockIdx.x == 0 && (k) < 16) reinterpret_cast<long long*>(a.status + 64)[((who) * 4 + (ev)) * 16 + (k)] = clock64(); \
-    } while (0)
-#else
-#define QTB_GEMM_STAMP(who, ev, k) do { } while (0)
-#endif
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count)); }
@@ -175,250 +200,276 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes,
 // Instruction descriptor for kind::i8: S32 accumulator (2 at bit 4), signed 8-bit A and B (1 at bits 7 and 10), both K-major,
 // N / 8 at bit 17, M / 16 at bit 24.
 __device__ __forceinline__ uint32_t instr_desc_i8(int m, int n) { return (2u << 4) | (1u << 7) | (1u << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(m >> 4) << 24); }
-__device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    const uint32_t zero = 0;  // no output lane is disabled
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(tmem_d),
-        "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(zero)
-        : "memory");
-}
-// The same instruction with the A operand in tensor memory (128 lanes = rows, 32-bit columns of four consecutive K elements).
-__device__ __forceinline__ void mma_i8_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    const uint32_t zero = 0;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(zero)
-        : "memory");
-}
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// ---- pairs of blocks (cta_group::2) ----
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The address, in the cluster's window, of what lies at `addr` in block `rank`'s shared memory.
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+// An arrival at a barrier of either block. It orders nothing but what the tcgen05 fences and waits around it order (operands in tensor memory, accumulator reads) and
+// copies whose completion the arriving thread has seen: with .release.cluster an arrival, and .acquire.cluster a wait, cost about 3000 and 250 cycles.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ void raise_abort(uint32_t flag_addr, uint32_t rank) {  // in the other block too
+    asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(flag_addr, rank ^ 1)), "r"(1u) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+// 256 rows (128 in the tensor memory of either block) x N x 32; the first half of B's rows lies in the first block's shared memory, the rest in the second's.
+__device__ __forceinline__ void mma_i8_ts_pair(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// Arrives at the barrier of that offset in both blocks once the MMAs issued so far are done.
+__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(static_cast<uint16_t>(3)) : "memory");
+}
+// 16 columns of the two-bit copy -> four words of four int8 operands. A nibble of the masked word selects a byte of (-1, 0, 1, 0): its low two bits are a code, bit 2
+// picks the second operand of the permute (the same word), bit 3 (sign fill) is masked away.
+__device__ __forceinline__ void decode16(uint32_t w, uint32_t* v) {
+    const uint32_t m0 = w & 0x77777777u, m1 = (w >> 2) & 0x77777777u;
+    constexpr uint32_t kTrits = 0x000100FFu;
+    asm("prmt.b32 %0, %1, %1, %2;" : "=r"(v[0]) : "r"(kTrits), "r"(m0));
+    asm("prmt.b32 %0, %1, %1, %2;" : "=r"(v[1]) : "r"(kTrits), "r"(m0 >> 16));
+    asm("prmt.b32 %0, %1, %1, %2;" : "=r"(v[2]) : "r"(kTrits), "r"(m1));
+    asm("prmt.b32 %0, %1, %1, %2;" : "=r"(v[3]) : "r"(kTrits), "r"(m1 >> 16));
+}
+__device__ __forceinline__ void tmem_store32(uint32_t addr, const uint32_t* v) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, "
+        "%29, %30, %31, %32};" ::"r"(addr),
+        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]),
+        "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]),
+        "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_load8(uint32_t addr, uint32_t* v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(addr));
 }
 
 }  // namespace gemm_detail
 
-__global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap act_map, GemmArgs a) {
+// The end of an item: this thread's row of `own` (a multiple of eight) accumulator columns is read, the accumulator released, and the first `valid` of them written, `ldo` apart.
+// Out of line: its 64 values would crowd the decoding loop's registers.
+__device__ __noinline__ void gemm_write_out(uint32_t tmem, uint32_t released, int own, int32_t* dst, int ldo, int valid) {
+    using namespace gemm_detail;
+    constexpr int kMost = kGemmMaxN / kGemmGroups;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    uint32_t v[kMost];
+#pragma unroll
+    for (int c = 0; c < kMost; c += 8)
+        if (c < own) tmem_load8(tmem + c, v + c);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive_cluster(released);
+#pragma unroll
+    for (int c = 0; c < kMost; c += 8) {
+        if (c >= valid) break;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (c + i < valid) dst[static_cast<size_t>(static_cast<uint32_t>((c + i) * ldo))] = static_cast<int32_t>(v[c + i]);
+    }
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap act_map, GemmArgs a) {
     using namespace gemm_detail;
     extern __shared__ unsigned char gemm_smem_raw[];
-    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gemm_smem_raw) + 1023) & ~uintptr_t(1023));
+    const uint32_t smem0 = (smem_u32(gemm_smem_raw) + 1023u) & ~1023u;  // the same offset in both blocks, as the descriptors want it
+    unsigned char* smem = gemm_smem_raw + (smem0 - smem_u32(gemm_smem_raw));
     const int S = a.stages, n = a.n;
-    unsigned char* b_tiles = smem;                                        // S stages of four n * 32-byte activation tiles
-    unsigned char* raw_tiles = b_tiles + size_t(S) * n * kGemmBlockCols;  // S stages of the 128 x 32 weight bytes of a block, as they lie in memory
-    uint32_t* lut = reinterpret_cast<uint32_t*>(raw_tiles + size_t(S) * kGemmM * 32);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(lut) + kGemmLutBytes);
-    // barriers: loaded[S] (weight bytes and activations of a stage have landed), empty[S] (the MMAs that read the stage are done);
-    // a_full[G], a_empty[G] (the int8 operand of group g in tensor memory is written / its MMAs are done); acc_full, acc_empty (the accumulator)
+    const uint32_t act_bytes = uint32_t(n / 2) * kGemmStageCols;
+    const uint32_t b_base = smem0;                                        // S stages of two tiles of n / 2 vectors x 128 bytes
+    const uint32_t raw_base = smem0 + S * act_bytes;                      // S stages of the weight bytes of this block's tile
+    const unsigned char* raw_tiles = smem + S * act_bytes;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S * (act_bytes + kGemmStageBytes));
+    // barriers of each block: loaded[S] (its weight bytes and activations of a stage have landed), empty[S] (the MMAs of the stage are done: it may be loaded again, and the
+    // group may write its next operand), acc_full (those of an item); of the first block only: a_full[G] (group g's operand is written in both blocks), acc_empty (both have read the accumulator)
     const uint32_t bar0 = smem_u32(bars);
     auto loaded = [&](int s) { return bar0 + 8u * s; };
     auto empty = [&](int s) { return bar0 + 8u * (kGemmMaxStages + s); };
     auto a_full = [&](int g) { return bar0 + 8u * (2 * kGemmMaxStages + g); };
-    auto a_empty = [&](int g) { return bar0 + 8u * (2 * kGemmMaxStages + kGemmGroups + g); };
-    const uint32_t acc_full = bar0 + 8u * (2 * kGemmMaxStages + 2 * kGemmGroups), acc_empty = acc_full + 8u;
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * kGemmMaxStages + 2 * kGemmGroups + 2);  // 26 barriers, then these two words
-    volatile unsigned int* abort_flag = reinterpret_cast<volatile unsigned int*>(bars + 2 * kGemmMaxStages + 2 * kGemmGroups + 3);
+    const uint32_t acc_full = bar0 + 8u * (2 * kGemmMaxStages + kGemmGroups), acc_empty = acc_full + 8u;
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * kGemmMaxStages + kGemmGroups + 2);  // 30 barriers, then these two words
+    volatile unsigned int* abort_flag = reinterpret_cast<volatile unsigned int*>(bars + 2 * kGemmMaxStages + kGemmGroups + 3);
+    const uint32_t abort_addr = acc_empty + 16u;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // work items: (row tile, K part), taken round-robin by the CTAs; an item is `per` blocks of one tile
-    const int per = a.blocks_per_cta, parts = (a.blocks + per - 1) / per, items = (a.rows_padded / kGemmM) * parts;
-    // tensor memory: the accumulator in columns [0, n), then the int8 operand of each decode group (128 rows x 128 K = 32 columns of four bytes)
-    uint32_t tmem_cols = 32;
-    while (tmem_cols < static_cast<uint32_t>(n) + 32u * kGemmGroups) tmem_cols <<= 1;
+    const uint32_t rank = cluster_rank();
+    // work items: (pair of row tiles, K part), taken round-robin by the pairs; an item is `per` stages of one pair of tiles
+    const int per = a.blocks_per_item, parts = (a.blocks + per - 1) / per, items = a.pairs * parts, first = blockIdx.x >> 1, step = gridDim.x >> 1;
+    constexpr uint32_t kOperandCol = 256;  // tensor memory: the accumulator in columns [0, n), the operands of group g in 64 columns from 256 + 64 g
 
-    // ---- set-up: byte -> int8x4 table, barriers, tensor memory ----
-    for (int v = tid; v < 256; v += kGemmThreads) {
-        uint32_t word = 0;
-        for (int q = 0; q < 4; ++q) {
-            const int code = (v >> (2 * q)) & 3;
-            word |= uint32_t(uint8_t(code == 3 ? 0 : code - 1)) << (8 * q);  // code 3 does not occur; it reads as trit 0
-        }
-        for (int copy = 0; copy < 32; ++copy) lut[v * 32 + ((copy + v) & 31)] = word;  // entry v of copy c at v * 128 + c * 4 (rotated fill: no bank conflicts here)
-    }
     if (tid == 0) {
         for (int s = 0; s < S; ++s) {
-            mbar_init(loaded(s), 2);  // the expect_tx arrivals of the two loader threads
+            mbar_init(loaded(s), 1);  // the expect_tx arrival of the loading thread
             mbar_init(empty(s), 1);   // tcgen05.commit
         }
-        for (int g = 0; g < kGemmGroups; ++g) {
-            mbar_init(a_full(g), kGemmDecodeWarps / kGemmGroups);  // one arrival per warp of the group
-            mbar_init(a_empty(g), 1);                              // tcgen05.commit
-        }
-        mbar_init(acc_full, 1);                  // tcgen05.commit after the last MMA of an item
-        mbar_init(acc_empty, kGemmDecodeWarps);  // every epilogue warp has read its part
+        for (int g = 0; g < kGemmGroups; ++g) mbar_init(a_full(g), 2 * kGemmDecodeWarps / kGemmGroups);  // one arrival per warp of the group in either block
+        mbar_init(acc_full, 1);                      // tcgen05.commit after the last MMA of an item
+        mbar_init(acc_empty, 2 * kGemmDecodeWarps);  // every warp that reads the accumulator has read its part
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(const_cast<uint32_t*>(tmem_slot))), "r"(tmem_cols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(const_cast<uint32_t*>(tmem_slot))), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    cluster_sync_all();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0 || warp == 2 + kGemmDecodeWarps) {
-        // ---- loads, by two threads so that neither's fixed cost per block bounds the pipe: warp 0 fetches the weight bytes of a block (one bulk
-        // copy of the tile's 4096 bytes), the last warp its activations (one TMA box: 32 bytes x n vectors x four K tiles) ----
-        if (lane == 0) {
-            const bool weights = warp == 0;
-            int it = 0, s = 0;
-            uint32_t ph = 0;  // stage and phase of the ring, advanced by hand (S is a run-time value)
-            bool okay = true;
-            const uint32_t b_base = smem_u32(b_tiles), raw_base = smem_u32(raw_tiles);
-            for (int item = blockIdx.x; item < items && okay; item += gridDim.x) {
-                const int row0 = (item / parts) * kGemmM, kb0 = (item % parts) * per, nkb = min(per, a.blocks - kb0);
-                const uint8_t* src = a.w + (size_t(kb0) * a.rows_padded + row0) * 32;
-                const size_t pitch = size_t(a.rows_padded) * 32;
-                for (int k = 0; k < nkb; ++k, ++it) {
-                    QTB_GEMM_STAMP(0, 0, it);
-                    if (!(okay = mbar_wait(empty(s), ph ^ 1, abort_flag, a.spin_limit))) break;
-                    QTB_GEMM_STAMP(0, 1, it);
-                    if (weights) {
-                        mbar_expect_tx(loaded(s), kGemmM * 32u);
-                        bulk_load(raw_base + s * (kGemmM * 32), src, kGemmM * 32, loaded(s));
-                        src += pitch;
-                    } else {
-                        mbar_expect_tx(loaded(s), 4u * n * 32u);
-                        tma_load_3d(b_base + s * n * kGemmBlockCols, &act_map, 0, 0, (kb0 + k) * 4, loaded(s));
-                    }
-                    QTB_GEMM_STAMP(0, 2, it);
-                    if (++s == S) s = 0, ph ^= 1;
+    if (warp > kGemmDecodeWarps) {
+        // ---- loads: one thread issues, but the warp stays together, so that addresses live in uniform registers ----
+        const int mine = warp - kGemmDecodeWarps - 1;
+        int it0 = 0, until = 0;  // stages of the sequence before this item; behind this warp's last issued stage
+        bool okay = true;
+        for (int item = first; item < items && okay; item += step) {
+            const int tile = (item / parts) * 2 + static_cast<int>(rank), kb0 = (item % parts) * per, nkb = min(per, a.blocks - kb0);
+            const uint8_t* src = a.w + (size_t(tile) * a.blocks + kb0) * kGemmStageBytes;
+            for (int k = (mine - it0) & (kGemmLoadWarps - 1); k < nkb; k += kGemmLoadWarps) {
+                const int it = it0 + k, s = it % S;
+                if (!(okay = __all_sync(0xffffffffu, mbar_wait(empty(s), ((it / S) & 1) ^ 1, abort_flag, a.spin_limit)))) break;
+                if (elect_one()) {
+                    const uint32_t dst = b_base + s * act_bytes;
+                    const int x = (kb0 + k) * kGemmStageCols, y = static_cast<int>(rank) * (n / 2);
+                    mbar_expect_tx(loaded(s), kGemmStageBytes + act_bytes);
+                    bulk_load(raw_base + s * kGemmStageBytes, src + size_t(k) * kGemmStageBytes, kGemmStageBytes, loaded(s));
+                    tma_load_2d(dst, &act_map, x, y, loaded(s));
+                    tma_load_2d(dst + act_bytes / 2, &act_map, x + 128, y, loaded(s));
                 }
+                __syncwarp();
+                until = it + 1;
             }
-            // its own copies in flight land before the CTA leaves: the last min(it, S) uses of the ring, newest first
-            for (int back = 0; back < min(it, S); ++back) {
-                if (--s < 0) s = S - 1, ph ^= 1;
-                mbar_wait(loaded(s), ph, abort_flag, a.spin_limit, false);
-            }
+            it0 += nkb;
         }
-    } else if (warp == 1) {
-        // ---- tensor cores: four MMAs per block (A from tensor memory, B from shared memory), all issued by one thread ----
-        if (lane == 0) {
-            const uint32_t idesc = instr_desc_i8(kGemmM, n);
+        if (!okay && lane == 0) raise_abort(abort_addr, rank);
+        // its own copies in flight land before the block leaves (stages before the last S are long used up)
+        for (int it = max(0, it0 - S); it < until; ++it)
+            if ((it & (kGemmLoadWarps - 1)) == mine) mbar_wait(loaded(it % S), (it / S) & 1, abort_flag, a.spin_limit, false);
+    } else if (warp == kGemmDecodeWarps) {
+        // ---- tensor cores of both blocks: eight MMAs per stage (A from tensor memory, B from shared memory), issued by one thread of the first block. The warp
+        // stays together around them, so that descriptors live in uniform registers (one lane alone took 80 cycles an instruction) ----
+        if (rank == 0) {
+            const uint32_t idesc = instr_desc_i8(2 * kGemmM, n);
             int j = 0, s = 0, it = 0;
-            uint32_t ph = 0;
             bool okay = true;
-            // descriptor of stage 0, K tile 0; a stage or a tile further on only moves the start address field (16-byte units)
-            const uint64_t b_desc0 = smem_desc(smem_u32(b_tiles), 16, 256, 6);
-            const uint32_t b_stage16 = uint32_t(n * kGemmBlockCols) >> 4, b_tile16 = uint32_t(n * 32) >> 4;
-            for (int item = blockIdx.x; item < items && okay; item += gridDim.x, ++j) {
+            // descriptor of stage 0, K tile 0 (128-byte swizzle, 8-row groups 1024 bytes apart); a stage or a tile further on only moves the start address field (16-byte units)
+            const uint64_t b_desc0 = smem_desc(b_base, 16, 1024, 2);
+            const uint32_t b_stage16 = act_bytes >> 4, b_half16 = act_bytes >> 5;
+            for (int item = first; item < items && okay; item += step, ++j) {
                 const int kb0 = (item % parts) * per, nkb = min(per, a.blocks - kb0);
-                if (!(okay = mbar_wait(acc_empty, (j & 1) ^ 1, abort_flag, a.spin_limit))) break;  // the epilogue of the previous item has drained the accumulator
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (!(okay = __all_sync(0xffffffffu, mbar_wait(acc_empty, (j & 1) ^ 1, abort_flag, a.spin_limit)))) break;  // the previous item's accumulator has been read
                 for (int k = 0; k < nkb; ++k, ++it) {
                     const int g = it & (kGemmGroups - 1);
-                    QTB_GEMM_STAMP(1, 0, k + 100 * j);
-                    // the group's arrival also stands for the stage's loads: the group waited for them before it decoded
-                    if (!(okay = mbar_wait(a_full(g), (it / kGemmGroups) & 1, abort_flag, a.spin_limit))) break;
-                    QTB_GEMM_STAMP(1, 1, k + 100 * j);
+                    // the groups' arrivals also stand for the stage's loads: each waited for its block's before it decoded
+                    if (!(okay = __all_sync(0xffffffffu, mbar_wait(a_full(g), (it / kGemmGroups) & 1, abort_flag, a.spin_limit)))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t b_desc = b_desc0 + uint64_t(s * b_stage16);
-                    const uint32_t a_tmem = tmem_base + uint32_t(n + 32 * g);
+                    const uint32_t a_tmem = tmem_base + kOperandCol + 64u * g;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int p = 0; p < 4; ++p) mma_i8_ts(tmem_base, a_tmem + 8 * p, b_desc + uint64_t(p * b_tile16), idesc, (k | p) != 0 ? 1u : 0u);
-                    mma_commit(empty(s));     // the stage may be loaded again ...
-                    mma_commit(a_empty(g));   // ... and the group may write its next operand, once these MMAs are done
-                    QTB_GEMM_STAMP(1, 2, k + 100 * j);
-                    if (++s == S) s = 0, ph ^= 1;
+                        for (int p = 0; p < 8; ++p) mma_i8_ts_pair(tmem_base, a_tmem + 8 * p, b_desc + uint64_t((p >> 2) * b_half16 + (p & 3) * 2), idesc, (k | p) != 0 ? 1u : 0u);
+                        mma_commit_pair(empty(s));
+                        if (k + 1 == nkb) mma_commit_pair(acc_full);  // arrives when every MMA issued so far has finished
+                    }
+                    __syncwarp();
+                    if (++s == S) s = 0;
                 }
-                mma_commit(acc_full);  // arrives when every MMA issued so far has finished (also on the way out after a failed wait)
+                if (!okay) {  // what was issued is done before anyone leaves
+                    if (elect_one()) mma_commit_pair(acc_full);
+                    __syncwarp();
+                    mbar_wait(acc_full, j & 1, abort_flag, a.spin_limit, false);
+                }
             }
+            if (!okay && lane == 0) raise_abort(abort_addr, rank);
         }
     } else {
-        // ---- decode warps: a weight row (32 bytes of a block = 128 int8 operands) per thread, in groups of four warps ----
-        // Group g takes the blocks g, g + 4, ... of the CTA's block sequence. A warp owns the 32 lanes of tensor memory that its index modulo 4
+        // ---- decode warps: a weight row (64 bytes of a stage = 256 int8 operands) per thread, in groups of four warps ----
+        // Group g takes the stages g, g + 4, ... of the pair's sequence. A warp owns the 32 lanes of tensor memory that its index modulo 4
         // selects, so thread (warp, lane) takes row 32 (warp & 3) + lane of the tile and writes the row's operand into that lane with tcgen05.st:
         // no shared-memory store, so no proxy fence between the decode and the tensor cores.
-        const int group = (warp - 2) >> 2, quarter = warp & 3, r = quarter * 32 + lane;
-        const uint32_t* lut_lane = lut + lane;  // this lane's copy of the table: entry v at lut_lane[v * 32]
-        const unsigned char* raw_mine = raw_tiles + r * 32;
-        const uint32_t a_tmem = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(n + 32 * group);
+        const int group = warp >> 2, quarter = warp & 3, r = quarter * 32 + lane;
+        const uint32_t lanes = tmem_base + (uint32_t(quarter * 32) << 16), a_tmem = lanes + kOperandCol + 64u * group;
+        const uint32_t to_full = cluster_addr(a_full(group), 0), to_empty = cluster_addr(acc_empty, 0);
+        const int own = n / kGemmGroups, c0 = group * own;  // accumulator columns (a multiple of eight) that this group writes out
         bool okay = true;
-        int j = 0, it = 0, s = group % S, use = 0;  // stage and phase of this group's next block (block `group` of the sequence); its count of blocks so far
-        uint32_t ph = (group / S) & 1;
-        for (int item = blockIdx.x; item < items && okay; item += gridDim.x, ++j) {
-            const int row0 = (item / parts) * kGemmM, nkb = min(per, a.blocks - (item % parts) * per);
-            for (int k = 0; k < nkb && okay; ++k, ++it) {
-                if ((it & (kGemmGroups - 1)) != group) continue;
-                if (warp == 2) QTB_GEMM_STAMP(2, 0, k + 100 * j);
-                // The block's bytes have landed and the MMAs of this group's previous operand are done. With fewer stages than groups a group can be a
-                // whole use of the stage ahead of the loader; a parity wait only tells the last two phases apart, so the previous use is waited for first.
-                if (lane == 0)
-                    okay = (S >= kGemmGroups || it < S || mbar_wait(loaded(s), ph ^ 1, abort_flag, a.spin_limit)) && mbar_wait(loaded(s), ph, abort_flag, a.spin_limit) &&
-                           mbar_wait(a_empty(group), (use & 1) ^ 1, abort_flag, a.spin_limit);
-                okay = __shfl_sync(0xffffffffu, okay ? 1 : 0, 0) != 0;
+        auto finish = [&](int item, int j) {  // item `item`, the pair's j-th
+            okay = __all_sync(0xffffffffu, mbar_wait(acc_full, j & 1, abort_flag, a.spin_limit));
+            if (!okay) return;
+            const int row = ((item / parts) * 2 + static_cast<int>(rank)) * kGemmM + r;
+            gemm_write_out(lanes + c0, to_empty, own, a.out + (size_t(item % parts) * a.batch + c0) * a.ldo + row, a.ldo, row < a.rows ? min(own, a.batch - c0) : 0);
+        };
+        int j = 0, it0 = 0, before = -1;  // `before`: the item whose accumulator has not been written out yet
+        for (int item = first; item < items && okay; item += step, ++j) {
+            const int nkb = min(per, a.blocks - (item % parts) * per);
+            // A group decodes its first stage of an item before it writes out the item before. (All groups' reads before any store, or the reads first, or whichever is
+            // ready first: 0 to 3 us slower of 37 at 46080 x 3072, 256 vectors.)
+            bool owed = before >= 0;
+            for (int k = (group - it0) & (kGemmGroups - 1); k < nkb && okay; k += kGemmGroups) {
+                const int it = it0 + k, s = it % S;
+                // The MMAs of this group's previous operand are done - and with them all loads up to that stage, so that the parity of the stage's barrier
+                // is not mistaken - and the stage's bytes have landed. (S >= kGemmGroups: the barrier of that operand's stage cannot be a use further on.)
+                const int last = it - kGemmGroups;
+                if (!okay) break;
+                okay = (last < 0 || mbar_wait(empty(last % S), (last / S) & 1, abort_flag, a.spin_limit)) && mbar_wait(loaded(s), (it / S) & 1, abort_flag, a.spin_limit);
+                okay = __all_sync(0xffffffffu, okay);
                 if (!okay) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (warp == 2) QTB_GEMM_STAMP(2, 1, k + 100 * j);
-                const uint4* raw = reinterpret_cast<const uint4*>(raw_mine + s * (kGemmM * 32));
-                const uint4 lo = raw[0], hi = raw[1];
-                const uint32_t words[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+                const uint4* raw = reinterpret_cast<const uint4*>(raw_tiles + s * kGemmStageBytes) + r;
 #pragma unroll
-                for (int t = 0; t < 4; ++t) {  // K tile t: input words 2 t and 2 t + 1 become eight columns of four operands
-                    uint32_t v[8];
-#pragma unroll
-                    for (int m = 0; m < 2; ++m) {
-                        const uint32_t w = words[2 * t + m];
-                        v[4 * m + 0] = lut_lane[(w & 0xffu) << 5];
-                        v[4 * m + 1] = lut_lane[((w >> 8) & 0xffu) << 5];
-                        v[4 * m + 2] = lut_lane[((w >> 16) & 0xffu) << 5];
-                        v[4 * m + 3] = lut_lane[(w >> 24) << 5];
-                    }
-                    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(a_tmem + 8 * t), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
-                                 "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
-                                 : "memory");
+                for (int half = 0; half < 2; ++half) {
+                    const uint4 x = raw[(2 * half) * kGemmM], y = raw[(2 * half + 1) * kGemmM];
+                    uint32_t v[32];
+                    decode16(x.x, v), decode16(x.y, v + 4), decode16(x.z, v + 8), decode16(x.w, v + 12);
+                    decode16(y.x, v + 16), decode16(y.y, v + 20), decode16(y.z, v + 24), decode16(y.w, v + 28);
+                    tmem_store32(a_tmem + 32 * half, v);
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                if (warp == 2) QTB_GEMM_STAMP(2, 2, k + 100 * j);
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) mbar_arrive(a_full(group));
-                if (warp == 2) QTB_GEMM_STAMP(2, 3, k + 100 * j);
-                ++use;
-                s += kGemmGroups;  // this group's next block is four uses of the ring further on
-                while (s >= S) s -= S, ph ^= 1;
+                if (lane == 0) mbar_arrive_cluster(to_full);
+                if (owed) finish(before, j - 1), owed = false;
             }
-            if (!okay) break;
-            // ---- epilogue of the item: accumulator row -> out[b][row] ----
-            if (lane == 0) okay = mbar_wait(acc_full, j & 1, abort_flag, a.spin_limit);
-            okay = __shfl_sync(0xffffffffu, okay ? 1 : 0, 0) != 0;
-            if (!okay) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int row = row0 + r;
-            for (int c0 = group * 16; c0 < n; c0 += 16 * kGemmGroups) {  // the four warps that share a lane quarter alternate over the column chunks
-                uint32_t v[16];
-                const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(c0);
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
-                      "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                    : "r"(taddr));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (row < a.rows) {
-                    int32_t* dst = a.out + (size_t(item % parts) * a.batch + c0) * a.ldo + row;
-                    const int valid = min(16, a.batch - c0);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        if (i < valid) *dst = static_cast<int32_t>(v[i]);
-                        dst += a.ldo;
-                    }
-                }
-            }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty);
+            if (owed && okay) finish(before, j - 1);
+            before = item, it0 += nkb;
         }
+        if (okay && before >= 0) finish(before, j - 1);
+        if (!okay && lane == 0) raise_abort(abort_addr, rank);
     }
-    // ---- leave: everyone is past its last use of tensor memory ----
+    // ---- leave: everyone is past its last use of tensor memory and of the other block's barriers ----
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (tid == 0 && *abort_flag) atomicExch(a.status, kGemmStatusTimeout);
+    cluster_sync_all();
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
     }
 }
 

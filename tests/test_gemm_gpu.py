@@ -58,3 +58,12 @@ def test_arguments():
     assert lib.quintrit_b200_gemm_i32(m.handle, act.ctypes.data_as(i8p), 160, 1, out.ctypes.data_as(i32p), 10) == 4
     assert lib.quintrit_b200_gemm_i32(m.handle, None, 160, 1, out.ctypes.data_as(i32p), 64) == 1
     assert lib.quintrit_b200_gemm_i32(None, act.ctypes.data_as(i8p), 160, 1, out.ctypes.data_as(i32p), 64) == 14
+
+
+@pytest.mark.parametrize("rows,cols,batch", [(1, 5, 1), (127, 255, 31), (128, 256, 32), (129, 257, 33), (255, 272, 64), (256, 512, 224), (257, 1040, 225), (384, 3088, 255), (640, 768, 256), (19200, 336, 33), (38144, 512, 256)])
+def test_edges_of_the_batched_projection(rows, cols, batch):
+    """Row tiles that fill a pair of blocks or half of one, columns around a stage, batches around a step of the instruction's N, vectors read in place
+    and copied, one item for a pair of blocks and several: exact integers."""
+    trits, acts = _case(rows, cols, batch, 3 * rows + cols + batch)
+    got = q.Matrix.from_trits(trits, rows, cols).gemm_i32(acts)
+    assert np.array_equal(got, (acts.astype(np.float32) @ trits.astype(np.float32).T).astype(np.int64))  # sums below 2^24: floats hold them exactly
