@@ -2159,6 +2159,7 @@ namespace {
 
 std::mutex g_gemm_lock;
 constexpr int kGemmMaxParts = kAccPartsMax;
+constexpr size_t kGemmPartRows = size_t(kGemmMaxParts) * kGemmMaxN;  // rows of a buffer for partial sums: parts x vectors is no more
 constexpr size_t kGemmSmemLimit = 227 * 1024;  // dynamic shared memory a CTA may ask for on this device
 // Writes a matrix into a two-bit copy from row tile `tile0` on; the copy's bytes are 0x55 (on the default stream, before).
 cudaError_t gemm_copy_weights(const quintrit_b200_matrix* m, uint8_t* copy, int tile0) {
@@ -2192,11 +2193,11 @@ int gemm_prepare(quintrit_b200_matrix* m) {
     return QUINTRIT_OK;
 }
 
-// One launch for up to kGemmMaxN activation vectors that are on the device ([batch][cols]); d_out is [batch][rows].
+// One launch for `batch` activation vectors that are on the device ([batch][cols]); d_out is [batch][rows]. (Vectors whose pitch or address the TMA cannot take: up to kGemmMaxN.)
 // With `defer`, a product whose K dimension is split leaves its parts where they are and describes them in *defer for the kernel that consumes the
 // sums (which adds them); otherwise a second kernel adds the parts into d_out.
 // `status` is the word a time-out is reported in: the matrix's own by default, a decoder's for the launches a decoder makes (one read-back per call).
-// `parts` is the buffer for the partial sums of a split K dimension (kGemmMaxParts x kGemmMaxN x rows values): the matrix's own, made on first need, by default.
+// `parts` is the buffer for the partial sums of a split K dimension (kGemmPartRows x rows values): the matrix's own, made on first need, by default.
 int gemm_launch(quintrit_b200_matrix* m, const int8_t* d_act, int batch, int32_t* d_out, cudaStream_t stream, int ldo = 0, AccView* defer = nullptr, unsigned int* status = nullptr,
                 int32_t* parts = nullptr) {
     if (ldo == 0) ldo = static_cast<int>(m->rows);
@@ -2205,7 +2206,8 @@ int gemm_launch(quintrit_b200_matrix* m, const int8_t* d_act, int batch, int32_t
     int rc = tensor_map_encoder(&encode);
     if (rc != QUINTRIT_OK) return rc;
     const int gblocks = static_cast<int>(gemm_blocks(m->cols));
-    const int n = (batch + 31) / 32 * 32, k_pad = gblocks * kGemmStageCols;  // the pair's instruction takes multiples of 32
+    const int tiles = (batch + kGemmMaxN - 1) / kGemmMaxN, n = ((batch + tiles - 1) / tiles + 31) / 32 * 32;  // token tiles of equal size; the pair's instruction takes multiples of 32
+    const int k_pad = gblocks * kGemmStageCols;
     // The TMA reads the caller's vectors in place when their pitch and address allow it (columns and vectors beyond the matrix read as zeros);
     // otherwise they are first copied into a zero-padded matrix with a pitch of whole stages.
     const bool in_place = m->cols % 16 == 0 && reinterpret_cast<uintptr_t>(d_act) % 16 == 0;
@@ -2226,37 +2228,38 @@ int gemm_launch(quintrit_b200_matrix* m, const int8_t* d_act, int batch, int32_t
     GemmArgs a;
     a.w = m->d_gemm_w, a.out = d_out, a.status = status != nullptr ? status : m->d_gemm_status;
     a.rows = static_cast<int>(m->rows), a.pairs = static_cast<int>(gemm_row_tiles(m->rows) / 2), a.blocks = gblocks;
-    a.n = n, a.batch = batch, a.ldo = ldo;
+    a.n = n, a.batch = batch, a.token_tiles = tiles, a.ldo = ldo;
     a.stages = gemm_stages_for(n, kGemmSmemLimit);
     if (const char* v = std::getenv("QUINTRIT_B200_GEMM_STAGES")) a.stages = std::max(kGemmGroups, std::min(std::atoi(v), a.stages));  // experiments: fewer stages (one a decode group at least)
     a.spin_limit = 1u << 16;  // polls of up to 20 us each: about a second before a wait gives up
-    // Work items are (pair of row tiles, K part); K is split (at most kGemmMaxParts parts) where the items of whole rows would leave multiprocessors idle: the cost of a split, in
+    // Work items are (pair of row tiles, K part, token tile); K is split (at most kGemmMaxParts parts, and no more than their buffer holds) where the items of whole rows would leave multiprocessors idle: the cost of a split, in
     // cycles, is the largest number of items a pair gets times (the stages of an item at four cycles a vector, or what handing them on takes, plus an end), plus the
     // bytes of the partial sums, written here and read by the consumer, at about 4 TB/s.
     const int sm_pairs = m->sm_count / 2;
     const long stage = std::max(4 * n + 36, 700), end = 2000 + 16 * n;
     int ksplit = 1;
     long best = -1;
-    for (int ks = 1; ks <= std::min(kGemmMaxParts, a.blocks); ++ks) {
+    const int most = std::max(1, std::min({kGemmMaxParts, a.blocks, static_cast<int>(kGemmPartRows / batch)}));
+    for (int ks = 1; ks <= most; ++ks) {
         const int per = (a.blocks + ks - 1) / ks, parts = (a.blocks + per - 1) / per;
-        const long waves = (long(a.pairs) * parts + sm_pairs - 1) / sm_pairs;
+        const long waves = (long(a.pairs) * parts * tiles + sm_pairs - 1) / sm_pairs;
         const long cost = waves * (per * stage + end) + (parts > 1 ? static_cast<long>(2.0 * parts * double(batch) * double(m->rows) * 4.0 / 2160.0) : 0);
         if (best < 0 || cost < best) best = cost, ksplit = parts;
     }
-    if (const char* v = std::getenv("QUINTRIT_B200_GEMM_KSPLIT")) ksplit = std::max(1, std::min({std::atoi(v), a.blocks, kGemmMaxParts}));
+    if (const char* v = std::getenv("QUINTRIT_B200_GEMM_KSPLIT")) ksplit = std::max(1, std::min(std::atoi(v), most));
     a.blocks_per_item = (a.blocks + ksplit - 1) / ksplit;
     ksplit = (a.blocks + a.blocks_per_item - 1) / a.blocks_per_item;
     if (ksplit > 1) {
         if (parts == nullptr) {
             if (m->d_gemm_parts == nullptr) {
                 std::lock_guard<std::mutex> hold(g_gemm_lock);
-                if (m->d_gemm_parts == nullptr) QTB_CUDA(cudaMalloc(&m->d_gemm_parts, size_t(kGemmMaxParts) * kGemmMaxN * m->rows * sizeof(int32_t)));
+                if (m->d_gemm_parts == nullptr) QTB_CUDA(cudaMalloc(&m->d_gemm_parts, kGemmPartRows * m->rows * sizeof(int32_t)));
             }
             parts = m->d_gemm_parts;
         }
         a.out = parts, a.ldo = static_cast<int>(m->rows);
     }
-    gemm_i8_tcgen05_kernel<<<2 * std::min(a.pairs * ksplit, sm_pairs), kGemmThreads, gemm_smem_bytes(n, a.stages), stream>>>(map, a);
+    gemm_i8_tcgen05_kernel<<<2 * std::min(a.pairs * ksplit * tiles, sm_pairs), kGemmThreads, gemm_smem_bytes(n, a.stages), stream>>>(map, a);
     ++g_launches;
     if (ksplit > 1 && defer != nullptr) {
         *defer = AccView{parts, ksplit, size_t(batch) * m->rows, static_cast<int>(m->rows)};
@@ -2337,7 +2340,12 @@ extern "C" int quintrit_b200_gemm_i32(quintrit_b200_matrix_t* matrix, const int8
 // ---- prompt ingestion: a chunk of tokens per pass, projections on the tensor cores -------------------------------------------------
 namespace {
 
-constexpr int kPrefillMax = kGemmMaxN;
+// Tokens of a pass. Attention's blocks are as long as the cache before their tokens, products are tiles of 256 vectors on 74 pairs of multiprocessors: with more of both in a
+// launch less of the last wave is empty. The feed-forward half goes in portions of kPortionMax, whose 32-bit gate and up sums (184 KB a token of the
+// Falcon3-10B shape) stay in L2 on their way to the activation step. 1000 tokens through four such layers: 4654 us in passes of 256, 3466 so.
+constexpr int kPrefillMax = 1024, kPortionMax = 512;
+inline int prefill_rows(const quintrit_b200_decoder* d) { return std::max(kGemmMaxN, std::min(kPrefillMax, (d->ctx + 255) / 256 * 256)); }  // tokens that the step buffers hold
+inline int prefill_portions(const quintrit_b200_decoder* d) { return (prefill_rows(d) + kPortionMax - 1) / kPortionMax; }
 
 // The batched products of a decoder: q | k | v and gate | up of a layer are stacked row-wise into one matrix each where their row counts are whole
 // tiles (one launch instead of three or two, and no launch too small to fill the device); o and down keep their own two-bit copies. The partial
@@ -2395,7 +2403,8 @@ int decoder_gemm_prepare(quintrit_b200_decoder* d) {
         bool all_stacked = true;
         for (int l = 0; l < d->layers; ++l) all_stacked = all_stacked && d->pf.stack[size_t(l) * 2 + (kind == 0 ? 0 : 1)] != nullptr;
         if (second_of_stack && all_stacked && (kind == 0 || kind == 2)) continue;  // the stack's one buffer is parts[first of the kind]
-        if ((rc = dev_alloc(d, &d->pf.parts[k], size_t(kGemmMaxParts) * kGemmMaxN * rows_kind[kind], false)) != QUINTRIT_OK) return rc;
+        const size_t portions = k == 6 ? prefill_portions(d) : 1;  // the down sums of every portion wait for the next layer's norm
+        if ((rc = dev_alloc(d, &d->pf.parts[k], portions * kGemmPartRows * rows_kind[kind], false)) != QUINTRIT_OK) return rc;
     }
     QTB_CUDA(cudaFuncSetAttribute(gemm_i8_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmemLimit)));
     QTB_CUDA(cudaDeviceSynchronize());
@@ -2405,15 +2414,15 @@ int decoder_gemm_prepare(quintrit_b200_decoder* d) {
 
 int prefill_buffers(quintrit_b200_decoder* d) {
     if (d->pf.x != nullptr || d->lay) return QUINTRIT_OK;  // (a layered decoder made its buffers when it was created)
-    const size_t B = kPrefillMax, H = d->hidden, I = d->inter, qd = d->q_dim, kvd = d->kv_dim, hd = d->head_dim;
+    const size_t B = prefill_rows(d), P = std::min<size_t>(B, kPortionMax), H = d->hidden, I = d->inter, qd = d->q_dim, kvd = d->kv_dim, hd = d->head_dim;
     int rc;
     if ((rc = dev_alloc(d, &d->pf.tokens, B)) != QUINTRIT_OK || (rc = dev_alloc(d, &d->pf.pos, 4)) != QUINTRIT_OK || (rc = dev_alloc(d, &d->pf.x, B * H)) != QUINTRIT_OK ||
         (rc = dev_alloc(d, &d->pf.q, B * qd)) != QUINTRIT_OK || (rc = dev_alloc(d, &d->pf.part_acc, B * d->q_heads * 4 * hd)) != QUINTRIT_OK ||
         (rc = dev_alloc(d, &d->pf.part_ms, B * d->q_heads * 8)) != QUINTRIT_OK || (rc = dev_alloc(d, &d->pf.s_h, B)) != QUINTRIT_OK ||
         (rc = dev_alloc(d, &d->pf.s_q, B)) != QUINTRIT_OK || (rc = dev_alloc(d, &d->pf.s_i, B)) != QUINTRIT_OK || (rc = dev_alloc(d, &d->pf.a8_h, B * H)) != QUINTRIT_OK ||
-        (rc = dev_alloc(d, &d->pf.a8_q, B * qd)) != QUINTRIT_OK || (rc = dev_alloc(d, &d->pf.a8_i, B * I)) != QUINTRIT_OK ||
+        (rc = dev_alloc(d, &d->pf.a8_q, B * qd)) != QUINTRIT_OK || (rc = dev_alloc(d, &d->pf.a8_i, P * I)) != QUINTRIT_OK ||
         (rc = dev_alloc(d, &d->pf.acc_qkv, B * (qd + 2 * kvd))) != QUINTRIT_OK || (rc = dev_alloc(d, &d->pf.acc_o, B * H)) != QUINTRIT_OK ||
-        (rc = dev_alloc(d, &d->pf.acc_gu, B * 2 * I)) != QUINTRIT_OK || (rc = dev_alloc(d, &d->pf.acc_down, B * H)) != QUINTRIT_OK)
+        (rc = dev_alloc(d, &d->pf.acc_gu, P * 2 * I)) != QUINTRIT_OK || (rc = dev_alloc(d, &d->pf.acc_down, B * H)) != QUINTRIT_OK)
         return rc;
     return QUINTRIT_OK;
 }
@@ -2448,19 +2457,22 @@ int prefill_layers(quintrit_b200_decoder* d, int n, const BatchTarget& tg) {
     // Projections whose K dimension is split leave their parts to the kernel that consumes the sums (AccView); only the last layer's down
     // projection is completed by a pass of its own, because the final norm of a later launch reads it.
     const bool defer = std::getenv("QUINTRIT_B200_GEMM_DEFER_OFF") == nullptr;
-    AccView v_q{}, v_k{}, v_v{}, v_o{}, v_gate{}, v_up{}, v_down{};
+    AccView v_q{}, v_k{}, v_v{}, v_o{}, v_gate{}, v_up{};
+    std::vector<AccView> v_down(prefill_portions(d));
     auto view = [&](AccView* v) { return defer ? v : nullptr; };
     unsigned int* st = d->d_counters + 2;  // the decoder's status word: a time-out in a batched product is read back with the decoder's other failures
     for (int l = 0; l < d->layers; ++l) {
         const float* sc = d->scales.data() + l * 7;
-        NormQuantArgs n1{};
-        n1.x = d->pf.x, n1.b_x = H;
-        if (l > 0) n1.acc_prev = d->pf.acc_down, n1.b_acc = H, n1.scale_prev = d->pf.s_i, n1.ws_prev = d->scales[(l - 1) * 7 + 6];
-        n1.norm_w = d->norms[l * 4 + 0], n1.eps = d->eps, n1.n = H;
-        n1.q_out = d->pf.a8_h, n1.b_q = H, n1.scale_out = d->pf.s_h, n1.b_scale = 1;
-        if (l > 0) n1.v_prev = defer ? v_down : AccView{d->pf.acc_down, 1, 0, H};
-        launch_norm_quant_rows(n1, n, s);
-        QTB_LAUNCH_CHECK();
+        for (int t0 = 0; t0 < n; t0 += l > 0 ? kPortionMax : n) {  // (the sums of the layer before lie in portions)
+            NormQuantArgs n1{};
+            n1.x = d->pf.x + size_t(t0) * H, n1.b_x = H;
+            if (l > 0) n1.acc_prev = d->pf.acc_down + size_t(t0) * H, n1.b_acc = H, n1.scale_prev = d->pf.s_i + t0, n1.ws_prev = d->scales[(l - 1) * 7 + 6];
+            n1.norm_w = d->norms[l * 4 + 0], n1.eps = d->eps, n1.n = H;
+            n1.q_out = d->pf.a8_h + size_t(t0) * H, n1.b_q = H, n1.scale_out = d->pf.s_h + t0, n1.b_scale = 1;
+            if (l > 0) n1.v_prev = defer ? v_down[t0 / kPortionMax] : AccView{d->pf.acc_down + size_t(t0) * H, 1, 0, H};
+            launch_norm_quant_rows(n1, l > 0 ? std::min(kPortionMax, n - t0) : n, s);
+            QTB_LAUNCH_CHECK();
+        }
         if (quintrit_b200_matrix* sq = d->pf.stack[size_t(l) * 2]) {  // q | k | v as one product
             if ((rc = gemm_launch(sq, d->pf.a8_h, n, d->pf.acc_qkv, s, qkv, &v_q, st, d->pf.parts[0])) != QUINTRIT_OK) return rc;
             v_k = v_q, v_k.base += qd;
@@ -2505,24 +2517,31 @@ int prefill_layers(quintrit_b200_decoder* d, int n, const BatchTarget& tg) {
         n2.v_prev = defer ? v_o : AccView{d->pf.acc_o, 1, 0, H};
         launch_norm_quant_rows(n2, n, s);
         QTB_LAUNCH_CHECK();
-        if (quintrit_b200_matrix* sg = d->pf.stack[size_t(l) * 2 + 1]) {  // gate | up as one product
-            if ((rc = gemm_launch(sg, d->pf.a8_h, n, d->pf.acc_gu, s, 2 * I, &v_gate, st, d->pf.parts[4])) != QUINTRIT_OK) return rc;
-            v_up = v_gate, v_up.base += I;
-        } else if ((rc = gemm_launch(mat(l, 4), d->pf.a8_h, n, d->pf.acc_gu, s, 2 * I, view(&v_gate), st, d->pf.parts[4])) != QUINTRIT_OK ||
-                   (rc = gemm_launch(mat(l, 5), d->pf.a8_h, n, d->pf.acc_gu + I, s, 2 * I, view(&v_up), st, d->pf.parts[5])) != QUINTRIT_OK) {
-            return rc;
+        for (int t0 = 0; t0 < n; t0 += kPortionMax) {
+            const int m = std::min(kPortionMax, n - t0), portion = t0 / kPortionMax;
+            const int8_t* a8 = d->pf.a8_h + size_t(t0) * H;
+            if (quintrit_b200_matrix* sg = d->pf.stack[size_t(l) * 2 + 1]) {  // gate | up as one product
+                if ((rc = gemm_launch(sg, a8, m, d->pf.acc_gu, s, 2 * I, &v_gate, st, d->pf.parts[4])) != QUINTRIT_OK) return rc;
+                v_up = v_gate, v_up.base += I;
+            } else if ((rc = gemm_launch(mat(l, 4), a8, m, d->pf.acc_gu, s, 2 * I, view(&v_gate), st, d->pf.parts[4])) != QUINTRIT_OK ||
+                       (rc = gemm_launch(mat(l, 5), a8, m, d->pf.acc_gu + I, s, 2 * I, view(&v_up), st, d->pf.parts[5])) != QUINTRIT_OK) {
+                return rc;
+            }
+            const bool gu_views = defer || d->pf.stack[size_t(l) * 2 + 1] != nullptr;
+            ActQuantArgs aq{};
+            aq.acc_gate = d->pf.acc_gu, aq.acc_up = d->pf.acc_gu + I, aq.b_acc = 2 * I, aq.act_scale = d->pf.s_h + t0, aq.b_scale = 1;
+            aq.ws_gate = sc[4], aq.ws_up = sc[5];
+            aq.n = I, aq.relu2 = d->arch == QUINTRIT_B200_ARCH_BITNET;
+            aq.sub_norm_w = d->norms[l * 4 + 3], aq.eps = d->eps;
+            aq.q_out = d->pf.a8_i, aq.b_q = I, aq.scale_out = d->pf.s_i + t0;
+            aq.v_gate = gu_views ? v_gate : AccView{aq.acc_gate, 1, 0, aq.b_acc}, aq.v_up = gu_views ? v_up : AccView{aq.acc_up, 1, 0, aq.b_acc};
+            launch_act_quant_rows(aq, m, s);
+            QTB_LAUNCH_CHECK();
+            const size_t rows = mat(l, 6)->rows;
+            if ((rc = gemm_launch(mat(l, 6), d->pf.a8_i, m, d->pf.acc_down + size_t(t0) * H, s, 0, l + 1 < d->layers ? view(&v_down[portion]) : nullptr, st,
+                                  d->pf.parts[6] + portion * kGemmPartRows * rows)) != QUINTRIT_OK)
+                return rc;
         }
-        const bool gu_views = defer || d->pf.stack[size_t(l) * 2 + 1] != nullptr;
-        ActQuantArgs aq{};
-        aq.acc_gate = d->pf.acc_gu, aq.acc_up = d->pf.acc_gu + I, aq.b_acc = 2 * I, aq.act_scale = d->pf.s_h, aq.b_scale = 1;
-        aq.ws_gate = sc[4], aq.ws_up = sc[5];
-        aq.n = I, aq.relu2 = d->arch == QUINTRIT_B200_ARCH_BITNET;
-        aq.sub_norm_w = d->norms[l * 4 + 3], aq.eps = d->eps;
-        aq.q_out = d->pf.a8_i, aq.b_q = I, aq.scale_out = d->pf.s_i;
-        aq.v_gate = gu_views ? v_gate : AccView{aq.acc_gate, 1, 0, aq.b_acc}, aq.v_up = gu_views ? v_up : AccView{aq.acc_up, 1, 0, aq.b_acc};
-        launch_act_quant_rows(aq, n, s);
-        QTB_LAUNCH_CHECK();
-        if ((rc = gemm_launch(mat(l, 6), d->pf.a8_i, n, d->pf.acc_down, s, 0, l + 1 < d->layers ? view(&v_down) : nullptr, st, d->pf.parts[6])) != QUINTRIT_OK) return rc;
     }
     return QUINTRIT_OK;
 }
@@ -2532,7 +2551,7 @@ int enqueue_prefill_chunk(quintrit_b200_decoder* d, int n, uint32_t pos0, bool w
     const int H = d->hidden;
     QTB_CUDA(cudaMemcpyAsync(d->pf.pos, &pos0, sizeof pos0, cudaMemcpyHostToDevice, s));
     int rc;
-    // A full chunk is about 1200 launches; from the third full chunk on they are replayed as one CUDA graph (the first runs as it is and makes
+    // A full pass is about 500 launches of 40 layers; from the third full chunk on they are replayed as one CUDA graph (the first runs as it is and makes
     // every lazy allocation, the second is captured). The position and the tokens are read from device memory, so one graph serves every chunk.
     if (n == kPrefillMax && tg.own && d->pf.graph_ready) {
         QTB_CUDA(cudaGraphLaunch(d->pf.graph, s));
@@ -3142,7 +3161,7 @@ extern "C" int quintrit_b200_batch_create(quintrit_b200_decoder_t* decoder, uint
         int rc = check_decoder(decoder);
         if (rc != QUINTRIT_OK) return rc;
         quintrit_b200_decoder* d = decoder;
-        if (sequences == 0 || sequences > static_cast<uint32_t>(kPrefillMax)) return fail(QUINTRIT_ERR_INVALID_ARGUMENT, "sequences must be in [1, %d], got %u", kPrefillMax, sequences);
+        if (sequences == 0 || sequences > static_cast<uint32_t>(kGemmMaxN)) return fail(QUINTRIT_ERR_INVALID_ARGUMENT, "sequences must be in [1, %d], got %u", kGemmMaxN, sequences);
         if (!prefill_available(d)) return fail(QUINTRIT_ERR_UNSUPPORTED, "this decoder has no batched pass (block-scaled or tensor-parallel model)");
         DeviceGuard g(d->device);
         if ((rc = prefill_buffers(d)) != QUINTRIT_OK) return rc;

@@ -11,8 +11,8 @@
 // made on the device the first time a matrix is used here: two bits per trit (0.25 bytes per weight), placed so that a mask, at most two shifts and one
 // byte permute turn a quarter of a word into four int8 operands that are already in K order. The product runs as tcgen05.mma.kind::i8 on pairs of
 // multiprocessors (cta_group::2) with the accumulator in tensor memory:
-//   * a work item is 256 weight rows (the M of the instruction, 128 a block of the pair) times a range of 256-column stages (K); the batch is the N
-//     (32..256). Each block of a pair holds half of the batch's activations, so a stage costs it n / 2 x 256 + 8192 bytes of shared memory and of L2 traffic: with a
+//   * a work item is 256 weight rows (the M of the instruction, 128 a block of the pair) times a range of 256-column stages (K) times up to 256 vectors (the N).
+//     Each block of a pair holds half of the batch's activations, so a stage costs it n / 2 x 256 + 8192 bytes of shared memory and of L2 traffic: with a
 //     block for itself (n x 256 + 8192) the activations' way through L2 would be longer than the products;
 //   * sixteen warps decode, in four groups that take the stages round-robin: a thread takes a row's 64 bytes of a stage from shared memory and writes the row's
 //     256 int8 operands into its lane of TENSOR MEMORY with tcgen05.st (64 columns a group). Operands that threads
@@ -66,9 +66,10 @@ struct GemmArgs {
     int rows, pairs;       // weight rows; pairs of row tiles
     int blocks;            // stages (256 columns) of a row
     int ldo;               // elements between the results of consecutive vectors in `out` (rows, or more when the results go into a wider row)
-    int n;                 // instruction N: the batch rounded up to a multiple of 32
-    int batch;             // activation vectors actually present (columns of the accumulator that are written out)
-    int blocks_per_item;   // stages of one work item (a pair of row tiles x a K part)
+    int n;                 // instruction N: vectors of a token tile, a multiple of 32
+    int batch;             // activation vectors actually present
+    int token_tiles;       // of n vectors each; the last may be ragged
+    int blocks_per_item;   // stages of one work item (a pair of row tiles x a K part x a token tile)
     int stages;
     unsigned int spin_limit;
 };
@@ -319,8 +320,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rank = cluster_rank();
-    // work items: (pair of row tiles, K part), taken round-robin by the pairs; an item is `per` stages of one pair of tiles
-    const int per = a.blocks_per_item, parts = (a.blocks + per - 1) / per, items = a.pairs * parts, first = blockIdx.x >> 1, step = gridDim.x >> 1;
+    // work items: (pair of row tiles, K part, token tile), taken round-robin by the pairs; an item is `per` stages of one pair of tiles. The token tiles of the
+    // same weights are neighbours, so that HBM is read for one of them
+    const int per = a.blocks_per_item, parts = (a.blocks + per - 1) / per, tiles = a.token_tiles, items = a.pairs * parts * tiles, first = blockIdx.x >> 1, step = gridDim.x >> 1;
+    auto part_of = [&](int item) { return item / tiles % parts; };
+    auto pair_of = [&](int item) { return item / (tiles * parts); };
     constexpr uint32_t kOperandCol = 256;  // tensor memory: the accumulator in columns [0, n), the operands of group g in 64 columns from 256 + 64 g
 
     if (tid == 0) {
@@ -350,14 +354,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
         int it0 = 0, until = 0;  // stages of the sequence before this item; behind this warp's last issued stage
         bool okay = true;
         for (int item = first; item < items && okay; item += step) {
-            const int tile = (item / parts) * 2 + static_cast<int>(rank), kb0 = (item % parts) * per, nkb = min(per, a.blocks - kb0);
+            const int tile = pair_of(item) * 2 + static_cast<int>(rank), kb0 = part_of(item) * per, nkb = min(per, a.blocks - kb0);
             const uint8_t* src = a.w + (size_t(tile) * a.blocks + kb0) * kGemmStageBytes;
             for (int k = (mine - it0) & (kGemmLoadWarps - 1); k < nkb; k += kGemmLoadWarps) {
                 const int it = it0 + k, s = it % S;
                 if (!(okay = __all_sync(0xffffffffu, mbar_wait(empty(s), ((it / S) & 1) ^ 1, abort_flag, a.spin_limit)))) break;
                 if (elect_one()) {
                     const uint32_t dst = b_base + s * act_bytes;
-                    const int x = (kb0 + k) * kGemmStageCols, y = static_cast<int>(rank) * (n / 2);
+                    const int x = (kb0 + k) * kGemmStageCols, y = item % tiles * n + static_cast<int>(rank) * (n / 2);
                     mbar_expect_tx(loaded(s), kGemmStageBytes + act_bytes);
                     bulk_load(raw_base + s * kGemmStageBytes, src + size_t(k) * kGemmStageBytes, kGemmStageBytes, loaded(s));
                     tma_load_2d(dst, &act_map, x, y, loaded(s));
@@ -383,7 +387,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
             const uint64_t b_desc0 = smem_desc(b_base, 16, 1024, 2);
             const uint32_t b_stage16 = act_bytes >> 4, b_half16 = act_bytes >> 5;
             for (int item = first; item < items && okay; item += step, ++j) {
-                const int kb0 = (item % parts) * per, nkb = min(per, a.blocks - kb0);
+                const int kb0 = part_of(item) * per, nkb = min(per, a.blocks - kb0);
                 if (!(okay = __all_sync(0xffffffffu, mbar_wait(acc_empty, (j & 1) ^ 1, abort_flag, a.spin_limit)))) break;  // the previous item's accumulator has been read
                 for (int k = 0; k < nkb; ++k, ++it) {
                     const int g = it & (kGemmGroups - 1);
@@ -422,12 +426,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
         auto finish = [&](int item, int j) {  // item `item`, the pair's j-th
             okay = __all_sync(0xffffffffu, mbar_wait(acc_full, j & 1, abort_flag, a.spin_limit));
             if (!okay) return;
-            const int row = ((item / parts) * 2 + static_cast<int>(rank)) * kGemmM + r;
-            gemm_write_out(lanes + c0, to_empty, own, a.out + (size_t(item % parts) * a.batch + c0) * a.ldo + row, a.ldo, row < a.rows ? min(own, a.batch - c0) : 0);
+            const int row = (pair_of(item) * 2 + static_cast<int>(rank)) * kGemmM + r, vector = item % tiles * n + c0;
+            gemm_write_out(lanes + c0, to_empty, own, a.out + (size_t(part_of(item)) * a.batch + vector) * a.ldo + row, a.ldo, row < a.rows ? min(own, a.batch - vector) : 0);
         };
         int j = 0, it0 = 0, before = -1;  // `before`: the item whose accumulator has not been written out yet
         for (int item = first; item < items && okay; item += step, ++j) {
-            const int nkb = min(per, a.blocks - (item % parts) * per);
+            const int nkb = min(per, a.blocks - part_of(item) * per);
             // A group decodes its first stage of an item before it writes out the item before. (All groups' reads before any store, or the reads first, or whichever is
             // ready first: 0 to 3 us slower of 37 at 46080 x 3072, 256 vectors.)
             bool owed = before >= 0;

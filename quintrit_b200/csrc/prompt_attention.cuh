@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(kTokenTileThreads, 2) attention_tile_kernel(At
     float2* s_vs = reinterpret_cast<float2*>(s_q + R * hd);                              // [R][64]: vs twice (packed operand); before that the score
     float* s_ms = reinterpret_cast<float*>(s_vs + R * kTokenTileRows);                        // [R][64]
     const int kvh = blockIdx.x, c = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h0 = kvh * G;
-    const int pos0 = static_cast<int>(a.pos[0]), first = (pos0 / kTokenTile + static_cast<int>(blockIdx.z)) * kTokenTile;
+    const int pos0 = static_cast<int>(a.pos[0]), first = (pos0 / kTokenTile + static_cast<int>(gridDim.z - 1 - blockIdx.z)) * kTokenTile;  // the last tokens, whose rows are most, first
     const int last = min(first + kTokenTile, pos0 + a.tokens) - 1;  // the last position of the tile that is a token of the chunk
     if (last < first) return;
     const int n_kv = min(max((last + 1 + 255) / 256 * 256, 256), a.ctx);

@@ -99,3 +99,21 @@ def test_many_chunks_replay_one_graph():
     la, ta = a.forward(want_next, 800)
     lb, tb = b.forward(got_next, 800)
     assert np.array_equal(la.view(np.uint32), lb.view(np.uint32)) and ta == tb
+
+
+@pytest.mark.parametrize("arch,inter,n", [(q.ARCH_LLAMA, 512, 513), (q.ARCH_LLAMA, 4128, 1000), (q.ARCH_BITNET, 512, 1025), (q.ARCH_LLAMA, 512, 1600)])
+def test_long_passes_equal_short_ones(arch, inter, n):
+    """Passes of up to 1024 tokens, their feed-forward half in portions of 512, products over several token tiles: a portion of one token, ragged
+    tiles, a second pass of one token and a longer one, against calls of at most 200 tokens (one token tile, one portion)."""
+    spec = synth.make_model(arch, arch == q.ARCH_BITNET, 256, inter, 2, 4, 2, 64, 300, 1792, 500000.0, 1e-5, config=n, random_norms=True, tied=arch == q.ARCH_BITNET)
+    tokens = synth.prompt_tokens(9, n, spec["vocab"])
+    a, b = q.Decoder(spec), q.Decoder(spec)
+    for at in range(0, n, 200):
+        want, want_next = a.prefill(tokens[at:at + 200], at)
+    got, got_next = b.prefill(tokens)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32)) and got_next == want_next
+    for step in range(3):  # the caches are the same
+        la, ta = a.forward(want_next, n + step)
+        lb, tb = b.forward(got_next, n + step)
+        assert np.array_equal(la.view(np.uint32), lb.view(np.uint32)) and ta == tb
+        want_next = got_next = ta
