@@ -603,6 +603,7 @@ __global__ void __launch_bounds__(kAttnThreads) attention_kernel(AttnArgs a) {
 }
 
 // ---- the same attention for all query heads of a KV head at once --------------------------------------------------------
+// For head sizes that row_attention.cuh has no kernel for (it is faster where it has one).
 // Grid (kv_heads, chunks, tokens), 288 threads: the G query heads that share a KV head (grouped-query attention) share one
 // pass over its keys and values. The arithmetic per head is attention_kernel's, operation for operation (the reference's
 // order: attention.rs:402-469); what changes is who does it and how the rows arrive:

@@ -11,6 +11,7 @@
 #include "gemv_lut.cuh"
 #include "megakernel.cuh"
 #include "prompt_attention.cuh"
+#include "row_attention.cuh"
 #include "row_kernels.cuh"
 
 namespace qtb {
@@ -54,6 +55,7 @@ struct quintrit_b200_decoder {
     qtb::AttnGqaKernel attn_gqa = nullptr;     // one-launch-per-step and batched paths: the grouped attention kernel, if this model's shape has one
     size_t attn_gqa_smem = 0;
     qtb::AttnGqaKernel attn_tile = nullptr;    // prompt chunks: eight tokens per block, if this model's shape has that kernel
+    qtb::AttnGqaKernel attn_rows = nullptr;    // the same for the head sizes it exists for, packed operations
     size_t attn_gqa_pad = 0;                   // experiments: extra shared memory per block, which lowers the number of resident blocks
     float* attn_out = nullptr;
     float *fac = nullptr, *fac_M = nullptr;
@@ -187,7 +189,10 @@ inline void launch_attention(quintrit_b200_decoder* d, AttnArgs at, int n, cudaS
         return;
     }
     // several tokens: the query heads of a KV head share one pass over its rows; one token: more, wider blocks pull the rows faster
-    if (d->attn_gqa != nullptr && n > 1)
+    const int group = d->q_heads / d->kv_heads;
+    if (d->attn_rows != nullptr && n > 1)
+        d->attn_rows<<<dim3(d->kv_heads, 4, n), kRowAttnThreads, row_attn_smem(group, d->head_dim), s>>>(at);
+    else if (d->attn_gqa != nullptr && n > 1)
         d->attn_gqa<<<dim3(d->kv_heads, 4, n), kAttnGqaThreads, d->attn_gqa_smem + d->attn_gqa_pad, s>>>(at);
     else
         attention_kernel<<<dim3(d->q_heads, 4, n), kAttnThreads, attention_smem(d->head_dim), s>>>(at);
