@@ -5,6 +5,7 @@
 #include <sys/stat.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <mutex>
@@ -1067,7 +1068,7 @@ int decoder_create_impl(const quintrit_b200_decoder_desc_t* desc, quintrit_b200_
         (rc = dev_alloc(d, &d->d_history, ctx + 1)) != QUINTRIT_OK || (rc = dev_alloc(d, &d->d_counters, 4)) != QUINTRIT_OK)
         return rc;
 
-    if ((rc = dev_alloc(d, &d->q8_d, std::max<size_t>({H, I, qd}) / 32 + 1)) != QUINTRIT_OK) return rc;
+    if ((rc = dev_alloc(d, &d->q8_d, std::max<size_t>({H, I, qd}) / 32 + 1)) != QUINTRIT_OK || (rc = decoder_report_init(d)) != QUINTRIT_OK) return rc;
     // The limit is a property of the kernel, shared by every decoder of the process: it is set to the most the device allows, so that a
     // later, smaller model does not lower it under an earlier, larger one.
     int smem_optin = 0;
@@ -1279,6 +1280,7 @@ int mega_setup(quintrit_b200_decoder* d, const quintrit_b200_decoder_desc_t* des
     a.q_dim_full = d->q_dim_full, a.inter_full = d->inter_full, a.vocab_base = d->tp_rank * d->vocab, a.h_slice = H / d->tp_world;
     if (d->tp_world > 1) a.v_inter = reinterpret_cast<float*>(d->tp_box + off_v);
     a.best_val = d->best_val, a.best_idx = d->best_idx, a.token = d->d_token, a.pos = d->d_pos, a.history = d->d_history;
+    a.steps = d->d_steps, a.report = d->report;
     a.bar = d->bar, a.status = d->d_counters + 2, a.trace = nullptr;
     d->mega_smem = mega_smem_bytes(a.attn_region, std::max(H, d->q_dim_full), H, L);
     // the table-base constant: measured once per device like the GEMV kernel's
@@ -1300,15 +1302,17 @@ int mega_setup(quintrit_b200_decoder* d, const quintrit_b200_decoder_desc_t* des
 int decoder_step(quintrit_b200_decoder* d) {
     if (d->tp_world > 1 && !d->tp_attached) return fail(QUINTRIT_ERR_INVALID_ARGUMENT, "the tensor-parallel group is not attached yet (quintrit_b200_decoder_tp_attach)");
     if (d->use_mega) {
-        QTB_CUDA(cudaMemsetAsync(d->bar, 0, 16 * sizeof(unsigned int), d->stream));
+        if (!d->bar_cleared) QTB_CUDA(cudaMemsetAsync(d->bar, 0, 16 * sizeof(unsigned int), d->stream));
+        d->bar_cleared = false;
         void* args[] = {&d->mega};
         QTB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(d->mega_kernel), dim3(d->sm_count), dim3(kMegaThreads), args, d->mega_smem, d->stream));
-        ++g_launches;
+        ++g_launches, ++d->launched;
         return QUINTRIT_OK;
     }
     int rc = decoder_graph(d);
     if (rc != QUINTRIT_OK) return rc;
     QTB_CUDA(cudaGraphLaunch(d->graph_step, d->stream));
+    ++d->launched;
     return QUINTRIT_OK;
 }
 
@@ -1327,6 +1331,32 @@ int decoder_check_status(quintrit_b200_decoder* d) {
     QTB_CUDA(cudaStreamSynchronize(d->stream));
     if (flag != 0) {  // the word is sticky on the device: clear it so that the decoder stays usable after the error
         cudaMemsetAsync(d->d_counters + 2, 0, sizeof(unsigned int), d->stream);
+        cudaMemcpyAsync(&d->launched, d->d_steps, sizeof(uint32_t), cudaMemcpyDeviceToHost, d->stream);  // steps that gave up have not been counted
+        cudaStreamSynchronize(d->stream);
+        return kernel_status_error(flag);
+    }
+    return QUINTRIT_OK;
+}
+
+// Waits until the last step launched has reported: everything it did is done then, though its last kernel may still be leaving. (Copies of the token and of the status word
+// and a wait for the stream took 12 to 20 us behind a step.) A kernel that gave up reports nothing: the stream runs dry, and its status tells why.
+int decoder_wait_report(quintrit_b200_decoder* d) {
+    const volatile uint32_t* steps = &d->report->steps;
+    for (unsigned int spins = 1; *steps != d->launched; ++spins) {
+#if defined(__x86_64__)
+        __builtin_ia32_pause();
+#endif
+        if (spins % 4096 != 0) continue;
+        const cudaError_t e = cudaStreamQuery(d->stream);
+        if (e == cudaErrorNotReady) continue;
+        if (e != cudaSuccess) return cuda_fail(e, "a decode step");
+        if (*steps == d->launched) break;
+        const int rc = decoder_check_status(d);
+        return rc != QUINTRIT_OK ? rc : fail(QUINTRIT_ERR_DEVICE, "a decode step ended without a result on the CUDA device");
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    if (const unsigned int flag = d->report->status) {
+        QTB_CUDA(cudaMemsetAsync(d->d_counters + 2, 0, sizeof(unsigned int), d->stream));  // sticky on the device: cleared so that the decoder stays usable after the error
         return kernel_status_error(flag);
     }
     return QUINTRIT_OK;
@@ -1861,8 +1891,9 @@ extern "C" int quintrit_b200_decoder_forward(quintrit_b200_decoder_t* decoder, u
         DeviceGuard g(d->device);
         if ((rc = decoder_set(d, token, pos)) != QUINTRIT_OK || (rc = decoder_step(d)) != QUINTRIT_OK) return rc;
         if (logits) QTB_CUDA(cudaMemcpyAsync(logits, d->logits, size_t(d->vocab) * sizeof(float), cudaMemcpyDeviceToHost, d->stream));
-        if (out_token) QTB_CUDA(cudaMemcpyAsync(out_token, d->d_token, sizeof(uint32_t), cudaMemcpyDeviceToHost, d->stream));
-        if ((rc = decoder_check_status(d)) != QUINTRIT_OK) return rc;
+        if ((rc = decoder_wait_report(d)) != QUINTRIT_OK) return rc;
+        if (logits) QTB_CUDA(cudaStreamSynchronize(d->stream));
+        if (out_token) *out_token = d->report->token;
         d->host_pos = pos + 1;
         return ok();
     });
@@ -3066,7 +3097,7 @@ struct quintrit_b200_batch {
     __half* x16 = nullptr;                 // [n_seq][hidden]: the final norm's output
     LayeredStore layered;                  // layered models: states and windows of the sequences instead of kc / vc
     std::vector<uint32_t> host_pos;        // tokens cached per sequence
-    std::vector<uint32_t> staged;          // host copy of the ids given to an asynchronous copy
+    std::vector<uint32_t> staged;          // host copy of a prompt's ids for the asynchronous copies
     std::vector<void*> allocs;
     // The launches of a step of n tokens (about 500 for 40 layers) are replayed as one CUDA graph from the third step of that size on: tokens,
     // sequence list and positions are read from device memory, so the graph of a size serves every step of that size.
@@ -3280,28 +3311,21 @@ extern "C" int quintrit_b200_batch_step(quintrit_b200_batch_t* batch, const uint
         if (logits != nullptr && logits_capacity < count * static_cast<size_t>(d->vocab)) return fail(QUINTRIT_ERR_BUFFER_TOO_SMALL, "logits hold %zu values, %zu are needed", logits_capacity, count * static_cast<size_t>(d->vocab));
         DeviceGuard g(d->device);
         cudaStream_t s = d->stream;
-        // the ids of both copies below, complete before the first copy is enqueued; the sequence list is always read from device memory (one
-        // graph per step size), so "all sequences in order" is written out
+        // The sequence list is always read from device memory (one graph per step size), so "all sequences in order" is written out; list and tokens travel by value.
         // Inside the step the tokens are ordered by the length of their sequences, longest first: the attention blocks of a launch are handed to the
         // multiprocessors in order, and with that order every multiprocessor gets long and short ones alike. order[k] = the caller's index z.
         std::vector<uint32_t> order(count);
         for (size_t z = 0; z < count; ++z) order[z] = static_cast<uint32_t>(z);
         auto seq_at = [&](uint32_t z) { return sequences != nullptr ? sequences[z] : z; };
         std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return b->host_pos[seq_at(x)] > b->host_pos[seq_at(y)]; });
-        b->staged.resize(count * (tokens != nullptr ? 2 : 1));
+        BatchBegin begin;
         for (size_t k = 0; k < count; ++k) {
-            b->staged[k] = seq_at(order[k]);
-            if (tokens != nullptr) b->staged[count + k] = tokens[order[k]];
+            begin.slot[k] = seq_at(order[k]);
+            begin.token[k] = tokens != nullptr ? tokens[order[k]] : 0u;
         }
         const uint32_t* slot = b->d_slot;
-        uint32_t* step_tokens = d->lay ? d->lay->tokens : d->pf.tokens;
-        QTB_CUDA(cudaMemcpyAsync(b->d_slot, b->staged.data(), count * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-        if (tokens != nullptr) {
-            QTB_CUDA(cudaMemcpyAsync(step_tokens, b->staged.data() + count, count * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-        } else {
-            gather_tokens_kernel<<<(n + 255) / 256, 256, 0, s>>>(step_tokens, b->d_last, slot, n);
-            QTB_LAUNCH_CHECK();
-        }
+        batch_begin_kernel<<<1, kReportTokens, 0, s>>>(begin, b->d_slot, d->lay ? d->lay->tokens : d->pf.tokens, tokens != nullptr ? nullptr : b->d_last, n);
+        QTB_LAUNCH_CHECK();
         BatchTarget tg;
         tg.kc = b->kc, tg.vc = b->vc, tg.pos = b->d_pos, tg.own = false;
         tg.seq.slot = slot, tg.seq.pos_stride = 1, tg.seq.cache_stride = batch_cache_stride(d);
@@ -3309,7 +3333,7 @@ extern "C" int quintrit_b200_batch_step(quintrit_b200_batch_t* batch, const uint
             int r = d->lay ? layered_batch_layers(b, n, tg) : prefill_layers(d, n, tg);
             if (r == QUINTRIT_OK) r = batch_head(b, n);
             if (r != QUINTRIT_OK) return r;
-            advance_batch_kernel<<<(n + 255) / 256, 256, 0, s>>>(b->d_pos, b->d_last, b->d_chosen, slot, n);
+            advance_batch_kernel<<<1, kReportTokens, 0, s>>>(b->d_pos, b->d_last, b->d_chosen, slot, n, d->d_steps, d->d_counters + 2, d->report);
             QTB_LAUNCH_CHECK();
             return QUINTRIT_OK;
         };
@@ -3336,14 +3360,14 @@ extern "C" int quintrit_b200_batch_step(quintrit_b200_batch_t* batch, const uint
             if ((rc = enqueue()) != QUINTRIT_OK) return rc;
             b->warm[n] = 1;
         }
-        std::vector<uint32_t> chosen(out_tokens != nullptr ? count : 0);
-        if (out_tokens) QTB_CUDA(cudaMemcpyAsync(chosen.data(), b->d_chosen, count * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        ++d->launched;
         if (logits)
             for (size_t k = 0; k < count; ++k)
                 QTB_CUDA(cudaMemcpyAsync(logits + size_t(order[k]) * d->vocab, b->logits + k * d->vocab, size_t(d->vocab) * sizeof(float), cudaMemcpyDeviceToHost, s));
-        if ((rc = decoder_check_status(d)) != QUINTRIT_OK) return rc;  // (waits for the stream)
+        if ((rc = decoder_wait_report(d)) != QUINTRIT_OK) return rc;
+        if (logits) QTB_CUDA(cudaStreamSynchronize(s));
         if (out_tokens)
-            for (size_t k = 0; k < count; ++k) out_tokens[order[k]] = chosen[k];
+            for (size_t k = 0; k < count; ++k) out_tokens[order[k]] = d->report->chosen[k];
         for (int z = 0; z < n; ++z) b->host_pos[sequences != nullptr ? sequences[z] : static_cast<uint32_t>(z)] += 1;
         return ok();
     });

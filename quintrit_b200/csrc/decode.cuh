@@ -1449,23 +1449,59 @@ __global__ void __launch_bounds__(kSampleThreads) sample_topk_kernel(const float
     *token = chosen;
 }
 
-// next position (the generation loop runs on the device: the token comes from argmax_kernel, the position from here)
-__global__ void advance_kernel(uint32_t* pos, uint32_t* history, const uint32_t* token) {
-    history[pos[0]] = token[0];
-    pos[0] += 1;
-}
-// the same for a step of several sequences: token z of the step belongs to sequence slot[z] (or z)
-__global__ void advance_batch_kernel(uint32_t* pos, uint32_t* last, const uint32_t* chosen, const uint32_t* slot, int n) {
-    const int z = blockIdx.x * blockDim.x + threadIdx.x;
-    if (z >= n) return;
-    const uint32_t s = slot != nullptr ? slot[z] : static_cast<uint32_t>(z);
-    last[s] = chosen[z];
-    pos[s] += 1;
-}
-// tokens of a step: the given ones, or the last chosen token of every listed sequence
-__global__ void gather_tokens_kernel(uint32_t* tokens, const uint32_t* last, const uint32_t* slot, int n) {
-    const int z = blockIdx.x * blockDim.x + threadIdx.x;
-    if (z < n) tokens[z] = last[slot != nullptr ? slot[z] : static_cast<uint32_t>(z)];
+// What a step tells the host: pinned host memory that the device writes, so that nothing has to be copied and no stream waited for. `steps` is written last, behind
+// everything else the step did.
+constexpr int kReportTokens = 256;
+struct StepReport {
+    uint32_t steps;   // steps done so far (a device-side count)
+    uint32_t status;  // the decoder's status word
+    uint32_t token;   // the greedy token of a single step
+    uint32_t chosen[kReportTokens];  // of a step of several sequences
+};
+__device__ __forceinline__ void report_step(StepReport* r, uint32_t* steps, const unsigned int* status) {  // one thread, behind its and (synchronised) others' writes to *r
+    *reinterpret_cast<volatile uint32_t*>(&r->status) = *reinterpret_cast<const volatile unsigned int*>(status);
+    const uint32_t n = *steps + 1;
+    *steps = n;
+    __threadfence_system();
+    *reinterpret_cast<volatile uint32_t*>(&r->steps) = n;
 }
 
+// token and position of a step (given by value: a copy from pageable memory each took 4 us of the stream and some of the host's), and the grid barrier's counter of the token kernel
+__global__ void step_begin_kernel(uint32_t* token, uint32_t* pos, uint32_t t, uint32_t p, unsigned int* bar) {
+    if (bar != nullptr && threadIdx.x < 16) bar[threadIdx.x] = 0u;
+    if (threadIdx.x == 0) *token = t, *pos = p;
+}
+
+// next position (the generation loop runs on the device: the token comes from argmax_kernel, the position from here)
+__global__ void advance_kernel(uint32_t* pos, uint32_t* history, const uint32_t* token, uint32_t* steps, const unsigned int* status, StepReport* report) {
+    const uint32_t t = token[0];
+    history[pos[0]] = t;
+    pos[0] += 1;
+    *reinterpret_cast<volatile uint32_t*>(&report->token) = t;
+    report_step(report, steps, status);
+}
+// the same for a step of several sequences (one block): token z of the step belongs to sequence slot[z]
+__global__ void __launch_bounds__(kReportTokens) advance_batch_kernel(uint32_t* pos, uint32_t* last, const uint32_t* chosen, const uint32_t* slot, int n, uint32_t* steps, const unsigned int* status,
+                                                                      StepReport* report) {
+    const int z = threadIdx.x;
+    if (z < n) {
+        const uint32_t s = slot[z], t = chosen[z];
+        last[s] = t;
+        pos[s] += 1;
+        *reinterpret_cast<volatile uint32_t*>(&report->chosen[z]) = t;
+        __threadfence_system();
+    }
+    __syncthreads();
+    if (z == 0) report_step(report, steps, status);
+}
+// the sequences of a step and, where they are given, its tokens
+struct BatchBegin {
+    uint32_t slot[kReportTokens], token[kReportTokens];
+};
+__global__ void __launch_bounds__(kReportTokens) batch_begin_kernel(const __grid_constant__ BatchBegin b, uint32_t* slot, uint32_t* tokens, const uint32_t* last, int n) {
+    const int z = threadIdx.x;
+    if (z >= n) return;
+    slot[z] = b.slot[z];
+    tokens[z] = last != nullptr ? last[b.slot[z]] : b.token[z];
+}
 }  // namespace qtb

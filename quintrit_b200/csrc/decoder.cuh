@@ -40,6 +40,10 @@ struct quintrit_b200_decoder {
     float *s_h, *s_q, *s_i;
     int32_t *acc_qkv, *acc_o, *acc_gu, *acc_down;
     uint32_t *d_token, *d_pos, *d_history;
+    uint32_t* d_steps = nullptr;              // steps done, counted on the device; `launched` counts them here
+    uint32_t launched = 0;
+    qtb::StepReport* report = nullptr;        // pinned host memory that steps write
+    bool bar_cleared = false;                 // step_begin_kernel of the next step has cleared the grid barrier's counter
     unsigned long long* d_rng = nullptr;       // state of the sampler's xorshift64 generator (runtime level, sampling on the device)
     unsigned int* d_counters;
     qtb::GemvItem* d_items;
@@ -140,6 +144,7 @@ inline void destroy_decoder(quintrit_b200_decoder* d) {
     for (quintrit_b200_matrix* m : d->pf.stacked_objects) qtb_release_stacked(m);
     if (d->stream) cudaStreamDestroy(d->stream);
     for (void* p : d->allocs) cudaFree(p);
+    if (d->report) cudaFreeHost(d->report);
     if (d->lay) layered_release(d);
     if (prev >= 0) cudaSetDevice(prev);
     d->magic = 0;
@@ -356,9 +361,17 @@ inline int enqueue_token(quintrit_b200_decoder* d, bool with_head) {
 
 // Sets the device-side position and token from host values.
 inline int decoder_set(quintrit_b200_decoder* d, uint32_t token, uint32_t pos) {
-    QTB_CUDA(cudaMemcpyAsync(d->d_token, &token, sizeof token, cudaMemcpyHostToDevice, d->stream));
-    QTB_CUDA(cudaMemcpyAsync(d->d_pos, &pos, sizeof pos, cudaMemcpyHostToDevice, d->stream));
+    step_begin_kernel<<<1, 32, 0, d->stream>>>(d->d_token, d->d_pos, token, pos, d->use_mega ? d->bar : nullptr);
+    QTB_LAUNCH_CHECK();
+    d->bar_cleared = d->use_mega;
     return QUINTRIT_OK;
+}
+inline int decoder_report_init(quintrit_b200_decoder* d) {
+    void* p = nullptr;
+    QTB_CUDA(cudaHostAlloc(&p, sizeof(StepReport), cudaHostAllocPortable | cudaHostAllocMapped));
+    d->report = static_cast<StepReport*>(p);
+    *d->report = StepReport{};
+    return dev_alloc(d, &d->d_steps, 1);
 }
 
 // Captures [one token + advance] into a graph the first time it is needed.
@@ -368,7 +381,7 @@ inline int decoder_graph(quintrit_b200_decoder* d) {
     QTB_CUDA(cudaStreamBeginCapture(d->stream, cudaStreamCaptureModeThreadLocal));
     int rc = enqueue_token(d, true);
     if (rc == QUINTRIT_OK) {
-        advance_kernel<<<1, 1, 0, d->stream>>>(d->d_pos, d->d_history, d->d_token);
+        advance_kernel<<<1, 1, 0, d->stream>>>(d->d_pos, d->d_history, d->d_token, d->d_steps, d->d_counters + 2, d->report);
         ++g_launches;
     }
     cudaError_t e = cudaStreamEndCapture(d->stream, &g);

@@ -1239,7 +1239,7 @@ int layered_decoder_create(const std::shared_ptr<LayeredModel>& model, uint32_t 
     int rc;
     QTB_CUDA(cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking));
     if ((rc = dev_alloc(d, &d->logits, d->vocab)) || (rc = dev_alloc(d, &d->d_token, 4)) || (rc = dev_alloc(d, &d->d_pos, 4)) || (rc = dev_alloc(d, &d->d_history, size_t(ctx) + 1)) ||
-        (rc = dev_alloc(d, &d->d_counters, 4)))
+        (rc = dev_alloc(d, &d->d_counters, 4)) || (rc = decoder_report_init(d)))
         return rc;
     return layered_decoder_setup(d, model);
 }

@@ -62,7 +62,9 @@ struct MegaArgs {
     uint32_t* token;
     uint32_t* pos;
     uint32_t* history;
-    unsigned int* bar;        // grid barrier counter, cleared by the host before every launch
+    uint32_t* steps;          // steps done (device), and what the host is told of them
+    StepReport* report;
+    unsigned int* bar;        // grid barrier counter, cleared before every launch
     unsigned int* status;     // 0 = fine, 1 = wrong shared-memory base, 2 = a barrier timed out
     unsigned long long* trace; // optional: CTA 0 stores the global timer at every phase boundary (14 per layer + 3)
     // Tensor parallelism over tp_world GPUs (1 = none). q_heads, kv_heads, inter and vocab above are this rank's shares; the
@@ -1953,7 +1955,10 @@ __device__ __noinline__ void phase_finish(const MegaArgs& a, unsigned int seq_ba
         a.amax_bits[3] = 0u;
         if (a.attn_v2)
             for (int k = 0; k < a.kv_heads; ++k) a.fac_done[k] = 0u;
+        *reinterpret_cast<volatile uint32_t*>(&a.report->token) = tok;
     }
+    __syncthreads();  // (the clearing above)
+    if (tid == 0) report_step(a.report, a.steps, a.status);
 }
 
 template <uint32_t BASE>

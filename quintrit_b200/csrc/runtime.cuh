@@ -213,8 +213,9 @@ int rt_forward(quintrit_session* s, uint32_t token, uint32_t pos, bool want_logi
     if ((rc = decoder_step(d)) != QUINTRIT_OK) return rc;
     if ((rc = rt_enqueue_sample(d, sample)) != QUINTRIT_OK) return rc;  // replaces the greedy choice in d_token by the sampled one
     if (want_logits) QTB_CUDA(cudaMemcpyAsync(s->logits.data(), d->logits, size_t(d->vocab) * sizeof(float), cudaMemcpyDeviceToHost, d->stream));
-    if (greedy) QTB_CUDA(cudaMemcpyAsync(greedy, d->d_token, sizeof(uint32_t), cudaMemcpyDeviceToHost, d->stream));
-    if ((rc = decoder_check_status(d)) != QUINTRIT_OK) return rc;
+    if (greedy && sample != nullptr) QTB_CUDA(cudaMemcpyAsync(greedy, d->d_token, sizeof(uint32_t), cudaMemcpyDeviceToHost, d->stream));  // (the report holds the step's own choice)
+    if ((rc = sample != nullptr || want_logits ? decoder_check_status(d) : decoder_wait_report(d)) != QUINTRIT_OK) return rc;
+    if (greedy && sample == nullptr) *greedy = d->report->token;
     if (s->cached.size() >= pos) {
         s->cached.resize(pos);
         s->cached.push_back(token);
