@@ -1161,14 +1161,26 @@ __global__ void __launch_bounds__(kHeadThreads, 1) lm_head_batch_kernel(const __
         const unsigned char* sx = st + kRows * kHeadRowStride + group * kHeadTokens * kHeadCols * 2 + j * 4;
 #pragma unroll
         for (int i = 0; i < kHeadCols / 32; ++i) {
-            unsigned long long wf[8];
+            if constexpr (BF16) {
+                unsigned long long wf[8];
 #pragma unroll
-            for (int r = 0; r < 8; ++r) wf[r] = head_widen<BF16>(*reinterpret_cast<const uint32_t*>(sw + 2 * r * kHeadRowStride + i * 64));
+                for (int r = 0; r < 8; ++r) wf[r] = widen_bf162(*reinterpret_cast<const uint32_t*>(sw + 2 * r * kHeadRowStride + i * 64));
 #pragma unroll
-            for (int t = 0; t < kHeadTokens; ++t) {
-                const unsigned long long x = head_widen<BF16>(*reinterpret_cast<const uint32_t*>(sx + t * kHeadCols * 2 + i * 64));
+                for (int t = 0; t < kHeadTokens; ++t) {
+                    const unsigned long long x = widen_bf162(*reinterpret_cast<const uint32_t*>(sx + t * kHeadCols * 2 + i * 64));
 #pragma unroll
-                for (int r = 0; r < 8; ++r) acc[r * 8 + t] = head_step<BF16>(wf[r], x, acc[r * 8 + t]);
+                    for (int r = 0; r < 8; ++r) acc[r * 8 + t] = head_step<BF16>(wf[r], x, acc[r * 8 + t]);
+                }
+            } else {
+                uint32_t wh[8];
+#pragma unroll
+                for (int r = 0; r < 8; ++r) wh[r] = *reinterpret_cast<const uint32_t*>(sw + 2 * r * kHeadRowStride + i * 64);
+#pragma unroll
+                for (int t = 0; t < kHeadTokens; ++t) {
+                    const uint32_t x = *reinterpret_cast<const uint32_t*>(sx + t * kHeadCols * 2 + i * 64);
+#pragma unroll
+                    for (int r = 0; r < 8; ++r) acc[r * 8 + t] = fma_half2_mixed(x, wh[r], acc[r * 8 + t]);
+                }
             }
         }
         if ((it + 1) % chunks == 0) {

@@ -35,6 +35,15 @@ __device__ __forceinline__ unsigned long long widen_half2(uint32_t h) {
     const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
     return pack_f32x2(f.x, f.y);
 }
+// acc + x y, two F16 products added to two floats: the product of two F16 numbers is exact in F32, so this has the bits of fma_f32x2 on the widened operands,
+// without widening them (which, like packed operations, only the heavy half of the FMA pipe does, two cycles an instruction); two instructions, one cycle each.
+__device__ __forceinline__ unsigned long long fma_half2_mixed(uint32_t x, uint32_t y, unsigned long long acc) {
+    unsigned long long r;
+    asm("{\n\t.reg .b16 xl, xu, yl, yu;\n\t.reg .f32 a, b;\n\tmov.b32 {xl, xu}, %1;\n\tmov.b32 {yl, yu}, %2;\n\tmov.b64 {a, b}, %3;\n\tfma.rn.f32.f16 a, xl, yl, a;\n\tfma.rn.f32.f16 b, xu, yu, b;\n\tmov.b64 %0, {a, b};\n\t}"
+        : "=l"(r)
+        : "r"(x), "r"(y), "l"(acc));
+    return r;
+}
 __device__ __forceinline__ unsigned long long widen_bf162(uint32_t h) { return pack_f32x2(__uint_as_float(h << 16), __uint_as_float(h & 0xffff0000u)); }
 
 __device__ __forceinline__ unsigned long long shfl_xor_f32x2(unsigned long long v, int mask) { return __shfl_xor_sync(0xffffffffu, v, mask); }
