@@ -44,31 +44,39 @@ __device__ __forceinline__ float block_max_f32(float v, float* sh) {
 // The published table algorithm of glibc's single-precision exp: N = 32 entries of 2^(i/N) (bits, minus i << 47), a
 // cubic evaluated in double. The table is filled by the host (exp2_table_bits) so that no constant list is copied.
 __device__ __constant__ unsigned long long c_exp2_tab[32];
+__device__ unsigned long long g_exp2_tab[32];  // the same for a warp that reads it whole: from constant memory the 32 entries come one after another (about 1000 cycles)
 
-__device__ __forceinline__ float device_expf(float x) {
+// With the table's entry from `entry(i)`.
+template <typename Entry>
+__device__ __forceinline__ float device_expf_from(float x, Entry entry) {
     const double inv_ln2_n = 0x1.71547652b82fep0 * 32.0, shift = 0x1.8p52;
     const double c0 = 0x1.c6af84b912394p-5 / 32.0 / 32.0 / 32.0, c1 = 0x1.ebfce50fac4f3p-3 / 32.0 / 32.0, c2 = 0x1.62e42ff0c52d6p-1 / 32.0;
-    const uint32_t ix = __float_as_uint(x), abstop = (ix >> 20) & 0x7ffu;
-    if (abstop >= 0x42bu) {
-        if (ix == 0xff800000u) return 0.0f;
-        if (abstop >= 0x7f8u) return __fadd_rn(x, x);
-        if (x > 0x1.62e42ep6f) return __uint_as_float(0x7f800000u);
-        if (x < -0x1.9fe368p6f) return 0.0f;
-    }
     const double xd = static_cast<double>(x);
     const double z0 = __dmul_rn(inv_ln2_n, xd);
     double kd = __dadd_rn(z0, shift);
     const unsigned long long ki = static_cast<unsigned long long>(__double_as_longlong(kd));
     kd = __dsub_rn(kd, shift);
     const double r = __dsub_rn(z0, kd);
-    const unsigned long long t = c_exp2_tab[ki & 31ull] + (ki << 47);
+    const unsigned long long t = entry(static_cast<int>(ki & 31ull)) + (ki << 47);
     const double s = __longlong_as_double(static_cast<long long>(t));
     const double z = __fma_rn(c0, r, c1);
     const double r2 = __dmul_rn(r, r);
     double y = __fma_rn(c2, r, 1.0);
     y = __fma_rn(z, r2, y);
     y = __dmul_rn(y, s);
-    return __double2float_rn(y);
+    // Selects, not branches, so that several exponentials of a thread overlap; for an infinite or NaN argument the computation above means nothing.
+    const uint32_t ix = __float_as_uint(x), abstop = (ix >> 20) & 0x7ffu;
+    float result = __double2float_rn(y);
+    result = abstop >= 0x42bu && x > 0x1.62e42ep6f ? __uint_as_float(0x7f800000u) : result;
+    result = abstop >= 0x42bu && x < -0x1.9fe368p6f ? 0.0f : result;
+    return abstop >= 0x7f8u && ix != 0xff800000u ? __fadd_rn(x, x) : result;
+}
+__device__ __forceinline__ float device_expf(float x) {
+    return device_expf_from(x, [](int i) { return c_exp2_tab[i]; });
+}
+// The same for a whole warp at once (every lane calls it): lane i brings entry i, g_exp2_tab[lane]. Lanes that look different entries up in constant memory wait for one another.
+__device__ __forceinline__ float device_expf_warp(float x, unsigned long long lane_entry) {
+    return device_expf_from(x, [&](int i) { return __shfl_sync(0xffffffffu, lane_entry, i); });
 }
 
 // ---- ggml's vector expf, one lane (ops.rs:316-387), and SiLU (ops.rs:389-399) ---------------------------------------

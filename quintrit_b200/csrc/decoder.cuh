@@ -62,8 +62,6 @@ struct quintrit_b200_decoder {
     qtb::AttnGqaKernel attn_rows = nullptr;    // the same for the head sizes it exists for, packed operations
     size_t attn_gqa_pad = 0;                   // experiments: extra shared memory per block, which lowers the number of resident blocks
     float* attn_out = nullptr;
-    float *fac = nullptr, *fac_M = nullptr;
-    unsigned int *fac_flags = nullptr, *fac_done = nullptr;
     unsigned long long* trace;  // phase timestamps of the last traced step (13 per layer + 3)
     cudaStream_t stream;
     cudaGraphExec_t graph_step;               // one token: embed ... argmax (token and position read from device memory)

@@ -10,6 +10,9 @@
 //   F1 SwiGLU on a slice per CTA, maximum through atomicMax
 //   F2 down GEMV, quantising its activations on the fly in the table fill
 // and the token ends with the final norm, the output head (rows split over CTAs), the greedy choice and pos += 1.
+// Between two grid barriers a phase lasts 1 to 8 us, so every trip to L2 before its work counts: the kernel's arguments, the position and the cos/sin row
+// of the position lie in shared memory (read through a reference to the kernel's parameter, each argument was a global load behind every barrier). With scores by
+// four threads a row: 62.8 -> 58.5 us a layer of the Falcon3-10B shape at context 1024, 59.8 -> 53.5 of the BitNet-2B shape (cycle stamps of block 0).
 // All arithmetic is the device functions of decode.cuh / gemv_lut.cuh, so the bits equal the per-kernel path and the
 // reference CPU runtime. Every wait is bounded: a barrier that does not complete sets status and the kernel returns.
 #pragma once
@@ -23,6 +26,7 @@ namespace qtb {
 constexpr int kMegaThreads = 512;
 constexpr int kMegaWarps = kMegaThreads / 32;
 constexpr int kMegaMaxHeads = 64;
+constexpr int kMegaCosSin = 256;  // floats of a row of the cos/sin table: rope_dims <= head_dim <= 256
 constexpr unsigned int kBarrierSpinLimit = 1u << 21;  // polls of one L2 round trip each (~0.7 us): about 1.5 s, then the kernel gives up
 
 struct MegaLayer {
@@ -73,15 +77,6 @@ struct MegaArgs {
     // number) pairs that the readers poll.
     int attn_v2;               // attention second half by (KV head, 8 coordinates) units that also combine the chunks
     float* attn_out;           // their result: the attention output before the o projection's quantiser (q_dim floats)
-    // Softmax factors of the current token, computed once per (head, chunk) by the CTAs that have no values unit and read by
-    // every unit of the head's group: rows of fac_stride floats, ms rows of all (head, chunk slot) first, then the vs rows;
-    // one word of move flags per (head, chunk slot, group of eight positions); the maximum of every (head, chunk slot);
-    // fac_done[kv head] counts the (head, chunk) tasks finished since the token began.
-    float* fac;
-    unsigned int* fac_flags;
-    float* fac_M;
-    unsigned int* fac_done;
-    int fac_stride;
     int l2_prefetch;           // request the weights of later phases into L2 ahead of their streams (QUINTRIT_B200_L2_PREFETCH=0 switches it off)
     int bf16_tables;           // embedding and output head hold BF16 instead of F16 bit patterns
     int neox;                  // BitNet: RoPE pairs (i, i + rope_dims / 2) instead of (2i, 2i + 1) (config.rs:464-467)
@@ -340,12 +335,9 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-__device__ __forceinline__ void cp_async4(void* smem_dst, const void* gsrc) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst))), "l"(gsrc) : "memory");
-}
 // Requests the n norm weights that the next norm needs (one copy group); they land while other phases run.
 __device__ __forceinline__ void request_norm_weights(float* w_s, const float* __restrict__ w, int n) {
-    for (int i = threadIdx.x; i < n; i += kMegaThreads) cp_async4(w_s + i, w + i);
+    for (int i = threadIdx.x; i < n / 4; i += kMegaThreads) cp_async16(w_s + 4 * i, w + 4 * i);  // (n: a multiple of 32)
     cp_async_commit();
 }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
@@ -442,41 +434,39 @@ __device__ __forceinline__ void stage_rows(unsigned char* dst, const __half* src
     }
 }
 
-// Score of one staged key row against the query, by ONE thread: the 32 accumulator lanes of the reference's dot product
-// (ggml_vec_dot_f16: element e goes to lane e mod 32, lanes are summed by a fixed tree) live in 32 registers, so the
-// 32 chains run interleaved and the tree needs no shuffles.
+// Score of one staged key row against the query, by four neighbouring threads: the 32 accumulator lanes of the reference's dot product
+// (ggml_vec_dot_f16: element e goes to lane e mod 32, lanes are summed by a fixed tree) live in eight registers of each, so a chunk of 32 elements is one
+// 16-byte load, and the tree's first two levels are exchanges. (One thread a row had 32 chains of its own and kept 84 of the 512 threads busy at
+// context 1024: 2.3 us of a layer.) Every thread of the warp calls it; all four have the result.
 template <bool F32>
 __device__ __forceinline__ float key_score(const unsigned char* buf, int r, int hd, const float* s_q) {
-    float acc[32];
+    const int sub = threadIdx.x & 3, sw = r & 7;
+    float acc[8];
 #pragma unroll
-    for (int l = 0; l < 32; ++l) acc[l] = 0.0f;
-    const int row_bytes = hd * 2;
-    const unsigned char* row = buf + r * row_bytes;
-    const int sw = r & 7;
+    for (int l = 0; l < 8; ++l) acc[l] = 0.0f;
+    const unsigned char* row = buf + r * hd * 2;
+    const float* q = s_q + 8 * sub;
+#pragma unroll 4
     for (int i = 0; i < hd; i += 32) {
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-            const uint4 kk = *reinterpret_cast<const uint4*>(row + ((((i >> 3) + cc) ^ sw) << 4));
-            const float4 q0 = *reinterpret_cast<const float4*>(s_q + i + 8 * cc), q1 = *reinterpret_cast<const float4*>(s_q + i + 8 * cc + 4);
-            const __half2 h0 = *reinterpret_cast<const __half2*>(&kk.x), h1 = *reinterpret_cast<const __half2*>(&kk.y);
-            const __half2 h2 = *reinterpret_cast<const __half2*>(&kk.z), h3 = *reinterpret_cast<const __half2*>(&kk.w);
-            acc[8 * cc + 0] = __fmaf_rn(__low2float(h0), q0.x, acc[8 * cc + 0]);
-            acc[8 * cc + 1] = __fmaf_rn(__high2float(h0), q0.y, acc[8 * cc + 1]);
-            acc[8 * cc + 2] = __fmaf_rn(__low2float(h1), q0.z, acc[8 * cc + 2]);
-            acc[8 * cc + 3] = __fmaf_rn(__high2float(h1), q0.w, acc[8 * cc + 3]);
-            acc[8 * cc + 4] = __fmaf_rn(__low2float(h2), q1.x, acc[8 * cc + 4]);
-            acc[8 * cc + 5] = __fmaf_rn(__high2float(h2), q1.y, acc[8 * cc + 5]);
-            acc[8 * cc + 6] = __fmaf_rn(__low2float(h3), q1.z, acc[8 * cc + 6]);
-            acc[8 * cc + 7] = __fmaf_rn(__high2float(h3), q1.w, acc[8 * cc + 7]);
-        }
+        const uint4 kk = *reinterpret_cast<const uint4*>(row + ((((i >> 3) + sub) ^ sw) << 4));
+        const float4 q0 = *reinterpret_cast<const float4*>(q + i), q1 = *reinterpret_cast<const float4*>(q + i + 4);
+        const __half2 h0 = *reinterpret_cast<const __half2*>(&kk.x), h1 = *reinterpret_cast<const __half2*>(&kk.y);
+        const __half2 h2 = *reinterpret_cast<const __half2*>(&kk.z), h3 = *reinterpret_cast<const __half2*>(&kk.w);
+        acc[0] = __fmaf_rn(__low2float(h0), q0.x, acc[0]);
+        acc[1] = __fmaf_rn(__high2float(h0), q0.y, acc[1]);
+        acc[2] = __fmaf_rn(__low2float(h1), q0.z, acc[2]);
+        acc[3] = __fmaf_rn(__high2float(h1), q0.w, acc[3]);
+        acc[4] = __fmaf_rn(__low2float(h2), q1.x, acc[4]);
+        acc[5] = __fmaf_rn(__high2float(h2), q1.y, acc[5]);
+        acc[6] = __fmaf_rn(__low2float(h3), q1.z, acc[6]);
+        acc[7] = __fmaf_rn(__high2float(h3), q1.w, acc[7]);
     }
-    if (F32) {  // ggml_vec_dot_f16 summed as (a0+a1)+(a2+a3), then ((l0+l4)+(l2+l6))+((l1+l5)+(l3+l7)): dot_lane_reduce_f16_f32
+    // F32: (a0+a1)+(a2+a3), then ((l0+l4)+(l2+l6))+((l1+l5)+(l3+l7)) (dot_lane_reduce_f16_f32); else (a0+a2)+(a1+a3) (dot_lane_reduce_f16)
+    constexpr int kNear = F32 ? 1 : 2, kFar = 3 - kNear;
 #pragma unroll
-        for (int l = 0; l < 8; ++l) acc[l] = __fadd_rn(__fadd_rn(acc[l], acc[l + 8]), __fadd_rn(acc[l + 16], acc[l + 24]));
-    } else {    // (a0+a2)+(a1+a3): dot_lane_reduce_f16
+    for (int l = 0; l < 8; ++l) acc[l] = __fadd_rn(acc[l], __shfl_xor_sync(0xffffffffu, acc[l], kNear));
 #pragma unroll
-        for (int l = 0; l < 8; ++l) acc[l] = __fadd_rn(__fadd_rn(acc[l], acc[l + 16]), __fadd_rn(acc[l + 8], acc[l + 24]));
-    }
+    for (int l = 0; l < 8; ++l) acc[l] = __fadd_rn(acc[l], __shfl_xor_sync(0xffffffffu, acc[l], kFar));
 #pragma unroll
     for (int l = 0; l < 4; ++l) acc[l] = __fadd_rn(acc[l], acc[l + 4]);
     if (F32) return __fadd_rn(__fadd_rn(acc[0], acc[2]), __fadd_rn(acc[1], acc[3]));
@@ -541,9 +531,9 @@ struct KvSplit {
     int pos, seq_len, n_kv, chunk;  // chunk = positions per chunk (n_kv when there is a single chunk)
     bool split;
 };
-__device__ __forceinline__ KvSplit kv_split(const MegaArgs& a) {
+__device__ __forceinline__ KvSplit kv_split(const MegaArgs& a, int pos) {
     KvSplit s;
-    s.pos = static_cast<int>(a.pos[0]);
+    s.pos = pos;
     s.seq_len = s.pos + 1;
     s.n_kv = (s.seq_len + 255) / 256 * 256;
     if (s.n_kv < 256) s.n_kv = 256;
@@ -559,7 +549,7 @@ __device__ __forceinline__ KvSplit kv_split(const MegaArgs& a) {
 // key and value rows, appends them to the cache and scores the new key from shared memory. Scores go to
 // a.scores[head][position]. `smem` is the CTA's dynamic shared memory from its start: the staged block overlays the GEMV
 // table, whose zero rows are restored before returning.
-__device__ __noinline__ void mega_scores_unit(const MegaArgs& a, const MegaLayer& ly, int kvh, int r0, int rows, float s_in, unsigned char* smem) {
+__device__ __noinline__ void mega_scores_unit(const MegaArgs& a, const MegaLayer& ly, int pos, const float* cs, int kvh, int r0, int rows, float s_in, unsigned char* smem) {
     const int tid = threadIdx.x;
     const int hd = a.head_dim, gqa = a.q_heads / a.kv_heads;
     const int qd = a.q_heads * hd, kvd = a.kv_heads * hd, row_bytes = hd * 2;
@@ -569,13 +559,11 @@ __device__ __noinline__ void mega_scores_unit(const MegaArgs& a, const MegaLayer
     __half* s_vcur = s_kcur + hd;
     const bool f32v = a.f32_values != 0;
     const float attn_scale = a.attn_scale;
-    const int pos = static_cast<int>(a.pos[0]);
     const bool has_cur = pos >= r0 && pos < r0 + rows;
     const int len_old = has_cur ? pos - r0 : rows;  // rows that come from the cache
     const __half* kbase = ly.kc + static_cast<size_t>(kvh) * hd + static_cast<size_t>(r0) * kvd;
     const bool live = s_in > 0.0f;
     const float pq = live ? __fdiv_rn(ly.ws[0], s_in) : 0.0f, pk = live ? __fdiv_rn(ly.ws[1], s_in) : 0.0f, pv = live ? __fdiv_rn(ly.ws[2], s_in) : 0.0f;
-    const float* cs = a.cos_sin + static_cast<size_t>(pos) * a.rope_dims;
     const int half = hd / 2, hr = a.rope_dims / 2;
     const int n_pairs = (gqa + (has_cur ? 1 : 0)) * half;
     // Pair idx of the rotated, rescaled query heads (and of the new key / value rows): head g, pair p. Its two elements are
@@ -648,10 +636,14 @@ __device__ __noinline__ void mega_scores_unit(const MegaArgs& a, const MegaLayer
     cp_async_wait<0>();
     __syncthreads();
     QTB_FINE(a, 27);
-    for (int t = tid; t < rows * gqa; t += kMegaThreads) {
-        const int g = t / rows, r = t - g * rows;
-        const float sc = f32v ? key_score<true>(blk, r, hd, s_q + g * hd) : key_score<false>(blk, r, hd, s_q + g * hd);
-        a.scores[static_cast<size_t>(kvh * gqa + g) * a.ctx + r0 + r] = __fmul_rn(sc, attn_scale);
+    {
+        // (head, row) of four threads; the rows of a group of eight in the order 0 4 1 5 2 6 3 7, whose pieces lie in different banks two by two
+        const int rows8 = (rows + 7) / 8 * 8, tasks = rows8 * gqa;
+        for (int t0 = 0; t0 < tasks; t0 += kMegaThreads / 4) {  // (whole warps: the scores' sums are exchanges)
+            const int t = min(t0 + (tid >> 2), tasks - 1), g = t / rows8, k = t - g * rows8, r = (k & ~7) | ((k & 1) << 2) | ((k >> 1) & 3);
+            const float sc = f32v ? key_score<true>(blk, r, hd, s_q + g * hd) : key_score<false>(blk, r, hd, s_q + g * hd);
+            if ((tid & 3) == 0 && t0 + (tid >> 2) < tasks && r < rows) a.scores[static_cast<size_t>(kvh * gqa + g) * a.ctx + r0 + r] = __fmul_rn(sc, attn_scale);
+        }
     }
     __syncthreads();
     QTB_FINE(a, 28);
@@ -674,11 +666,11 @@ __host__ __device__ constexpr size_t values_unit_bytes(int len, int gqa) {
 // every query head of the group (phase B of attention_kernel, recomputed by every slice) and the value accumulation
 // (phase C). The V slice of the whole chunk is staged in shared memory in four copy groups; warp g runs the chains of
 // query head g, one coordinate per lane, strictly in position order. Slice 0 also produces M and S of each head.
-__device__ __noinline__ void mega_values_unit(const MegaArgs& a, const MegaLayer& ly, int kvh, int c, int slice, unsigned char* smem) {
+__device__ __noinline__ void mega_values_unit(const MegaArgs& a, const MegaLayer& ly, int pos, int kvh, int c, int slice, unsigned char* smem) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int hd = a.head_dim, gqa = a.q_heads / a.kv_heads, kvd = a.kv_heads * hd;
     const bool f32v = a.f32_values != 0;
-    const KvSplit ks = kv_split(a);
+    const KvSplit ks = kv_split(a, pos);
     int start = 0, end = ks.seq_len;
     if (ks.split) {
         start = c * ks.chunk;
@@ -847,13 +839,12 @@ __device__ __noinline__ void mega_values_unit(const MegaArgs& a, const MegaLayer
 // maximum that the quantiser of the o projection needs. What is left after the next grid barrier is a load and a rounding.
 // Staging is asynchronous copies only (no registers, everything in flight at once): the unit's 16-byte piece of every
 // cached V row into [chunk][position][8 halves], the scores of its heads into one row per (head, chunk). The softmax
-// factors (attention.rs:448-462) are computed by all threads, eight consecutive positions each: maxima of the groups, a
-// barrier, the maximum before the group from the earlier groups' maxima, then one exponential per position. A word per
-// head and group of eight positions tells whether any chunk's running maximum moved there; groups without a move run
-// branch-free.
+// factors (attention.rs:448-462) are made by the unit itself, a warp per (head, chunk) (v2_factors). The positions at which any chunk's running maximum
+// moved are known per head and group of eight; groups without a move run branch-free.
 constexpr int kV2Dims = 16;      // coordinates per unit: two warps of eight coordinates x four chunks per query head
 constexpr int kV2WarpsPerHead = kV2Dims / 8;
 constexpr int kV2MaxCtx = 4096;
+static_assert(kV2MaxCtx / 4 / 8 < 256, "a group's number fits the low byte of the table of next groups");
 constexpr int kV2MaxGqa = 7;     // chain warps (two per head) + the warp of the sum chains must fit the 16 warps of the CTA
 
 // Row length (floats) of the factor rows for chunks of `chunk` positions: a multiple of 8, at least `chunk`.
@@ -864,7 +855,7 @@ __host__ __device__ constexpr int values2_clr(int chunk) { return values2_clp(ch
 __host__ __device__ constexpr size_t values2_bytes(int ctx, int gqa) {
     const int nch = ctx >= 512 ? 4 : 1, chunk = ctx >= 512 ? (ctx + 3) / 4 : ctx, clp = values2_clp(chunk);
     return static_cast<size_t>(nch) * values2_clr(chunk) * kV2Dims * 2 + static_cast<size_t>(2) * gqa * nch * clp * 4 + static_cast<size_t>(gqa) * (clp / 8) * 4 +
-           static_cast<size_t>(gqa) * 8 * 4 + static_cast<size_t>(gqa) * nch * 8 + 64;
+           static_cast<size_t>(gqa) * 8 * 4 + static_cast<size_t>(gqa) * nch * (8 + clp / 8) + 64;
 }
 
 template <bool F32>
@@ -890,12 +881,13 @@ __device__ __noinline__ float v2_chain(uint32_t v_off, uint32_t w_off, uint32_t 
 #pragma unroll
     for (int j = 0; j < 8; ++j) vn[j] = *reinterpret_cast<const __half*>(vrow + j * (kV2Dims * 2));
     float4 w0n = *reinterpret_cast<const float4*>(wrow), w1n = *reinterpret_cast<const float4*>(wrow + 4);
-    // `nx[g]` is the first group at or after g in which some chunk's running maximum moved (ngr if none). Up to there the loop
+    // The low byte of `nx[g]` is the first group at or after g in which some chunk's running maximum moved (ngr if none), the high one the positions of group g at
+    // which it did. Up to there the loop
     // has no branch but its own, so the compiler overlaps the loads of the next group with the eight dependent steps.
     const unsigned short* nx = reinterpret_cast<const unsigned short*>(fl);
     int grp = 0;
     while (grp < ngr) {
-        const int stop = min(static_cast<int>(nx[grp]), ngr);
+        const int stop = min(static_cast<int>(nx[grp] & 0xffu), ngr);
         for (; grp < stop; ++grp) {
             float v[8];
 #pragma unroll
@@ -909,8 +901,9 @@ __device__ __noinline__ float v2_chain(uint32_t v_off, uint32_t w_off, uint32_t 
             for (int j = 0; j < 8; ++j) acc = v2_round<F32>(__fmaf_rn(v[j], w[j], acc));
         }
         if (grp < ngr) {
-            // a group with a move: its rescale factors are loaded once; the multiply of a position is skipped where this lane's
-            // chunk did not move (a factor of one would change nothing, but cost a step's latency)
+            // a group with a move: its rescale factors are loaded once; a position at which no chunk's maximum moved has no multiply (a factor of one, which
+            // the other chunks' lanes have, changes nothing). The mask is the head's, so the branches are the whole warp's.
+            const unsigned int mask = nx[grp] >> 8;
             float v[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) v[j] = __half2float(vn[j]);
@@ -923,7 +916,7 @@ __device__ __noinline__ float v2_chain(uint32_t v_off, uint32_t w_off, uint32_t 
             w1n = *reinterpret_cast<const float4*>(wrow + 8 * (grp + 1) + 4);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                if (m[j] != 1.0f) acc = v2_round<F32>(__fmul_rn(acc, m[j]));
+                if (mask & (1u << j)) acc = v2_round<F32>(__fmul_rn(acc, m[j]));
                 acc = v2_round<F32>(__fmaf_rn(v[j], w[j], acc));
             }
             ++grp;
@@ -959,116 +952,83 @@ __device__ __noinline__ float v2_sum_chain(uint32_t m_off, uint32_t w_off, int l
     return S;
 }
 
-// One helper task of the values phase: the softmax factors of head `h`, chunk `c` (attention.rs:448-462), two consecutive
-// positions per thread. The running maximum before a position comes from a scan over the block; then one exponential per
-// position: ms = exp(m_before - score), vs = 1 where the score exceeds the maximum so far, else ms = 1, vs = exp(score -
-// m_before). Positions behind the chunk's end up to the common chain length get vs = 0, ms = 1: such a step leaves a sum
-// unchanged bit for bit. Rows, move flags (bit j of a word: the maximum moved at position 8 group + j, and by a factor other
-// than one) and the chunk's maximum go to global memory; the count of finished tasks of the KV head is raised last.
-__device__ __noinline__ void v2_factors_task(const MegaArgs& a, int h, int c, unsigned char* smem) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const KvSplit ks = kv_split(a);
-    const int nch = ks.split ? 4 : 1, CL = ks.chunk, seq = ks.seq_len;
-    auto chunk_len = [&](int cc) {
-        if (!ks.split) return cc == 0 ? seq : 0;
-        const int start = cc * CL;
-        return max(0, min(min(start + CL, ks.n_kv), seq) - start);
-    };
-    int ngr = 0;
-    for (int cc = 0; cc < nch; ++cc) ngr = max(ngr, (chunk_len(cc) + 7) / 8);
-    const int len = chunk_len(c), slot = h * 4 + c;
-    const float* src = a.scores + static_cast<size_t>(h) * a.ctx + c * CL;
-    float* ms_out = a.fac + static_cast<size_t>(slot) * a.fac_stride;
-    float* vs_out = a.fac + static_cast<size_t>(a.q_heads * 4 + slot) * a.fac_stride;
-    unsigned int* fl_out = a.fac_flags + static_cast<size_t>(slot) * (a.fac_stride / 8);
-    float* s_wt = reinterpret_cast<float*>(smem);  // one maximum per warp
-    // chunks of up to 512 positions: one position per thread; up to 1024: two consecutive ones
-    const bool two = ngr * 8 > kMegaThreads;
-    const int p0 = two ? 2 * tid : tid, p1 = p0 + 1;
-    const float s0 = p0 < len ? __ldcg(src + p0) : -INFINITY, s1 = two && p1 < len ? __ldcg(src + p1) : -INFINITY;
-    float incl = fmaxf(s0, s1);
-    for (int o = 1; o < 32; o <<= 1) {
-        const float t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl = fmaxf(incl, t);
-    }
-    float before = __shfl_up_sync(0xffffffffu, incl, 1);
-    if (lane == 0) before = -INFINITY;
-    __syncthreads();  // the table region is free
-    if (lane == 31) s_wt[warp] = incl;
-    __syncthreads();
-    float total = -INFINITY;
+// The softmax factors (attention.rs:448-462) of one (head, chunk), by one warp, 128 positions at a time, four neighbouring ones a lane: the running maximum before a
+// lane's positions comes from a scan over the lanes' maxima; ms = exp(m_before - score), vs = 1 where a score exceeds the maximum so far, else ms = 1, vs =
+// exp(score - m_before). Positions behind the chunk's end up to the common chain length (ngr groups of eight) get vs = 0, ms = 1: such a step leaves a sum
+// unchanged bit for bit. moved[g]: bit k = the maximum moved, by a factor other than one, at position k of group g. Returns the chunk's maximum. The first
+// 256 scores come with the call, requested before the copies of the values, behind which they would wait.
+// (Blocks without a unit made them once per KV head and handed them on through global memory: 5.4 us of a layer of the Falcon3-10B shape at 1024 positions from the start
+// of the phase to the chains, 5.2 now, and without those blocks. What a phase runs once a layer waits for its instructions: 32 positions a turn cost 0.9 us
+// more, eight a lane side by side 1.4.)
+struct Scores8 {
+    float s[8];  // positions 4 lane .. 4 lane + 3 of the first 128 and of the next
+};
+__device__ __forceinline__ Scores8 v2_load_scores(const float* __restrict__ scores, int len, int first) {
+    Scores8 r;
+    const bool wide = (reinterpret_cast<uintptr_t>(scores) & 15) == 0;
 #pragma unroll
-    for (int w = 0; w < kMegaWarps; ++w) {
-        const float t = s_wt[w];
-        if (w < warp) before = fmaxf(before, t);
-        total = fmaxf(total, t);
-    }
-    auto factor = [&](int p, float sc, float m_before, float& ms, float& vs) {
-        ms = 1.0f, vs = 0.0f;
-        bool moved = false;
-        if (p < len) {
-            vs = 1.0f;
-            if (sc > m_before) {
-                ms = device_expf(__fsub_rn(m_before, sc));
-                moved = ms != 1.0f;  // exp(0) = 1: a maximum that moved by nothing needs no rescale
-            } else {
-                vs = device_expf(__fsub_rn(sc, m_before));
-            }
-        }
-        return moved;
-    };
-    float ms0, vs0, ms1 = 1.0f, vs1 = 0.0f;
-    const bool mv0 = factor(p0, s0, before, ms0, vs0);
-    bool mv1 = false;
-    if (two) mv1 = factor(p1, s1, fmaxf(before, s0), ms1, vs1);
-    const unsigned int b0 = __ballot_sync(0xffffffffu, mv0), b1 = __ballot_sync(0xffffffffu, mv1);
-    if (two) {
-        if (p0 < ngr * 8) {
-            *reinterpret_cast<float2*>(ms_out + p0) = make_float2(ms0, ms1);
-            *reinterpret_cast<float2*>(vs_out + p0) = make_float2(vs0, vs1);
-        }
-        if ((lane & 3) == 0) {  // four lanes = eight positions = one group
-            unsigned int bits = 0;
+    for (int h = 0; h < 2; ++h) {
+        const int p = first + 128 * h + 4 * (threadIdx.x & 31);
+        if (wide && p + 4 <= len) {
+            const float4 x = __ldcg(reinterpret_cast<const float4*>(scores + p));
+            r.s[4 * h] = x.x, r.s[4 * h + 1] = x.y, r.s[4 * h + 2] = x.z, r.s[4 * h + 3] = x.w;
+        } else {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) bits |= (((b0 >> (lane + i)) & 1u) << (2 * i)) | (((b1 >> (lane + i)) & 1u) << (2 * i + 1));
-            const int grp = warp * 8 + (lane >> 2);
-            if (grp < ngr) fl_out[grp] = bits;
-        }
-    } else {
-        if (p0 < ngr * 8) {
-            ms_out[p0] = ms0;
-            vs_out[p0] = vs0;
-        }
-        if ((lane & 7) == 0) {  // eight lanes = one group
-            const int grp = warp * 4 + (lane >> 3);
-            if (grp < ngr) fl_out[grp] = (b0 >> lane) & 0xFFu;
+            for (int k = 0; k < 4; ++k) r.s[4 * h + k] = p + k < len ? __ldcg(scores + p + k) : -INFINITY;
         }
     }
-    if (tid == 0) a.fac_M[slot] = total;
-    __syncthreads();
-    if (tid == 0) {
-        __threadfence();
-        atomicAdd(a.fac_done + h / (a.q_heads / a.kv_heads), 1u);
+    return r;
+}
+__device__ __noinline__ float v2_factors(Scores8 in, const float* __restrict__ scores, int len, int ngr, float* ms_row, float* vs_row, unsigned char* moved, unsigned long long exp_entry) {
+    const int lane = threadIdx.x & 31, n = ngr * 8;
+    float carry = -INFINITY;
+#pragma unroll 1
+    for (int b = 0; b < n; b += 128) {
+        if (b > 0) {
+            if (b % 256 == 0) in = v2_load_scores(scores, len, b);
+            else in.s[0] = in.s[4], in.s[1] = in.s[5], in.s[2] = in.s[6], in.s[3] = in.s[7];
+        }
+        const int p = b + 4 * lane;
+        float top = fmaxf(fmaxf(in.s[0], in.s[1]), fmaxf(in.s[2], in.s[3]));
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float t = __shfl_up_sync(0xffffffffu, top, o);
+            if (lane >= o) top = fmaxf(top, t);
+        }
+        float run = __shfl_up_sync(0xffffffffu, top, 1);
+        run = lane == 0 ? carry : fmaxf(carry, run);
+        carry = fmaxf(carry, __shfl_sync(0xffffffffu, top, 31));
+        float arg[4], ms[4], vs[4];
+        bool up[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            up[k] = p + k < len && in.s[k] > run;
+            arg[k] = p + k >= len ? 0.0f : up[k] ? __fsub_rn(run, in.s[k]) : __fsub_rn(in.s[k], run);
+            if (up[k]) run = in.s[k];
+        }
+        unsigned int bits = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float ex = device_expf_warp(arg[k], exp_entry);
+            ms[k] = up[k] ? ex : 1.0f;
+            vs[k] = up[k] ? 1.0f : p + k < len ? ex : 0.0f;
+            bits |= ms[k] != 1.0f ? 1u << k : 0u;  // exp(0) = 1: a maximum that moved by nothing needs no rescale
+        }
+        bits |= __shfl_down_sync(0xffffffffu, bits, 1) << 4;
+        if (p < n) {
+            *reinterpret_cast<float4*>(ms_row + p) = make_float4(ms[0], ms[1], ms[2], ms[3]);
+            *reinterpret_cast<float4*>(vs_row + p) = make_float4(vs[0], vs[1], vs[2], vs[3]);
+            if ((lane & 1) == 0) moved[p >> 3] = static_cast<unsigned char>(bits);
+        }
     }
+    return carry;
 }
 
-#ifdef QTB_DEBUG_V2
-__device__ long long g_v2_clock[16];
-#define QTB_V2_CLOCK(k)                                  \
-    do {                                                 \
-        if (threadIdx.x == 0 && blockIdx.x == 0) g_v2_clock[k] = clock64(); \
-    } while (0)
-#else
-#define QTB_V2_CLOCK(k) \
-    do {                \
-    } while (0)
-#endif
-
 template <bool F32>
-__device__ __noinline__ void mega_values2_unit(const MegaArgs& a, const MegaLayer& ly, int l, int kvh, int slice, unsigned char* smem) {
+__device__ __noinline__ void mega_values2_unit(const MegaArgs& a, const MegaLayer& ly, int l, int pos, unsigned long long exp_entry, int kvh, int slice, unsigned char* smem) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int hd = a.head_dim, gqa = a.q_heads / a.kv_heads, kvd = a.kv_heads * hd;
-    const KvSplit ks = kv_split(a);
+    const KvSplit ks = kv_split(a, pos);
     const int nch = ks.split ? 4 : 1, CL = ks.chunk, clp = values2_clp(CL), clr = values2_clr(CL), seq = ks.seq_len;
     const int ngr8 = clp / 8, npairs = gqa * nch;
     constexpr int kPiece = kV2Dims * 2;                                                  // bytes of a cached row a unit takes
@@ -1078,7 +1038,7 @@ __device__ __noinline__ void mega_values2_unit(const MegaArgs& a, const MegaLaye
     unsigned short* s_next = reinterpret_cast<unsigned short*>(f_vs + npairs * clp);     // [gqa][ngr8 + 2]: next group with a move
     float* s_scale = reinterpret_cast<float*>(s_next + gqa * (ngr8 + 2) + ((gqa * (ngr8 + 2)) & 1));  // [gqa][4][2]: chunk-combine factors
     float* s_MS = s_scale + gqa * 8;                                                     // [gqa][nch][2]: M, S
-    int* s_ok = reinterpret_cast<int*>(s_MS + npairs * 2);
+    unsigned char* s_moved = reinterpret_cast<unsigned char*>(s_MS + npairs * 2);         // [gqa][nch][ngr8]: positions of a group at which the maximum moves
     auto chunk_len = [&](int c) {
         if (!ks.split) return c == 0 ? seq : 0;
         const int start = c * CL;
@@ -1086,53 +1046,31 @@ __device__ __noinline__ void mega_values2_unit(const MegaArgs& a, const MegaLaye
     };
     int ngr = 0;  // groups of eight positions of the longest chunk: the length of every chain of this unit
     for (int cc = 0; cc < nch; ++cc) ngr = max(ngr, (chunk_len(cc) + 7) / 8);
+    auto scores_of = [&](int pair) { return a.scores + static_cast<size_t>(kvh * gqa + pair / nch) * a.ctx + (pair % nch) * CL; };
+    Scores8 first = v2_load_scores(scores_of(min(warp, npairs - 1)), chunk_len(min(warp, npairs - 1) % nch), 0);
     __syncthreads();  // every thread is done with the table the arrays overlay
     QTB_FINE(a, 8);
-    QTB_V2_CLOCK(0);
     {
         const __half* vsrc = ly.vc + static_cast<size_t>(kvh) * hd + slice * kV2Dims;
-        for (int i = tid; i < seq * 2; i += kMegaThreads) {  // two 16-byte copies per cached row
-            const int p = i >> 1, h = i & 1, c = ks.split ? p / CL : 0;
-            cp_async16(Vr + static_cast<size_t>(c * clr + (p - c * CL)) * kPiece + h * 16, vsrc + static_cast<size_t>(p) * kvd + h * 8);
+        for (int c = 0; c < nch; ++c) {  // two 16-byte copies per cached row
+            const __half* rows = vsrc + static_cast<size_t>(c) * CL * kvd;
+            unsigned char* dst = Vr + static_cast<size_t>(c * clr) * kPiece;
+            const int n = chunk_len(c) * 2;
+            for (int i = tid; i < n; i += kMegaThreads) cp_async16(dst + i * 16, rows + static_cast<size_t>(i >> 1) * kvd + (i & 1) * 8);
         }
         cp_async_commit();
         // zero values behind a chunk's end up to the common chain length (the last chunk, mostly)
         for (int c = 0; c < nch; ++c)
             for (int i = chunk_len(c) * 2 + tid; i < ngr * 16; i += kMegaThreads) *reinterpret_cast<uint4*>(Vr + static_cast<size_t>(c * clr) * kPiece + i * 16) = make_uint4(0u, 0u, 0u, 0u);
-        // The factors of this group's heads come from the helper CTAs of this phase (v2_factors_task): wait, bounded, until
-        // all (head, chunk) tasks of the KV head have been counted.
-        if (tid == 0) {
-            const unsigned int target = static_cast<unsigned int>(l + 1) * static_cast<unsigned int>(npairs);
-            int okay = 1;
-            for (unsigned int spins = 0;; ++spins) {
-                unsigned int v;
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.fac_done + kvh));
-                if (v >= target) break;
-                if (spins > kBarrierSpinLimit || *reinterpret_cast<volatile unsigned int*>(a.bar) >= kBarFail) {
-                    report_failure(a.bar, a.status, 2u);
-                    okay = 0;
-                    break;
-                }
-            }
-            *s_ok = okay;
-        }
+    }
+    for (int pair = warp; pair < npairs; pair += kMegaWarps) {
+        if (pair >= kMegaWarps) first = v2_load_scores(scores_of(pair), chunk_len(pair % nch), 0);
+        const float M = v2_factors(first, scores_of(pair), chunk_len(pair % nch), ngr, f_ms + pair * clp, f_vs + pair * clp, s_moved + pair * ngr8, exp_entry);
+        if (lane == 0) s_MS[pair * 2] = M;
     }
     __syncthreads();
-    if (*s_ok == 0) return;  // the grid barrier that follows ends the kernel
     QTB_FINE(a, 2);
-    QTB_V2_CLOCK(1);
     {
-        const int rows4 = a.q_heads * 4, fl_stride = a.fac_stride / 8;
-        for (int pair = warp; pair < npairs; pair += kMegaWarps) {
-            const int g = pair / nch, c = pair - g * nch, slot = (kvh * gqa + g) * 4 + c;
-            const float* ms_src = a.fac + static_cast<size_t>(slot) * a.fac_stride;
-            const float* vs_src = a.fac + static_cast<size_t>(rows4 + slot) * a.fac_stride;
-            for (int q = lane; q < ngr * 2; q += 32) {
-                cp_async16(f_ms + pair * clp + q * 4, ms_src + q * 4);
-                cp_async16(f_vs + pair * clp + q * 4, vs_src + q * 4);
-            }
-        }
-        cp_async_commit();
         // For every head and group the first group at or after it in which any chunk moved (the chain runs branch-free up to
         // there): one warp per head, 32 groups at a time from the end with the carry of the later groups.
         for (int g = warp; g < gqa; g += kMegaWarps) {
@@ -1141,33 +1079,29 @@ __device__ __noinline__ void mega_values2_unit(const MegaArgs& a, const MegaLaye
             if (lane == 0) nx[ngr] = static_cast<unsigned short>(ngr);
             for (int hi = (ngr + 31) / 32 * 32; hi > 0; hi -= 32) {
                 const int grp = hi - 32 + lane;
-                unsigned int bits = 0;
+                unsigned int mask = 0;
                 if (grp < ngr)
-                    for (int c = 0; c < nch; ++c) bits |= __ldcg(a.fac_flags + static_cast<size_t>((kvh * gqa + g) * 4 + c) * fl_stride + grp);
-                const unsigned int any = __ballot_sync(0xffffffffu, bits != 0u);
-                const unsigned int later = any >> lane;  // bit 0: this group
+                    for (int c = 0; c < nch; ++c) mask |= s_moved[(g * nch + c) * ngr8 + grp];
+                const unsigned int later = __ballot_sync(0xffffffffu, mask != 0u) >> lane;  // bit 0: this group
                 const int nxt = later ? hi - 32 + lane + (__ffs(later) - 1) : carry;
-                if (grp < ngr) nx[grp] = static_cast<unsigned short>(nxt);
+                if (grp < ngr) nx[grp] = static_cast<unsigned short>(nxt | mask << 8);
                 carry = __shfl_sync(0xffffffffu, nxt, 0);
             }
         }
-        if (tid < npairs) s_MS[tid * 2] = __ldcg(a.fac_M + (kvh * gqa + tid / nch) * 4 + tid % nch);
-        if (ks.split && tid < gqa * 8) {
+        if (ks.split && tid >= kMegaThreads - gqa * 8) {
             // The factors that fold chunk c into the running result (attention.rs:510-541): the maximum before the chunk is
             // that of the earlier non-empty chunks, so the eight exponentials of a head are independent: one thread each.
-            const int g = tid >> 3, c = (tid >> 1) & 3, which = tid & 1;
-            const float* Mg = a.fac_M + (kvh * gqa + g) * 4;
+            const int t = tid - (kMegaThreads - gqa * 8), g = t >> 3, c = (t >> 1) & 3, which = t & 1;
             float m_before = -INFINITY;
             for (int k = 0; k < c; ++k)
-                if (chunk_len(k) > 0) m_before = fmaxf(m_before, __ldcg(Mg + k));
-            const float M = __ldcg(Mg + c), m_new = fmaxf(m_before, M);
-            s_scale[tid] = device_expf(__fsub_rn(which == 0 ? m_before : M, m_new));
+                if (chunk_len(k) > 0) m_before = fmaxf(m_before, s_MS[(g * nch + k) * 2]);
+            const float M = s_MS[(g * nch + c) * 2], m_new = fmaxf(m_before, M);
+            s_scale[t] = device_expf(__fsub_rn(which == 0 ? m_before : M, m_new));
         }
         cp_async_wait<0>();
     }
     __syncthreads();
     QTB_FINE(a, 3);
-    QTB_V2_CLOCK(3);
     float acc = 0.0f;
     const int head = warp / kV2WarpsPerHead, part8 = warp % kV2WarpsPerHead;  // chain warps: (query head, eight of the unit's coordinates)
     if (warp < gqa * kV2WarpsPerHead) {
@@ -1180,7 +1114,6 @@ __device__ __noinline__ void mega_values2_unit(const MegaArgs& a, const MegaLaye
         const uint32_t f_off = static_cast<uint32_t>(reinterpret_cast<const unsigned char*>(s_next + head * (ngr8 + 2)) - smem);
         acc = v2_chain<F32>(v_off, w_off, m_off, f_off, ngr);
         QTB_FINE(a, 9);
-        QTB_V2_CLOCK(4);
     } else {
         // S of every (head, chunk), one thread each, meanwhile
         const int pair = (warp - gqa * kV2WarpsPerHead) * 32 + lane;
@@ -1190,7 +1123,6 @@ __device__ __noinline__ void mega_values2_unit(const MegaArgs& a, const MegaLaye
     }
     __syncthreads();
     QTB_FINE(a, 12);
-    QTB_V2_CLOCK(5);
     if (warp < gqa * kV2WarpsPerHead) {
         // combine the chunks (attention.rs:497-541); every lane of a coordinate computes the same value
         const int d = lane & 7;
@@ -1243,7 +1175,7 @@ __device__ __noinline__ void mega_values2_unit(const MegaArgs& a, const MegaLaye
 // the group's queries, the new key/value rows), a values unit for the longest chunk, or the output head's activations (floats).
 // It is never smaller than kMegaRegionMin, which together with the vectors behind it decides which models take this kernel: wider ones
 // (past 8 to 9 thousand values) have not been run through it and take one kernel per step.
-constexpr size_t kMegaRegionMin = 129 * 1024;
+constexpr size_t kMegaRegionMin = 127 * 1024;
 __host__ __device__ constexpr size_t mega_attn_region(int ctx, int gqa, int head_dim, int hidden, bool v2) {
     const int len_max = ctx < 512 ? ctx : (ctx + 3) / 4;
     size_t need = static_cast<size_t>(kAttnBlockBytes) + static_cast<size_t>(gqa) * head_dim * 4 + static_cast<size_t>(head_dim) * 4 + 64;
@@ -1253,10 +1185,12 @@ __host__ __device__ constexpr size_t mega_attn_region(int ctx, int gqa, int head
     if (kMegaRegionMin > need) need = kMegaRegionMin;
     return (need + 1023) / 1024 * 1024;
 }
-// After the small arrays: the norm weights of the next norm (hidden floats) and a copy of every layer's descriptor.
+// After the small arrays: the norm weights of the next norm (hidden floats), a row of the cos/sin table, the kernel's arguments and a copy of every layer's descriptor.
+constexpr size_t kMegaArgsBytes = 1024;
+static_assert(sizeof(MegaArgs) <= kMegaArgsBytes, "the token kernel's arguments do not fit their place");
 __host__ __device__ constexpr size_t mega_smem_bytes(size_t attn_region, int maxvec, int hidden, int layers) {
     return attn_region + static_cast<size_t>(maxvec) * 4 + (static_cast<size_t>(maxvec) + 15) / 16 * 16 + 4096 +
-           (static_cast<size_t>(hidden) * 4 + 15) / 16 * 16 + static_cast<size_t>(layers) * sizeof(MegaLayer);
+           (static_cast<size_t>(hidden) * 4 + 15) / 16 * 16 + static_cast<size_t>(kMegaCosSin) * 4 + kMegaArgsBytes + static_cast<size_t>(layers) * sizeof(MegaLayer);
 }
 
 // ---- the token kernel ---------------------------------------------------------------------------------------------------
@@ -1271,10 +1205,14 @@ struct MegaSmem {
     double* sh_d;    // 32 doubles
     float* sh_f;     // 32 floats
     float* pair;     // chunk-combine factors: q_heads * (4 * 2 + 4) floats (q_heads <= kMegaMaxHeads)
+    unsigned long long* exp_tab;  // the exponential's table (g_exp2_tab)
     float* scale;    // [0] attention-input scale, [1] o-input scale, [2] ffn-input scale, [3] down-input scale (previous layer)
     int* flag;
+    int* pos;        // the token's position (a global load behind every grid barrier is a round trip to L2)
     float* w;        // weights of the next norm
+    float* cs;       // the position's row of the cos/sin table
     MegaLayer* layers;
+    MegaArgs* args;  // the kernel's arguments: a reference to the parameter itself makes every field a global load, which misses L1 behind every grid barrier
 };
 __device__ __forceinline__ MegaSmem mega_smem_views(unsigned char* smem, const MegaArgs& a) {
     MegaSmem v;
@@ -1286,10 +1224,14 @@ __device__ __forceinline__ MegaSmem mega_smem_views(unsigned char* smem, const M
     v.sh_d = reinterpret_cast<double*>(small);
     v.sh_f = reinterpret_cast<float*>(small + 256);
     v.pair = reinterpret_cast<float*>(small + 384);
+    v.exp_tab = reinterpret_cast<unsigned long long*>(small + 3456);
     v.scale = reinterpret_cast<float*>(small + 3968);
     v.flag = reinterpret_cast<int*>(small + 4000);
+    v.pos = reinterpret_cast<int*>(small + 4008);
     v.w = reinterpret_cast<float*>(small + 4096);
-    v.layers = reinterpret_cast<MegaLayer*>(small + 4096 + (static_cast<size_t>(a.hidden) * 4 + 15) / 16 * 16);
+    v.cs = v.w + (a.hidden + 3) / 4 * 4;
+    v.args = reinterpret_cast<MegaArgs*>(v.cs + kMegaCosSin);
+    v.layers = reinterpret_cast<MegaLayer*>(reinterpret_cast<unsigned char*>(v.args) + kMegaArgsBytes);
     return v;
 }
 
@@ -1459,14 +1401,14 @@ __device__ __noinline__ void phase_scores(const MegaArgs& a, int l, unsigned cha
     const MegaSmem v = mega_smem_views(smem, a);
     const int tid = threadIdx.x, cta = blockIdx.x, G = gridDim.x;
     const MegaLayer& ly = v.layers[l];
-    const KvSplit ks = kv_split(a);
+    const KvSplit ks = kv_split(a, *v.pos);
     int R = (a.kv_heads * ks.seq_len + G - 1) / G;
     R = max(16, min(R, kAttnBlockPos));
     const int per_head = (ks.seq_len + R - 1) / R;
     const float s_h = v.scale[0];
     for (int u = cta; u < a.kv_heads * per_head; u += G) {
         const int kvh = u / per_head, r0 = (u - kvh * per_head) * R;
-        mega_scores_unit(a, ly, kvh, r0, min(R, ks.seq_len - r0), s_h, smem);
+        mega_scores_unit(a, ly, ks.pos, v.cs, kvh, r0, min(R, ks.seq_len - r0), s_h, smem);
     }
     if (cta == G - 1) {
         for (int i = tid; i < a.hidden; i += kMegaThreads) a.acc_down[i] = 0;  // read by every CTA in phase A, rewritten by down
@@ -1481,7 +1423,7 @@ __device__ __noinline__ void phase_scores(const MegaArgs& a, int l, unsigned cha
 __device__ __noinline__ void phase_values(const MegaArgs& a, int l, unsigned char* smem) {
     const MegaSmem v = mega_smem_views(smem, a);
     const int cta = blockIdx.x, G = gridDim.x;
-    const KvSplit ks = kv_split(a);
+    const KvSplit ks = kv_split(a, *v.pos);
     const int nchunks = ks.split ? 4 : 1, slices = a.head_dim / kAttnSlice;
     // The value chains are pure latency (one dependent step per position) and leave the memory system idle: the o, gate, up
     // and down weights of this layer are requested into L2 now.
@@ -1489,37 +1431,19 @@ __device__ __noinline__ void phase_values(const MegaArgs& a, int l, unsigned cha
         for (int k = 3; k < 7; ++k) prefetch_weights(v.layers[l], k);
     for (int u = cta; u < a.kv_heads * nchunks * slices; u += G) {
         const int slice = u % slices, c = (u / slices) % nchunks, kvh = u / (slices * nchunks);
-        mega_values_unit(a, v.layers[l], kvh, c, slice, smem);
+        mega_values_unit(a, v.layers[l], ks.pos, kvh, c, slice, smem);
     }
 }
 
-// Phase C2, second form: one unit per (KV head, 8 coordinates); see mega_values2_unit.
+// Phase C2, second form: one unit per (KV head, 16 coordinates); see mega_values2_unit.
 __device__ __noinline__ void phase_values2(const MegaArgs& a, int l, unsigned char* smem) {
     const MegaSmem v = mega_smem_views(smem, a);
-    const int slices = a.head_dim / kV2Dims, units = a.kv_heads * slices, G = gridDim.x, cta = blockIdx.x;
-    if (cta < units) {  // the host chose this form only if units < gridDim.x
-        if (a.f32_values)
-            mega_values2_unit<true>(a, v.layers[l], l, cta / slices, cta % slices, smem);
-        else
-            mega_values2_unit<false>(a, v.layers[l], l, cta / slices, cta % slices, smem);
-        return;
-    }
-    // helpers: the factor tasks, interleaved over the KV heads so that every head's first tasks start at once
-    const KvSplit ks = kv_split(a);
-    const int nch = ks.split ? 4 : 1, tasks = a.q_heads * nch;
-    int done = 0;
-    for (int t = cta - units; t < tasks; t += G - units) {
-        v2_factors_task(a, t / nch, t % nch, smem);
-        ++done;
-    }
-    if (done) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < 13 * 64; i += kMegaThreads) {  // the zero rows of the table the tasks wrote over
-            const int k = i >> 6;
-            reinterpret_cast<int*>(smem)[(k < 9 ? 28 * k + 27 : 243 + k) * 64 + (i & 63)] = 0;
-        }
-        __syncthreads();
-    }
+    const int slices = a.head_dim / kV2Dims, cta = blockIdx.x;
+    if (cta >= a.kv_heads * slices) return;  // the host chose this form only if there are no more units than blocks
+    if (a.f32_values)
+        mega_values2_unit<true>(a, v.layers[l], l, *v.pos, v.exp_tab[threadIdx.x & 31], cta / slices, cta % slices, smem);
+    else
+        mega_values2_unit<false>(a, v.layers[l], l, *v.pos, v.exp_tab[threadIdx.x & 31], cta / slices, cta % slices, smem);
 }
 
 // Phase D after phase_values2: the attention output is complete in a.attn_out and, without a sub-norm, so is its maximum;
@@ -1573,7 +1497,7 @@ __device__ __noinline__ bool phase_combine(const MegaArgs& a, int l, unsigned in
     const MegaSmem v = mega_smem_views(smem, a);
     const int tid = threadIdx.x, hd = a.head_dim, qd = a.q_heads * hd;
     float* s_pair = v.pair;
-    const KvSplit ks = kv_split(a);
+    const KvSplit ks = kv_split(a, *v.pos);
     QTB_FINE(a, 21);
     // every chunk value of a thread's coordinates is requested before the factors are needed
     float amax = 0.0f;
@@ -1953,8 +1877,6 @@ __device__ __noinline__ void phase_finish(const MegaArgs& a, unsigned int seq_ba
         a.amax_bits[1] = 0u;
         a.amax_bits[2] = 0u;
         a.amax_bits[3] = 0u;
-        if (a.attn_v2)
-            for (int k = 0; k < a.kv_heads; ++k) a.fac_done[k] = 0u;
         *reinterpret_cast<volatile uint32_t*>(&a.report->token) = tok;
     }
     __syncthreads();  // (the clearing above)
@@ -1962,23 +1884,29 @@ __device__ __noinline__ void phase_finish(const MegaArgs& a, unsigned int seq_ba
 }
 
 template <uint32_t BASE>
-__global__ void __launch_bounds__(kMegaThreads, 1) decode_token_kernel(const __grid_constant__ MegaArgs a) {
+__global__ void __launch_bounds__(kMegaThreads, 1) decode_token_kernel(const __grid_constant__ MegaArgs params) {
     extern __shared__ __align__(1024) unsigned char smem[];
     const int tid = threadIdx.x, cta = blockIdx.x, G = gridDim.x;
     if (static_cast<uint32_t>(__cvta_generic_to_shared(smem)) != BASE) {
-        if (tid == 0) atomicMax(a.status, 1u);
+        if (tid == 0) atomicMax(params.status, 1u);
         return;
     }
+    const MegaArgs& a = *mega_smem_views(smem, params).args;
     {
-        const MegaSmem v = mega_smem_views(smem, a);
+        const MegaSmem v = mega_smem_views(smem, params);
+        for (int i = tid; i < static_cast<int>(sizeof(MegaArgs) / 4); i += kMegaThreads) reinterpret_cast<uint32_t*>(v.args)[i] = reinterpret_cast<const uint32_t*>(&params)[i];
         for (int i = tid; i < 13 * 64; i += kMegaThreads) {  // byte values that are no velurex code look up zero
             const int k = i >> 6;
             v.tab[(k < 9 ? 28 * k + 27 : 243 + k) * 64 + (i & 63)] = 0;
         }
-        request_norm_weights(v.w, a.n_layers > 0 ? a.layers[0].attn_norm : a.out_norm, a.hidden);
-        for (int i = tid; i < a.n_layers * static_cast<int>(sizeof(MegaLayer) / 4); i += kMegaThreads)
-            reinterpret_cast<uint32_t*>(v.layers)[i] = reinterpret_cast<const uint32_t*>(a.layers)[i];
+        request_norm_weights(v.w, params.n_layers > 0 ? params.layers[0].attn_norm : params.out_norm, params.hidden);
+        for (int i = tid; i < params.n_layers * static_cast<int>(sizeof(MegaLayer) / 4); i += kMegaThreads)
+            reinterpret_cast<uint32_t*>(v.layers)[i] = reinterpret_cast<const uint32_t*>(params.layers)[i];
         if (tid < 4) v.scale[tid] = 0.0f;
+        if (tid < 32) v.exp_tab[tid] = g_exp2_tab[tid];
+        const int pos = static_cast<int>(params.pos[0]);
+        if (tid == 0) *v.pos = pos;
+        for (int i = tid; i < params.rope_dims; i += kMegaThreads) v.cs[i] = params.cos_sin[static_cast<size_t>(pos) * params.rope_dims + i];
         __syncthreads();
         if (a.l2_prefetch && a.n_layers > 0)
             for (int k = 0; k < 3; ++k) prefetch_weights(v.layers[0], k);  // the first layer's q, k and v

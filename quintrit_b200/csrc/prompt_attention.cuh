@@ -88,6 +88,7 @@ __global__ void __launch_bounds__(kTokenTileThreads, 2) attention_tile_kernel(At
 #pragma unroll
         for (int e = 0; e < E / 2; ++e) acc[g][e] = 0ull;
     }
+    const unsigned long long exp_entry = g_exp2_tab[lane];
     const int j = lane & 15, row0 = 8 * warp + 4 * (lane >> 4);  // phase A: accumulator lanes 2j, 2j + 1 of four rows
     for (int base = 0; base < len_block; base += kTokenTileRows) {
         asm volatile("cp.async.wait_group 1;" ::: "memory");  // the keys; the values may still be on their way
@@ -157,7 +158,7 @@ __global__ void __launch_bounds__(kTokenTileThreads, 2) attention_tile_kernel(At
                 if (lane == 0) excl = -INFINITY;
                 const float m_old = fmaxf(carry[g], excl);
                 const bool up = sc > m_old;
-                const float ex = device_expf(up ? __fsub_rn(m_old, sc) : __fsub_rn(sc, m_old));
+                const float ex = device_expf_warp(up ? __fsub_rn(m_old, sc) : __fsub_rn(sc, m_old), exp_entry);
                 if (r < rows) {
                     ms_g[r] = up ? ex : 1.0f;
                     vs_g[r] = up ? make_float2(1.0f, 1.0f) : make_float2(ex, ex);

@@ -80,6 +80,7 @@ __global__ void __launch_bounds__(kRowAttnThreads, 4) attention_rows_kernel(Attn
 #pragma unroll
     for (int k = 0; k < kChains; ++k) acc[k] = 0ull;
     float S = 0.0f;
+    const unsigned long long exp_entry = g_exp2_tab[lane];
     int s = 0;
     auto next_stage = [&]() -> const unsigned char* {  // its rows have landed; the buffer of the stage before is filled again
         asm volatile("cp.async.wait_group %0;" ::"n"(kRowAttnBuffers - 2) : "memory");
@@ -152,7 +153,7 @@ __global__ void __launch_bounds__(kRowAttnThreads, 4) attention_rows_kernel(Attn
             if (lane == 0) excl = -INFINITY;
             const float m_old = fmaxf(carry, excl);
             const bool up = sc > m_old;
-            const float ex = device_expf(up ? __fsub_rn(m_old, sc) : __fsub_rn(sc, m_old));
+            const float ex = device_expf_warp(up ? __fsub_rn(m_old, sc) : __fsub_rn(sc, m_old), exp_entry);
             if (p < rows) {
                 s_ms[g * kRowAttnRound + p] = up ? ex : 1.0f;
                 s_vs[g * kRowAttnRound + p] = up ? make_float2(1.0f, 1.0f) : make_float2(ex, ex);
