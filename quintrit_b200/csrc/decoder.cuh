@@ -40,6 +40,7 @@ struct quintrit_b200_decoder {
     float *s_h, *s_q, *s_i;
     int32_t *acc_qkv, *acc_o, *acc_gu, *acc_down;
     uint32_t *d_token, *d_pos, *d_history;
+    qtb::StepEnd* step_end = nullptr;
     uint32_t* d_steps = nullptr;              // steps done, counted on the device; `launched` counts them here
     uint32_t launched = 0;
     qtb::StepReport* report = nullptr;        // pinned host memory that steps write
@@ -351,8 +352,6 @@ inline int enqueue_token(quintrit_b200_decoder* d, bool with_head) {
         QTB_LAUNCH_CHECK();
         launch_lm_head(d->lm_head, d->x16, H, d->vocab, d->logits, d->bf16_tables, d->sm_count, s);
         QTB_LAUNCH_CHECK();
-        argmax_kernel<<<1, 1024, 0, s>>>(d->logits, d->vocab, d->d_token);
-        QTB_LAUNCH_CHECK();
     }
     return QUINTRIT_OK;
 }
@@ -369,17 +368,18 @@ inline int decoder_report_init(quintrit_b200_decoder* d) {
     QTB_CUDA(cudaHostAlloc(&p, sizeof(StepReport), cudaHostAllocPortable | cudaHostAllocMapped));
     d->report = static_cast<StepReport*>(p);
     *d->report = StepReport{};
-    return dev_alloc(d, &d->d_steps, 1);
+    const int rc = dev_alloc(d, &d->step_end, 1);
+    return rc != QUINTRIT_OK ? rc : dev_alloc(d, &d->d_steps, 1);
 }
 
-// Captures [one token + advance] into a graph the first time it is needed.
+// Captures [one token + the step's end] into a graph the first time it is needed.
 inline int decoder_graph(quintrit_b200_decoder* d) {
     if (d->graph_ready) return QUINTRIT_OK;
     cudaGraph_t g = nullptr;
     QTB_CUDA(cudaStreamBeginCapture(d->stream, cudaStreamCaptureModeThreadLocal));
     int rc = enqueue_token(d, true);
     if (rc == QUINTRIT_OK) {
-        advance_kernel<<<1, 1, 0, d->stream>>>(d->d_pos, d->d_history, d->d_token, d->d_steps, d->d_counters + 2, d->report);
+        step_end_kernel<<<step_end_blocks(d->vocab), kEndThreads, 0, d->stream>>>(d->logits, d->vocab, d->step_end, d->d_token, d->d_pos, d->d_history, d->d_steps, d->d_counters + 2, d->report);
         ++g_launches;
     }
     cudaError_t e = cudaStreamEndCapture(d->stream, &g);

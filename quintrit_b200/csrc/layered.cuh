@@ -1154,14 +1154,11 @@ inline int layered_logits_rows(quintrit_b200_decoder* d, int first, int n, float
     return d->lay->model->f32 ? layered_head_rows<float>(d, nullptr, first, n, logits) : layered_head_rows<bf16>(d, nullptr, first, n, logits);
 }
 
-// One token (id and position in device memory), logits and greedy choice: the body of the decoder's step graph.
+// One token (id and position in device memory) and its logits: the body of the decoder's step graph.
 int layered_enqueue_token(quintrit_b200_decoder* d, bool with_head) {
     int rc = layered_run(d, d->d_token, 1, layered_own(d, d->d_pos));
     if (rc != QUINTRIT_OK || !with_head) return rc;
-    if ((rc = layered_logits(d, 0, d->logits)) != QUINTRIT_OK) return rc;
-    argmax_kernel<<<1, 1024, 0, d->stream>>>(d->logits, d->vocab, d->d_token);
-    QTB_LAUNCH_CHECK();
-    return QUINTRIT_OK;
+    return layered_logits(d, 0, d->logits);
 }
 
 // Tokens at positions pos0 .. pos0 + count - 1 of a sequence, in chunks; logits at the places `want` (ascending indices into tokens) go to
