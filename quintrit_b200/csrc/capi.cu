@@ -2691,6 +2691,10 @@ struct quintrit_b200_moe {
     // into pinned memory; behind it is room for the inputs on their way up.
     char *pack = nullptr, *host = nullptr;
     size_t pack_out = 0, host_x = 0;  // bytes in front of `out`; bytes in front of the inputs
+    // The two copies and eight launches of a whole block's forward as one graph per batch size, from the second forward of that size on (the host took longer to issue
+    // them than the device to run the short ones).
+    std::vector<cudaGraphExec_t> graph;  // [max_batch + 1], nullptr until captured
+    std::vector<char> warm;
     char* on_host(const void* p) const { return host + (static_cast<const char*>(p) - pack); }  // where a part of the piece lies in the host's copy
     cudaStream_t stream = nullptr;
 };
@@ -2707,6 +2711,8 @@ int check_moe(const quintrit_b200_moe* m) {
 void destroy_moe(quintrit_b200_moe* m) {
     if (m == nullptr) return;
     DeviceGuard g(m->device);
+    for (cudaGraphExec_t g : m->graph)
+        if (g != nullptr) cudaGraphExecDestroy(g);
     if (m->stream) cudaStreamDestroy(m->stream);
     for (void* p : m->allocs) cudaFree(p);
     if (m->host) cudaFreeHost(m->host);
@@ -2837,13 +2843,44 @@ int moe_whole(quintrit_b200_moe* m, const float* x, size_t batch, float* out, ui
     const int B = static_cast<int>(batch), K = m->top_k;
     const size_t x_bytes = batch * m->hidden * sizeof(float), bytes = m->pack_out + x_bytes;
     std::memcpy(m->host + m->host_x, x, x_bytes);
-    QTB_CUDA(cudaMemcpyAsync(m->x, m->host + m->host_x, x_bytes, cudaMemcpyHostToDevice, s));
-    int rc = moe_enqueue(m, B);
-    if (rc != QUINTRIT_OK) return rc;
+    int rc = QUINTRIT_OK;
     m->n_local = B * K, m->last_batch = B;  // (local_z counts up from zero in such a block)
+    auto enqueue = [&]() -> int {
+        QTB_CUDA(cudaMemcpyAsync(m->x, m->host + m->host_x, x_bytes, cudaMemcpyHostToDevice, s));
+        int r = moe_enqueue(m, B);
+        if (r == QUINTRIT_OK) r = moe_enqueue_experts(m, B, true);
+        if (r == QUINTRIT_OK) QTB_CUDA(cudaMemcpyAsync(m->host, m->pack, bytes, cudaMemcpyDeviceToHost, s));
+        return r;
+    };
+    if (m->graph.size() <= batch) m->graph.resize(batch + 1, nullptr), m->warm.resize(batch + 1, 0);  // (batch <= max_batch)
+    if (m->graph[batch] == nullptr && m->warm[batch]) {
+        cudaGraph_t g = nullptr;
+        QTB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        rc = enqueue();
+        const cudaError_t e = cudaStreamEndCapture(s, &g);
+        if (rc != QUINTRIT_OK) {
+            if (g) cudaGraphDestroy(g);
+            return rc;
+        }
+        if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture(mixture of experts)");
+        const cudaError_t ei = cudaGraphInstantiate(&m->graph[batch], g, 0);
+        cudaGraphDestroy(g);
+        if (ei != cudaSuccess) {
+            m->graph[batch] = nullptr;
+            return cuda_fail(ei, "cudaGraphInstantiate(mixture of experts)");
+        }
+    }
+    if (m->graph[batch] != nullptr) {
+        QTB_CUDA(cudaGraphLaunch(m->graph[batch], s));
+    } else {
+        if ((rc = enqueue()) != QUINTRIT_OK) return rc;
+        m->warm[batch] = 1;
+    }
     for (bool again = false;; again = true) {
-        if ((rc = moe_enqueue_experts(m, B, true)) != QUINTRIT_OK) return rc;
-        QTB_CUDA(cudaMemcpyAsync(m->host, m->pack, bytes, cudaMemcpyDeviceToHost, s));
+        if (again) {
+            if ((rc = moe_enqueue_experts(m, B, true)) != QUINTRIT_OK) return rc;
+            QTB_CUDA(cudaMemcpyAsync(m->host, m->pack, bytes, cudaMemcpyDeviceToHost, s));
+        }
         QTB_CUDA(cudaStreamSynchronize(s));
         if (reinterpret_cast<unsigned int*>(m->on_host(m->counters))[2] != 0) return fail(QUINTRIT_ERR_DEVICE, "GEMV kernel on the CUDA device found its shared-memory table at an unexpected address");
         bool ties = false;
