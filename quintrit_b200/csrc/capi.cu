@@ -2520,7 +2520,8 @@ int prefill_layers(quintrit_b200_decoder* d, int n, const BatchTarget& tg) {
         if (qkv_views) rk.v_q = v_q, rk.v_k = v_k, rk.v_v = v_v;
         rk.k_cache = tg.kc + static_cast<size_t>(l) * d->ctx * kvd;
         rk.v_cache = tg.vc + static_cast<size_t>(l) * d->ctx * kvd;
-        rope_kv_kernel<<<dim3(((qd + kvd) / 2 + kvd + 255) / 256, 1, n), 256, 0, s>>>(rk);
+        if (rope_rows_fit(rk)) rope_kv_rows_kernel<<<dim3(((qd + 2 * kvd) / 8 + kRopeThreads - 1) / kRopeThreads, 1, n), kRopeThreads, 0, s>>>(rk);
+        else rope_kv_kernel<<<dim3(((qd + kvd) / 2 + kvd + 255) / 256, 1, n), 256, 0, s>>>(rk);
         QTB_LAUNCH_CHECK();
         AttnArgs at{};
         at.q = d->pf.q, at.b_q = qd;

@@ -175,6 +175,70 @@ __global__ void __launch_bounds__(1024) norm_quant_rows_kernel(const __grid_cons
     if (threadIdx.x == 0) a.scale_out[a.b_scale ? z : 0] = s;
 }
 
+// Rotation of queries and keys and the cache's new rows (rope_kv_kernel's operations) for many tokens: eight elements a thread - eight neighbours, or with NEOX pairing
+// four neighbours and their four partners - in 16-byte loads and stores. Grid (blocks of 128 threads over a token's elements, 1, tokens). Bound by its instructions where
+// an element a thread was divided, scaled and looked up by itself (1000 tokens of 12 + 2 x 4 heads of 256: 30 us at 75 % of the issue slots; see rope_rows_fit).
+constexpr int kRopeThreads = 128;
+inline bool rope_rows_fit(const RopeKvArgs& a) { return !a.block_scaled && a.v_q.base != nullptr && a.rope_dims % 8 == 0 && a.head_dim % 8 == 0; }
+__device__ __forceinline__ void scaled4(const AccView& v, int i, float post, bool live, float (&x)[4]) {
+    const int4 s = acc_view_read4(v, blockIdx.z, i);
+    x[0] = live ? __fmul_rn(static_cast<float>(s.x), post) : 0.0f, x[1] = live ? __fmul_rn(static_cast<float>(s.y), post) : 0.0f;
+    x[2] = live ? __fmul_rn(static_cast<float>(s.z), post) : 0.0f, x[3] = live ? __fmul_rn(static_cast<float>(s.w), post) : 0.0f;
+}
+__device__ __forceinline__ uint2 halves4(const float (&x)[4]) {
+    const __half2 lo = __floats2half2_rn(x[0], x[1]), hi = __floats2half2_rn(x[2], x[3]);
+    return make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+}
+__global__ void __launch_bounds__(kRopeThreads) rope_kv_rows_kernel(const __grid_constant__ RopeKvArgs a) {
+    const size_t z = blockIdx.z;
+    const int qk = (a.q_dim + a.kv_dim) / 8, t = blockIdx.x * kRopeThreads + threadIdx.x;
+    if (t >= qk + a.kv_dim / 8) return;
+    const float s = a.act_scale[a.b_scale ? z : 0];
+    const bool live = s > 0.0f;
+    const uint32_t pos = seq_position(a.seq, a.pos, blockIdx.z);
+    const size_t row = seq_cache_offset(a.seq, blockIdx.z) + static_cast<size_t>(pos) * a.kv_dim;
+    float x[4], y[4];
+    if (t >= qk) {  // values: scale and append
+        const int i = (t - qk) * 8;
+        const float post = live ? __fdiv_rn(a.ws_v, s) : 0.0f;
+        scaled4(a.v_v, i, post, live, x), scaled4(a.v_v, i + 4, post, live, y);
+        *reinterpret_cast<uint2*>(a.v_cache + row + i) = halves4(x);
+        *reinterpret_cast<uint2*>(a.v_cache + row + i + 4) = halves4(y);
+        return;
+    }
+    const int per_head = a.head_dim / 8, h = t / per_head, item = t - h * per_head, base = h * a.head_dim;
+    const bool is_q = base < a.q_dim, rot = item < a.rope_dims / 8;
+    const float post = live ? __fdiv_rn(is_q ? a.ws_q : a.ws_k, s) : 0.0f;
+    // where x and y lie in the head: neighbours, or (NEOX, rotated part) half the rotated dimensions apart
+    const bool apart = a.neox && rot;
+    const int d0 = apart ? item * 4 : item * 8, d1 = apart ? d0 + a.rope_dims / 2 : d0 + 4;
+    const AccView& v = is_q ? a.v_q : a.v_k;
+    const int from = is_q ? base : base - a.q_dim;
+    scaled4(v, from + d0, post, live, x), scaled4(v, from + d1, post, live, y);
+    if (rot) {
+        const float* cs = a.cos_sin + static_cast<size_t>(pos) * a.rope_dims;
+        auto turn = [](float& p, float& q, float c, float sn) {
+            const float r0 = __fmaf_rn(p, c, -__fmul_rn(q, sn)), r1 = __fmaf_rn(p, sn, __fmul_rn(q, c));
+            p = r0, q = r1;
+        };
+        if (apart) {
+            const float4 c0 = *reinterpret_cast<const float4*>(cs + 2 * d0), c1 = *reinterpret_cast<const float4*>(cs + 2 * d0 + 4);
+            turn(x[0], y[0], c0.x, c0.y), turn(x[1], y[1], c0.z, c0.w), turn(x[2], y[2], c1.x, c1.y), turn(x[3], y[3], c1.z, c1.w);
+        } else {
+            const float4 c0 = *reinterpret_cast<const float4*>(cs + d0), c1 = *reinterpret_cast<const float4*>(cs + d1);
+            turn(x[0], x[1], c0.x, c0.y), turn(x[2], x[3], c0.z, c0.w), turn(y[0], y[1], c1.x, c1.y), turn(y[2], y[3], c1.z, c1.w);
+        }
+    }
+    if (is_q) {
+        float* q = a.q_out + z * a.b_q + base;
+        *reinterpret_cast<float4*>(q + d0) = make_float4(x[0], x[1], x[2], x[3]);
+        *reinterpret_cast<float4*>(q + d1) = make_float4(y[0], y[1], y[2], y[3]);
+    } else {
+        *reinterpret_cast<uint2*>(a.k_cache + row + from + d0) = halves4(x);
+        *reinterpret_cast<uint2*>(a.k_cache + row + from + d1) = halves4(y);
+    }
+}
+
 // The factors of a head's four chunks (attn_combine_chunks), which are the same for all its coordinates.
 struct ChunkFactors {
     float older[4], newer[4], inv;

@@ -117,3 +117,18 @@ def test_long_passes_equal_short_ones(arch, inter, n):
         lb, tb = b.forward(got_next, n + step)
         assert np.array_equal(la.view(np.uint32), lb.view(np.uint32)) and ta == tb
         want_next = got_next = ta
+
+
+@pytest.mark.parametrize("arch,rope_dims", [(q.ARCH_LLAMA, 64), (q.ARCH_LLAMA, 32), (q.ARCH_LLAMA, 20), (q.ARCH_BITNET, 64), (q.ARCH_BITNET, 40), (q.ARCH_BITNET, 12)])
+def test_rotated_dimensions_of_a_chunk(arch, rope_dims):
+    """Heads rotated whole, in part (whole eights: rope_kv_rows_kernel; others: rope_kv_kernel), neighbouring and distant pairs, against single steps."""
+    spec = _spec(arch, arch == q.ARCH_BITNET, 3 + rope_dims, tied=arch == q.ARCH_BITNET)
+    spec["rope_dims"] = rope_dims
+    tokens = synth.prompt_tokens(13, 45, spec["vocab"])
+    a, b = q.Decoder(spec), q.Decoder(spec)
+    for pos, t in enumerate(tokens):
+        want, want_next = a.forward(int(t), pos)
+    got, got_next = b.prefill(tokens)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32)) and got_next == want_next
+    la, lb = a.forward(want_next, 45)[0], b.forward(got_next, 45)[0]
+    assert np.array_equal(la.view(np.uint32), lb.view(np.uint32))
