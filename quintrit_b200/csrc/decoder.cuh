@@ -82,7 +82,7 @@ struct quintrit_b200_decoder {
     unsigned int* tp_seq = nullptr;
     bool tp_attached = false;
     void* tp_peer[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};  // peer boxes opened through IPC
-    // prompt ingestion in chunks of up to kPrefillMax tokens (batched projections on the tensor cores): per-token rows of the step buffers, made on first use
+    // prompt ingestion in passes of up to kPrefillMax tokens (batched projections on the tensor cores): per-token rows of the step buffers, made on first use
     struct Prefill {
         uint32_t* tokens = nullptr;
         uint32_t* pos = nullptr;

@@ -12,7 +12,7 @@
 // and the token ends with the final norm, the output head (rows split over CTAs), the greedy choice and pos += 1.
 // Between two grid barriers a phase lasts 1 to 8 us, so every trip to L2 before its work counts: the kernel's arguments, the position and the cos/sin row
 // of the position lie in shared memory (read through a reference to the kernel's parameter, each argument was a global load behind every barrier). With scores by
-// four threads a row: 62.8 -> 58.5 us a layer of the Falcon3-10B shape at context 1024, 59.8 -> 53.5 of the BitNet-2B shape (cycle stamps of block 0).
+// four threads a row: 62.8 -> 57.5 us a layer of the Falcon3-10B shape at context 1024, 59.8 -> 56.2 of the BitNet-2B shape (cycle stamps of block 0).
 // All arithmetic is the device functions of decode.cuh / gemv_lut.cuh, so the bits equal the per-kernel path and the
 // reference CPU runtime. Every wait is bounded: a barrier that does not complete sets status and the kernel returns.
 #pragma once
@@ -831,7 +831,7 @@ __device__ __noinline__ void mega_values_unit(const MegaArgs& a, const MegaLayer
     __syncthreads();
 }
 
-// ---- attention, second half, second form: one unit per (KV head, 8 coordinates) -----------------------------------------
+// ---- attention, second half, second form: one unit per (KV head, 16 coordinates) -----------------------------------------
 // The value accumulation is a chain of one dependent step per position (about 16 cycles: multiply-add, round to half,
 // widen), so its length, not the work, sets the time. A unit therefore takes ALL chunks of its coordinates at once: lane
 // (chunk, coordinate) of warp g runs the chain of query head g for that chunk, the four chunks of the reference's split

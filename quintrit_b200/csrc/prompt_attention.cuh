@@ -12,7 +12,8 @@
 // Bound by instruction issue and, in C, by the heavy half of the FMA pipe, which converts between F16 and F32 (ncu, 232 tokens at positions 768 to 999, 12 /
 // 4 heads of 256: 201 us, while a multiprocessor is active 54 % of the issue slots and 58 % of that pipe; 40 warp instructions per token, head and
 // position with the tiles' overhang, of which the source has 9 in a score and 22 in the chains). The 1000-token prompt of a 4-layer Falcon3-10B shape:
-// 8.03 -> 6.11 ms against a block per token (attention_gqa_kernel).
+// 8.03 -> 6.11 ms against a block per token (attention_gqa_kernel). With all 1000 tokens in one launch, the last first: 580 -> 418 us a layer; still half the issue slots and half of the
+// heavy side busy, 3.8 warps a scheduler (128 registers, 110 KB a block). Widening by mixed-precision additions, which either side takes: 3 % slower.
 #pragma once
 #include "decode.cuh"
 #include "packed_f32.cuh"

@@ -232,7 +232,7 @@ int rt_feed(quintrit_session* s, const uint32_t* ids, size_t n, uint32_t pos0, b
     quintrit_b200_decoder* d = s->dec;
     DeviceGuard g(d->device);
     if (n >= 8 && prefill_available(d) && std::getenv("QUINTRIT_B200_NO_PREFILL") == nullptr) {
-        // a prompt goes in chunks of up to 256 tokens with the projections on the tensor cores; the result is that of n single steps
+        // a prompt goes in passes of up to 1024 tokens with the projections on the tensor cores; the result is that of n single steps
         int rc = decoder_prefill(d, ids, n, pos0);
         if (rc != QUINTRIT_OK) return rc;
         if ((rc = rt_enqueue_sample(d, sample)) != QUINTRIT_OK) return rc;
