@@ -2241,6 +2241,7 @@ int gemm_launch(quintrit_b200_matrix* m, const int8_t* d_act, int batch, int32_t
     const bool in_place = m->cols % 16 == 0 && reinterpret_cast<uintptr_t>(d_act) % 16 == 0;
     const void* base = d_act;
     cuuint64_t pitch = m->cols, vectors = static_cast<cuuint64_t>(batch);
+    if (!in_place && (batch > kGemmMaxN || m->d_gemm_act == nullptr)) return fail(QUINTRIT_ERR_INVALID_ARGUMENT, "%d vectors of %zu values cannot be read in place", batch, m->cols);
     if (!in_place) {
         gemm_pad_activations_kernel<<<std::min((n * k_pad + 255) / 256, 148 * 8), 256, 0, stream>>>(d_act, m->d_gemm_act, batch, n, static_cast<int>(m->cols), k_pad);
         ++g_launches;
