@@ -412,17 +412,15 @@ inline void layered_store_view(const LayeredModel& m, const LayeredStore& st, si
     c.pk = static_cast<char*>(c.pk) + pools * dp, c.pv = static_cast<char*>(c.pv) + pools * vp;
 }
 
-// Shares a decode step's attention is cut into: enough blocks for the device, none below 16 keys (logistic) or 32 (pooled). A block's time is mostly a chain
-// of waits, but its keys count too: with shares of a whole tile (128, 64) 348 keys were 3 and 6 blocks a head group, a Tosevik step of six layers took 252 us, now 246, a
-// Lasosun step 152, now 148 (8 keys: 152).
+// Shares a decode step's attention is cut into: enough blocks for the device, none below one tile of keys.
 inline int attention_splits(const MixerSpec& l, int ctx, int n, int sm_count) {
     if (l.kind == MixerKind::kLogistic) {
         const int gqa = l.heads / l.kv_heads, per = logistic_heads(gqa), groups = l.kv_heads * ((gqa + per - 1) / per) * n;
-        return std::max(1, std::min({(ctx + 15) / 16, (sm_count + groups - 1) / groups, 64}));
+        return std::max(1, std::min({(ctx + kLaKeys - 1) / kLaKeys, (sm_count + groups - 1) / groups, 64}));
     }
     const int groups = l.kv_heads * ((l.heads / l.kv_heads + kPaHeads - 1) / kPaHeads) * n;
     const int keys = std::min(ctx, l.window) + (l.pool > 0 ? ctx / l.pool : 0);
-    return std::max(1, std::min({(keys + 31) / 32, 4 * sm_count / groups, 64}));
+    return std::max(1, std::min({(keys + kPaTile - 1) / kPaTile, 4 * sm_count / groups, 64}));
 }
 typedef void (*LogisticStep)(LogisticArgs, int, int);
 template <typename T, bool OWN> LogisticStep logistic_step_for(int heads) {

@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kPaThreads) pooled_attention_kernel(const __gr
     const float* prow = a.p + size_t(z) * a.ld;
     if (tid < kPaHeads) m_run[tid] = -INFINITY, l_run[tid] = 0.0f;
     const int nb = pooled_blocks_seen(pos, a.window, a.pool), lo = max(0, pos - a.window + 1), total = nb + pos - lo + 1;
-    const int per = ((total + a.splits - 1) / a.splits + 7) / 8 * 8;
+    const int per = ((total + a.splits - 1) / a.splits + kPaTile - 1) / kPaTile * kPaTile;
     const int begin = min(split * per, total), end = min(begin + per, total);
     const T* ring_k = static_cast<const T*>(a.cache.k) + (size_t(slot) * a.cache.ring * a.kv_heads + kvh) * dp;
     const T* ring_v = static_cast<const T*>(a.cache.v) + (size_t(slot) * a.cache.ring * a.kv_heads + kvh) * vp;

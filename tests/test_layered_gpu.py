@@ -186,6 +186,18 @@ def test_the_ring_of_the_cache_is_used_again(tmp_path, dtype):
     check(in_portions(s, ids, [700]), want, dtype)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_keys_within_a_tile_are_one_share_whatever_the_session_holds(tmp_path, dtype):
+    """A share of a step's keys is at least one tile of 64, so while all keys fit a tile the order of every sum, and so every bit, is the same in a small and in a large session."""
+    config = mf.lasosun_config([A(6, 3, 24, 40, 400, 16, ff=48), A(4, 1, 32, 16, 300, 8)], 56, 45, 400)
+    small, w = build(tmp_path, config, 31, dtype, context=70)
+    large = Model.load(small.path, dtype=dtype, context=400)
+    ids = ids_for(32, 62, 45)
+    a, b = (in_portions(m.new_session(), ids, [1]) for m in (small, large))
+    check(a, plain.lasosun(config, w, ids), dtype)
+    assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
 @pytest.mark.parametrize("kind", ["mamba2", "hgrn2"])
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_a_state_carries_over_hundreds_of_tokens_and_strong_decays(tmp_path, kind, dtype):

@@ -228,6 +228,18 @@ def test_one_key_far_back_and_at_the_borders_of_tiles_and_shares(tmp_path, temp,
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+def test_a_session_of_one_tile_of_keys_takes_one_share(tmp_path, dtype):
+    """Sessions of up to 128 positions, the keys of a tile, cut nothing: the order of every sum, and so every bit, is the same in a small and in a full one."""
+    config = mf.tosevik_config([PL(A(6, 3, 24, 40, every=17), R(4, 16, 24)), PL(A(8, 1, 40, 20, scale=0.3), R(2, 32, 16))], 56, 45)
+    small, w = build(tmp_path, config, 31, dtype, mf.random_tosevik(config, 31), context=60)
+    large = Model.load(small.path, dtype=dtype, context=128)
+    ids = ids_for(32, 60, 45)
+    a, b = (in_portions(m.new_session(), ids, [1]) for m in (small, large))
+    check(a, plain.tosevik(config, w, ids), dtype)
+    assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_distance_slopes_and_biases_of_every_head(tmp_path, dtype):
     """Queries and keys that all agree: the weights follow the distance alone, head by head."""
     config = mf.tosevik_config([PL(A(6, 2, 16, 24, coef=0.0, scale=0.01), R(1, 8, 8))], 64, 30)
