@@ -44,6 +44,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include "gemm_turns.hpp"
 #include "gemv_lut.cuh"
 
 namespace qtb {
@@ -51,7 +52,6 @@ namespace qtb {
 constexpr int kGemmM = 128;     // weight rows of a block; a pair takes two such tiles
 constexpr int kGemmDecodeWarps = 16;
 constexpr int kGemmGroups = 4;  // the decode warps work in groups of four; group g decodes the stages it, it + 4, ... of the pair's sequence on its own
-constexpr int kGemmLoadWarps = 2;  // load warp w fetches the stages w, w + 4, ...: the fixed cost of a stage (about 600 cycles in one warp) would bound small batches
 constexpr int kGemmThreads = 32 * (kGemmDecodeWarps + 1 + kGemmLoadWarps);  // decode warps, the MMA warp, load warps
 constexpr int kGemmMaxStages = 12;
 constexpr int kGemmMaxN = 256;  // 256 accumulator columns + 4 x 64 operand columns are the 512 columns of tensor memory
@@ -373,8 +373,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
             it0 += nkb;
         }
         if (!okay && lane == 0) raise_abort(abort_addr, rank);
-        // its own copies in flight land before the block leaves (stages before the last S are long used up)
-        for (int it = max(0, it0 - S); it < until; ++it)
+        // its own copies in flight land before the block leaves
+        for (int it = gemm_drain_from(until, S); it < until; ++it)
             if ((it & (kGemmLoadWarps - 1)) == mine) mbar_wait(loaded(it % S), (it / S) & 1, abort_flag, a.spin_limit, false);
     } else if (warp == kGemmDecodeWarps) {
         // ---- tensor cores of both blocks: eight MMAs per stage (A from tensor memory, B from shared memory), issued by one thread of the first block. The warp
@@ -388,7 +388,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
             const uint32_t b_stage16 = act_bytes >> 4, b_half16 = act_bytes >> 5;
             for (int item = first; item < items && okay; item += step, ++j) {
                 const int kb0 = part_of(item) * per, nkb = min(per, a.blocks - kb0);
-                if (!(okay = __all_sync(0xffffffffu, mbar_wait(acc_empty, (j & 1) ^ 1, abort_flag, a.spin_limit)))) break;  // the previous item's accumulator has been read
+                if (!(okay = __all_sync(0xffffffffu, mbar_wait(acc_empty, (j & 1) ^ 1, abort_flag, a.spin_limit)))) {  // the previous item's accumulator has been read
+                    if (j > 0) mbar_wait(acc_full, (j - 1) & 1, abort_flag, a.spin_limit, false);  // its products are done before anyone leaves (their end is committed already)
+                    break;
+                }
                 for (int k = 0; k < nkb; ++k, ++it) {
                     const int g = it & (kGemmGroups - 1);
                     // the groups' arrivals also stand for the stage's loads: each waited for its block's before it decoded

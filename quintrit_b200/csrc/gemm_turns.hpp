@@ -1,0 +1,20 @@
+// The order in which the load warps of the batched projection (gemm_tc.cuh) take the stages, as far as its exits need it: plain integers, so that it
+// can be followed without a device.
+#pragma once
+
+#ifdef __CUDACC__
+#define QTB_TURNS_FN __host__ __device__ inline constexpr
+#else
+#define QTB_TURNS_FN inline constexpr
+#endif
+
+namespace qtb {
+
+constexpr int kGemmLoadWarps = 2;  // load warp w fetches the stages w, w + 2, ... of the pair's sequence: the fixed cost of a stage (about 600 cycles in one warp) would bound small batches
+
+// The first stage whose copies a load warp waits for before its block leaves, when it has issued none from `until` on. Stage `it` is issued only after the products of
+// stage it - S, which lay in the same buffer, are done, and they read all stages up to it: of the stages before until - S nothing is in flight any more. It holds wherever the
+// warp stopped, also in the middle of an item: what counts is how far it came, not where the item would have ended.
+QTB_TURNS_FN int gemm_drain_from(int until, int stages) { return until > stages ? until - stages : 0; }
+
+}  // namespace qtb
