@@ -317,6 +317,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * kGemmMaxStages + kGemmGroups + 2);  // 30 barriers, then these two words
     volatile unsigned int* abort_flag = reinterpret_cast<volatile unsigned int*>(bars + 2 * kGemmMaxStages + kGemmGroups + 3);
     const uint32_t abort_addr = acc_empty + 16u;
+    volatile int* turn_until = reinterpret_cast<volatile int*>(bars + 2 * kGemmMaxStages + kGemmGroups + 4);  // how far the load warps came
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rank = cluster_rank();
@@ -374,7 +375,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
         }
         if (!okay && lane == 0) raise_abort(abort_addr, rank);
         // its own copies in flight land before the block leaves
-        for (int it = gemm_drain_from(until, S); it < until; ++it)
+        turn_until[mine] = until;
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * kGemmLoadWarps) : "memory");  // the load warps
+        int furthest = until;
+        for (int w = 0; w < kGemmLoadWarps; ++w) furthest = max(furthest, turn_until[w]);
+        for (int it = gemm_drain_from(furthest, S); it < until; ++it)
             if ((it & (kGemmLoadWarps - 1)) == mine) mbar_wait(loaded(it % S), (it / S) & 1, abort_flag, a.spin_limit, false);
     } else if (warp == kGemmDecodeWarps) {
         // ---- tensor cores of both blocks: eight MMAs per stage (A from tensor memory, B from shared memory), issued by one thread of the first block. The warp

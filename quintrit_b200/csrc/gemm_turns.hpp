@@ -12,9 +12,10 @@ namespace qtb {
 
 constexpr int kGemmLoadWarps = 2;  // load warp w fetches the stages w, w + 2, ... of the pair's sequence: the fixed cost of a stage (about 600 cycles in one warp) would bound small batches
 
-// The first stage whose copies a load warp waits for before its block leaves, when it has issued none from `until` on. Stage `it` is issued only after the products of
-// stage it - S, which lay in the same buffer, are done, and they read all stages up to it: of the stages before until - S nothing is in flight any more. It holds wherever the
-// warp stopped, also in the middle of an item: what counts is how far it came, not where the item would have ended.
+// The first stage whose copies a block's load warps wait for before it leaves; `until` is behind the last stage that any of them issued. That one was issued only after the
+// products of the stage S before it, which lay in the same buffer, were done, and they read all stages up to it: of the stages before until - S nothing is in flight
+// any more. From there on no buffer has been used again, so a stage's barrier is still in the phase behind its copies. It holds wherever the warps stopped, also in the middle of
+// an item: what counts is how far they came, not where the item would have ended.
 QTB_TURNS_FN int gemm_drain_from(int until, int stages) { return until > stages ? until - stages : 0; }
 
 }  // namespace qtb

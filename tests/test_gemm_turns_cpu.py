@@ -1,5 +1,6 @@
 """The exits of the batched projection's load warps (csrc/gemm_turns.hpp), followed on the host: wherever a warp stops, what it waits for is what may still be in flight."""
 import ctypes
+import itertools
 import os
 import subprocess
 
@@ -17,23 +18,21 @@ def turns(tmp_path_factory):
     return ctypes.CDLL(str(d / "turns.so"))
 
 
-def stages_of(warp, warps, total):
-    return range(warp, total, warps)
-
-
-@pytest.mark.parametrize("stages", [4, 5, 12])
-@pytest.mark.parametrize("items,per", [(1, 3), (1, 90), (2, 90), (3, 12), (5, 1)])
-def test_a_load_warp_that_stops_anywhere_waits_for_its_own_copies(turns, stages, items, per):
-    """The warp stops in front of any stage (in the middle of an item of 90 stages too, of which only a few are in flight) or behind the last."""
-    warps, total = turns.load_warps(), items * per
-    for warp in range(warps):
-        mine = list(stages_of(warp, warps, total))
-        for stop in range(len(mine) + 1):
-            issued = mine[:stop]
-            until = issued[-1] + 1 if issued else 0
-            # the products of stage i - stages were seen done before i was issued, and with them everything up to it
-            read = max((i - stages for i in issued), default=-1)
-            in_flight = {i for i in issued if i > read}
-            waited = {i for i in range(turns.drain_from(until, stages), until) if i % warps == warp}
-            assert waited == in_flight
-            assert len({i % stages for i in waited}) == len(waited)  # every buffer's barrier once: its last use
+@pytest.mark.parametrize("stages", [4, 5, 7, 12])
+@pytest.mark.parametrize("total", [1, 3, 13, 30])
+def test_load_warps_that_stop_anywhere_wait_for_their_own_copies(turns, stages, total):
+    """Either warp stops in front of any stage or behind the last, in the middle of an item too: together they wait for what may be in flight, and only at buffers that have
+    not been used again (a barrier two phases on would never show the phase that is waited for)."""
+    warps = turns.load_warps()
+    stops = range(total + warps)
+    for ends in itertools.product(stops, repeat=warps):
+        issued = sorted(it for w in range(warps) for it in range(w, min(ends[w], total), warps))
+        gap = next((it for it in range(total) if it not in issued), total)  # the products get no further than the first stage that is missing
+        if any(it - stages >= gap for it in issued):
+            continue  # a stage is issued when the one in its buffer has been multiplied
+        until = [max((it + 1 for it in issued if it % warps == w), default=0) for w in range(warps)]
+        read = max((it - stages for it in issued), default=-1)  # seen done by one warp or the other
+        waited = [it for w in range(warps) for it in range(turns.drain_from(max(until), stages), until[w]) if it % warps == w]
+        assert {it for it in issued if it > read} == set(waited)
+        for it in waited:
+            assert it + stages not in issued
