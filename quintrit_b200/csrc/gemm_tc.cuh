@@ -19,7 +19,9 @@
 //     store to shared memory need a proxy fence before the tensor cores may read them, and that fence was measured at more than a
 //     thousand cycles a block; operands in tensor memory need none;
 //   * two load warps, taking the stages in turn, fetch the tile's 8192 weight bytes (one bulk copy) and the matching activations (two
-//     TMA boxes of n / 2 vectors x 128 bytes, 128-byte swizzle, in place from the caller's vectors where their pitch allows it), completing on one mbarrier;
+//     TMA boxes of n / 2 vectors x 128 bytes, 128-byte swizzle, in place from the caller's vectors where their pitch allows it). What a block loads completes on one
+//     mbarrier of its own, but for the second block's activations: only the tensor cores read them, on the first block's command, so they complete on a barrier of the
+//     first block (the cta_group::2 form of the copy), where a decode warp sees it before it hands its operand to the issuing thread;
 //   * one thread of the pair's first block issues eight MMAs (256 x N x 32, A from tensor memory, B from shared memory) per stage and releases the stage
 //     and the group's operand columns in both blocks with tcgen05.commit; a ring of 5 to 12 stages (as many as fit) keeps the loads ahead;
 //   * the kernel is persistent: a pair takes items round-robin;
@@ -219,19 +221,22 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
-// An arrival at a barrier of either block. It orders nothing but what the tcgen05 fences and waits around it order (operands in tensor memory, accumulator reads) and
-// copies whose completion the arriving thread has seen: with .release.cluster an arrival, and .acquire.cluster a wait, cost about 3000 and 250 cycles.
+// An arrival at a barrier of either block. It orders nothing but what the tcgen05 fences and waits around it order (operands in tensor memory, accumulator reads), and nothing
+// else is handed over by it: with .release.cluster an arrival, and .acquire.cluster a wait, cost about 3000 and 250 cycles.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
     return p != 0;
 }
-__device__ __forceinline__ void raise_abort(uint32_t flag_addr, uint32_t rank) {  // in the other block too
-    asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(flag_addr, rank ^ 1)), "r"(1u) : "memory");
-}
+__device__ __forceinline__ void store_cluster(uint32_t addr, uint32_t value) { asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(value) : "memory"); }
+__device__ __forceinline__ void raise_abort(uint32_t flag_addr, uint32_t rank) { store_cluster(cluster_addr(flag_addr, rank ^ 1), 1u); }  // in the other block too
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+// The same with a barrier that may be the other block's (`bar`: an address in the cluster's window).
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
 }
 // 256 rows (128 in the tensor memory of either block) x N x 32; the first half of B's rows lies in the first block's shared memory, the rest in the second's.
 __device__ __forceinline__ void mma_i8_ts_pair(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
@@ -307,17 +312,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
     const uint32_t raw_base = smem0 + S * act_bytes;                      // S stages of the weight bytes of this block's tile
     const unsigned char* raw_tiles = smem + S * act_bytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S * (act_bytes + kGemmStageBytes));
-    // barriers of each block: loaded[S] (its weight bytes and activations of a stage have landed), empty[S] (the MMAs of the stage are done: it may be loaded again, and the
-    // group may write its next operand), acc_full (those of an item); of the first block only: a_full[G] (group g's operand is written in both blocks), acc_empty (both have read the accumulator)
+    // barriers of each block: loaded[S] (its weight bytes of a stage, and in the first block the activations, have landed), empty[S] (the MMAs of the stage are done: it may be loaded
+    // again, and the group may write its next operand), acc_full (those of an item); of the first block only: a_full[G] (group g's operand is written in both blocks), acc_empty (both
+    // have read the accumulator), peer_acts[S] (the second block's activations have landed in its shared memory)
     const uint32_t bar0 = smem_u32(bars);
     auto loaded = [&](int s) { return bar0 + 8u * s; };
     auto empty = [&](int s) { return bar0 + 8u * (kGemmMaxStages + s); };
     auto a_full = [&](int g) { return bar0 + 8u * (2 * kGemmMaxStages + g); };
     const uint32_t acc_full = bar0 + 8u * (2 * kGemmMaxStages + kGemmGroups), acc_empty = acc_full + 8u;
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * kGemmMaxStages + kGemmGroups + 2);  // 30 barriers, then these two words
-    volatile unsigned int* abort_flag = reinterpret_cast<volatile unsigned int*>(bars + 2 * kGemmMaxStages + kGemmGroups + 3);
-    const uint32_t abort_addr = acc_empty + 16u;
-    volatile int* turn_until = reinterpret_cast<volatile int*>(bars + 2 * kGemmMaxStages + kGemmGroups + 4);  // how far the load warps came
+    auto peer_acts = [&](int s) { return acc_empty + 8u * (1 + s); };
+    constexpr int kBarriers = 3 * kGemmMaxStages + kGemmGroups + 2;
+    static_assert(kBarriers * 8 + 8 + 8 * kGemmLoadWarps <= 512, "the barriers and words do not fit their place");
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + kBarriers);
+    volatile unsigned int* abort_flag = reinterpret_cast<volatile unsigned int*>(tmem_slot + 1);
+    volatile int* turn_until = reinterpret_cast<volatile int*>(tmem_slot + 2);  // how far the load warps came; in the first block, behind them: the second block's
+    const uint32_t abort_addr = bar0 + 8u * kBarriers + 4u, peer_until_addr = abort_addr + 4u + 4u * kGemmLoadWarps;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rank = cluster_rank();
@@ -332,6 +341,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
         for (int s = 0; s < S; ++s) {
             mbar_init(loaded(s), 1);  // the expect_tx arrival of the loading thread
             mbar_init(empty(s), 1);   // tcgen05.commit
+            mbar_init(peer_acts(s), 1);  // the expect_tx arrival of the first block's loading thread
         }
         for (int g = 0; g < kGemmGroups; ++g) mbar_init(a_full(g), 2 * kGemmDecodeWarps / kGemmGroups);  // one arrival per warp of the group in either block
         mbar_init(acc_full, 1);                      // tcgen05.commit after the last MMA of an item
@@ -353,6 +363,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
         // ---- loads: one thread issues, but the warp stays together, so that addresses live in uniform registers ----
         const int mine = warp - kGemmDecodeWarps - 1;
         int it0 = 0, until = 0;  // stages of the sequence before this item; behind this warp's last issued stage
+        const uint32_t own_bytes = rank == 0 ? kGemmStageBytes + act_bytes : kGemmStageBytes, acts_landed = rank == 0 ? loaded(0) : cluster_addr(peer_acts(0), 0);
         bool okay = true;
         for (int item = first; item < items && okay; item += step) {
             const int tile = pair_of(item) * 2 + static_cast<int>(rank), kb0 = part_of(item) * per, nkb = min(per, a.blocks - kb0);
@@ -363,24 +374,28 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
                 if (elect_one()) {
                     const uint32_t dst = b_base + s * act_bytes;
                     const int x = (kb0 + k) * kGemmStageCols, y = item % tiles * n + static_cast<int>(rank) * (n / 2);
-                    mbar_expect_tx(loaded(s), kGemmStageBytes + act_bytes);
+                    // (the second block's copies may complete on peer_acts before the first one has announced them: the phase waits for the announcement's arrival)
+                    const uint32_t acts = acts_landed + 8u * s;
+                    mbar_expect_tx(loaded(s), own_bytes);
+                    if (rank == 0) mbar_expect_tx(peer_acts(s), act_bytes);
                     bulk_load(raw_base + s * kGemmStageBytes, src + size_t(k) * kGemmStageBytes, kGemmStageBytes, loaded(s));
-                    tma_load_2d(dst, &act_map, x, y, loaded(s));
-                    tma_load_2d(dst + act_bytes / 2, &act_map, x + 128, y, loaded(s));
+                    tma_load_2d_pair(dst, &act_map, x, y, acts);
+                    tma_load_2d_pair(dst + act_bytes / 2, &act_map, x + 128, y, acts);
                 }
                 __syncwarp();
                 until = it + 1;
             }
             it0 += nkb;
         }
-        if (!okay && lane == 0) raise_abort(abort_addr, rank);
-        // its own copies in flight land before the block leaves
+        // its own copies in flight land before the block leaves (the second block's activations: at the end)
         turn_until[mine] = until;
+        if (rank == 1 && lane == 0) store_cluster(cluster_addr(peer_until_addr + 4u * mine, 0), static_cast<uint32_t>(until));
         asm volatile("bar.sync 1, %0;" ::"n"(32 * kGemmLoadWarps) : "memory");  // the load warps
         int furthest = until;
         for (int w = 0; w < kGemmLoadWarps; ++w) furthest = max(furthest, turn_until[w]);
         for (int it = gemm_drain_from(furthest, S); it < until; ++it)
-            if ((it & (kGemmLoadWarps - 1)) == mine) mbar_wait(loaded(it % S), (it / S) & 1, abort_flag, a.spin_limit, false);
+            if ((it & (kGemmLoadWarps - 1)) == mine) okay &= mbar_wait(loaded(it % S), (it / S) & 1, abort_flag, a.spin_limit, false);
+        if (!__all_sync(0xffffffffu, okay) && lane == 0) raise_abort(abort_addr, rank);
     } else if (warp == kGemmDecodeWarps) {
         // ---- tensor cores of both blocks: eight MMAs per stage (A from tensor memory, B from shared memory), issued by one thread of the first block. The warp
         // stays together around them, so that descriptors live in uniform registers (one lane alone took 80 cycles an instruction) ----
@@ -399,7 +414,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
                 }
                 for (int k = 0; k < nkb; ++k, ++it) {
                     const int g = it & (kGemmGroups - 1);
-                    // the groups' arrivals also stand for the stage's loads: each waited for its block's before it decoded
+                    // the arrivals of the first block's warps also stand for the activations of both blocks, which they have seen land
                     if (!(okay = __all_sync(0xffffffffu, mbar_wait(a_full(g), (it / kGemmGroups) & 1, abort_flag, a.spin_limit)))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t b_desc = b_desc0 + uint64_t(s * b_stage16);
@@ -429,6 +444,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
         const int group = warp >> 2, quarter = warp & 3, r = quarter * 32 + lane;
         const uint32_t lanes = tmem_base + (uint32_t(quarter * 32) << 16), a_tmem = lanes + kOperandCol + 64u * group;
         const uint32_t to_full = cluster_addr(a_full(group), 0), to_empty = cluster_addr(acc_empty, 0);
+        const bool sees_peer = rank == 0 && quarter == 0;  // one warp of a group waits for the second block's activations too (in the issuing warp, which every stage passes through, a step of 32 sequences took 3 % longer)
         const int own = n / kGemmGroups, c0 = group * own;  // accumulator columns (a multiple of eight) that this group writes out
         bool okay = true;
         auto finish = [&](int item, int j) {  // item `item`, the pair's j-th
@@ -449,7 +465,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
                 // is not mistaken - and the stage's bytes have landed. (S >= kGemmGroups: the barrier of that operand's stage cannot be a use further on.)
                 const int last = it - kGemmGroups;
                 if (!okay) break;
-                okay = (last < 0 || mbar_wait(empty(last % S), (last / S) & 1, abort_flag, a.spin_limit)) && mbar_wait(loaded(s), (it / S) & 1, abort_flag, a.spin_limit);
+                okay = (last < 0 || mbar_wait(empty(last % S), (last / S) & 1, abort_flag, a.spin_limit)) && mbar_wait(loaded(s), (it / S) & 1, abort_flag, a.spin_limit) &&
+                       (!sees_peer || mbar_wait(peer_acts(s), (it / S) & 1, abort_flag, a.spin_limit));
                 okay = __all_sync(0xffffffffu, okay);
                 if (!okay) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -479,6 +496,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
     __syncthreads();
     if (tid == 0 && *abort_flag) atomicExch(a.status, kGemmStatusTimeout);
     cluster_sync_all();
+    if (*abort_flag) {  // the same in both blocks: who raised it raised it in both, before the barrier
+        // the second block's activations in flight land before it leaves: the first block's barriers show it, once what it had not come to announce is announced
+        if (rank == 0 && warp > kGemmDecodeWarps) {
+            const int mine = warp - kGemmDecodeWarps - 1, until = turn_until[mine], theirs = turn_until[kGemmLoadWarps + mine];
+            int furthest = theirs;
+            for (int w = 0; w < kGemmLoadWarps; ++w) furthest = max(furthest, turn_until[kGemmLoadWarps + w]);
+            for (int it = gemm_drain_from(furthest, S); it < theirs; ++it) {
+                if ((it & (kGemmLoadWarps - 1)) != mine) continue;
+                if (!gemm_announced(it, until) && elect_one()) mbar_expect_tx(peer_acts(it % S), act_bytes);
+                __syncwarp();
+                mbar_wait(peer_acts(it % S), (it / S) & 1, abort_flag, a.spin_limit, false);
+            }
+        }
+        cluster_sync_all();
+    }
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");

@@ -18,4 +18,7 @@ constexpr int kGemmLoadWarps = 2;  // load warp w fetches the stages w, w + 2, .
 // an item: what counts is how far they came, not where the item would have ended.
 QTB_TURNS_FN int gemm_drain_from(int until, int stages) { return until > stages ? until - stages : 0; }
 
+// Whether the first block has announced (expect_tx) the second one's activations of a stage: its load warp of the same turn, which came to `until`, does so when it issues its own.
+QTB_TURNS_FN bool gemm_announced(int it, int until) { return it < until; }
+
 }  // namespace qtb
