@@ -1142,15 +1142,15 @@ int decoder_create_impl(const quintrit_b200_decoder_desc_t* desc, quintrit_b200_
     // the single-kernel path stages KV rows with a piece permutation that needs a power-of-two head_dim of at least 64
     // and one values unit of the longest chunk must fit the shared memory of an SM next to the activation vectors
     const int gqa_n = d->q_heads / d->kv_heads;
-    // the second form of the attention's second half (units that take all chunks of 8 coordinates) where its arrays fit
+    // the second form of the attention's second half (units that take all chunks of 16 coordinates) where its arrays fit
     d->attn_v2 = tp_world == 1 && d->ctx <= static_cast<uint32_t>(kV2MaxCtx) && gqa_n <= kV2MaxGqa && qd_full <= size_t(kNormPer) * kMegaThreads && hd % kV2Dims == 0 &&
                  d->kv_heads * (hd / kV2Dims) <= static_cast<uint32_t>(d->sm_count);
     if (const char* v2 = std::getenv("QUINTRIT_B200_ATTN_V2")) d->attn_v2 = d->attn_v2 && v2[0] != '0';  // experiments: "0" keeps the first form
-    auto bytes_for = [&](bool v2) {
-        return mega_smem_bytes(mega_attn_region(d->ctx, gqa_n, hd, H, v2), static_cast<int>(std::max<size_t>(H, qd_full)), static_cast<int>(H), static_cast<int>(L));
+    auto charge = [&](bool v2) {
+        return mega_charge(static_cast<int>(d->ctx), gqa_n, static_cast<int>(hd), static_cast<int>(H), static_cast<int>(std::max<size_t>(H, qd_full)), static_cast<int>(L), v2);
     };
-    if (d->attn_v2 && bytes_for(true) > static_cast<size_t>(smem_optin)) d->attn_v2 = false;
-    const size_t mega_bytes = bytes_for(d->attn_v2);
+    if (d->attn_v2 && charge(true) > static_cast<size_t>(smem_optin)) d->attn_v2 = false;
+    const size_t mega_bytes = charge(d->attn_v2);
     const bool staged_ok = hd >= 64 && (hd & (hd - 1)) == 0 && gqa_n <= 16 && mega_bytes <= static_cast<size_t>(smem_optin);
     if (staged_ok && d->q_heads <= kMegaMaxHeads && !(mode && std::strcmp(mode, "kernels") == 0)) {
         if ((rc = mega_setup(d, desc)) != QUINTRIT_OK) return rc;

@@ -20,13 +20,10 @@
 
 #include "decode.cuh"
 #include "gemv_lut.cuh"
+#include "mega_plan.hpp"
 
 namespace qtb {
 
-constexpr int kMegaThreads = 512;
-constexpr int kMegaWarps = kMegaThreads / 32;
-constexpr int kMegaMaxHeads = 64;
-constexpr int kMegaCosSin = 256;  // floats of a row of the cos/sin table: rope_dims <= head_dim <= 256
 constexpr unsigned int kBarrierSpinLimit = 1u << 21;  // polls of one L2 round trip each (~0.7 us): about 1.5 s, then the kernel gives up
 
 struct MegaLayer {
@@ -35,11 +32,11 @@ struct MegaLayer {
     const float* ffn_norm;
     const float* attn_sub_norm;  // BitNet: RMSNorm of the attention output before o (q_dim weights), else nullptr
     const float* ffn_sub_norm;   // BitNet: RMSNorm of the gated activations before down (inter weights), else nullptr
-    float ws[7];
     __half* kc;               // [ctx][kv_dim]
     __half* vc;
     const unsigned char* wbase[7];  // the seven weight matrices of the layer in the stream layout, for the L2 prefetches
     unsigned int wbytes[7];
+    float ws[7];
 };
 
 struct MegaArgs {
@@ -414,9 +411,6 @@ __device__ __forceinline__ void residual_add_ll(float* y_s, const float* x, cons
     }
 }
 
-constexpr int kAttnBlockPos = 128;                          // positions staged in shared memory at a time
-constexpr int kAttnBlockBytes = kAttnBlockPos * 256 * 2;    // one staged block (head_dim <= 256 halves per row)
-
 // Byte offset of 16-byte piece `c` of row `r` inside a staged block. The pieces of a row are permuted by the low three
 // bits of the row number, so that 8 threads reading the same piece of 8 consecutive rows, or one row's consecutive
 // pieces, always touch 8 different 16-byte bank groups (head_dim >= 64, i.e. at least 8 pieces per row).
@@ -654,14 +648,6 @@ __device__ __noinline__ void mega_scores_unit(const MegaArgs& a, const MegaLayer
     __syncthreads();
 }
 
-constexpr int kAttnSlice = 32;  // coordinates of a head that one values unit accumulates (one warp per query head)
-
-// Shared memory a values unit needs for chunks of `len` positions and `gqa` query heads per KV head.
-__host__ __device__ constexpr size_t values_unit_bytes(int len, int gqa) {
-    return (static_cast<size_t>(len) * kAttnSlice * 2 + 15) / 16 * 16 + static_cast<size_t>(2) * gqa * len * 4 + (kMegaWarps + 16) * 4 +
-           (static_cast<size_t>(gqa) * ((len + 7) / 8 + 1) * 3 + 15) / 16 * 16;
-}
-
 // Attention, second half: for one KV head, one chunk of positions and one slice of 32 coordinates, the softmax factors of
 // every query head of the group (phase B of attention_kernel, recomputed by every slice) and the value accumulation
 // (phase C). The V slice of the whole chunk is staged in shared memory in four copy groups; warp g runs the chains of
@@ -841,23 +827,6 @@ __device__ __noinline__ void mega_values_unit(const MegaArgs& a, const MegaLayer
 // cached V row into [chunk][position][8 halves], the scores of its heads into one row per (head, chunk). The softmax
 // factors (attention.rs:448-462) are made by the unit itself, a warp per (head, chunk) (v2_factors). The positions at which any chunk's running maximum
 // moved are known per head and group of eight; groups without a move run branch-free.
-constexpr int kV2Dims = 16;      // coordinates per unit: two warps of eight coordinates x four chunks per query head
-constexpr int kV2WarpsPerHead = kV2Dims / 8;
-constexpr int kV2MaxCtx = 4096;
-static_assert(kV2MaxCtx / 4 / 8 < 256, "a group's number fits the low byte of the table of next groups");
-constexpr int kV2MaxGqa = 7;     // chain warps (two per head) + the warp of the sum chains must fit the 16 warps of the CTA
-
-// Row length (floats) of the factor rows for chunks of `chunk` positions: a multiple of 8, at least `chunk`.
-__host__ __device__ constexpr int values2_clp(int chunk) { return (chunk + 7) / 8 * 8; }
-// Positions per chunk in the staged V block: odd, so that the 32-byte pieces the four chunks' lanes read at one step fall into
-// four different bank groups.
-__host__ __device__ constexpr int values2_clr(int chunk) { return values2_clp(chunk) + 1; }
-__host__ __device__ constexpr size_t values2_bytes(int ctx, int gqa) {
-    const int nch = ctx >= 512 ? 4 : 1, chunk = ctx >= 512 ? (ctx + 3) / 4 : ctx, clp = values2_clp(chunk);
-    return static_cast<size_t>(nch) * values2_clr(chunk) * kV2Dims * 2 + static_cast<size_t>(2) * gqa * nch * clp * 4 + static_cast<size_t>(gqa) * (clp / 8) * 4 +
-           static_cast<size_t>(gqa) * 8 * 4 + static_cast<size_t>(gqa) * nch * (8 + clp / 8) + 64;
-}
-
 template <bool F32>
 __device__ __forceinline__ float v2_round(float x) {
     return F32 ? x : __half2float(__float2half_rn(x));
@@ -1170,28 +1139,8 @@ __device__ __noinline__ void mega_values2_unit(const MegaArgs& a, const MegaLaye
     __syncthreads();
 }
 
-// Shared-memory plan of the token kernel (bytes from the dynamic base): attention region (its first 64 KiB double as the
-// GEMV table) | y (floats) | a8 | small. The attention region holds whichever is largest: a scores unit (staged key block,
-// the group's queries, the new key/value rows), a values unit for the longest chunk, or the output head's activations (floats).
-// It is never smaller than kMegaRegionMin, which together with the vectors behind it decides which models take this kernel: wider ones
-// (past 8 to 9 thousand values) have not been run through it and take one kernel per step.
-constexpr size_t kMegaRegionMin = 127 * 1024;
-__host__ __device__ constexpr size_t mega_attn_region(int ctx, int gqa, int head_dim, int hidden, bool v2) {
-    const int len_max = ctx < 512 ? ctx : (ctx + 3) / 4;
-    size_t need = static_cast<size_t>(kAttnBlockBytes) + static_cast<size_t>(gqa) * head_dim * 4 + static_cast<size_t>(head_dim) * 4 + 64;
-    const size_t vals = v2 ? values2_bytes(ctx, gqa) : values_unit_bytes(len_max, gqa), head = static_cast<size_t>(hidden) * 4;
-    if (vals > need) need = vals;
-    if (head > need) need = head;
-    if (kMegaRegionMin > need) need = kMegaRegionMin;
-    return (need + 1023) / 1024 * 1024;
-}
-// After the small arrays: the norm weights of the next norm (hidden floats), a row of the cos/sin table, the kernel's arguments and a copy of every layer's descriptor.
-constexpr size_t kMegaArgsBytes = 1024;
-static_assert(sizeof(MegaArgs) <= kMegaArgsBytes, "the token kernel's arguments do not fit their place");
-__host__ __device__ constexpr size_t mega_smem_bytes(size_t attn_region, int maxvec, int hidden, int layers) {
-    return attn_region + static_cast<size_t>(maxvec) * 4 + (static_cast<size_t>(maxvec) + 15) / 16 * 16 + 4096 +
-           (static_cast<size_t>(hidden) * 4 + 15) / 16 * 16 + static_cast<size_t>(kMegaCosSin) * 4 + kMegaArgsBytes + static_cast<size_t>(layers) * sizeof(MegaLayer);
-}
+static_assert(sizeof(MegaArgs) <= kMegaArgsBytes && kMegaArgsBytes - sizeof(MegaArgs) < 16, "the plan's place for the arguments");
+static_assert(sizeof(MegaLayer) == kMegaLayerBytes, "the plan's place for a layer");
 
 // ---- the token kernel ---------------------------------------------------------------------------------------------------
 // Every phase is its own non-inlined function and the kernel body keeps almost nothing alive across the calls (scalars
@@ -1202,9 +1151,8 @@ struct MegaSmem {
     int* tab;
     float* y;        // activation vector (max(hidden, q_dim) floats)
     int8_t* a8;      // its int8 codes
-    double* sh_d;    // 32 doubles
-    float* sh_f;     // 32 floats
-    float* pair;     // chunk-combine factors: q_heads * (4 * 2 + 4) floats (q_heads <= kMegaMaxHeads)
+    double* sh_d;    // a double per warp
+    float* sh_f;     // a float per warp
     unsigned long long* exp_tab;  // the exponential's table (g_exp2_tab)
     float* scale;    // [0] attention-input scale, [1] o-input scale, [2] ffn-input scale, [3] down-input scale (previous layer)
     int* flag;
@@ -1222,13 +1170,12 @@ __device__ __forceinline__ MegaSmem mega_smem_views(unsigned char* smem, const M
     v.a8 = reinterpret_cast<int8_t*>(v.y + maxvec);
     unsigned char* small = reinterpret_cast<unsigned char*>(v.a8) + (maxvec + 15) / 16 * 16;
     v.sh_d = reinterpret_cast<double*>(small);
-    v.sh_f = reinterpret_cast<float*>(small + 256);
-    v.pair = reinterpret_cast<float*>(small + 384);
-    v.exp_tab = reinterpret_cast<unsigned long long*>(small + 3456);
-    v.scale = reinterpret_cast<float*>(small + 3968);
-    v.flag = reinterpret_cast<int*>(small + 4000);
-    v.pos = reinterpret_cast<int*>(small + 4008);
-    v.w = reinterpret_cast<float*>(small + 4096);
+    v.sh_f = reinterpret_cast<float*>(small + kMegaSmallSumF);
+    v.exp_tab = reinterpret_cast<unsigned long long*>(small + kMegaSmallExp);
+    v.scale = reinterpret_cast<float*>(small + kMegaSmallScale);
+    v.flag = reinterpret_cast<int*>(small + kMegaSmallFlag);
+    v.pos = reinterpret_cast<int*>(small + kMegaSmallPos);
+    v.w = reinterpret_cast<float*>(small + kMegaSmallBytes);
     v.cs = v.w + (a.hidden + 3) / 4 * 4;
     v.args = reinterpret_cast<MegaArgs*>(v.cs + kMegaCosSin);
     v.layers = reinterpret_cast<MegaLayer*>(reinterpret_cast<unsigned char*>(v.args) + kMegaArgsBytes);
@@ -1496,7 +1443,7 @@ __device__ __noinline__ void phase_combine2(const MegaArgs& a, int l, unsigned c
 __device__ __noinline__ bool phase_combine(const MegaArgs& a, int l, unsigned int seq, unsigned char* smem) {
     const MegaSmem v = mega_smem_views(smem, a);
     const int tid = threadIdx.x, hd = a.head_dim, qd = a.q_heads * hd;
-    float* s_pair = v.pair;
+    float* s_pair = reinterpret_cast<float*>(v.tab);  // chunk-combine factors: q_heads * (4 * 2 + 4) floats; between two GEMVs the table's rows before its first zero row are free
     const KvSplit ks = kv_split(a, *v.pos);
     QTB_FINE(a, 21);
     // every chunk value of a thread's coordinates is requested before the factors are needed
@@ -1676,7 +1623,7 @@ __device__ __noinline__ void phase_ffn_sub_norm(const MegaArgs& a, int l, unsign
     const float* w = v.layers[l].ffn_sub_norm;
     // the per-CTA partial sums: fetched by one thread each (one L2 round trip in all), then added by every thread in the
     // same fixed order (four interleaved chains)
-    double* s_part = reinterpret_cast<double*>(v.y);  // the activation vector is not in use between SwiGLU and down
+    double* s_part = reinterpret_cast<double*>(v.tab);  // between two GEMVs the table's rows before its first zero row are free (the activation vector may be shorter than the sums)
     for (int c = tid; c < G; c += kMegaThreads) s_part[c] = __ldcg(a.sumsq_part + c);
     __syncthreads();
     double p0 = 0.0, p1 = 0.0, p2 = 0.0, p3 = 0.0;
@@ -1810,7 +1757,7 @@ __device__ __noinline__ bool phase_head(const MegaArgs& a, unsigned int seq_base
     __syncthreads();
     if (a.l2_prefetch && a.n_layers > 0)  // the next token starts with the first layer's attention projections
         for (int k = 0; k < 3; ++k) prefetch_weights(v.layers[0], k);
-    float* s_bv = v.sh_f;  // 32 floats: one candidate per warp
+    float* s_bv = v.sh_f;  // one candidate per warp
     unsigned int* s_bi = reinterpret_cast<unsigned int*>(v.sh_d);
     if (lane == 0) {
         s_bv[warp] = bv;

@@ -204,3 +204,47 @@ def test_context_of_several_thousand_positions(oracle, f32_values, head_dim, q_h
     spec = synth.make_model(q.ARCH_LLAMA, f32_values, hidden, 256, 1, q_heads, kv_heads, head_dim, 264, 3584, 10000.0, 1e-6, config=29, tied=True)
     rng = np.random.default_rng(5)
     _run(spec, rng.integers(0, 264, 3400), oracle, check_every=211)
+
+
+LIMIT = 227 * 1024  # shared memory a block may ask for
+
+
+def _charge(ctx, group, head_dim, hidden, layers, second):
+    """What decides whether a model takes the token kernel, and with which form of the attention's second half (csrc/mega_plan.hpp)."""
+    chunks, chunk = (4, (ctx + 3) // 4) if ctx >= 512 else (1, ctx)
+    eights, up = (chunk + 7) // 8 * 8, lambda n, k: (n + k - 1) // k * k
+    if second:
+        values = chunks * (eights + 1) * 32 + 2 * group * chunks * eights * 4 + group * (eights // 8) * 4 + group * 32 + group * chunks * 8 + 64
+    else:
+        values = up(chunk * 64, 16) + 2 * group * chunk * 4 + 128 + up(group * ((chunk + 7) // 8 + 1) * 3, 16)
+    region = up(max(65536 + group * head_dim * 4 + head_dim * 4 + 64, values, hidden * 4, 129 * 1024), 1024)
+    return region + 5 * hidden + 4096 + 4 * hidden + 200 * layers
+
+
+@pytest.mark.parametrize("group,ctx,second,f32_values", [(4, 2816, True, False), (7, 2048, True, True), (3, 3840, True, False), (4, 8192, False, False), (12, 4608, False, True)])
+def test_the_widest_models_that_take_the_token_kernel(monkeypatch, group, ctx, second, f32_values):
+    """As wide as the token kernel takes them at a context that sets its shared memory: it is the path that runs, with the bits of one kernel per step, up to the last
+    position."""
+    hidden = max(h for h in range(64 * group, 9000, 32) if _charge(ctx, group, 64, h, 1, second) <= LIMIT)
+    assert _charge(ctx, group, 64, hidden, 1, second) > LIMIT - 300
+    spec = synth.make_model(q.ARCH_LLAMA, f32_values, hidden, 256, 1, group, 1, 64, 300, ctx, 500000.0, 1e-5, config=80 + group, random_norms=True)
+    spec["scales"] = (spec["scales"] * np.float32(0.06)).astype(np.float32)  # scores of a few units: weights spread over many positions
+    tokens = synth.prompt_tokens(17, ctx, spec["vocab"])
+    one = q.Decoder(spec)
+    monkeypatch.setenv("QUINTRIT_B200_DECODE", "kernels")
+    steps = q.Decoder(spec)
+    for d in (one, steps):
+        d.prefill(tokens[:ctx - 12])
+    for pos in range(ctx - 12, ctx - 1):
+        (a, ta), (b, tb) = one.forward(int(tokens[pos]), pos), steps.forward(int(tokens[pos]), pos)
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32)) and ta == tb, pos
+    assert len(one.trace_step()) > 0  # refused where one kernel per step runs
+    with pytest.raises(q.QuintritError) as e:
+        steps.trace_step()
+    assert e.value.code == 6
+
+
+def test_a_sub_norm_over_more_blocks_than_the_vector_has_room(oracle):
+    """The partial sums of all blocks take more bytes than the activation vector of so narrow a model."""
+    spec = synth.make_model(q.ARCH_BITNET, True, 64, 160, 2, 1, 1, 64, 100, 256, 500000.0, 1e-5, config=14, random_norms=True, tied=True)
+    _run(spec, np.random.default_rng(5).integers(0, 100, 12), oracle)
