@@ -5,7 +5,6 @@
 #include <sys/stat.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <mutex>
@@ -16,6 +15,7 @@
 #include "gemv_lut.cuh"
 #include "transcode.cuh"
 #include "gemm_tc.cuh"
+#include "step_wait.hpp"
 #include "tensor_map.cuh"
 #include "block_scaled.cuh"
 
@@ -1320,14 +1320,19 @@ int kernel_status_error(unsigned int flag) {
     return QUINTRIT_OK;
 }
 
+// Steps that gave up have not been counted by the device: the count of launched ones becomes its own (behind a stream that has run dry).
+void decoder_recount_steps(quintrit_b200_decoder* d) {
+    cudaMemcpyAsync(&d->launched, d->d_steps, sizeof(uint32_t), cudaMemcpyDeviceToHost, d->stream);
+    cudaStreamSynchronize(d->stream);
+}
+
 int decoder_check_status(quintrit_b200_decoder* d) {
     unsigned int flag = 0;
     QTB_CUDA(cudaMemcpyAsync(&flag, d->d_counters + 2, sizeof flag, cudaMemcpyDeviceToHost, d->stream));
     QTB_CUDA(cudaStreamSynchronize(d->stream));
     if (flag != 0) {  // the word is sticky on the device: clear it so that the decoder stays usable after the error
         cudaMemsetAsync(d->d_counters + 2, 0, sizeof(unsigned int), d->stream);
-        cudaMemcpyAsync(&d->launched, d->d_steps, sizeof(uint32_t), cudaMemcpyDeviceToHost, d->stream);  // steps that gave up have not been counted
-        cudaStreamSynchronize(d->stream);
+        decoder_recount_steps(d);
         return kernel_status_error(flag);
     }
     return QUINTRIT_OK;
@@ -1336,20 +1341,23 @@ int decoder_check_status(quintrit_b200_decoder* d) {
 // Waits until the last step launched has reported: everything it did is done then, though its last kernel may still be leaving. (Copies of the token and of the status word
 // and a wait for the stream took 12 to 20 us behind a step.) A kernel that gave up reports nothing: the stream runs dry, and its status tells why.
 int decoder_wait_report(quintrit_b200_decoder* d) {
-    const volatile uint32_t* steps = &d->report->steps;
-    for (unsigned int spins = 1; *steps != d->launched; ++spins) {
-#if defined(__x86_64__)
-        __builtin_ia32_pause();
-#endif
-        if (spins % 4096 != 0) continue;
-        const cudaError_t e = cudaStreamQuery(d->stream);
-        if (e == cudaErrorNotReady) continue;
-        if (e != cudaSuccess) return cuda_fail(e, "a decode step");
-        if (*steps == d->launched) break;
+    struct {
+        quintrit_b200_decoder* d;
+        cudaError_t error;
+        uint32_t reported() const { return *const_cast<const volatile uint32_t*>(&d->report->steps); }
+        uint32_t launched() const { return d->launched; }
+        StepStream stream() {
+            error = cudaStreamQuery(d->stream);
+            return error == cudaSuccess ? StepStream::kDry : error == cudaErrorNotReady ? StepStream::kBusy : StepStream::kFailed;
+        }
+        void recount() { decoder_recount_steps(d); }
+    } steps{d, cudaSuccess};
+    const StepOutcome outcome = wait_for_steps(steps);
+    if (outcome == StepOutcome::kStreamFailed) return cuda_fail(steps.error, "a decode step");
+    if (outcome == StepOutcome::kNoReport) {
         const int rc = decoder_check_status(d);
         return rc != QUINTRIT_OK ? rc : fail(QUINTRIT_ERR_DEVICE, "a decode step ended without a result on the CUDA device");
     }
-    std::atomic_thread_fence(std::memory_order_acquire);
     if (const unsigned int flag = d->report->status) {
         QTB_CUDA(cudaMemsetAsync(d->d_counters + 2, 0, sizeof(unsigned int), d->stream));  // sticky on the device: cleared so that the decoder stays usable after the error
         return kernel_status_error(flag);

@@ -121,6 +121,30 @@ def test_a_silent_rank_ends_in_an_error_not_in_a_hang(monkeypatch):
     lone.free()
 
 
+def test_a_decoder_is_used_again_after_steps_that_gave_up(monkeypatch):
+    """A step that gave up has reported nothing; the calls after it wait for their own steps, end in the same error at once when their wait runs out too (one step or several
+    behind one another), and nobody waits for the reports that never came."""
+    import time
+
+    import quintrit_b200 as q
+    from quintrit_b200 import synth
+
+    monkeypatch.setenv("QUINTRIT_B200_TP_WAIT_MS", "50")
+    spec = synth.make_model(q.ARCH_LLAMA, False, 256, 512, 2, 4, 2, 64, 512, 256, 500000.0, 1e-5, config=22, random_norms=True)
+    group = [q.Decoder(synth.shard_spec(spec, r, 2), device=0) for r in range(2)]
+    for d in group:
+        d.tp_attach_local(group)
+    group[1].info()  # nothing of rank 1 ever launches
+    for call in (lambda: group[0].forward(1, 0), lambda: group[0].generate([1, 2], 2), lambda: group[0].forward(1, 0, want_logits=False), lambda: group[0].forward(2, 0)):
+        t0 = time.perf_counter()
+        with pytest.raises(q.QuintritError) as e:
+            call()
+        assert e.value.code == 15 and "another rank" in str(e.value)
+        assert time.perf_counter() - t0 < 1.0
+    for d in group:
+        d.free()
+
+
 def test_a_grid_barrier_that_cannot_complete_gives_up():
     """The barrier's give-up path, made to run out without a fault or a hang: four resident CTAs wait for a fifth arrival
     with 5000 polls of patience. Status 2 comes back as QUINTRIT_ERR_DEVICE, every CTA was released by the failure bit and
