@@ -1130,7 +1130,6 @@ int decoder_create_impl(const quintrit_b200_decoder_desc_t* desc, quintrit_b200_
         if (kq != nullptr && bytes + 1024 <= static_cast<size_t>(smem_optin)) {
             if ((rc = allow_max_dynamic_smem(kq, smem_optin)) != QUINTRIT_OK) return rc;
             d->attn_gqa = kq, d->attn_gqa_smem = bytes;
-            if (const char* pad = std::getenv("QUINTRIT_B200_ATTN_SMEM_PAD")) d->attn_gqa_pad = std::min<size_t>(static_cast<size_t>(std::atoi(pad)), smem_optin - 1024 - bytes);
         }
         d->attn_rows = attention_rows_for(group, static_cast<int>(hd), d->f32_values != 0);
         if (d->attn_rows != nullptr && (rc = allow_max_dynamic_smem(d->attn_rows, smem_optin)) != QUINTRIT_OK) return rc;

@@ -61,7 +61,6 @@ struct quintrit_b200_decoder {
     size_t attn_gqa_smem = 0;
     qtb::AttnGqaKernel attn_tile = nullptr;    // prompt chunks: eight tokens per block, if this model's shape has that kernel
     qtb::AttnGqaKernel attn_rows = nullptr;    // the same for the head sizes it exists for, packed operations
-    size_t attn_gqa_pad = 0;                   // experiments: extra shared memory per block, which lowers the number of resident blocks
     float* attn_out = nullptr;
     unsigned long long* trace;  // phase timestamps of the last traced step (13 per layer + 3)
     cudaStream_t stream;
@@ -197,7 +196,7 @@ inline void launch_attention(quintrit_b200_decoder* d, AttnArgs at, int n, cudaS
     if (d->attn_rows != nullptr && n > 1)
         d->attn_rows<<<dim3(d->kv_heads, 4, n), kRowAttnThreads, row_attn_smem(group, d->head_dim), s>>>(at);
     else if (d->attn_gqa != nullptr && n > 1)
-        d->attn_gqa<<<dim3(d->kv_heads, 4, n), kAttnGqaThreads, d->attn_gqa_smem + d->attn_gqa_pad, s>>>(at);
+        d->attn_gqa<<<dim3(d->kv_heads, 4, n), kAttnGqaThreads, d->attn_gqa_smem, s>>>(at);
     else
         attention_kernel<<<dim3(d->q_heads, 4, n), kAttnThreads, attention_smem(d->head_dim), s>>>(at);
 }

@@ -85,20 +85,28 @@ def test_arguments():
     assert e.value.code == 2
 
 
-def test_many_chunks_replay_one_graph():
-    """From the third full chunk on the launches of a chunk are replayed as a CUDA graph: 800 tokens = 3 full chunks + a tail."""
-    spec = _spec(q.ARCH_LLAMA, False, 79, ctx=1024)
-    tokens = synth.prompt_tokens(6, 800, spec["vocab"])
+@pytest.mark.parametrize("arch", [q.ARCH_LLAMA, q.ARCH_BITNET])
+def test_many_chunks_replay_one_graph(arch):
+    """From the third full pass on the launches of a pass are replayed as a CUDA graph: 3200 tokens = 3 full passes of 1024 (as they are, captured, replayed) and a tail, then
+    another prompt on the same decoder, whose full passes are all replays. Against single steps, which take none of it."""
+    spec = _spec(arch, arch == q.ARCH_BITNET, 79, ctx=4096, tied=arch == q.ARCH_BITNET)
     a, b = q.Decoder(spec), q.Decoder(spec)
-    for pos, t in enumerate(tokens):
-        want, want_next = a.forward(int(t), pos)
-    got, got_next = b.prefill(tokens)
-    assert np.array_equal(got.view(np.uint32), want.view(np.uint32)) and got_next == want_next
-    again, _ = b.prefill(tokens)  # a second prompt on the same decoder: every full chunk is a replay now
-    assert np.array_equal(again.view(np.uint32), want.view(np.uint32))
-    la, ta = a.forward(want_next, 800)
-    lb, tb = b.forward(got_next, 800)
-    assert np.array_equal(la.view(np.uint32), lb.view(np.uint32)) and ta == tb
+    launches = []
+    for seed, n in ((6, 3200), (7, 3100)):
+        tokens = synth.prompt_tokens(seed, n, spec["vocab"])
+        for pos, t in enumerate(tokens):
+            want, want_next = a.forward(int(t), pos, want_logits=pos == n - 1)
+        before = q.launch_count()
+        got, got_next = b.prefill(tokens)
+        launches.append(q.launch_count() - before)
+        assert np.array_equal(got.view(np.uint32), want.view(np.uint32)) and got_next == want_next
+        for step in range(2):  # the caches are the same
+            la, ta = a.forward(want_next, n + step)
+            lb, tb = b.forward(got_next, n + step)
+            assert np.array_equal(la.view(np.uint32), lb.view(np.uint32)) and ta == tb
+            want_next = got_next = ta
+    assert launches[1] < launches[0] / 2  # a replay launches nothing one by one: of the second prompt only the tail and the head
+
 
 
 @pytest.mark.parametrize("arch,inter,n", [(q.ARCH_LLAMA, 512, 513), (q.ARCH_LLAMA, 4128, 1000), (q.ARCH_BITNET, 512, 1025), (q.ARCH_LLAMA, 512, 1600)])

@@ -34,10 +34,11 @@ def test_portions_equal_single_steps(group, head_dim, f32_values):
 
 
 @pytest.mark.parametrize("f32_values", [False, True])
-@pytest.mark.parametrize("group,head_dim", [(1, 64), (4, 64), (2, 128), (3, 128), (1, 256), (3, 256)])
+@pytest.mark.parametrize("group,head_dim", [(1, 64), (4, 64), (2, 128), (3, 128), (1, 256), (3, 256), (3, 32), (2, 96), (3, 96), (3, 224)])
 def test_short_portions_behind_long_contexts(group, head_dim, f32_values):
-    """Portions too short for tiles of tokens (attention_rows_kernel, a block per token, KV head and chunk) where a chunk takes more than one round of 256
-    positions, with a round of one position (chunks of 320 and 576: rounds of 64; position 1281 leaves one row in the last chunk), against single steps."""
+    """Portions too short for tiles of tokens (attention_rows_kernel, for the head sizes it does not take attention_gqa_kernel: a block per token, KV head and chunk) where a
+    chunk takes more than one round of 256 positions, with a round of one position (chunks of 320 and 576: rounds of 64; position 1281 leaves one row in the last chunk),
+    against single steps."""
     kv_heads = 1 if head_dim == 256 else 2
     spec = synth.make_model(q.ARCH_LLAMA, f32_values, 256, 512, 1, group * kv_heads, kv_heads, head_dim, 300, 2304, 500000.0, 1e-5, config=70 + group, random_norms=True)
     spec["scales"] = (spec["scales"] * np.float32(0.06)).astype(np.float32)  # scores of a few units: weights spread over many positions
