@@ -248,13 +248,14 @@ def run_decode(args, local_rank: int):
     try:
         dec.prefill(prompt[:16])  # makes the two-bit copies of the weights and the chunk buffers
         t0 = time.perf_counter()
-        _, nxt = dec.prefill(prompt)  # the first prompt: its second full chunk is captured into the graph that later chunks replay
+        _, nxt = dec.prefill(prompt)  # the first prompt
         first_s = time.perf_counter() - t0
+        dec.prefill(prompt)  # a decoder's second full pass is captured into the graph that later ones replay
         t0 = time.perf_counter()
         _, nxt2 = dec.prefill(prompt)
         chunk_s = time.perf_counter() - t0
         ingest = {"prompt_tokens": int(len(prompt)), "token_by_token_tokens_per_s": round(len(prompt) / serial_s, 1), "chunked_tokens_per_s": round(len(prompt) / chunk_s, 1),
-                  "chunked_ms": round(chunk_s * 1e3, 2), "first_prompt_ms": round(first_s * 1e3, 2), "chunk": 256, "same_next_token": bool(int(nxt) == int(first[0]) == int(nxt2)),
+                  "chunked_ms": round(chunk_s * 1e3, 2), "first_prompt_ms": round(first_s * 1e3, 2), "chunk": 1024, "same_next_token": bool(int(nxt) == int(first[0]) == int(nxt2)),
                   "kernel": "gemm_i8_tcgen05_kernel for the projections, the step kernels with a token index in the grid"}
     except q.QuintritError as e:
         ingest = {"error": str(e)}

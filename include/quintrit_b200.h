@@ -369,7 +369,7 @@ int quintrit_b200_selftest_barrier(uint32_t device_index, uint32_t ctas, uint32_
 int quintrit_b200_selftest_clear(uint32_t device_index, uint32_t spin_limit, uint32_t* out_kept);
 
 /*
- * Prompt ingestion: `count` tokens at positions pos .. pos + count - 1 in chunks of up to 256, every projection of a chunk as one
+ * Prompt ingestion: `count` tokens at positions pos .. pos + count - 1 in passes of up to 1024, every projection of a pass as one
  * batched product on the tensor cores (quintrit_b200_gemm_i32). The reference ingests a prompt token by token
  * (quintrit-c/src/runtime.rs:430-436); the result here is bit for bit that of `count` calls of quintrit_b200_decoder_forward:
  * the KV cache, the position, and - for the last token - the logits and the greedy choice (logits and out_token may be NULL).

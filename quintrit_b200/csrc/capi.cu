@@ -2216,8 +2216,8 @@ int gemm_prepare(quintrit_b200_matrix* m) {
     cudaError_t e = cudaMemsetAsync(w, 0x55, bytes, nullptr);
     if (e == cudaSuccess) e = gemm_copy_weights(m, w, 0);
     if (e == cudaSuccess) e = cudaMalloc(&m->d_gemm_act, size_t(kGemmMaxN) * k_pad);
-    if (e == cudaSuccess) e = cudaMalloc(&m->d_gemm_status, 4096);  // the status word; the rest is used by debug builds only
-    if (e == cudaSuccess) e = cudaMemset(m->d_gemm_status, 0, 4096);
+    if (e == cudaSuccess) e = cudaMalloc(&m->d_gemm_status, sizeof(unsigned int));
+    if (e == cudaSuccess) e = cudaMemset(m->d_gemm_status, 0, sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_i8_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmemLimit));
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
@@ -2248,6 +2248,7 @@ int gemm_launch(quintrit_b200_matrix* m, const int8_t* d_act, int batch, int32_t
     const bool in_place = m->cols % 16 == 0 && reinterpret_cast<uintptr_t>(d_act) % 16 == 0;
     const void* base = d_act;
     cuuint64_t pitch = m->cols, vectors = static_cast<cuuint64_t>(batch);
+    // (no caller comes here: decoders have whole 16 columns, single matrices give up to kGemmMaxN vectors a launch)
     if (!in_place && (batch > kGemmMaxN || m->d_gemm_act == nullptr)) return fail(QUINTRIT_ERR_INVALID_ARGUMENT, "%d vectors of %zu values cannot be read in place", batch, m->cols);
     if (!in_place) {
         gemm_pad_activations_kernel<<<std::min((n * k_pad + 255) / 256, 148 * 8), 256, 0, stream>>>(d_act, m->d_gemm_act, batch, n, static_cast<int>(m->cols), k_pad);
@@ -2588,8 +2589,8 @@ int enqueue_prefill_chunk(quintrit_b200_decoder* d, int n, uint32_t pos0, bool w
     const int H = d->hidden;
     QTB_CUDA(cudaMemcpyAsync(d->pf.pos, &pos0, sizeof pos0, cudaMemcpyHostToDevice, s));
     int rc;
-    // A full pass is about 500 launches of 40 layers; from the third full chunk on they are replayed as one CUDA graph (the first runs as it is and makes
-    // every lazy allocation, the second is captured). The position and the tokens are read from device memory, so one graph serves every chunk.
+    // A full pass is about 500 launches of 40 layers; from the third full pass on they are replayed as one CUDA graph (the first runs as it is and makes
+    // every lazy allocation, the second is captured). The position and the tokens are read from device memory, so one graph serves every pass.
     if (n == kPrefillMax && tg.own && d->pf.graph_ready) {
         QTB_CUDA(cudaGraphLaunch(d->pf.graph, s));
     } else if (n == kPrefillMax && tg.own && d->pf.warm && std::getenv("QUINTRIT_B200_PREFILL_GRAPH_OFF") == nullptr) {
@@ -3413,12 +3414,5 @@ extern "C" int quintrit_b200_batch_step(quintrit_b200_batch_t* batch, const uint
         return ok();
     });
 }
-
-#ifdef QTB_GEMM_TRACE
-extern "C" int quintrit_b200_debug_gemm_trace(quintrit_b200_matrix_t* m, long long* out) {  // debug builds: 4 roles x 4 events x 16 blocks of cycle stamps
-    cudaDeviceSynchronize();
-    return cudaMemcpy(out, m->d_gemm_status + 64, 4 * 4 * 16 * sizeof(long long), cudaMemcpyDeviceToHost);
-}
-#endif
 
 #include "runtime.cuh"

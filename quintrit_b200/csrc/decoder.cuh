@@ -88,7 +88,7 @@ struct quintrit_b200_decoder {
         float *x = nullptr, *q = nullptr, *part_acc = nullptr, *part_ms = nullptr, *s_h = nullptr, *s_q = nullptr, *s_i = nullptr;
         int8_t *a8_h = nullptr, *a8_q = nullptr, *a8_i = nullptr;
         int32_t *acc_qkv = nullptr, *acc_o = nullptr, *acc_gu = nullptr, *acc_down = nullptr;
-        bool warm = false, graph_ready = false;  // a full chunk ran once (lazy allocations done); the graph of a full chunk exists
+        bool warm = false, graph_ready = false;  // a full pass ran once (lazy allocations done); the graph of a full pass exists
         cudaGraphExec_t graph = nullptr;
         // batched products: per layer the row-wise stacks q | k | v and gate | up (nullptr: separate launches), and the buffers for the partial
         // sums of split products, one per projection kind (q, k, v, o, gate, up, down; a stack uses the first of its kind)
@@ -182,7 +182,7 @@ inline int decoder_gemv_bs(quintrit_b200_decoder* d, int layer, int first, const
 
 // Attention of n tokens: all query heads of a KV head in one block where an instantiation exists, else one query head per block. `end`: positions
 // after the last token of a prompt chunk (0 for tokens of several sequences). A chunk's tokens go eight to a block where that fills the machine:
-// with 64 tokens or more once the cache is divided into four chunks (end above 512), which are blocks of their own, and with full chunks of 256
+// with 64 tokens or more once the cache is divided into four chunks (end above 512), which are blocks of their own, and with 256 or more
 // anywhere. Passes of four layers with 12 / 4 heads of 256 and F16 accumulators: 256 tokens at position 900 2713 -> 1654 us, at 0 1067 -> 1045; 64
 // at 900 997 -> 752, but at 200 714 -> 737; 32 at 900 731 -> 718, at 200 574 -> 672. With 8 / 2 heads of 128: 64 at 900 674 -> 628, 48 560 -> 596.
 inline void launch_attention(quintrit_b200_decoder* d, AttnArgs at, int n, cudaStream_t s, size_t end = 0) {

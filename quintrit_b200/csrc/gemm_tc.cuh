@@ -148,7 +148,7 @@ __global__ void gemm_reduce_parts_kernel(const int32_t* __restrict__ partial, in
     }
 }
 
-// int8 activation vectors [batch][cols] -> the zero-padded matrix [n][blocks * 128] the TMA reads
+// int8 activation vectors [batch][cols] -> the zero-padded matrix [n][whole stages of 256] the TMA reads
 __global__ void gemm_pad_activations_kernel(const int8_t* __restrict__ act, int8_t* __restrict__ padded, int batch, int n, int cols, int k_pad) {
     const size_t total = size_t(n) * k_pad;
     for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {

@@ -72,7 +72,7 @@ struct MegaArgs {
     // vectors that every rank needs whole (o and down results, attention output, SwiGLU output) live in a "box" of which
     // every rank has one; ranks write their slices straight into the boxes of all ranks over NVLink as (value, sequence
     // number) pairs that the readers poll.
-    int attn_v2;               // attention second half by (KV head, 8 coordinates) units that also combine the chunks
+    int attn_v2;               // attention second half by (KV head, 16 coordinates) units that also combine the chunks
     float* attn_out;           // their result: the attention output before the o projection's quantiser (q_dim floats)
     int l2_prefetch;           // request the weights of later phases into L2 ahead of their streams (QUINTRIT_B200_L2_PREFETCH=0 switches it off)
     int bf16_tables;           // embedding and output head hold BF16 instead of F16 bit patterns
@@ -823,8 +823,8 @@ __device__ __noinline__ void mega_values_unit(const MegaArgs& a, const MegaLayer
 // (chunk, coordinate) of warp g runs the chain of query head g for that chunk, the four chunks of the reference's split
 // (attention.rs:510-533) side by side, and the unit also combines them (attention.rs:497-541) and contributes to the
 // maximum that the quantiser of the o projection needs. What is left after the next grid barrier is a load and a rounding.
-// Staging is asynchronous copies only (no registers, everything in flight at once): the unit's 16-byte piece of every
-// cached V row into [chunk][position][8 halves], the scores of its heads into one row per (head, chunk). The softmax
+// Staging is asynchronous copies only (no registers, everything in flight at once): the unit's 32 bytes of every
+// cached V row into [chunk][position][16 halves], the scores of its heads into one row per (head, chunk). The softmax
 // factors (attention.rs:448-462) are made by the unit itself, a warp per (head, chunk) (v2_factors). The positions at which any chunk's running maximum
 // moved are known per head and group of eight; groups without a move run branch-free.
 template <bool F32>
