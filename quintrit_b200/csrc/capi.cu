@@ -1331,6 +1331,13 @@ int decoder_check_status(quintrit_b200_decoder* d) {
     QTB_CUDA(cudaStreamSynchronize(d->stream));
     if (flag != 0) {  // the word is sticky on the device: clear it so that the decoder stays usable after the error
         cudaMemsetAsync(d->d_counters + 2, 0, sizeof(unsigned int), d->stream);
+        if (d->use_mega) {  // what a token kernel that gave up had added up: its launches begin with zeros
+            cudaMemsetAsync(d->acc_qkv, 0, (size_t(d->q_dim) + 2 * size_t(d->kv_dim)) * sizeof(int32_t), d->stream);
+            cudaMemsetAsync(d->acc_o, 0, size_t(d->hidden) * sizeof(int32_t), d->stream);
+            cudaMemsetAsync(d->acc_gu, 0, 2 * size_t(d->inter) * sizeof(int32_t), d->stream);
+            cudaMemsetAsync(d->acc_down, 0, size_t(d->hidden) * sizeof(int32_t), d->stream);
+            cudaMemsetAsync(d->amax_bits, 0, 4 * sizeof(unsigned int), d->stream);
+        }
         decoder_recount_steps(d);
         return kernel_status_error(flag);
     }
